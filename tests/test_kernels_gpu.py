@@ -565,6 +565,75 @@ def test_a_refused_row_stays_flagged_over_later_steps():
     assert status.tolist() == [1, 0]
 
 
+@pytest.mark.parametrize("vocab", [1, 5, 31, 1024, 1025, 4097, 32003, 128256])
+@pytest.mark.parametrize("steps", [0, 3, 60])
+def test_sample_rows_over_a_cluster(vocab, steps):
+    """Rows shared by the blocks of a cluster: shares that are empty, end inside four entries or differ in
+    size; continuous logits (the select ends after one digit) and logits on a grid of `steps` values (runs of
+    equal ones at the cut, more of them in a bin than the candidate buffer holds): tokens, windows and generators
+    of the plain chain, or refused together with it."""
+    n = 4
+    top = min(vocab, 40)
+    params = [[0.7, 0.75, 0.25, 1.1], [1.0, 0.9, 0.0, 1.0], [0.0, 0.75, 0.25, 1.2], [1.3, 2.0, 0.1, 1.0]]
+    iparams = [[top if top < vocab else 0, 8], [1, 0], [0, 8], [min(1024, max(vocab - 1, 1)), 0]]
+    state_gpu = _sampler_state(n, params, iparams, [3, 4, 5, 6])
+    state_cpu = [t.cpu().clone() for t in state_gpu]
+    for draw in range(3):
+        logits = randn(n, vocab, seed=300 + draw, scale=2.0)
+        if steps:
+            logits = torch.round(logits * steps) / steps
+        ranked = [v if 0 < v[0] < vocab or vocab <= 1024 else None for v in iparams]
+        ties = [ranked[r] is not None and params[r][0] > 0 and iparams[r][0] > 0
+                and int((logits[r] >= torch.topk(logits[r], min(iparams[r][0], vocab)).values[-1]).sum()) > 2048 for r in range(n)]
+        cpu_logits = logits.cpu().clone()
+        ops().sample_rows(logits, *state_gpu, record=True)
+        plain_ops.sample_rows(cpu_logits, *state_cpu, record=True)
+        for r in range(n):
+            if ties[r] or int(state_gpu[6][r]) != 0:
+                assert int(state_gpu[6][r]) == 1 and (ties[r] or int(state_cpu[6][r]) == 1), (r, draw)
+                for g, c in zip(state_gpu, state_cpu):           # the same state for the draws that follow
+                    c[r] = g[r].cpu()
+                continue
+            assert int(state_gpu[5][r]) == int(state_cpu[5][r]), (r, draw)
+            assert state_gpu[4][r] == state_cpu[4][r].to(DEV) and state_gpu[2][r].tolist() == state_cpu[2][r].tolist()
+
+
+@pytest.mark.parametrize("rows,vocab", [(1, 1), (3, 7), (2, 33), (5, 4099), (33, 128256)])
+def test_argmax_over_a_cluster(rows, vocab):
+    """First maximum over the blocks' shares, also with equal maxima in several shares and rows of -inf and NaN."""
+    x = randn(rows, vocab, seed=310)
+    x[0] = float("-inf")
+    if rows > 1:
+        x[1, vocab // 2:] = 7.0                                   # equal maxima from there on
+        x[1, 0] = float("nan")
+    want = [0 if r == 0 else vocab // 2 if r == 1 else int(x[r].argmax()) for r in range(rows)]
+    if rows > 1 and vocab // 2 == 0:
+        want[1] = 0
+    assert ops().argmax_rows(x).tolist() == want
+
+
+@pytest.mark.parametrize("n,k", [(16, 4), (17, 64), (64, 172), (344, 64), (1000, 68), (100, 4096), (4099, 260)])
+@pytest.mark.parametrize("residual", [False, True])
+def test_linear_of_few_rows_in_32_bit(n, k, residual):
+    """Up to 8 rows run a kernel of their own: the bits of the tiled kernel for the same rows (9 of them), for every
+    number of rows, with edges in the columns, in the last tile of k, and a bias."""
+    x, w, b = randn(9, k, seed=320), randn(n, k, seed=321), randn(n, seed=322)
+    start = randn(9, n, seed=323)
+
+    def run(m):
+        if residual:
+            acc = start[:m].clone()
+            ops().linear(x[:m], w, b, residual=acc)
+            return acc
+        return ops().linear(x[:m], w, b, out_dtype=torch.float32)
+
+    whole = run(9)
+    for m in range(1, 9):
+        assert torch.equal(run(m), whole[:m]), m
+    want = (x.double() @ w.double().T + b.double() + (start.double() if residual else 0.0)).float()
+    assert torch.allclose(whole, want, atol=k * 2.0 ** -24 * float((x.abs() @ w.abs().T).max()), rtol=1e-6)
+
+
 # ----------------------------------------------------------------------------- what rides in a product's epilogue
 
 def _sums_in_parts(x, parts, seed):
