@@ -40,15 +40,21 @@ constexpr int WARPS = 4;
 // the result rows hold n_heads * value_dim elements).
 template <typename T, int AHEAD, int MAX_PER_LANE>
 __global__ void __launch_bounds__(WARPS * 32)
-attention_generic_kernel(const T* __restrict__ q, int q_stride, const T* __restrict__ k_cache,
-                         const T* __restrict__ v_cache, const int* __restrict__ block_table,
+attention_generic_kernel(const T* q, int q_stride, const T* k_cache,
+                         const T* v_cache, const int* __restrict__ block_table,
                          int table_stride, int ring_pages, const int* __restrict__ tok_pos,
                          const int* __restrict__ tok_seq, T* __restrict__ out, int out_stride,
                          int n_heads, int n_kv_heads, int head_dim, float scale, int window,
-                         const float* __restrict__ sinks, const T* __restrict__ gate, int gate_stride,
+                         const float* __restrict__ sinks, const T* gate, int gate_stride,
                          float out_scale, float softcap, int value_dim, const float* __restrict__ bias, int span) {
     int t = blockIdx.x, head = blockIdx.y;
     const bool values_are_keys = k_cache == v_cache;
+    griddep_launch();
+    griddep_wait();
+    q = behind_wait(q);
+    k_cache = behind_wait(k_cache);
+    v_cache = behind_wait(v_cache);
+    gate = behind_wait(gate);
     int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int kv_head = head / (n_heads / n_kv_heads);
     int pos = tok_pos[t];
@@ -165,7 +171,7 @@ LLMB_EXPORT int llmb_attention_generic(const void* q, int q_stride, const void* 
     bool few = (long long)n_tokens * n_heads < 4096;       // the result is the same either way
     bool wide = head_dim > LLMB_MAX_HEAD_DIM || value_dim > LLMB_MAX_HEAD_DIM;              // twice the registers a lane: only where the head needs them
 #define LLMB_GENERIC_AS(T, AHEAD, PER)                                                                  \
-    attention_generic_kernel<T, AHEAD, PER><<<grid, WARPS * 32, 0, stream>>>(                            \
+    llmb::launch(attention_generic_kernel<T, AHEAD, PER>, grid, dim3(WARPS * 32), 0, stream, true,       \
         (const T*)q, q_stride, (const T*)k_cache, (const T*)v_cache, block_table, table_stride,         \
         ring_pages, tok_pos, tok_seq, (T*)out, out_stride, n_heads, n_kv_heads, head_dim, scale, window, \
         sinks, (const T*)gate, gate_stride, out_scale, softcap, value_dim, bias, span)

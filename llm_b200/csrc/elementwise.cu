@@ -352,6 +352,8 @@ __global__ void rope_cache_kernel(T* __restrict__ qkv, const float* __restrict__
                                   int ring_pages, T* __restrict__ k_cache, T* __restrict__ v_cache,
                                   int n_heads, int n_kv_heads, int head_dim, int n_rot, int interleaved,
                                   int write_cache) {
+    griddep_launch();
+    griddep_wait();                      // (src is written too: nothing is read through a constant pointer but tables)
     int t = blockIdx.x;
     int head = blockIdx.y;               // [0, Hq): q; [Hq, Hq+Hkv): k; then v
     int pos = tok_pos[t];
@@ -498,11 +500,11 @@ LLMB_EXPORT int llmb_rope_cache_write(void* qkv, int dtype, const float* table,
     dim3 grid(n_tokens, n_heads + 2 * n_kv_heads);
     int threads = head_dim / 2 >= 64 ? 64 : 32;
     if (dtype == LLMB_DTYPE_F32)
-        rope_cache_kernel<float><<<grid, threads, 0, stream>>>(
+        llmb::launch(rope_cache_kernel<float>, grid, dim3(threads), 0, stream, true,
             (float*)qkv, table, tok_pos, tok_seq, block_table, table_stride, ring_pages,
             (float*)k_cache, (float*)v_cache, n_heads, n_kv_heads, head_dim, n_rot, interleaved, write_cache);
     else if (dtype == LLMB_DTYPE_BF16)
-        rope_cache_kernel<__nv_bfloat16><<<grid, threads, 0, stream>>>(
+        llmb::launch(rope_cache_kernel<__nv_bfloat16>, grid, dim3(threads), 0, stream, true,
             (__nv_bfloat16*)qkv, table, tok_pos, tok_seq, block_table, table_stride, ring_pages,
             (__nv_bfloat16*)k_cache, (__nv_bfloat16*)v_cache, n_heads, n_kv_heads, head_dim, n_rot,
             interleaved, write_cache);
@@ -588,8 +590,11 @@ __device__ __forceinline__ float gated(float gate, float up, float linear, float
 }
 
 template <typename T>
-__global__ void swiglu_kernel(const T* __restrict__ gu, T* __restrict__ act, long long total,
+__global__ void swiglu_kernel(const T* gu, T* __restrict__ act, long long total,
                               int width, float linear, float cubic) {
+    griddep_launch();
+    griddep_wait();
+    gu = behind_wait(gu);
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     long long stride = (long long)gridDim.x * blockDim.x;
     for (; i < total; i += stride) {
@@ -639,9 +644,9 @@ LLMB_EXPORT int llmb_swiglu(const void* gu, void* act, int dtype, int n_tokens, 
     }
     int blocks = (int)((total + 255) / 256 < 148 * 16 ? (total + 255) / 256 : 148 * 16);
     if (dtype == LLMB_DTYPE_F32)
-        swiglu_kernel<float><<<blocks, 256, 0, stream>>>((const float*)gu, (float*)act, total, width, linear, cubic);
+        llmb::launch(swiglu_kernel<float>, blocks, 256, 0, stream, true, (const float*)gu, (float*)act, total, width, linear, cubic);
     else if (dtype == LLMB_DTYPE_BF16)
-        swiglu_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>((const __nv_bfloat16*)gu, (__nv_bfloat16*)act, total, width, linear, cubic);
+        llmb::launch(swiglu_kernel<__nv_bfloat16>, blocks, 256, 0, stream, true, (const __nv_bfloat16*)gu, (__nv_bfloat16*)act, total, width, linear, cubic);
     else
         return fail(LLMB_ERR_ARGUMENT, "swiglu: unknown dtype %d", dtype);
     return check_launch("swiglu");
