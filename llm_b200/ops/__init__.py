@@ -25,7 +25,7 @@ from .build import all_sources, ensure_built, load_library
 
 PAGE = native.plan_constant("page")              # positions per cache page (csrc/plan.h)
 BFLOAT16_ONLY = ("gemm_tc", "gemm_skinny", "attention_decode", "attention_decode_window", "attention_prefill",
-                 "attention_prefill_tc", "latent_prefill_tc")     # (diff_attention holds the 32-bit kernel too)
+                 "attention_prefill_tc", "latent_prefill_tc", "sigmoid_attention_tc")     # (diff_attention holds the 32-bit kernel too)
 
 _DTYPE_CODE = {torch.float32: 0, torch.bfloat16: 1}
 _c_int, _c_float, _c_void = ctypes.c_int, ctypes.c_float, ctypes.c_void_p
@@ -1092,7 +1092,8 @@ def check_device_status() -> None:
     """Raise if a kernel of a loaded library reported a wait that ran out. Cheap (it
     reads a word of host memory); meaningful after the stream was synchronised."""
     from .build import _loaded
-    for name in ("gemm_tc", "attention_prefill_tc", "routed_experts", "latent_prefill_tc", "latent_attention"):
+    for name in ("gemm_tc", "attention_prefill_tc", "routed_experts", "latent_prefill_tc", "latent_attention",
+                 "sigmoid_attention_tc"):
         if name in _loaded:
             code = getattr(_loaded[name], f"llmb_{name}_status")()
             if code != 0:
@@ -1609,16 +1610,31 @@ def sigmoid_attention_replay_key(step, spec):
     return (False, max(step.new_counts))
 
 
+SIGMOID_MIXED_BYTES = 256 << 20     # room for the mixed queries of a prefill; more heads than fit run one group after the other
+
+
+def sigmoid_mixed_heads(n_tokens: int, n_heads: int, n_kv_heads: int, dim: int, vdim: int) -> int:
+    """How many heads' mixed queries (bfloat16 [n_tokens, n_kv_heads * dim] each) the tcgen05 prefill of the sigmoid
+    attention keeps at once, or 0 for head sizes and groups that it does not serve."""
+    if dim not in (64, 128) or vdim not in (64, 128) or n_heads % n_kv_heads or n_heads // n_kv_heads not in (1, 2, 4, 8) \
+            or n_heads > 128:
+        return 0
+    most = max(1, min(n_heads, SIGMOID_MIXED_BYTES // max(1, n_tokens * n_kv_heads * dim * 2)))
+    groups = (n_heads + most - 1) // most
+    return (n_heads + groups - 1) // groups             # groups of equal size
+
+
 def sigmoid_attention(q, k_cache, v_cache, block_table, ring_pages, tok_pos, tok_seq, n_heads, n_kv_heads, dim, vdim,
                       scale, window, talk, head_bias, out_scale, out, decode=False, seq_lens=None, max_len=0,
-                      cu_seqlens=None, max_new=0, seq_order=None):
+                      cu_seqlens=None, max_new=0, seq_order=None, mixed=None):
     """Causal grouped-query attention without a softmax, of the new tokens' queries q [T, H * dim]
     over the paged cache (keys [pages, G, 64, dim], values [pages, G, 64, vdim]), which already
     holds the new tokens. For query t at position p and every key j with j <= p (and p - j <
     window, where window > 0): s_a = scale q_a . k_g(a),j; with `talk` (float32 [H, H])
     s_a <- sum_b talk[a, b] s_b; with `head_bias` (float32 [H]) s_a += head_bias[a]; then
     out[t, a] = out_scale * sum_j sigmoid(s_a) v_g(a),j. Scores, weights and sums are 32-bit.
-    `out` [T, H * vdim] in q's dtype may be a range of columns of a wider buffer."""
+    `out` [T, H * vdim] in q's dtype may be a range of columns of a wider buffer. `mixed` (bfloat16
+    [sigmoid_mixed_heads(..), T, G * dim], optional): scratch of a prefill with `talk`."""
     _require_cuda(q, k_cache, v_cache, block_table, tok_pos, tok_seq, talk, head_bias, out)
     n = q.shape[0]
     _check_rows(q, n, n_heads * dim, q.dtype, "sigmoid_attention: q")
@@ -1649,6 +1665,24 @@ def sigmoid_attention(q, k_cache, v_cache, block_table, ring_pages, tok_pos, tok
               _ptr(out), _c_int(out.stride(0)), _ptr(scratch), ctypes.c_longlong(scratch.numel()), _c_int(n),
               _c_int(n_heads), _c_int(n_kv_heads), _c_int(dim), _c_int(vdim), _c_float(scale), _c_int(window),
               _ptr(talk), _ptr(head_bias), _c_float(out_scale), _c_int(splits), _stream(), kernels=3 if splits > 1 else 2)
+        return out
+    heads_at_once = 0
+    if variant == "sigmoid_attention_tiles" and talk is not None and out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0 \
+            and k_cache.data_ptr() % 16 == 0 and v_cache.data_ptr() % 16 == 0:
+        # With a mixing matrix the scores are a contraction over all key heads, a matrix product by size: tcgen05 wherever
+        # the kernel is built for the sizes. Without one they are one head long, and the tiles on mma.sync stay.
+        heads_at_once = sigmoid_mixed_heads(n, n_heads, n_kv_heads, dim, vdim)
+    if heads_at_once:
+        shape = (heads_at_once, n, n_kv_heads * dim)
+        if mixed is None:
+            mixed = torch.empty(shape, dtype=torch.bfloat16, device=q.device)
+        _check_out(mixed, shape, torch.bfloat16, "sigmoid_attention: mixed")
+        _call("sigmoid_attention_tc", "llmb_sigmoid_attention_tc", _ptr(q), _c_int(q.stride(0)), _c_int(n), _ptr(k_cache),
+              _ptr(v_cache), _c_int(k_cache.shape[0]), _ptr(block_table), _c_int(block_table.shape[1]), _c_int(ring_pages),
+              _ptr(cu_seqlens), _ptr(seq_lens), _ptr(seq_order), _ptr(out), _c_int(out.stride(0)), _ptr(mixed),
+              _c_int(heads_at_once), _c_int(cu_seqlens.numel() - 1), _c_int(max_new), _c_int(n_heads), _c_int(n_kv_heads),
+              _c_int(dim), _c_int(vdim), _c_float(scale), _c_int(window), _ptr(talk), _ptr(head_bias), _c_float(out_scale),
+              _stream(), kernels=2 * ((n_heads + heads_at_once - 1) // heads_at_once))
         return out
     if variant == "sigmoid_attention_tiles":
         _call("sigmoid_attention", "llmb_sigmoid_attention_tiles", _ptr(q), _c_int(q.stride(0)), _ptr(k_cache),
@@ -1820,6 +1854,6 @@ def required_libraries() -> list:
 __all__ = ["PAGE", "GLU_BLOCK", "glu_fusable", "embed", "scale_", "random_normal_", "begin_recording", "end_recording", "RecordedPass", "scratch_generation", "Emit", "FoldedNorm", "RopeWrite", "cast_sumsq", "SUMSQ_LD", "rmsnorm", "swiglu", "rope_cache_write", "linear", "attention",
            "softcap_", "add_rows_", "conv_rope_cache_write", "diff_attention", "tanh_norm", "norm_rope_cache_write",
            "sigmoid_attention", "gated_recurrence", "state_space", "attention_replay_key", "layernorm", "input_conv", "output_norm_add_", "forget_recurrence",
-           "latent_write", "head_products", "latent_attention", "latent_prefill", "attention_decode_splits", "sigmoid_attention_replay_key", "sigmoid_decode_splits",
+           "latent_write", "head_products", "latent_attention", "latent_prefill", "attention_decode_splits", "sigmoid_attention_replay_key", "sigmoid_decode_splits", "sigmoid_mixed_heads",
            "argmax_rows", "sample_rows", "launch_count", "count_launches", "tensor_core_status", "check_device_status", "ensure_built", "load_library", "all_sources",
            "required_libraries", "tactics"]

@@ -20,7 +20,8 @@ class SigmoidAttentionMixer(ProjectedMixer):
 
     Launches: norm + rotation + cache write (ops.norm_rope_cache_write), the attention
     (ops.sigmoid_attention)."""
-    libraries = ("elementwise", "gemm_simt", "gemm_skinny", "gemm_tc", "projection_norm", "sigmoid_attention")
+    libraries = ("elementwise", "gemm_simt", "gemm_skinny", "gemm_tc", "projection_norm", "sigmoid_attention",
+                 "sigmoid_attention_tc")
 
     def __init__(self, spec):
         s = spec
@@ -86,7 +87,18 @@ class SigmoidAttentionMixer(ProjectedMixer):
     def mix_scratch(self, n_tokens, dtype):
         from ..engine.workspace import BufferRequest
         # phases: 0 norm + rotation + cache write, 1 attention
-        return [BufferRequest("queries", (n_tokens, self.q_width), dtype, 0, 1)]
+        out = [BufferRequest("queries", (n_tokens, self.q_width), dtype, 0, 1)]
+        mixed = self._mixed_shape(n_tokens, dtype)
+        if mixed is not None:
+            out.append(BufferRequest("mixed_queries", mixed, dtype, 1, 1))
+        return out
+
+    def _mixed_shape(self, n_tokens, dtype):
+        """The mixed queries that a prefill keeps at once (None: the kernels that need none)."""
+        s = self.spec
+        heads = ops.sigmoid_mixed_heads(n_tokens, s.n_heads, s.n_kv_heads, s.head_dim, s.value_dim) \
+            if s.talk and dtype == torch.bfloat16 else 0
+        return (heads, n_tokens, self.k_width) if heads else None
 
     def mix_replay_key(self, step):
         return ops.sigmoid_attention_replay_key(step, self.spec)
@@ -111,10 +123,12 @@ class SigmoidAttentionMixer(ProjectedMixer):
                                   self.position.interleaved if self.position is not None else False,
                                   ctx.tok_pos, ctx.tok_seq, queries, table, ring, keys, values,
                                   write_cache=(entry == cache_entry))
+        mixed = self._mixed_shape(n, proj.dtype) if proj.is_cuda and not ctx.decode else None
+        extra = {} if mixed is None else {"mixed": scratch("mixed_queries", mixed, proj.dtype)}
         ops.sigmoid_attention(queries, keys, values, table, ring, ctx.tok_pos, ctx.tok_seq, s.n_heads, s.n_kv_heads,
                               s.head_dim, s.value_dim, s.scale, s.window, self.talk, self.head_bias, s.out_scale, out,
                               decode=ctx.decode, seq_lens=ctx.seq_lens, max_len=ctx.max_len, cu_seqlens=ctx.cu_seqlens,
-                              max_new=max(ctx.new_counts), seq_order=ctx.seq_order)
+                              max_new=max(ctx.new_counts), seq_order=ctx.seq_order, **extra)
 
 
 register_mixer("sigmoid_attention", SigmoidAttentionMixer)

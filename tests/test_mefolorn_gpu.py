@@ -281,6 +281,27 @@ def test_sigmoid_attention(dtype, case, generic):
         _close(got, want, dtype, (case, lengths))
 
 
+@pytest.mark.parametrize("case", [
+    # heads, kv heads, head size, value size, window, bias: what the tcgen05 prefill serves
+    (4, 4, 64, 64, 0, True), (8, 4, 64, 128, 257, False), (8, 1, 128, 64, 130, True), (16, 2, 128, 128, 0, True)])
+@pytest.mark.parametrize("room", [1 << 28, 1 << 20])
+def test_sigmoid_attention_prefill_at_the_edges_of_tiles(case, room, monkeypatch):
+    """Tiles of 128 queries, steps of four pages, windows that begin inside a page, one token behind many; all heads at
+    once and groups of them."""
+    ops = _ops()
+    heads, groups, dim, vdim, window, bias = case
+    monkeypatch.setattr(ops, "SIGMOID_MIXED_BYTES", room)
+    for lengths, new in (([127, 128, 129], [127, 128, 129]), ([256, 257, 321, 64], [256, 257, 129, 1]),
+                         ([1030, 515, 1], [513, 2, 1]), ([900], [640])):
+        batch = Batch(lengths, new, seed=3 + len(lengths))
+        assert ops.sigmoid_mixed_heads(batch.n_tokens, heads, groups, dim, vdim) > 0
+        got = _sigmoid(ops.sigmoid_attention, batch, heads, groups, dim, vdim, torch.bfloat16, window, True, bias)
+        want = _sigmoid(plain_ops.sigmoid_attention, batch, heads, groups, dim, vdim, torch.bfloat16, window, True, bias)
+        torch.cuda.synchronize()
+        ops.check_device_status()
+        _close(got, want, torch.bfloat16, (case, lengths))
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, "generic"])
 @pytest.mark.parametrize("decode", [False, True])
 def test_sigmoid_attention_planted_keys_and_mixing(dtype, decode):
