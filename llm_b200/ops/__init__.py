@@ -25,7 +25,7 @@ from .build import all_sources, ensure_built, load_library
 
 PAGE = native.plan_constant("page")              # positions per cache page (csrc/plan.h)
 BFLOAT16_ONLY = ("gemm_tc", "gemm_skinny", "attention_decode", "attention_decode_window", "attention_prefill",
-                 "attention_prefill_tc", "latent_prefill_tc", "sigmoid_attention_tc")     # (diff_attention holds the 32-bit kernel too)
+                 "attention_prefill_tc", "latent_prefill_tc", "sigmoid_attention_tc", "diff_attention_tc")     # (diff_attention holds the 32-bit kernel too)
 
 _DTYPE_CODE = {torch.float32: 0, torch.bfloat16: 1}
 _c_int, _c_float, _c_void = ctypes.c_int, ctypes.c_float, ctypes.c_void_p
@@ -1093,7 +1093,7 @@ def check_device_status() -> None:
     reads a word of host memory); meaningful after the stream was synchronised."""
     from .build import _loaded
     for name in ("gemm_tc", "attention_prefill_tc", "routed_experts", "latent_prefill_tc", "latent_attention",
-                 "sigmoid_attention_tc"):
+                 "sigmoid_attention_tc", "diff_attention_tc"):
         if name in _loaded:
             code = getattr(_loaded[name], f"llmb_{name}_status")()
             if code != 0:
@@ -1757,6 +1757,11 @@ def diff_attention_replay_key(step, spec):
     return (False, max(step.new_counts))
 
 
+def diff_attention_tc_serves(dim: int, vdim: int) -> bool:
+    """Whether the tcgen05 prefill of the differential attention is built for these map and value sizes."""
+    return (dim, vdim) in ((32, 64), (64, 64), (64, 128), (128, 128))
+
+
 def diff_attention(q, k_cache, v_cache, block_table, ring_pages, tok_pos, tok_seq, n_heads, n_kv_heads, dim,
                    vdim, scale, window, keep_first, lam, eps, out_scale, head_norm=True, out=None, decode=False,
                    seq_lens=None, max_len=0, cu_seqlens=None, max_new=0, seq_order=None):
@@ -1779,7 +1784,16 @@ def diff_attention(q, k_cache, v_cache, block_table, ring_pages, tok_pos, tok_se
     variant = tactics.choose_diff_attention(decode, q.dtype, n_heads, n_kv_heads, dim, vdim, window, keep_first,
                                             cu_seqlens is not None and seq_lens is not None,
                                             q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0)
-    if variant == "diff_attention_prefill":
+    # tcgen05 wherever it is built for the sizes (its tile of 128 queries is at no size slower than 64 on mma.sync)
+    if variant == "diff_attention_prefill" and diff_attention_tc_serves(dim, vdim) and scale > 0 and out.data_ptr() % 16 == 0 \
+            and k_cache.data_ptr() % 16 == 0 and v_cache.data_ptr() % 16 == 0:
+        _call("diff_attention_tc", "llmb_diff_attention_tc", _ptr(q), _c_int(q.stride(0)), _c_int(n), _ptr(k_cache),
+              _ptr(v_cache), _c_int(k_cache.shape[0]), _ptr(block_table), _c_int(block_table.shape[1]), _c_int(ring_pages),
+              _ptr(cu_seqlens), _ptr(seq_lens), _ptr(seq_order), _ptr(out), _c_int(out.stride(0)),
+              _c_int(cu_seqlens.numel() - 1), _c_int(max_new), _c_int(n_heads), _c_int(n_kv_heads), _c_int(dim),
+              _c_int(vdim), _c_float(scale), _c_int(window), _c_int(keep_first), _c_float(lam), _c_float(eps),
+              _c_float(out_scale), _c_int(1 if head_norm else 0), _stream())
+    elif variant == "diff_attention_prefill":
         _call("diff_attention", "llmb_diff_attention_prefill", _ptr(q), _c_int(q.stride(0)), _ptr(k_cache),
               _ptr(v_cache), _ptr(block_table), _c_int(block_table.shape[1]), _c_int(ring_pages), _ptr(cu_seqlens),
               _ptr(seq_lens), _ptr(out), _c_int(out.stride(0)), _c_int(cu_seqlens.numel() - 1), _c_int(max_new),

@@ -32,7 +32,8 @@ class DiffAttentionMixer(Mixer):
     cache holds both maps [2 * dim]; lambda is computed once at bind, in 32-bit."""
     graph_safe = True
     emits = True
-    libraries = ("elementwise", "gemm_simt", "gemm_skinny", "gemm_tc", "short_conv", "diff_attention")
+    libraries = ("elementwise", "gemm_simt", "gemm_skinny", "gemm_tc", "short_conv", "diff_attention",
+                 "diff_attention_tc")
 
     def __init__(self, spec):
         s = spec

@@ -180,6 +180,18 @@ def test_diff_attention_prefill_kernel(shape, window, keep_first):
     _close(got, want, torch.bfloat16, (shape, window, keep_first))
 
 
+@pytest.mark.parametrize("shape", [(32, 64), (64, 64), (64, 128), (128, 128)])
+@pytest.mark.parametrize("window,keep_first", [(0, 0), (130, 0), (257, 70)])
+def test_diff_attention_prefill_at_the_edges_of_tiles(shape, window, keep_first):
+    """The tcgen05 prefill: tiles of 128 queries, more pages than its rings hold, rows whose window begins pages behind
+    their tile's first key."""
+    dim, vdim = shape
+    batch = Batch([1500, 128, 129, 700, 127], [257, 128, 129, 2, 127], seed=window + dim)
+    got, want = _attention_both(batch, 8, 2, dim, vdim, torch.bfloat16, window, keep_first, variant="diff_attention_prefill")
+    _ops().check_device_status()
+    _close(got, want, torch.bfloat16, (shape, window, keep_first))
+
+
 @pytest.mark.parametrize("shape", SHAPES)
 @pytest.mark.parametrize("window,keep_first", [(0, 0), (70, 3), (64, 0), (33, 65), (200, 1)])
 def test_diff_attention_decode_kernel(shape, window, keep_first, monkeypatch):
