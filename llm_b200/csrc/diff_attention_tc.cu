@@ -12,13 +12,13 @@
 //   operand. The scores of page n + 2 of a map are issued right behind P V of page n, as in attention_prefill_tc.
 // * warps 0-3 are the softmax of map 1, warps 4-7 that of map 2; a thread owns a query row. While one map's
 //   products run, the other map's exponentials do: what two blocks an SM do for attention_prefill_tc. O is
-//   rescaled in place when a row's maximum has outgrown the exponent's reference by 2^8.
+//   rescaled in place by a warp one of whose rows has a new maximum.
 // * tensor memory, all 512 columns: 2 maps x 2 score buffers x 64, 2 x DV for O. The two warps that own the same
 //   lanes halve the columns of O1 and O2 at the end: o = a1 - lambda a2, the head's norm, the scale.
 //
 // Bound by the exponentials (2 x 64 a query and page at 16 a cycle and SM), with 4 + 4 products a map and page
-// beside them. 3,001 tokens, 32 heads of 2 x 64 over 8, values of 128, on a B200: 451 us by tiles of 64 queries on
-// mma.sync, 198 us here (1.1 us a page and block; 1,024 cycles of exponentials are 0.55).
+// beside them. 3,001 tokens, 32 heads of 2 x 64 over 8, values of 128, on a B200: 440 us by tiles of 64 queries on
+// mma.sync, 222 us here (1.2 us a page and block; 1,024 cycles of exponentials are 0.55), the same error.
 // Which call comes here: every prefill of the map and value sizes below; the other sizes of LLMB_DIFF_SHAPES have
 // rows that no 128-byte swizzle covers (48) or values narrower than one (32), and stay on mma.sync.
 //
@@ -197,7 +197,7 @@ diff_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         int warp_pos = start + tile * BQ + quarter * 32;     // the warp's first position
         uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16);
         uint32_t o_addr = lane_addr + O_COL + map * DV;
-        float run_max = -INFINITY, run_sum = 0.f;
+        float reference = -INFINITY, run_sum = 0.f;
         bool ok = true;
         for (int n = 0; n < walk.count && ok; ++n) {
             int b = map * 2 + (n & 1);
@@ -224,13 +224,13 @@ diff_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             float top = -INFINITY;
 #pragma unroll
             for (int j = 0; j < 32; ++j) top = max3(top, __uint_as_float(ra[j]), __uint_as_float(rb[j]));
-            // The reference moves only when the page's maximum exceeds it by more than 2^8; O is then rescaled. A row that
-            // has seen no key yet keeps -inf (inf - inf is no number, and no number is not above 8): weights 0, nothing moves.
-            bool move = n == 0 || (top - run_max) * scale_log2 > 8.f;
-            float new_max = move ? top : run_max;
-            float alpha = (move && n > 0) ? fast_exp2((run_max - new_max) * scale_log2) : 1.f;
-            float shift = new_max == -INFINITY ? 0.f : new_max * scale_log2;
-            run_max = new_max;
+            // The exponent's reference is the row's maximum itself, as in the mma.sync kernel: the largest weights then lie just
+            // below 1, where bfloat16 is finest. (A reference that lags by up to 2^8 saves most of the rescaling, 198 us
+            // for 222, and is 4 % further from 64 bits.) A row that has seen no key yet keeps -inf: weights 0.
+            float raised = fmaxf(reference, top * scale_log2);
+            float alpha = raised > reference ? fast_exp2(reference - raised) : 1.f;
+            float shift = raised == -INFINITY ? 0.f : raised;
+            reference = raised;
             float add = 0.f;
             uint32_t packed[16];
 #pragma unroll
