@@ -90,6 +90,129 @@ delta_prepare_kernel(const T* __restrict__ proj, int ld, const float* __restrict
     }
 }
 
+template <typename T, int N> struct alignas(N * sizeof(T)) Wide { T v[N]; };
+
+// The same for four taps and key sizes of 64 or 128: a warp takes pieces of the channels of TOK tokens that follow each other,
+// with everything a piece needs requested at once: the tokens' rows and the three before them (a row is read once for the
+// TOK tokens), and the taps. Where the tokens lie in their sequences is looked up once for all pieces, and nothing passes
+// through shared memory. Pieces: key head g's q and k (2 D channels), 32 * EPL channels of v, the gates of all heads.
+// A lane has EPL neighbouring channels, so that its loads and stores are EPL values wide. 8,192 channels: 24 tokens 32.5 -> 6.2 us (one token a
+// warp, all pieces side by side), 2,077 tokens 117 -> 83 us (four tokens, the pieces one after the other).
+template <typename T, int EPL, int TOK>
+__global__ void __launch_bounds__(THREADS, 2)
+delta_prepare_pieces_kernel(const T* __restrict__ proj, int ld, const float* __restrict__ taps,
+                            const float* __restrict__ state, long long state_stride, const int* __restrict__ tok_seq,
+                            const int* __restrict__ cu_seqlens, const int* __restrict__ slot_ids,
+                            const float* __restrict__ rate, const float* __restrict__ dt_bias, float unit_eps,
+                            float* __restrict__ work, int work_ld, int n_tokens, int H, int G, int V) {
+    constexpr int D = 32 * EPL, PIECE = 32 * EPL, N = 2 * EPL;
+    griddep_launch();
+    griddep_wait();
+    proj = behind_wait(proj);
+    state = behind_wait(state);
+    int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int GD = G * D, C = 2 * GD + H * V, v_pieces = (H * V + PIECE - 1) / PIECE;
+    int t0 = blockIdx.x * TOK, count = min(TOK, n_tokens - t0);
+    int inside[TOK];                       // a token's place among its sequence's new tokens
+    const float* held[TOK];                // its sequence's last inputs before this step
+    bool plain = count == TOK;             // all tokens are one sequence's, and so are the three before them
+#pragma unroll
+    for (int k = 0; k < TOK; ++k) {
+        int t = t0 + min(k, count - 1), seq = tok_seq[t];
+        inside[k] = t - cu_seqlens[seq];
+        held[k] = state + (long long)slot_ids[seq] * state_stride;
+        plain = plain && inside[k] >= 3 + k;
+    }
+    for (int piece = blockIdx.y * (THREADS / 32) + warp; piece <= G + v_pieces; piece += gridDim.y * (THREADS / 32)) {
+        if (piece == G + v_pieces) {
+            for (int k = 0; k < count; ++k) {
+                const T* in = proj + (size_t)(t0 + k) * ld + C + H * V;
+                float* out = work + (size_t)(t0 + k) * work_ld;
+                for (int a = lane; a < H; a += 32) {
+                    float b = to_float(in[a]);
+                    out[C + a] = 1.0f / (1.0f + expf(-b));
+                    float z = to_float(in[H + a]) + dt_bias[a];
+                    float sp = z > 20.0f ? z : log1pf(expf(z));
+                    out[C + H + a] = expf(rate[a] * sp);
+                }
+            }
+            break;
+        }
+        // a lane's channels: EPL from `first` on, a q and k piece has k's behind q's
+        bool keys = piece < G;
+        int first = lane * EPL + (keys ? piece * D : 2 * GD + (piece - G) * PIECE), used = keys ? N : EPL;
+        if (first >= C) continue;                
+        float x[N][TOK + 3], tap[N][4];
+#pragma unroll
+        for (int e = 0; e < N; ++e) {
+            if (e >= used) break;
+            float4 four = *reinterpret_cast<const float4*>(taps + (size_t)(first + (e / EPL) * GD + e % EPL) * 4);
+            tap[e][0] = four.x; tap[e][1] = four.y; tap[e][2] = four.z; tap[e][3] = four.w;
+        }
+#pragma unroll
+        for (int r = 0; r < TOK + 3; ++r) {
+            if (r < 3 && !plain) continue;
+            const T* row = proj + (size_t)(r < 3 ? t0 + r - 3 : t0 + min(r - 3, count - 1)) * ld + first;
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                if (half * EPL >= used) break;
+                Wide<T, EPL> v = *reinterpret_cast<const Wide<T, EPL>*>(row + half * GD);
+#pragma unroll
+                for (int e = 0; e < EPL; ++e) x[half * EPL + e][r] = to_float(v.v[e]);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < TOK; ++k) {
+            if (k >= count) break;
+            float row[N];
+#pragma unroll
+            for (int e = 0; e < N; ++e) {
+                if (e >= used) break;
+                float in[3];
+                int c = first + (e / EPL) * GD + e % EPL;
+#pragma unroll
+                for (int d = 3; d >= 1; --d)
+                    in[3 - d] = plain ? x[e][k + 3 - d]
+                                      : inside[k] >= d ? to_float(proj[(size_t)(t0 + k - d) * ld + c])
+                                                       : held[k][(size_t)(3 - (d - inside[k])) * C + c];
+                float acc = fmaf(tap[e][0], in[0], 0.f);
+                acc = fmaf(tap[e][1], in[1], acc);
+                acc = fmaf(tap[e][2], in[2], acc);
+                acc = fmaf(tap[e][3], x[e][k + 3], acc);
+                row[e] = silu(acc);
+            }
+            float* out = work + (size_t)(t0 + k) * work_ld;
+            if (keys) {
+                float sq = 0.f, sk = 0.f;
+#pragma unroll
+                for (int e = 0; e < EPL; ++e) {
+                    sq = fmaf(row[e], row[e], sq);
+                    sk = fmaf(row[EPL + e], row[EPL + e], sk);
+                }
+                float rq = 1.0f / sqrtf(warp_sum(sq) + unit_eps) * (1.0f / sqrtf((float)D));
+                float rk = 1.0f / sqrtf(warp_sum(sk) + unit_eps);
+                float dot = 0.f;
+                Wide<float, EPL> qs, ks;
+#pragma unroll
+                for (int e = 0; e < EPL; ++e) {
+                    qs.v[e] = row[e] * rq;
+                    ks.v[e] = row[EPL + e] * rk;
+                    dot = fmaf(qs.v[e], ks.v[e], dot);
+                }
+                *reinterpret_cast<Wide<float, EPL>*>(out + first) = qs;
+                *reinterpret_cast<Wide<float, EPL>*>(out + first + GD) = ks;
+                dot = warp_sum(dot);
+                if (lane == 0) out[C + 2 * H + piece] = dot;
+            } else {
+                Wide<float, EPL> vs;
+#pragma unroll
+                for (int e = 0; e < EPL; ++e) vs.v[e] = row[e];
+                *reinterpret_cast<Wide<float, EPL>*>(out + first) = vs;
+            }
+        }
+    }
+}
+
 template <typename T>
 __global__ void delta_conv_state_kernel(const T* __restrict__ proj, int ld, int n_taps, float* __restrict__ state,
                                         long long state_stride, const int* __restrict__ cu_seqlens,
@@ -126,7 +249,10 @@ constexpr int PAD = 4;           // floats between the slices of a staged q or k
 // DS threads share a pair of columns (DS a power of two up to 32), each DPT elements of both: lanes that follow each
 // other hold neighbouring column pairs of the same slice (their loads of q and k are one address), lanes 32 / DS
 // apart the slices. A step is a chain of dependent instructions (sums, shuffles, the update), so what counts is how
-// many warps a scheduler can turn to: DPT = 8 gives twice the warps of 16 for the same state.
+// many warps a scheduler can turn to: DPT = 8 gives twice the warps of 16 for the same state. From a key size of 64 on
+// the loads of q and k from shared memory (a slice of either for every column pair) weigh as much, and a slice of 32
+// elements wins: two sequences of 777 and 1,300 tokens, 32 heads of 128 x 128, take 502 us with 32 elements of two columns
+// a thread, 554 with 32 of one, 618 with 16 of two and 598 with 16 of four (the next token's q and k requested early).
 template <int DPT, int DS>
 __global__ void __launch_bounds__(SCAN_THREADS)
 delta_scan_kernel(const float* __restrict__ work, int work_ld, float* __restrict__ state, long long state_stride,
@@ -308,7 +434,8 @@ delta_finish_kernel(const float* __restrict__ o, int o_ld, const T* __restrict__
     griddep_wait();
     size_t t = blockIdx.x;
     int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int a = warp; a < H; a += THREADS / 32) {
+    int a = blockIdx.y * (THREADS / 32) + warp;              // a warp a head: its loads wait for nothing but themselves
+    if (a < H) {
         const float* row = o + t * o_ld + a * V;
         float sq = 0.f;
         for (int j = lane; j < V; j += 32) sq = fmaf(row[j], row[j], sq);
@@ -357,21 +484,35 @@ LLMB_EXPORT int llmb_delta_rule(const void* proj, int ld, int dtype, const float
         scan_configured[DPT == 32][level] = smem_scan;
     }
     long long s_offset = (long long)(n_taps - 1) * C;
+    // the prepare kernel by pieces: what a lane loads and stores at once starts on its boundary (a property of the model, so
+    // that a token's sums have one order in every step)
+    bool pieces = n_taps == 4 && (D == 64 || D == 128) && (H * V) % (D / 32) == 0 && ld % (D / 32) == 0 && work_ld % (D / 32) == 0 &&
+                  (((size_t)proj | (size_t)work | (size_t)taps) % 16) == 0;
 #define LLMB_DELTA(T)                                                                                              \
     do {                                                                                                           \
+        if (pieces) {                                                                                              \
+            int tok = n_tokens >= 4 * 148 ? 4 : 1;                                                                 \
+            auto kernel = D == 128 ? (tok == 4 ? delta_prepare_pieces_kernel<T, 4, 4> : delta_prepare_pieces_kernel<T, 4, 1>) \
+                                   : (tok == 4 ? delta_prepare_pieces_kernel<T, 2, 4> : delta_prepare_pieces_kernel<T, 2, 1>); \
+            dim3 grid((n_tokens + tok - 1) / tok, tok == 4 ? 1 : (G + (H * V + D - 1) / D + THREADS / 32) / (THREADS / 32)); \
+            LLMB_CUDA(llmb::launch(kernel, grid, dim3(THREADS), 0, stream, true, (const T*)proj, ld, taps,         \
+                                   (const float*)state, state_stride, tok_seq, cu_seqlens, slot_ids, rate, dt_bias, \
+                                   unit_eps, work, work_ld, n_tokens, H, G, V));                                   \
+        } else {                                                                                                   \
         if (smem_row > 48 * 1024)                                                                                  \
             LLMB_CUDA(cudaFuncSetAttribute(delta_prepare_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,   \
                                            (int)smem_row));                                                        \
         LLMB_CUDA(llmb::launch(delta_prepare_kernel<T>, dim3(n_tokens), dim3(THREADS), smem_row, stream, true,     \
                                (const T*)proj, ld, taps, n_taps, (const float*)state, state_stride, tok_seq,       \
                                cu_seqlens, slot_ids, rate, dt_bias, unit_eps, work, work_ld, H, G, D, V));         \
+        }                                                                                                          \
         if (n_taps > 1)                                                                                            \
             LLMB_CUDA(llmb::launch(delta_conv_state_kernel<T>, dim3((C + 127) / 128, n_seqs), dim3(128), 0, stream, \
                                    true, (const T*)proj, ld, n_taps, state, state_stride, cu_seqlens, slot_ids, C)); \
         LLMB_CUDA(llmb::launch(scan, scan_grid, dim3(SCAN_THREADS), smem_scan, stream, true,                       \
                                (const float*)work, work_ld, state, state_stride, s_offset, cu_seqlens, slot_ids,  \
                                o, H * V, H, G, D, V, vectors));                                                    \
-        LLMB_CUDA(llmb::launch(delta_finish_kernel<T>, dim3(n_tokens), dim3(THREADS), 0, stream, true,             \
+        LLMB_CUDA(llmb::launch(delta_finish_kernel<T>, dim3(n_tokens, (H + THREADS / 32 - 1) / (THREADS / 32)), dim3(THREADS), 0, stream, true,             \
                                (const float*)o, H * V, (const T*)proj + C, ld, norm_weight, eps, (T*)mixed,        \
                                mixed_ld, H, V));                                                                   \
     } while (0)
