@@ -1358,15 +1358,21 @@ def attention(qkv, k_cache, v_cache, block_table, ring_pages, tok_pos, tok_seq, 
             variant = "attention_prefill"
     if value_dim != head_dim:
         variant = "attention_generic"                 # the tile kernels take values of the keys' size
+    # With a window the choice is attention_prefill; its calls run on tcgen05 wherever that kernel is built for them (64 or 128
+    # elements a head, no bias, no soft cap, a positive scale, rows and pages on 16-byte boundaries).
+    windowed_tc = (variant == "attention_prefill" and window > 0 and head_dim in (64, 128) and bias is None and softcap <= 0.0
+                   and scale > 0 and not tactics.is_disabled("attention_prefill_tc") and qkv.stride(0) % 8 == 0
+                   and out.stride(0) % 8 == 0 and not any(t.data_ptr() % 16 for t in (qkv, out, k_cache, v_cache)))
     if variant == "attention_decode" and (qkv.stride(0) % 2 or qkv.data_ptr() % 4):
         variant = "attention_generic"
-    if variant == "attention_prefill_tc":
+    if variant == "attention_prefill_tc" or windowed_tc:
         _call("attention_prefill_tc", "llmb_attention_prefill_tc", _ptr(qkv), _c_int(qkv.stride(0)),
               _c_int(n), _ptr(k_cache), _ptr(v_cache), _c_int(k_cache.shape[0]), _ptr(block_table),
               _c_int(block_table.shape[1]), _c_int(ring_pages), _ptr(cu_seqlens), _ptr(seq_lens),
               _ptr(seq_order), _ptr(out), _c_int(out.stride(0)), _c_int(cu_seqlens.numel() - 1),
               _c_int(max_new), _c_int(n_heads), _c_int(n_kv_heads), _c_int(head_dim), _c_float(scale),
-              _c_int(window), _ptr(sinks), _ptr(bias), _c_int(span), _stream())
+              _c_int(window), _ptr(sinks), _ptr(bias), _c_int(span), _ptr(gate),
+              _c_int(gate.stride(0) if gate is not None else 0), _c_float(out_scale), _stream())
     elif variant == "attention_prefill":
         _call("attention_prefill", "llmb_attention_prefill", _ptr(qkv), _c_int(qkv.stride(0)),
               _ptr(k_cache), _ptr(v_cache), _ptr(block_table), _c_int(block_table.shape[1]),

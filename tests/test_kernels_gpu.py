@@ -449,6 +449,31 @@ def test_attention_finds_one_far_key(dtype):
     assert not torch.allclose(windowed[0], values[0][far, 0].to(dtype).float(), atol=0.1)
 
 
+@pytest.mark.parametrize("heads,kv_heads,dim", [(8, 2, 128), (4, 4, 64), (32, 1, 128)])
+@pytest.mark.parametrize("window", [1, 64, 130, 300])
+@pytest.mark.parametrize("extras", [False, True])
+def test_windowed_prefill_on_tcgen05(heads, kv_heads, dim, window, extras):
+    """Windows that begin inside a key block, blocks that only some rows of a tile see, with a sink, a gate and a scale."""
+    starts, counts = [0, 700, 63, 0], [300, 257, 1, 128]
+    lens = [s + c for s, c in zip(starts, counts)]
+    table, width, k_cache, v_cache = make_cache(4, lens, kv_heads, dim, torch.bfloat16, 96)
+    fill_cache(table, width, k_cache, v_cache, lens, 97)
+    tok_pos = torch.tensor([p for s, c in zip(starts, counts) for p in range(s, s + c)], dtype=torch.int32, device=DEV)
+    tok_seq = torch.tensor([b for b, c in enumerate(counts) for _ in range(c)], dtype=torch.int32, device=DEV)
+    cu = torch.tensor([sum(counts[:i]) for i in range(5)], dtype=torch.int32, device=DEV)
+    seq_lens = torch.tensor(lens, dtype=torch.int32, device=DEV)
+    n = tok_pos.numel()
+    q = randn(n, heads * dim, dtype=torch.bfloat16, seed=98)
+    more = dict(sinks=randn(heads, seed=99), gate=randn(n, heads, dtype=torch.bfloat16, seed=100), out_scale=0.7) if extras else {}
+    want = plain_ops.attention(q, k_cache, v_cache, table, width, tok_pos, tok_seq, heads, kv_heads, dim, dim ** -0.5, window, **more)
+    got = ops().attention(q, k_cache, v_cache, table, width, tok_pos, tok_seq, heads, kv_heads, dim, dim ** -0.5, window,
+                          seq_lens=seq_lens, max_len=max(lens), cu_seqlens=cu, max_new=max(counts), **more)
+    ops().check_device_status()
+    assert torch.allclose(got.float(), want.float(), atol=2e-2, rtol=2e-2)
+    g, w = got.float().view(-1, heads, dim), want.float().view(-1, heads, dim)
+    assert float(((g - w).norm(dim=-1) / w.norm(dim=-1).clamp_min(1e-3)).max()) < 0.03
+
+
 def test_attention_window_edge():
     """The key at position p - window is out, the key at p - window + 1 is in."""
     heads, kv_heads, dim, n, window = 2, 1, 32, 200, 64
