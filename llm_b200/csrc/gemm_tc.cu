@@ -1134,10 +1134,53 @@ __device__ __forceinline__ Unit pair_unit_of(int u, int tiles_a, int tiles_b) {
     return w;
 }
 
+// What the pairs do. The first n_full tiles (a multiple of the pairs, or all of them) run whole, one a pair and round. The
+// tail_tiles that are left would keep only some of the pairs busy for a whole tile's time, so their k-blocks, laid one
+// tile behind the other, are cut into pieces of tail_len (at most a tile's own number), one a pair: a pair gets the end of
+// one tile and the start of the next, or one part. Where a tile has several parts, each is left in scratch, and a kernel
+// behind (pair_tail_sum_kernel) adds them in the order of k and does what the epilogue would. (The block that brought the
+// last part doing that alone, 128 threads reading 128 KB a part, took some 30 us.)
+struct PairWork {
+    int n_kblocks, tiles_a, tiles_b, n_full, tail_tiles, tail_len;
+};
+struct PairPiece {
+    int tile_a, tile_b, k0, k1;      // the tile and its k-blocks [k0, k1)
+    int tail;                        // the tile's number among the tail's, or -1: the whole tile
+};
+// The i-th piece of pair `pair`; false: there is none.
+__device__ __forceinline__ bool pair_piece(const PairWork& w, int pair, int n_pairs, int i, PairPiece& p) {
+    int u = pair + i * n_pairs;
+    p.k0 = 0;
+    p.k1 = w.n_kblocks;
+    p.tail = -1;
+    if (u >= w.n_full) {
+        int done = w.n_full / n_pairs;                  // whole tiles of this pair (n_full is a multiple, where there is a tail)
+        int begin = pair * w.tail_len, end = min(begin + w.tail_len, w.tail_tiles * w.n_kblocks);
+        if (w.tail_tiles == 0 || begin >= end) return false;
+        int t = begin / w.n_kblocks + (i - done), at = t * w.n_kblocks;
+        if (at >= end) return false;
+        p.k0 = max(begin - at, 0);
+        p.k1 = min(end - at, w.n_kblocks);
+        if (p.k0 > 0 || p.k1 < w.n_kblocks) p.tail = t;
+        u = w.n_full + t;
+    }
+    Unit unit = pair_unit_of(u, w.tiles_a, w.tiles_b);
+    p.tile_a = unit.tile_a;
+    p.tile_b = unit.tile_b;
+    return true;
+}
+// A piece's place in scratch: two a pair, 256 x 256 values each, the halves of the pair's blocks one after the other, four
+// columns of a row together and the rows side by side (what a warp stores or loads at once is 512 bytes on end).
+constexpr int PIECE_FLOATS = 2 * BM * PAIR_BN;
+__device__ __forceinline__ float* piece_of(float* partials, const PairWork& w, int pair, int tail, uint32_t rank) {
+    int which = tail - pair * w.tail_len / w.n_kblocks;
+    return partials + (size_t)(pair * 2 + which) * PIECE_FLOATS + rank * (BM * PAIR_BN);
+}
+
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                    const __grid_constant__ CUtensorMap map_residual, Epilogue ep, int n_kblocks, int tiles_a,
-                    int n_units, int* status, int stages, int residual_by_tma) {
+                    const __grid_constant__ CUtensorMap map_residual, Epilogue ep, PairWork work, float* partials,
+                    int* status, int stages, int residual_by_tma) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     constexpr int A_BYTES = BM * BK * 2, B_BYTES = (PAIR_BN / 2) * BK * 2;
     constexpr int TMEM_COLS = 2 * PAIR_BN;
@@ -1190,14 +1233,14 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     // before this one may still be running; the tokens only after griddep_wait().
     griddep_launch();
     uint32_t early = 0;
-    if (warp == 0 && lane == 0 && pair < n_units) {
-        Unit w = pair_unit_of(pair, tiles_a, n_units / tiles_a);
-        early = (uint32_t)min(stages, n_kblocks);
+    PairPiece p;
+    if (warp == 0 && lane == 0 && pair_piece(work, pair, n_pairs, 0, p)) {
+        early = (uint32_t)min(stages, p.k1 - p.k0);
         for (uint32_t i = 0; i < early; ++i) {
             if (rank == 0) mbar_expect_tx(smem_u32(&full_bar[i]), 2 * (A_BYTES + B_BYTES));
             uint32_t bar = map_to_rank(smem_u32(&full_bar[i]), 0);
-            tma_load_2d_pair(smem_u32(b_tiles + (size_t)i * B_BYTES), &map_b, bar, (int)i * BK,
-                             w.tile_b * PAIR_BN + (int)rank * (PAIR_BN / 2));
+            tma_load_2d_pair(smem_u32(b_tiles + (size_t)i * B_BYTES), &map_b, bar, (p.k0 + (int)i) * BK,
+                             p.tile_b * PAIR_BN + (int)rank * (PAIR_BN / 2));
         }
     }
     griddep_wait();
@@ -1208,13 +1251,12 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             int s = 0;
             uint32_t round = 0;                                 // how often the ring has been walked through
             bool ok = true;
-            for (int u = pair; u < n_units && ok; u += n_pairs) {
-                Unit w = pair_unit_of(u, tiles_a, n_units / tiles_a);
-                for (int kb = 0; kb < n_kblocks; ++kb, ++it, s = (s + 1 == stages ? 0 : s + 1), round += (s == 0)) {
+            for (int i = 0; ok && pair_piece(work, pair, n_pairs, i, p); ++i) {
+                for (int kb = p.k0; kb < p.k1; ++kb, ++it, s = (s + 1 == stages ? 0 : s + 1), round += (s == 0)) {
                     if (it < early) {                           // armed above, the weight tile is in flight
                         tma_load_2d_pair(smem_u32(a_tiles + (size_t)s * A_BYTES), &map_a,
                                          map_to_rank(smem_u32(&full_bar[s]), 0), kb * BK,
-                                         w.tile_a * 2 * BM + (int)rank * BM);
+                                         p.tile_a * 2 * BM + (int)rank * BM);
                         continue;
                     }
                     ok = mbar_wait(smem_u32(&empty_bar[s]), (round & 1) ^ 1, abort_flag, status, 1);
@@ -1223,9 +1265,9 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     if (rank == 0) mbar_expect_tx(smem_u32(&full_bar[s]), 2 * (A_BYTES + B_BYTES));
                     uint32_t bar = map_to_rank(smem_u32(&full_bar[s]), 0);
                     tma_load_2d_pair(smem_u32(a_tiles + (size_t)s * A_BYTES), &map_a, bar, kb * BK,
-                                     w.tile_a * 2 * BM + (int)rank * BM);
+                                     p.tile_a * 2 * BM + (int)rank * BM);
                     tma_load_2d_pair(smem_u32(b_tiles + (size_t)s * B_BYTES), &map_b, bar, kb * BK,
-                                     w.tile_b * PAIR_BN + (int)rank * (PAIR_BN / 2));
+                                     p.tile_b * PAIR_BN + (int)rank * (PAIR_BN / 2));
                 }
             }
         }
@@ -1245,19 +1287,19 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             const uint64_t a_desc0 = smem_desc(smem_u32(a_tiles)), b_desc0 = smem_desc(smem_u32(b_tiles));
             const uint32_t full0 = smem_u32(&full_bar[0]), empty0 = smem_u32(&empty_bar[0]);
             bool ok = true;
-            for (int u = pair; u < n_units && ok; u += n_pairs, ++n_done) {
+            for (; ok && pair_piece(work, pair, n_pairs, (int)n_done, p); ++n_done) {
                 uint32_t buffer = n_done & 1, use = n_done >> 1;
                 ok = mbar_wait(smem_u32(&acc_empty_bar[buffer]), (use & 1) ^ 1, abort_flag, status, 4);
                 if (!ok) break;
                 tcgen05_fence_after();
                 uint32_t d_tmem = tmem_base + buffer * PAIR_BN;
-                for (int kb = 0; kb < n_kblocks; ++kb) {
+                for (int kb = p.k0; kb < p.k1; ++kb) {
                     ok = mbar_wait(full0 + 8 * s, phase, abort_flag, status, 2);
                     if (!ok) break;
                     tcgen05_fence_after();
                     uint64_t a_desc = a_desc0 + (uint64_t)(s * (A_BYTES >> 4));
                     uint64_t b_desc = b_desc0 + (uint64_t)(s * (B_BYTES >> 4));
-                    if (kb == 0) {
+                    if (kb == p.k0) {
                         tcgen05_mma_pair(d_tmem, a_desc, b_desc, idesc, 0u);
 #pragma unroll
                         for (int k = 1; k < BK / UMMA_K; ++k) tcgen05_mma_pair(d_tmem, a_desc + 2 * k, b_desc + 2 * k, idesc, 1u);
@@ -1276,12 +1318,11 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         int row = quarter * 32 + lane;
         uint32_t n_done = 0;
         bool ok = true;
-        for (int u = pair; u < n_units && ok; u += n_pairs, ++n_done) {
-            Unit w = pair_unit_of(u, tiles_a, n_units / tiles_a);
+        for (; ok && pair_piece(work, pair, n_pairs, (int)n_done, p); ++n_done) {
             uint32_t buffer = n_done & 1, use = n_done >> 1;
             const float* rstd = nullptr;
             if (ep.f.norm_sumsq) {                    // as in gemm_tc_kernel: while the products run
-                tile_rstd(ep, rstd_s[n_done & 1], quarter, w.tile_a * 2 * BM + (int)rank * BM, BM);
+                tile_rstd(ep, rstd_s[n_done & 1], quarter, p.tile_a * 2 * BM + (int)rank * BM, BM);
                 asm volatile("bar.sync 1, 128;" ::: "memory");
                 rstd = rstd_s[n_done & 1];
             }
@@ -1289,7 +1330,24 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             if (!ok) break;
             tcgen05_fence_after();
             uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + buffer * PAIR_BN;
-            int a_row = w.tile_a * 2 * BM + (int)rank * BM + row;
+            int a_row = p.tile_a * 2 * BM + (int)rank * BM + row;
+            if (p.tail >= 0) {                            // a part of a tile: the sums as they are
+                float* mine = piece_of(partials, work, pair, p.tail, rank) + row * 4;
+#pragma unroll 1
+                for (int c = 0; c < PAIR_BN; c += 32) {
+                    uint32_t r[32];
+                    tmem_ld32(taddr + c, r);
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        __stcg(reinterpret_cast<float4*>(mine + (size_t)(c + 4 * q) * BM),
+                               make_float4(__uint_as_float(r[4 * q]), __uint_as_float(r[4 * q + 1]),
+                                           __uint_as_float(r[4 * q + 2]), __uint_as_float(r[4 * q + 3])));
+                }
+                tcgen05_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_remote(map_to_rank(smem_u32(&acc_empty_bar[buffer]), 0));
+                continue;
+            }
             if (ep.glu) {
                 float r = rstd ? rstd[row] : 1.f;
                 __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(ep.out);
@@ -1298,7 +1356,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     uint32_t g[16], uu[16];
                     tmem_ld16(taddr + c, g);
                     tmem_ld16(taddr + c + 16, uu);
-                    int n0 = w.tile_b * PAIR_BN + c;
+                    int n0 = p.tile_b * PAIR_BN + c;
                     if (a_row < ep.tokens && n0 + 32 <= ep.outs) {
                         uint4 packed[2];
                         __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(packed);
@@ -1320,12 +1378,12 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 }
             } else if (residual_by_tma) {
                 float scale = rstd ? rstd[row] : 1.f;
-                int tile_row0 = w.tile_a * 2 * BM + (int)rank * BM;
+                int tile_row0 = p.tile_a * 2 * BM + (int)rank * BM;
 #pragma unroll 1
                 for (int c = 0; c < PAIR_BN; c += 32) {
                     uint32_t r[32];
                     tmem_ld32(taddr + c, r);
-                    int n0 = w.tile_b * PAIR_BN + c;
+                    int n0 = p.tile_b * PAIR_BN + c;
                     float* buffer_s = staging + ((c >> 5) & 1) * (BM * 32);
                     // the copy that last read this buffer (two pieces ago) must be done with it
                     if (threadIdx.x == 64) bulk_wait_read<1>();
@@ -1366,7 +1424,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     tmem_ld16(taddr + c, r);
 #pragma unroll
                     for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
-                    store_columns<PAIR_BN>(ep, 0, a_row, w.tile_b, c, v, nullptr, rstd, row);
+                    store_columns<PAIR_BN>(ep, 0, a_row, p.tile_b, c, v, nullptr, rstd, row);
                 }
             }
             tcgen05_fence_before();
@@ -1386,6 +1444,94 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     if (warp == 1) {
         tcgen05_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
+    }
+}
+
+// The tiles that the pairs left in parts. A block takes 64 rows and 64 columns of one tile; a warp 8 rows, a lane four
+// columns of one row in each of four column groups of 16 (its loads fall together to 128 bytes, its stores to 32 or 64): the
+// parts added in the order of k, then the row's scale, the bias, and the store, the sum or the gated activation.
+__global__ void __launch_bounds__(256)
+pair_tail_sum_kernel(float* partials, Epilogue ep, PairWork work) {
+    __shared__ float rstd[64];
+    griddep_launch();
+    griddep_wait();
+    int tail = blockIdx.x, first_part = tail * work.n_kblocks / work.tail_len;
+    int parts = ((tail + 1) * work.n_kblocks - 1) / work.tail_len - first_part + 1;
+    if (parts == 1) return;                                        // one pair ran the whole tile
+    Unit unit = pair_unit_of(work.n_full + tail, work.tiles_a, work.tiles_b);
+    int rows = (blockIdx.y >> 2) * 64, cols = (blockIdx.y & 3) * 64;
+    int token0 = unit.tile_a * 2 * BM + rows, n0 = unit.tile_b * PAIR_BN + cols;
+    if (token0 >= ep.tokens || n0 >= ep.outs) return;
+    int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int row = warp * 8 + (lane >> 2), quad = (lane & 3) * 4;       // of the block's rows; of a group's columns
+    int at = rows + row;
+    float4 sum[4];
+#pragma unroll
+    for (int g = 0; g < 4; ++g) sum[g] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 2
+    for (int i = 0; i < parts; ++i) {
+        const float* from = piece_of(partials, work, first_part + i, tail, at / BM) + (at % BM) * 4;
+        float4 v[4];
+#pragma unroll
+        for (int g = 0; g < 4; ++g) v[g] = __ldcg(reinterpret_cast<const float4*>(from + (size_t)(cols + g * 16 + quad) * BM));
+#pragma unroll
+        for (int g = 0; g < 4; ++g) { sum[g].x += v[g].x; sum[g].y += v[g].y; sum[g].z += v[g].z; sum[g].w += v[g].w; }
+    }
+    float scale = 1.f;
+    if (ep.f.norm_sumsq) {
+        if (threadIdx.x < 64) rstd[threadIdx.x] = token0 + (int)threadIdx.x < ep.tokens ? thread_row_rstd(ep.f, token0 + threadIdx.x) : 1.f;
+        __syncthreads();
+        scale = rstd[row];
+    }
+    int token = token0 + row;
+    if (token >= ep.tokens) return;
+    if (ep.glu) {
+        __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(ep.out) + (size_t)token * ep.ldo + n0 / 2 + quad;
+        bool wide = (ep.ldo & 3) == 0 && (reinterpret_cast<uintptr_t>(ep.out) & 7) == 0;
+#pragma unroll
+        for (int g = 0; g < 4; g += 2) {
+            if (n0 + g * 16 + 32 > ep.outs) break;
+            float a[4] = {gated(ep, sum[g].x * scale, sum[g + 1].x * scale), gated(ep, sum[g].y * scale, sum[g + 1].y * scale),
+                          gated(ep, sum[g].z * scale, sum[g + 1].z * scale), gated(ep, sum[g].w * scale, sum[g + 1].w * scale)};
+            if (wide) {
+                __nv_bfloat162 lo = __floats2bfloat162_rn(a[0], a[1]), hi = __floats2bfloat162_rn(a[2], a[3]);
+                *reinterpret_cast<uint2*>(o + g * 8) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+            } else {
+                for (int j = 0; j < 4; ++j) o[g * 8 + j] = __float2bfloat16_rn(a[j]);
+            }
+        }
+        return;
+    }
+    const void* target = ep.residual ? (const void*)ep.residual : ep.out;
+    bool wide = (ep.ldo & 3) == 0 && (reinterpret_cast<uintptr_t>(target) & 15) == 0;
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+        int n = n0 + g * 16 + quad;
+        float v[4] = {sum[g].x * scale, sum[g].y * scale, sum[g].z * scale, sum[g].w * scale};
+        if (ep.bias) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] += n + j < ep.outs ? ep.bias[n + j] : 0.f;
+        }
+        size_t place = (size_t)token * ep.ldo + n;
+        if (wide && n + 4 <= ep.outs) {
+            if (ep.residual) {
+                float4* r = reinterpret_cast<float4*>(ep.residual + place);
+                float4 old = *r;
+                *r = make_float4(old.x + v[0], old.y + v[1], old.z + v[2], old.w + v[3]);
+            } else if (ep.out_is_bf16) {
+                __nv_bfloat162 lo = __floats2bfloat162_rn(v[0], v[1]), hi = __floats2bfloat162_rn(v[2], v[3]);
+                *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(ep.out) + place) =
+                    make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+            } else {
+                *reinterpret_cast<float4*>(reinterpret_cast<float*>(ep.out) + place) = make_float4(v[0], v[1], v[2], v[3]);
+            }
+            continue;
+        }
+        for (int j = 0; j < 4 && n + j < ep.outs; ++j) {
+            if (ep.residual) ep.residual[place + j] += v[j];
+            else if (ep.out_is_bf16) reinterpret_cast<__nv_bfloat16*>(ep.out)[place + j] = __float2bfloat16_rn(v[j]);
+            else reinterpret_cast<float*>(ep.out)[place + j] = v[j];
+        }
     }
 }
 
@@ -1466,8 +1612,8 @@ int launch(const CUtensorMap& map_a, const CUtensorMap& map_b, const Epilogue& e
     return check_launch("gemm_tc (split-K sum)");
 }
 
-int launch_pair(const CUtensorMap& map_a, const CUtensorMap& map_b, const Epilogue& ep, int tiles_a,
-                int tiles_b, int n_kblocks, cudaStream_t stream) {
+int launch_pair(const CUtensorMap& map_a, const CUtensorMap& map_b, const Epilogue& ep, const PairWork& work, int n_pairs,
+                float* partials, cudaStream_t stream) {
     constexpr int STAGE_BYTES = BM * BK * 2 + (PAIR_BN / 2) * BK * 2;
     int stages = (192 * 1024) / STAGE_BYTES;
     if (stages > 8) stages = 8;
@@ -1487,41 +1633,65 @@ int launch_pair(const CUtensorMap& map_a, const CUtensorMap& map_b, const Epilog
         if (code) return code;
         residual_by_tma = 1;
     }
-    static int n_sms = 0;
-    if (n_sms == 0) {
-        int device = 0;
-        LLMB_CUDA(cudaGetDevice(&device));
-        LLMB_CUDA(cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, device));
-    }
     int* status = status_word();
     int* status_dev = nullptr;
     if (status) cudaHostGetDevicePointer((void**)&status_dev, status, 0);
-    int n_units = tiles_a * tiles_b;
-    int pairs = n_units < n_sms / 2 ? n_units : n_sms / 2;
-    llmb::launch(gemm_tc_pair_kernel, 2 * pairs, THREADS, smem, stream, true, map_a, map_b, map_residual, ep,
-                 n_kblocks, tiles_a, n_units, status_dev, stages, residual_by_tma);
-    return check_launch("gemm_tc_pair");
+    llmb::launch(gemm_tc_pair_kernel, 2 * n_pairs, THREADS, smem, stream, true, map_a, map_b, map_residual, ep, work, partials,
+                 status_dev, stages, residual_by_tma);
+    int code = check_launch("gemm_tc_pair");
+    if (code || work.tail_tiles == 0) return code;
+    llmb::launch(pair_tail_sum_kernel, dim3(work.tail_tiles, 16), 256, 0, stream, true, partials, ep, work);
+    return check_launch("gemm_tc_pair (the sums of the last round)");
 }
 
 struct Plan {
     int swap, bn, tiles_a, tiles_b, n_kblocks, per_split, splits;
 };
 
-// The weights take the 128-row side of the tiles (tokens in tiles of up to 128 on the other) and K
-// is split whenever the 256 x 256 tiles of the pair kernel would fill less than 0.6 of the GPU's 74
-// pairs of SMs: always up to 128 tokens, and up to 1,024 tokens for products with few output
-// columns. (With the tokens on the 128-row side a 128 x 4096 x 4096 product has 16 tiles and took
-// 38 us, a 256 x 4096 x 14336 product 103 us; this way they take 16 and 44 us. At 512 x 6144 x 4096
-// the 48 pair tiles are faster again: 28 against 34 us.)
+// The weights take the 128-row side of the tiles (tokens in tiles of up to 128 on the other) and K is split over blocks up to
+// 128 tokens, and up to 1,024 tokens where 256 x 256 tiles are too few for the pairs of SMs even when cut along K. (With the
+// tokens on the 128-row side a 128 x 4096 x 4096 product has 16 tiles and took 38 us; this way it takes 16. At 512 x 6144 x
+// 4096 the 48 pair tiles are faster again: 28 against 34 us.)
 constexpr int SWAP_TOKENS = 128, SWAP_TOKENS_MOST = 1024, PAIRS = 74;
+
+// How the pairs share the tiles (PairWork). A tile takes 0.4 us a k-block whatever the other pairs do, so a last round of R of
+// 74 tiles wastes (74 - R) / 74 of it. Cut into pieces (multiples of four k-blocks, at least an eighth of a tile) it takes
+// R / 74 of a tile's time, but leaving the parts and adding them in a kernel behind takes about 12 us, 30 k-blocks, and the
+// pairs, each at another k, no longer share what they read, about a third of a piece. The cut is made where it saves
+// more than that. Measured, whole tiles -> cut: 350 x 28672 x 4096 (224 tiles) 98.7 -> 93.4 us, 3001 x 28672 x 4096 (1,344)
+// 531 -> 494, 1300 x 4096 x 14336 (96) 150 -> 127, 256 x 6144 x 4096 (24) 26.4 -> 22.6; and not cut because slower:
+// 512 x 4096 x 4096 (32) 26.2 -> 29.2, 2048 x 4096 x 14336 (128) 174 -> 182.
+PairWork plan_pairs(int M, int N, int K, int* n_pairs) {
+    PairWork w;
+    w.n_kblocks = (K + BK - 1) / BK;
+    w.tiles_a = (M + 2 * BM - 1) / (2 * BM);
+    w.tiles_b = (N + PAIR_BN - 1) / PAIR_BN;
+    long long units = (long long)w.tiles_a * w.tiles_b;
+    int rest = (int)(units % PAIRS);
+    int length = (int)(((long long)rest * w.n_kblocks + PAIRS - 1) / PAIRS), least = (w.n_kblocks + 7) / 8;
+    length = ((length > least ? length : least) + 3) / 4 * 4;
+    if (rest > 0 && w.n_kblocks - length > 30 + (3 * length) / 10) {
+        w.n_full = (int)(units - rest);
+        w.tail_tiles = rest;
+        w.tail_len = length;
+        *n_pairs = w.n_full > 0 ? PAIRS : (rest * w.n_kblocks + length - 1) / length;
+    } else {
+        w.n_full = (int)units;
+        w.tail_tiles = 0;
+        w.tail_len = 1;
+        *n_pairs = units < PAIRS ? (int)units : PAIRS;
+    }
+    return w;
+}
+bool on_pairs(const Plan& p, int M, int N) { return !p.swap && M > 128 && N >= 256; }
 
 Plan make_plan(int M, int N, int K) {
     Plan p;
     p.n_kblocks = (K + BK - 1) / BK;
     long long pair_tiles = (long long)((M + 255) / 256) * ((N + 255) / 256);
-    // (a pair's tile of 64 k-blocks takes 26 us alone, whatever fills the other pairs: with a short K the
-    // pairs win from 24 tiles on, 256 x 6144 x 4096 in 25.9 against 30.5 us, 512 x 4096 x 4096 in 26.1 against 38.3;
-    // with a long K the split products stay ahead until the pairs are well filled)
+    // (a pair's tile of 64 k-blocks takes 26 us alone, whatever fills the other pairs: with a short K the pairs win from 24
+    // tiles on, 512 x 4096 x 4096 in 26.1 against 38.3 us; with a long K the split products stay ahead until the pairs are
+    // well filled, 350 x 4096 x 14336 in 59 us against 69 cut along K)
     bool few_tiles = p.n_kblocks <= 64 ? pair_tiles < 24 : pair_tiles * 5 < PAIRS * 3;
     p.swap = M <= SWAP_TOKENS || (M <= SWAP_TOKENS_MOST && few_tiles);
     if (p.swap) {
@@ -1567,16 +1737,23 @@ LLMB_EXPORT int llmb_gemm_tc_status() {
 // Floats of partial-sum scratch and counters a call needs (0 when it does not split K).
 LLMB_EXPORT long long llmb_gemm_tc_scratch_floats(int M, int N, int K) {
     Plan p = make_plan(M, N, K);
+    if (on_pairs(p, M, N)) {
+        int n_pairs;
+        return plan_pairs(M, N, K, &n_pairs).tail_tiles > 0 ? 2LL * n_pairs * PIECE_FLOATS : 0;
+    }
     return p.splits > 1 ? (long long)p.tiles_a * p.tiles_b * p.splits * p.bn * BM : 0;
 }
 LLMB_EXPORT int llmb_gemm_tc_counters(int M, int N, int K) {
     Plan p = make_plan(M, N, K);
+    if (on_pairs(p, M, N)) return 0;
     return p.tiles_a * p.tiles_b;
 }
 
 // Kernels a call launches (1, or 2 where the split-K sum is a kernel of its own).
 LLMB_EXPORT int llmb_gemm_tc_kernels(int M, int N, int K) {
     Plan p = make_plan(M, N, K);
+    int n_pairs;
+    if (on_pairs(p, M, N)) return plan_pairs(M, N, K, &n_pairs).tail_tiles > 0 ? 2 : 1;
     return 1 + sums_later(p.swap, p.splits, p.bn);
 }
 
@@ -1661,12 +1838,18 @@ LLMB_EXPORT int llmb_gemm_tc_ex(const void* x, int ldx, const void* w, const flo
     if (applied) *applied = did;
     CUtensorMap map_a, map_b;
     int code;
-    if (allow_pair && !p.swap && M > 128 && N >= 256) {
+    if (allow_pair && on_pairs(p, M, N)) {
         // 256 x 256 tiles over pairs of SMs; each block's boxes are 128 rows
+        int n_pairs;
+        PairWork work = plan_pairs(M, N, K, &n_pairs);
+        if (work.tail_tiles > 0 && (!partials || partial_floats < 2LL * n_pairs * PIECE_FLOATS)) {      // no room for parts: whole tiles only
+            work.n_full = work.tiles_a * work.tiles_b;
+            work.tail_tiles = 0;
+            n_pairs = work.n_full < PAIRS ? work.n_full : PAIRS;
+        }
         if ((code = make_map(&map_a, x, M, K, ldx, BM))) return code;
         if ((code = make_map(&map_b, w, N, K, K, PAIR_BN / 2))) return code;
-        return launch_pair(map_a, map_b, ep, (M + 2 * BM - 1) / (2 * BM), (N + PAIR_BN - 1) / PAIR_BN,
-                           p.n_kblocks, stream);
+        return launch_pair(map_a, map_b, ep, work, n_pairs, partials, stream);
     }
     if (p.swap) {
         if ((code = make_map(&map_a, w, N, K, K, BM))) return code;

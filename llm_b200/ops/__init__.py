@@ -1041,22 +1041,30 @@ _scratch: dict = {}
 _retired: list = []      # outgrown scratch buffers, kept alive for CUDA graphs that hold their address
 
 
+_SCRATCH_FLOATS, _SCRATCH_COUNTERS = 148 * 2 * 128 * 256, 1 << 14      # what a product on pairs of SMs asks for at most
+_SCRATCH_STREAMS = 8                  # streams of a device that keep a pair of their own; any further ones share the first
+
+
 def _split_scratch(device, floats: int, counters: int):
-    """Partial sums and tile counters of the split-K products, one pair per
-    device, shared by every call on the stream (calls run one after the other).
-    It grows when a call needs more; an outgrown pair is kept alive because a
-    captured step may still hold its address."""
-    held = _scratch.get(device)
+    """Partial sums and tile counters of the products that split K, one pair per device and stream (calls of a stream run
+    one after the other). It grows when a call needs more; an outgrown pair is kept alive because a captured step may
+    still hold its address. A step under capture takes a pair that the device has (a shape runs plainly before it is
+    captured, and what a capture allocates belongs to its graph)."""
+    capturing = device.type == "cuda" and torch.cuda.is_current_stream_capturing()
+    key = (device, 0 if device.type != "cuda" or capturing else _stream().value or 0)
+    if key not in _scratch and (capturing or sum(k[0] == device for k in _scratch) >= _SCRATCH_STREAMS):
+        key = next((k for k in _scratch if k[0] == device), key)
+    held = _scratch.get(key)
     if held is None or held[0].numel() < floats or held[1].numel() < counters:
-        n_floats = max(floats, held[0].numel() if held else 0, 1 << 23)
-        n_counters = max(counters, held[1].numel() if held else 0, 1 << 14)
+        n_floats = max(floats, held[0].numel() if held else 0, _SCRATCH_FLOATS)
+        n_counters = max(counters, held[1].numel() if held else 0, _SCRATCH_COUNTERS)
         global _scratch_generation
         if held is not None:
             _retired.append(held)
             _scratch_generation += 1
         held = (torch.empty(n_floats, dtype=torch.float32, device=device),
                 torch.zeros(n_counters, dtype=torch.int32, device=device))
-        _scratch[device] = held
+        _scratch[key] = held
     return held
 
 

@@ -169,6 +169,50 @@ def test_linear_with_gated_epilogue(m, f, k):
     assert ops().tensor_core_status() == 0
 
 
+@pytest.mark.parametrize("m,n,k", [(350, 4096, 4096), (129, 2048, 14336), (257, 2048, 8192), (1300, 4096, 4096),
+                                   (300, 2112, 2056), (777, 28672, 1024), (2077, 6144, 1600)])
+def test_linear_cuts_the_last_round_of_tiles(m, n, k):
+    """Products whose last round of 256 x 256 tiles leaves pairs idle: its tiles are cut along K over all pairs and their parts
+    added, for each epilogue, with one part order (two runs give the same bits). Largest error of a sum of k products of
+    bfloat16 values in 32 bits: k 2^-24 of the sum of magnitudes, far inside 2e-3 of the largest result."""
+    a = randn(m, k, dtype=torch.bfloat16, seed=201)
+    w = randn(n, k, dtype=torch.bfloat16, seed=202, scale=0.05)
+    bias = randn(n, seed=203)
+    plain = a.double() @ w.double().T
+    want = plain + bias.double()
+    scale = float(want.abs().max())
+    got = ops().linear(a, w, bias, out_dtype=torch.float32)
+    assert float((got - want).abs().max()) <= 2e-3 * scale
+    assert torch.equal(got, ops().linear(a, w, bias, out_dtype=torch.float32))
+    assert float((ops().linear(a, w, bias).double() - want).abs().max()) <= 1e-2 * scale
+    residual = randn(m, n, seed=204)
+    expect = residual.double() + want
+    ops().linear(a, w, bias, residual=residual)
+    assert float((residual - expect).abs().max()) <= 2e-3 * scale
+    if n % 32 == 0:
+        f = n // 2
+        gate, up = plain.view(m, f // 16, 2, 16).unbind(2)
+        act = (gate / (1 + torch.exp(-gate)) * up).reshape(m, f)
+        assert float((ops().linear(a, w, glu=True).double() - act).abs().max()) <= 1e-2 * float(act.abs().max())
+    assert ops().tensor_core_status() == 0
+
+
+def test_linear_on_two_streams_at_once():
+    """Products that leave parts in scratch, on two streams with nothing between them: each stream has its own."""
+    a = randn(350, 4096, dtype=torch.bfloat16, seed=205)
+    ws = [randn(4096, 4096, dtype=torch.bfloat16, seed=206 + i, scale=0.05) for i in range(2)]
+    want = [ops().linear(a, w) for w in ws]
+    streams = [torch.cuda.Stream() for _ in ws]
+    torch.cuda.synchronize()
+    got = [[], []]
+    for _ in range(10):
+        for i, stream in enumerate(streams):
+            with torch.cuda.stream(stream):
+                got[i].append(ops().linear(a, ws[i]))
+    torch.cuda.synchronize()
+    assert all(torch.equal(g, want[i]) for i in range(2) for g in got[i])
+
+
 def test_linear_rows_do_not_depend_on_the_batch():
     """32-bit: a row's product is bit-equal whether it is computed alone or among 200 rows."""
     a = randn(200, 172, seed=8)
