@@ -104,7 +104,9 @@ def test_tanh_norm(dtype, width):
     # query heads, key heads, head size, value heads, value size, rotated, norms, interleaved, columns behind
     (4, 2, 6, 2, 10, 4, True, False, 0), (3, 3, 10, 3, 7, 10, True, False, 5), (2, 1, 16, 1, 24, 0, True, False, 48),
     (4, 2, 64, 2, 32, 32, True, False, 192), (2, 2, 8, 2, 8, 8, False, True, 0), (1, 1, 12, 0, 0, 0, True, False, 3),
-    (1, 1, 9, 0, 0, 0, False, False, 0), (8, 2, 128, 2, 128, 64, True, False, 0)])
+    (1, 1, 9, 0, 0, 0, False, False, 0), (8, 2, 128, 2, 128, 64, True, False, 0),
+    # (eight columns a thread)
+    (3, 1, 64, 1, 40, 64, True, True, 8), (32, 8, 128, 8, 128, 128, True, False, 16), (2, 2, 32, 2, 32, 16, False, False, 0)])
 def test_norm_rope_cache_write(dtype, case):
     ops = _ops()
     heads, groups, dim, v_heads, vdim, n_rot, norms, interleaved, behind = case
@@ -358,11 +360,11 @@ def _recurrence_inputs(channels, blocks, taps, n_tokens, n_slots, dtype, seed):
     return wide, {k: v.to(DEV).contiguous() for k, v in params.items()}, state
 
 
-def _recurrence(fn, wide, params, state, batch, channels, dtype):
+def _recurrence(fn, wide, params, state, batch, channels, dtype, at=2):
     out_wide = torch.zeros((batch.n_tokens, channels + 9), dtype=dtype, device=DEV)
     work = torch.empty((3, batch.n_tokens, channels), device=DEV)
     p = params
-    fn(wide[:, 2:2 + channels], wide[:, 2 + channels:2 + 2 * channels], p["conv_w"], p["conv_b"], p["gate_a"], p["gate_a_bias"],
+    fn(wide[:, at:at + channels], wide[:, at + channels:at + 2 * channels], p["conv_w"], p["conv_b"], p["gate_a"], p["gate_a_bias"],
        p["gate_i"], p["gate_i_bias"], p["rate"], state, batch.tok_seq, batch.cu, batch.slots, out_wide[:, 4:4 + channels], 0.9, work,
        single_tokens=all(k == 1 for k in batch.new))
     return out_wide
@@ -383,6 +385,25 @@ def test_gated_recurrence(dtype, case):
         torch.cuda.synchronize()
         _close(got, want, dtype, (case, lengths, "out"))
         _close(states[0], states[1], torch.float32, (case, lengths, "state"))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("channels,blocks", [(32, 2), (1028, 4)])
+def test_gated_recurrence_of_aligned_rows(dtype, channels, blocks):
+    """Four channels a thread, four tokens or one: sequences that begin at every place of a group, and shorter ones than the
+    taps; chunks in which several sequences begin and end."""
+    ops = _ops()
+    for lengths, new in [([700, 64, 129, 5, 2, 3], [500, 3, 66, 5, 1, 3]), ([60, 900, 3, 131], [60, 320, 3, 131]),
+                         ([70, 5, 131, 64], [70, 2, 66, 1]), ([9, 200, 65], [1, 1, 1])]:
+        batch = Batch(lengths, new, seed=1)
+        _, params, state = _recurrence_inputs(channels, blocks, 4, batch.n_tokens, len(lengths) + 2, dtype, seed=channels)
+        wide = torch.randn((batch.n_tokens, 2 * channels + 8), generator=torch.Generator().manual_seed(7)).to(dtype).to(DEV)
+        states = [state.clone(), state.clone()]
+        got = _recurrence(ops.gated_recurrence, wide, params, states[0], batch, channels, dtype, at=0)
+        want = _recurrence(plain_ops.gated_recurrence, wide, params, states[1], batch, channels, dtype, at=0)
+        torch.cuda.synchronize()
+        _close(got, want, dtype, (channels, lengths, "out"))
+        _close(states[0], states[1], torch.float32, (channels, lengths, "state"))
 
 
 def test_gated_recurrence_carries_its_state_across_any_cut():
