@@ -530,9 +530,8 @@ using namespace llmb::tc;
 
 constexpr int GM = 128, GK = 64, G_THREADS = 192;
 constexpr int A_BYTES = GM * GK * 2;
-// tiles of 128 columns: a ring of three stages, two blocks an SM; tiles of 256 columns (two thirds of the operand bytes
-// per product): a ring of four, one block an SM
-__host__ __device__ constexpr int stages_of(int gn) { return gn == 128 ? 3 : 4; }
+// tiles of 128 columns: a ring of three stages, two blocks an SM
+__host__ __device__ constexpr int stages_of(int) { return 3; }
 __host__ __device__ constexpr size_t smem_of(int gn) { return 1024 + (size_t)stages_of(gn) * (A_BYTES + gn * GK * 2) + (2 * stages_of(gn) + 1) * 8 + 16; }
 
 // Xs[s, :] = h[sorted[s] / top, :]: the rows of h in the order of the plan (16 bytes a thread a time).
@@ -550,6 +549,69 @@ gather_rows_kernel(const __nv_bfloat16* __restrict__ h, int ld, int top, const i
     }
 }
 
+// The epilogue of one tile by one thread: row `row` of the tile's rows [first, first + rows) of the list, the GN accumulator
+// columns at taddr, the output columns from n0 on.
+template <bool GLU, int GN>
+__device__ __forceinline__ void store_row(uint32_t taddr, int row, int rows, int first, int n0, int N, __nv_bfloat16* act, float* y,
+                                          const int* sorted, const float* weights, Activation activation) {
+    bool live = row < rows;
+    if (GLU) {
+        float wgt = (live && weights) ? weights[sorted[first + row]] : 1.f;
+        __nv_bfloat16* out = act + (long long)(first + row) * N + n0;
+        bool vector = N % 8 == 0;
+#pragma unroll 1
+        for (int c = 0; c < GN / 2; c += 16) {
+            uint32_t g[16], u[16];
+            tmem_ld16(taddr + c, g);
+            tmem_ld16(taddr + GN / 2 + c, u);
+            if (!live || n0 + c >= N) continue;
+            float v[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                float gate = wgt * __uint_as_float(g[j]);
+                v[j] = activated(gate, wgt * __uint_as_float(u[j]), activation);
+            }
+            if (vector && n0 + c + 16 <= N) {
+                uint32_t packed[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    __nv_bfloat162 two = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+                    packed[j] = *reinterpret_cast<uint32_t*>(&two);
+                }
+                uint4* dst = reinterpret_cast<uint4*>(out + c);
+                dst[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+                dst[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
+            } else {
+#pragma unroll
+                for (int j = 0; j < 16; ++j)
+                    if (n0 + c + j < N) out[c + j] = __float2bfloat16_rn(v[j]);
+            }
+        }
+    } else {
+        int assignment = live ? sorted[first + row] : 0;
+        float wgt = live ? (weights ? weights[assignment] : 1.f) : 0.f;
+        float* out = y + (long long)assignment * N + n0;
+        bool vector = N % 4 == 0;
+#pragma unroll 1
+        for (int c = 0; c < GN; c += 16) {
+            uint32_t r[16];
+            tmem_ld16(taddr + c, r);
+            if (!live || n0 + c >= N) continue;
+            if (vector && n0 + c + 16 <= N) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    reinterpret_cast<float4*>(out + c)[j] =
+                        make_float4(wgt * __uint_as_float(r[4 * j]), wgt * __uint_as_float(r[4 * j + 1]),
+                                    wgt * __uint_as_float(r[4 * j + 2]), wgt * __uint_as_float(r[4 * j + 3]));
+            } else {
+#pragma unroll
+                for (int j = 0; j < 16; ++j)
+                    if (n0 + c + j < N) out[c + j] = wgt * __uint_as_float(r[j]);
+            }
+        }
+    }
+}
+
 // One block: the tile `blockIdx.y` of the plan (an expert's rows [first, first + rows) of the sorted list, at most
 // 128) times GN accumulator columns: the output columns [blockIdx.x * (GLU ? GN / 2 : GN), ..) of that expert. A: [rows of the list, K] behind
 // map_a. B: every expert's matrix stacked, [E * b_rows, K] behind map_b; GLU: an expert's b_rows = 2 N rows are N
@@ -557,7 +619,7 @@ gather_rows_kernel(const __nv_bfloat16* __restrict__ h, int ld, int top, const i
 // accumulator's first half are gates and its second half the ups. Warp 0: TMA producer. Warp 1: tensor memory and the
 // products. Warps 2..5: epilogue, a thread a row. Every wait is bounded and reports through `status`.
 template <bool GLU, int GN>
-__global__ void __launch_bounds__(G_THREADS, GN == 128 ? 2 : 1)
+__global__ void __launch_bounds__(G_THREADS, 2)
 expert_product_wide_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                            const int* __restrict__ plan, int E, int max_tiles, int b_rows, int N, int n_kblocks,
                            __nv_bfloat16* __restrict__ act, float* __restrict__ y, const int* __restrict__ sorted,
@@ -653,62 +715,7 @@ expert_product_wide_kernel(const __grid_constant__ CUtensorMap map_a, const __gr
         if (ok) {
             tcgen05_fence_after();
             uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16);
-            bool live = row < rows;
-            if (GLU) {
-                float wgt = (live && weights) ? weights[sorted[first + row]] : 1.f;
-                __nv_bfloat16* out = act + (long long)(first + row) * N + n0;
-                bool vector = N % 8 == 0;
-#pragma unroll 1
-                for (int c = 0; c < GN / 2; c += 16) {
-                    uint32_t g[16], u[16];
-                    tmem_ld16(taddr + c, g);
-                    tmem_ld16(taddr + GN / 2 + c, u);
-                    if (!live || n0 + c >= N) continue;
-                    float v[16];
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        float gate = wgt * __uint_as_float(g[j]);
-                        v[j] = activated(gate, wgt * __uint_as_float(u[j]), activation);
-                    }
-                    if (vector && n0 + c + 16 <= N) {
-                        uint32_t packed[8];
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) {
-                            __nv_bfloat162 two = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
-                            packed[j] = *reinterpret_cast<uint32_t*>(&two);
-                        }
-                        uint4* dst = reinterpret_cast<uint4*>(out + c);
-                        dst[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-                        dst[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 16; ++j)
-                            if (n0 + c + j < N) out[c + j] = __float2bfloat16_rn(v[j]);
-                    }
-                }
-            } else {
-                int assignment = live ? sorted[first + row] : 0;
-                float wgt = live ? (weights ? weights[assignment] : 1.f) : 0.f;
-                float* out = y + (long long)assignment * N + n0;
-                bool vector = N % 4 == 0;
-#pragma unroll 1
-                for (int c = 0; c < GN; c += 16) {
-                    uint32_t r[16];
-                    tmem_ld16(taddr + c, r);
-                    if (!live || n0 + c >= N) continue;
-                    if (vector && n0 + c + 16 <= N) {
-#pragma unroll
-                        for (int j = 0; j < 4; ++j)
-                            reinterpret_cast<float4*>(out + c)[j] =
-                                make_float4(wgt * __uint_as_float(r[4 * j]), wgt * __uint_as_float(r[4 * j + 1]),
-                                            wgt * __uint_as_float(r[4 * j + 2]), wgt * __uint_as_float(r[4 * j + 3]));
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 16; ++j)
-                            if (n0 + c + j < N) out[c + j] = wgt * __uint_as_float(r[j]);
-                    }
-                }
-            }
+            store_row<GLU, GN>(taddr, row, rows, first, n0, N, act, y, sorted, weights, activation);
         }
     }
 
@@ -722,6 +729,140 @@ expert_product_wide_kernel(const __grid_constant__ CUtensorMap map_a, const __gr
     if (warp == 1) {
         tcgen05_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(GN) : "memory");
+    }
+}
+
+// The same for tiles of 256 columns as a persistent kernel, one block an SM: the blocks take the tiles (an expert's 128 rows x
+// 256 columns, the column tile running fastest) in turn, the ring and two accumulators in tensor memory carry on from tile to
+// tile, and the epilogue of a tile runs under the products of the next. A k-block brings 48 KB for 4.2 MFLOP where the tile of
+// 128 columns brings 32 KB for 2.1: those were bound by what an SM can load. 8 of 32 experts of 4,096 x 1,792, the whole
+// feed-forward, tiles of 128 -> these: 128 tokens 305 -> 292 us, 777 485 -> 424, 2,077 1,084 -> 830, 8,192 3,628 -> 2,732.
+constexpr int SN = 256;
+constexpr size_t STREAM_SMEM = 1024 + 4 * (size_t)(A_BYTES + SN * GK * 2) + (2 * 4 + 4) * 8 + 16;
+template <bool GLU>
+__global__ void __launch_bounds__(G_THREADS, 1)
+expert_product_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                             const int* __restrict__ plan, int E, int max_tiles, int b_rows, int N, int n_kblocks,
+                             __nv_bfloat16* __restrict__ act, float* __restrict__ y, const int* __restrict__ sorted,
+                             const float* __restrict__ weights, Activation activation, int* status) {
+    constexpr int STAGES = 4, B_BYTES = SN * GK * 2;
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    unsigned char* a_tiles = base;
+    unsigned char* b_tiles = base + (size_t)STAGES * A_BYTES;
+    uint64_t* full_bar = reinterpret_cast<uint64_t*>(b_tiles + (size_t)STAGES * B_BYTES);
+    uint64_t* empty_bar = full_bar + STAGES;
+    uint64_t* acc_full = full_bar + 2 * STAGES;            // [2]
+    uint64_t* acc_empty = acc_full + 2;                    // [2]
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 4);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < STAGES; ++s) {
+            mbar_init(smem_u32(&full_bar[s]), 1);
+            mbar_init(smem_u32(&empty_bar[s]), 1);
+        }
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(smem_u32(&acc_full[i]), 1);
+            mbar_init(smem_u32(&acc_empty[i]), 4);         // the epilogue's warps
+        }
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                     ::"r"(smem_u32(tmem_slot)), "r"(2 * SN) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tcgen05_fence_before();
+    __syncthreads();
+    tcgen05_fence_after();
+    uint32_t tmem_base = *tmem_slot;
+    griddep_launch();                                      // behind the allocation: no block of the next kernel can hold this one's
+    griddep_wait();                                        // the plan is the work of a kernel before
+    plan = behind_wait(plan);
+    sorted = behind_wait(sorted);
+    const int* tile_expert = plan + E + 2;
+    constexpr int STEP = GLU ? SN / 2 : SN;                // output columns of a tile
+    int columns = (N + STEP - 1) / STEP, total = plan[E + 1] * columns;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            int s = 0;
+            uint32_t round = 0;
+            bool ok = true;
+            for (int u = blockIdx.x; u < total && ok; u += gridDim.x) {
+                int tile = u / columns, n0 = (u - tile * columns) * STEP;
+                int first = tile_expert[max_tiles + tile], b_row = tile_expert[tile] * b_rows + n0;
+                for (int kb = 0; kb < n_kblocks; ++kb) {
+                    ok = mbar_wait(smem_u32(&empty_bar[s]), (round & 1) ^ 1, abort_flag, status, 1);
+                    if (!ok) break;
+                    uint32_t bar = smem_u32(&full_bar[s]);
+                    mbar_expect_tx(bar, A_BYTES + B_BYTES);
+                    tma_load_2d(smem_u32(a_tiles + (size_t)s * A_BYTES), &map_a, bar, kb * GK, first);
+                    // boxes of 128 rows: the gate rows and the up rows of the same features, or 256 rows on end
+                    tma_load_2d(smem_u32(b_tiles + (size_t)s * B_BYTES), &map_b, bar, kb * GK, b_row);
+                    tma_load_2d(smem_u32(b_tiles + (size_t)s * B_BYTES + B_BYTES / 2), &map_b, bar, kb * GK, b_row + (GLU ? N : SN / 2));
+                    if (++s == STAGES) { s = 0; ++round; }
+                }
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            // instruction descriptor: D 32-bit, A and B bfloat16, both K-major, N = 256, M = 128
+            constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(SN >> 3) << 17) | ((uint32_t)(GM >> 4) << 24);
+            const uint64_t a_desc0 = smem_desc(smem_u32(a_tiles)), b_desc0 = smem_desc(smem_u32(b_tiles));
+            int s = 0;
+            uint32_t phase = 0, done = 0;
+            bool ok = true;
+            for (int u = blockIdx.x; u < total && ok; u += gridDim.x, ++done) {
+                uint32_t buffer = done & 1, use = done >> 1;
+                ok = mbar_wait(smem_u32(&acc_empty[buffer]), (use & 1) ^ 1, abort_flag, status, 4);
+                if (!ok) break;
+                tcgen05_fence_after();
+                for (int kb = 0; kb < n_kblocks; ++kb) {
+                    ok = mbar_wait(smem_u32(&full_bar[s]), phase, abort_flag, status, 2);
+                    if (!ok) break;
+                    tcgen05_fence_after();
+                    uint64_t a_desc = a_desc0 + (uint64_t)(s * (A_BYTES >> 4)), b_desc = b_desc0 + (uint64_t)(s * (B_BYTES >> 4));
+#pragma unroll
+                    for (int k = 0; k < GK / 16; ++k)
+                        tcgen05_mma(tmem_base + buffer * SN, a_desc + 2 * k, b_desc + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                    tcgen05_commit(smem_u32(&empty_bar[s]));
+                    if (++s == STAGES) { s = 0; phase ^= 1; }
+                }
+                if (ok) tcgen05_commit(smem_u32(&acc_full[buffer]));
+            }
+        }
+    } else {
+        int quarter = warp & 3, row = quarter * 32 + lane;
+        uint32_t done = 0;
+        for (int u = blockIdx.x; u < total; u += gridDim.x, ++done) {
+            int tile = u / columns, n0 = (u - tile * columns) * STEP;
+            int first = tile_expert[max_tiles + tile], rows = tile_expert[2 * max_tiles + tile];
+            uint32_t buffer = done & 1, use = done >> 1;
+            bool ok = mbar_wait(smem_u32(&acc_full[buffer]), use & 1, abort_flag, status, 3);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            tcgen05_fence_after();
+            store_row<GLU, SN>(tmem_base + ((uint32_t)(quarter * 32) << 16) + buffer * SN, row, rows, first, n0, N, act, y, sorted,
+                               weights, activation);
+            tcgen05_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&acc_empty[buffer]));
+        }
+    }
+
+    tcgen05_fence_before();
+    __syncthreads();
+    if (*abort_flag) {
+        for (int i = 0; i < 100; ++i) __nanosleep(10000);          // copies in flight land before shared memory is given up
+        __syncthreads();
+    }
+    if (warp == 1) {
+        tcgen05_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2 * SN) : "memory");
     }
 }
 
@@ -805,17 +946,17 @@ LLMB_EXPORT int llmb_routed_experts(const void* h, int ld, int dtype, const floa
     if (wide_tiles) {
         typedef __nv_bfloat16 B;
         using namespace wide;
-        // tiles of 256 columns for long lists (measured at width 4096, 8 of 32 experts of 1792: 3.65 against 3.86 ms at 8,192
-        // tokens, equal at 2,048, behind at width 2048) where the products are wide enough for them
-        bool wide256 = tensor_cores >= 3 && F >= 128 && hidden >= 256 && (long long)n_assign >= 1024LL * E;
-        int GN = wide256 ? 256 : 128;
+        // tiles of 256 columns wherever the products are wide enough for them (ahead at every length of the lists that comes
+        // here, 128 to 8,192 tokens, and at all four shapes that were measured)
+        bool wide256 = tensor_cores >= 3 && F >= 128 && hidden >= 256;
+        constexpr int GN = 128;
         size_t smem = smem_of(GN);
         static bool configured = false;
         if (!configured) {
             LLMB_CUDA(cudaFuncSetAttribute(expert_product_wide_kernel<true, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_of(128)));
             LLMB_CUDA(cudaFuncSetAttribute(expert_product_wide_kernel<false, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_of(128)));
-            LLMB_CUDA(cudaFuncSetAttribute(expert_product_wide_kernel<true, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_of(256)));
-            LLMB_CUDA(cudaFuncSetAttribute(expert_product_wide_kernel<false, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_of(256)));
+            LLMB_CUDA(cudaFuncSetAttribute(expert_product_stream_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)STREAM_SMEM));
+            LLMB_CUDA(cudaFuncSetAttribute(expert_product_stream_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)STREAM_SMEM));
             configured = true;
         }
         int* status_dev = nullptr;
@@ -823,7 +964,7 @@ LLMB_EXPORT int llmb_routed_experts(const void* h, int ld, int dtype, const floa
         if (status_host) LLMB_CUDA(cudaHostGetDevicePointer((void**)&status_dev, status_host, 0));
         CUtensorMap map_x, map_up, map_act, map_down;
         int code = llmb::tc::make_map_2d(&map_x, gathered, n_assign, hidden, hidden, GK, GM);
-        if (!code) code = llmb::tc::make_map_2d(&map_up, w_up, (long long)E * 2 * F, hidden, hidden, GK, GN / 2);
+        if (!code) code = llmb::tc::make_map_2d(&map_up, w_up, (long long)E * 2 * F, hidden, hidden, GK, wide256 ? 128 : GN / 2);
         if (!code) code = llmb::tc::make_map_2d(&map_act, act, n_assign, F, F, GK, GM);
         if (!code) code = llmb::tc::make_map_2d(&map_down, w_down, (long long)E * hidden, F, F, GK, GN);
         if (code) return code;
@@ -833,8 +974,18 @@ LLMB_EXPORT int llmb_routed_experts(const void* h, int ld, int dtype, const floa
         int gather_blocks = (int)((vectors + 255) / 256 < 148 * 8 ? (vectors + 255) / 256 : 148 * 8);
         LLMB_CUDA(llmb::launch(gather_rows_kernel, dim3(gather_blocks), dim3(256), 0, stream, true, (const B*)h, ld, top,
                                (const int*)sorted, (const int*)plan, E, hidden, (B*)gathered));
-        auto up = wide256 ? expert_product_wide_kernel<true, 256> : expert_product_wide_kernel<true, 128>;
-        auto down = wide256 ? expert_product_wide_kernel<false, 256> : expert_product_wide_kernel<false, 128>;
+        if (wide256) {
+            auto blocks = [&](int columns) { long long all = (long long)tiles * columns; return dim3((unsigned)(all < 148 ? all : 148)); };
+            LLMB_CUDA(llmb::launch(expert_product_stream_kernel<true>, blocks((F + 127) / 128), dim3(G_THREADS), STREAM_SMEM, stream,
+                                   true, map_x, map_up, (const int*)plan, E, max_tiles, 2 * F, F, (hidden + GK - 1) / GK, (B*)act,
+                                   (float*)nullptr, (const int*)sorted, up_weights, activation, status_dev));
+            LLMB_CUDA(llmb::launch(expert_product_stream_kernel<false>, blocks((hidden + 255) / 256), dim3(G_THREADS), STREAM_SMEM,
+                                   stream, true, map_act, map_down, (const int*)plan, E, max_tiles, hidden, hidden,
+                                   (F + GK - 1) / GK, (B*)nullptr, y, (const int*)sorted, down_weights, activation, status_dev));
+            return check_launch("routed_experts");
+        }
+        auto up = expert_product_wide_kernel<true, 128>;
+        auto down = expert_product_wide_kernel<false, 128>;
         LLMB_CUDA(llmb::launch(up, dim3((F + GN / 2 - 1) / (GN / 2), tiles), dim3(G_THREADS), smem, stream, true, map_x, map_up,
                                (const int*)plan, E, max_tiles, 2 * F, F, (hidden + GK - 1) / GK, (B*)act, (float*)nullptr,
                                (const int*)sorted, up_weights, activation, status_dev));

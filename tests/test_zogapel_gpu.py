@@ -53,6 +53,23 @@ def test_norm_add(out_dtype, width):
             _close(got, want, out_dtype, (terms, n, "next"))
 
 
+@pytest.mark.parametrize("width", [4, 2048, 2052, 4096, 6148, 8192, 8196])
+@pytest.mark.parametrize("terms", [1, 8])
+def test_norm_add_at_the_edges_of_rows_in_registers(width, terms):
+    ops = _ops()
+    gen = torch.Generator().manual_seed(width + terms)
+    for n in (1, 5):
+        x = (2.0 * torch.randn((n, width), generator=gen)).to(DEV)
+        y = (5.0 * torch.randn((n * terms, width), generator=gen)).to(DEV)
+        g1, g2 = (1.0 + 0.3 * torch.randn(width, generator=gen)).to(DEV), torch.randn(width, generator=gen).to(DEV)
+        xa, xb = x.clone(), x.clone()
+        got = ops.norm_add_(xa, y, g1, 1e-5, terms, g2, 1e-3, out=torch.zeros((n, width), dtype=torch.bfloat16, device=DEV),
+                            out_dtype=torch.bfloat16)
+        want = plain_ops.norm_add_(xb, y, g1, 1e-5, terms, g2, 1e-3, out_dtype=torch.bfloat16)
+        _close(xa, xb, torch.float32, (terms, n, "x"))
+        _close(got, want, torch.bfloat16, (terms, n, "next"))
+
+
 def test_norm_add_sums_a_token_s_rows_in_their_order():
     """Three rows a token whose sum in another order would round differently: 1e8 - 1e8 + 1 is 1, not 0."""
     ops = _ops()
@@ -223,6 +240,23 @@ def test_delta_rule(dtype, case):
         _close(states[0], states[1], torch.float32, (case, lengths, "state"))          # also the slots and columns that no one owns
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("case", [(2, 1, 128, 128, 4), (3, 1, 64, 40, 4), (4, 2, 64, 64, 4)])
+def test_delta_rule_of_long_steps(dtype, case):
+    """Steps whose convolution runs by pieces of four tokens: sequences that begin at every place of a piece, shorter ones than
+    the taps, values that fill no whole piece, a last piece of fewer tokens."""
+    ops = _ops()
+    H, G, D, V, K = case
+    batch = Batch([500, 64, 129, 5, 2, 40], [500, 3, 66, 5, 1, 40], seed=1)
+    proj, params, state = _delta_inputs(H, G, D, V, K, batch.n_tokens, 8, dtype, seed=D + V)
+    states = [state.clone(), state.clone()]
+    got = _delta(ops.delta_rule, proj, params, states[0], batch, H, G, D, V, dtype)
+    want = _delta(plain_ops.delta_rule, proj, params, states[1], batch, H, G, D, V, dtype)
+    torch.cuda.synchronize()
+    _close(got, want, dtype, (case, "out"))
+    _close(states[0], states[1], torch.float32, (case, "state"))
+
+
 def test_delta_rule_carries_its_state_across_any_cut():
     """A sequence in one step, and the same cut at every place into two steps (the second also token by
     token): the same results to the last bit in 32-bit, and the state that the cuts leave is the same."""
@@ -389,6 +423,29 @@ def test_routed_experts_on_tiles_of_256_columns():
         assert float((y - other_y).abs().max()) <= 2e-2 * float(other_y.abs().max())
     want = _experts(plain_ops.routed_experts, h[:64].contiguous(), router, None, w_up, w_down, top)[2]
     _close(y[:64], want, torch.bfloat16, "rows against the plain statement")
+
+
+@pytest.mark.parametrize("n", [511, 512, 515, 1184, 1191])
+@pytest.mark.parametrize("E,top,hidden", [(3, 2, 48), (32, 8, 132), (33, 4, 40)])
+def test_router_takes_several_tokens_a_block(n, E, top, hidden):
+    """Four and eight tokens a block, a last block of fewer, experts that fill no warp's four: every token's choice and
+    weights are bit for bit those of a step of few tokens."""
+    ops = _ops()
+    gen = torch.Generator().manual_seed(n + E)
+    F = 8
+    w_up = torch.zeros((E, 2 * F, hidden), device=DEV)
+    w_down = torch.zeros((E, hidden, F), device=DEV)
+    router = torch.randn((E, hidden), generator=gen).to(DEV)
+    bias = torch.randn(E, generator=gen).to(DEV)
+    h = torch.randn((n, hidden), generator=gen).to(DEV)
+    ids, weights, _ = _experts(ops.routed_experts, h, router, bias, w_up, w_down, top)
+    for first in range(0, n, 300):
+        some = h[first:first + 300].contiguous()
+        few_ids, few_weights, _ = _experts(ops.routed_experts, some, router, bias, w_up, w_down, top)
+        at = slice(first * top, (first + some.shape[0]) * top)
+        assert torch.equal(ids[at], few_ids) and torch.equal(weights[at], few_weights), first
+    logits = h.double() @ router.double().T + bias.double()
+    assert torch.equal(ids.view(n, top).long(), torch.topk(logits, top, -1).indices)
 
 
 def test_routed_experts_choice_ties_and_batch_independence():
