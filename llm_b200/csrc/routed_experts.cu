@@ -71,6 +71,8 @@ __device__ __forceinline__ void load4(const __nv_bfloat16* p, float (&x)[4]) {
     x[0] = lo.x; x[1] = lo.y; x[2] = hi.x; x[3] = hi.y;
 }
 
+constexpr int ROUTER_LOGITS = 48 * 1024 / (int)sizeof(float);      // values a block can keep without asking for more shared memory
+
 // A block takes TOK tokens and a warp EXP experts at a time: a weight row fetched once serves all of the tokens, a token's
 // elements all of the experts (bound by the loads: every block reads the whole matrix). A token's sum runs in the same order
 // whatever TOK and EXP are (a lane's elements in rising order, then the lanes as a butterfly). The choice is a warp's: a
@@ -920,17 +922,12 @@ LLMB_EXPORT int llmb_routed_experts(const void* h, int ld, int dtype, const floa
     int tile_m = wide_tiles ? wide::GM : TILE_M;
 #define LLMB_EXPERTS(T)                                                                                            \
     do {                                                                                                           \
-        if (n_tokens >= 512) {                                                                                     \
-            /* eight tokens a block once that still gives every SM one */                                          \
-            int tok = n_tokens >= 8 * 148 ? 8 : 4;                                                                 \
-            auto kernel = tok == 8 ? router_kernel<T, 8, 4> : router_kernel<T, 4, 4>;                              \
-            LLMB_CUDA(llmb::launch(kernel, dim3((n_tokens + tok - 1) / tok), dim3(256), sizeof(float) * tok * R,   \
-                                   stream, true, (const T*)h, ld, router, router_bias, hidden, R, top, ids,       \
-                                   weights, n_tokens, router_vectors, scoring, correction, weight_scale, groups, keep));        \
-        } else                                                                                                     \
-            LLMB_CUDA(llmb::launch(router_kernel<T, 1, 1>, dim3(n_tokens), dim3(512), sizeof(float) * R, stream,     \
-                                   true, (const T*)h, ld, router, router_bias, hidden, R, top, ids, weights,       \
-                                   n_tokens, router_vectors, scoring, correction, weight_scale, groups, keep));                  \
+        /* eight tokens a block once that still gives every SM one; fewer where their logits would not fit */      \
+        int tok = n_tokens >= 8 * 148 && 8 * R <= ROUTER_LOGITS ? 8 : n_tokens >= 512 && 4 * R <= ROUTER_LOGITS ? 4 : 1; \
+        auto router_of = tok == 8 ? router_kernel<T, 8, 4> : tok == 4 ? router_kernel<T, 4, 4> : router_kernel<T, 1, 1>; \
+        LLMB_CUDA(llmb::launch(router_of, dim3((n_tokens + tok - 1) / tok), dim3(tok > 1 ? 256 : 512),             \
+                               sizeof(float) * tok * R, stream, true, (const T*)h, ld, router, router_bias, hidden, R, \
+                               top, ids, weights, n_tokens, router_vectors, scoring, correction, weight_scale, groups, keep)); \
         if (pass_through > 0)                                                                                      \
             LLMB_CUDA(llmb::launch(pass_through_kernel<T>, dim3(n_assign), dim3(256), 0, stream, true, (const T*)h, \
                                    ld, top, (const int*)ids, (const float*)weights, E, hidden, y));                \

@@ -448,6 +448,23 @@ def test_router_takes_several_tokens_a_block(n, E, top, hidden):
     assert torch.equal(ids.view(n, top).long(), torch.topk(logits, top, -1).indices)
 
 
+@pytest.mark.parametrize("E,n", [(1536, 1184), (1537, 1184), (2048, 1191), (2048, 600), (1400, 1300)])
+def test_router_of_many_experts(E, n):
+    """Routers whose logits for eight tokens are more than a block's 48 KB of shared memory: the same choice as in a step of
+    few tokens, at every length of a step."""
+    ops = _ops()
+    gen = torch.Generator().manual_seed(E + n)
+    F, hidden, top = 8, 16, 4
+    w_up, w_down = torch.zeros((E, 2 * F, hidden), device=DEV), torch.zeros((E, hidden, F), device=DEV)
+    router, bias = torch.randn((E, hidden), generator=gen).to(DEV), torch.randn(E, generator=gen).to(DEV)
+    h = torch.randn((n, hidden), generator=gen).to(DEV)
+    ids, weights, _ = _experts(ops.routed_experts, h, router, bias, w_up, w_down, top)
+    for first in range(0, n, 500):
+        few_ids, few_weights, _ = _experts(ops.routed_experts, h[first:first + 500].contiguous(), router, bias, w_up, w_down, top)
+        at = slice(first * top, first * top + few_ids.numel())
+        assert torch.equal(ids[at], few_ids) and torch.equal(weights[at], few_weights), first
+
+
 def test_routed_experts_choice_ties_and_batch_independence():
     """The bias alone decides when the router's matrix is zero; equal logits go to the lower index; a
     token's rows do not depend on what else is in the step (bit for bit in 32-bit)."""
