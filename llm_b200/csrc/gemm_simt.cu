@@ -57,16 +57,13 @@ __device__ __forceinline__ void park_tile(float (*tile)[LD], const float (&held)
 // memory, are multiplied; the order of a thread's additions is k = 0, 1, 2, ... as before.
 template <typename TIn, typename TOut, int BM, int BN, int BK, int TM, int TN>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN))
-gemm_simt_kernel(const TIn* a, const TIn* __restrict__ w,
+gemm_simt_kernel(const TIn* __restrict__ a, const TIn* __restrict__ w,
                  const float* __restrict__ bias, TOut* __restrict__ out,
                  float* __restrict__ residual, int M, int N, int K, int lda, int ldc, int vector) {
     constexpr int THREADS = (BM / TM) * (BN / TN);
     constexpr int A_ITEMS = (BM * BK / 4 + THREADS - 1) / THREADS, W_ITEMS = (BN * BK / 4 + THREADS - 1) / THREADS;
     __shared__ float a_tile[BK][BM + 4];
     __shared__ float w_tile[BK][BN + 4];
-    griddep_launch();
-    griddep_wait();
-    a = behind_wait(a);
     int tid = threadIdx.x;
     int tx = tid % (BN / TN), ty = tid / (BN / TN);
     int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
@@ -222,12 +219,12 @@ static int launch(const void* a, const void* w, const float* bias, void* out, fl
     }
     if (M > 64) {
         dim3 grid(ceil_div(N, 128), ceil_div(M, 128));
-        LLMB_CUDA(llmb::launch(gemm_simt_kernel<TIn, TOut, 128, 128, 8, 8, 8>, grid, dim3(256), 0, stream, true,
-                               (const TIn*)a, (const TIn*)w, bias, (TOut*)out, residual, M, N, K, lda, ldc, vector));
+        gemm_simt_kernel<TIn, TOut, 128, 128, 8, 8, 8><<<grid, 256, 0, stream>>>(
+            (const TIn*)a, (const TIn*)w, bias, (TOut*)out, residual, M, N, K, lda, ldc, vector);
     } else {
         dim3 grid(ceil_div(N, 64), ceil_div(M, 32));
-        LLMB_CUDA(llmb::launch(gemm_simt_kernel<TIn, TOut, 32, 64, 16, 2, 4>, grid, dim3(256), 0, stream, true,
-                               (const TIn*)a, (const TIn*)w, bias, (TOut*)out, residual, M, N, K, lda, ldc, vector));
+        gemm_simt_kernel<TIn, TOut, 32, 64, 16, 2, 4><<<grid, 256, 0, stream>>>(
+            (const TIn*)a, (const TIn*)w, bias, (TOut*)out, residual, M, N, K, lda, ldc, vector);
     }
     return check_launch("gemm_simt");
 }
