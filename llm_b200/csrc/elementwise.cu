@@ -351,9 +351,11 @@ __global__ void rope_cache_kernel(T* __restrict__ qkv, const float* __restrict__
                                   const int* __restrict__ block_table, int table_stride,
                                   int ring_pages, T* __restrict__ k_cache, T* __restrict__ v_cache,
                                   int n_heads, int n_kv_heads, int head_dim, int n_rot, int interleaved,
-                                  int write_cache) {
-    griddep_launch();
-    griddep_wait();                      // (src is written too: nothing is read through a constant pointer but tables)
+                                  int write_cache, int dependent) {
+    if (dependent) {
+        griddep_launch();
+        griddep_wait();                  // (src is written too: nothing is read through a constant pointer but tables)
+    }
     int t = blockIdx.x;
     int head = blockIdx.y;               // [0, Hq): q; [Hq, Hq+Hkv): k; then v
     int pos = tok_pos[t];
@@ -499,15 +501,18 @@ LLMB_EXPORT int llmb_rope_cache_write(void* qkv, int dtype, const float* table,
     }
     dim3 grid(n_tokens, n_heads + 2 * n_kv_heads);
     int threads = head_dim / 2 >= 64 ? 64 : 32;
+    // A dependent launch saves a small step its gap; where the blocks take turns on the SMs, each pays for its wait
+    // (32-bit, 32 heads over 8 of 128: 2,048 tokens 52 us plainly launched, 101 us dependent; 64 tokens 2.9 and 3.6).
+    bool dependent = (long long)n_tokens * (n_heads + 2 * n_kv_heads) <= 4 * 148;
     if (dtype == LLMB_DTYPE_F32)
-        llmb::launch(rope_cache_kernel<float>, grid, dim3(threads), 0, stream, true,
+        llmb::launch(rope_cache_kernel<float>, grid, dim3(threads), 0, stream, dependent,
             (float*)qkv, table, tok_pos, tok_seq, block_table, table_stride, ring_pages,
-            (float*)k_cache, (float*)v_cache, n_heads, n_kv_heads, head_dim, n_rot, interleaved, write_cache);
+            (float*)k_cache, (float*)v_cache, n_heads, n_kv_heads, head_dim, n_rot, interleaved, write_cache, (int)dependent);
     else if (dtype == LLMB_DTYPE_BF16)
-        llmb::launch(rope_cache_kernel<__nv_bfloat16>, grid, dim3(threads), 0, stream, true,
+        llmb::launch(rope_cache_kernel<__nv_bfloat16>, grid, dim3(threads), 0, stream, dependent,
             (__nv_bfloat16*)qkv, table, tok_pos, tok_seq, block_table, table_stride, ring_pages,
             (__nv_bfloat16*)k_cache, (__nv_bfloat16*)v_cache, n_heads, n_kv_heads, head_dim, n_rot,
-            interleaved, write_cache);
+            interleaved, write_cache, (int)dependent);
     else
         return fail(LLMB_ERR_ARGUMENT, "rope: unknown dtype %d", dtype);
     return check_launch("rope_cache_write");
