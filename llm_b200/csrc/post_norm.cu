@@ -63,13 +63,14 @@ norm_add_kernel(const float* __restrict__ y, int terms, const float* __restrict_
         h[t * hidden + c] = from_float<TOut>(row[c] * rstd * gain_next[c]);
 }
 
-// The same for rows of a multiple of four values up to 8,192, all arrays on 16-byte boundaries: 512 threads hold a row in
-// registers, NV groups of four values each, and every load that does not wait for a sum is requested before the first one
-// is needed (the gains even before the kernel in front has ended). A row is one chain of load, sum, sum; the kernel above
-// walks it element by element, with a chain of `terms` loads for each. Rows of 4,096, some of them with eight terms: 24
-// rows 14.7 -> 4.2 us, 2,077 rows 44.7 -> 37.0 us. The choice depends on the row's width and the addresses' alignment
-// only, so that a row's sums have one order in every step.
-constexpr int WIDE_THREADS = 512;
+// The same for rows of a multiple of four values up to 8,192, all arrays on 16-byte boundaries: NT threads (as many as the row
+// has groups of four, up to 512) hold a row in registers, NV groups of four values each, and every load that does not wait
+// for a sum is requested before the first one is needed (the gains even before the kernel in front has ended). A row is one
+// chain of load, sum, sum; the kernel above walks it element by element, with a chain of `terms` loads for each. Rows of
+// 4,096, some of them with eight terms: 24 rows 14.7 -> 4.2 us, 2,077 rows 44.7 -> 37.0 us. Short rows, 4,096 of them with one
+// term: of 64 values 8.3 us by the kernel above, 19.3 with 512 threads a row, 4.7 so; of 1,024 values 17.6, 20.6 and 9.3. The
+// choice depends on the row's width and the addresses' alignment only, so that a row's sums have one order in every step.
+constexpr int WIDE_THREADS = 512;      // most threads a row
 template <typename TOut> __device__ __forceinline__ void store4(TOut* p, float4 v);
 template <> __device__ __forceinline__ void store4<float>(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
 template <> __device__ __forceinline__ void store4<__nv_bfloat16>(__nv_bfloat16* p, float4 v) {
@@ -80,18 +81,18 @@ __device__ __forceinline__ float square4(float4 v, float sum) {
     return fmaf(v.w, v.w, fmaf(v.z, v.z, fmaf(v.y, v.y, fmaf(v.x, v.x, sum))));
 }
 
-template <typename TOut, int NV>
-__global__ void __launch_bounds__(WIDE_THREADS)
+template <typename TOut, int NV, int NT>
+__global__ void __launch_bounds__(NT)
 norm_add_wide_kernel(const float* __restrict__ y, int terms, const float* __restrict__ gain_post, float eps_post,
                      float* __restrict__ x, const float* __restrict__ gain_next, float eps_next, TOut* __restrict__ h,
                      int hidden) {
-    __shared__ float scratch[2][WIDE_THREADS / 32];
+    __shared__ float scratch[2][NT / 32];
     int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     griddep_launch();
     float4 post[NV], next[NV];
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-        int c = (threadIdx.x + i * WIDE_THREADS) * 4;
+        int c = (threadIdx.x + i * NT) * 4;
         post[i] = next[i] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (c < hidden) {
             post[i] = *reinterpret_cast<const float4*>(gain_post + c);
@@ -106,7 +107,7 @@ norm_add_wide_kernel(const float* __restrict__ y, int terms, const float* __rest
     float4 s[NV], v[NV];
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-        int c = (threadIdx.x + i * WIDE_THREADS) * 4;
+        int c = (threadIdx.x + i * NT) * 4;
         v[i] = s[i] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (c < hidden) {
             v[i] = *reinterpret_cast<const float4*>(x_row + c);
@@ -123,7 +124,7 @@ norm_add_wide_kernel(const float* __restrict__ y, int terms, const float* __rest
         __syncthreads();
         float all = 0.f;
 #pragma unroll
-        for (int w = 0; w < WIDE_THREADS / 32; ++w) all += part[w];
+        for (int w = 0; w < NT / 32; ++w) all += part[w];
         return all;
     };
     float sq = 0.f;
@@ -133,7 +134,7 @@ norm_add_wide_kernel(const float* __restrict__ y, int terms, const float* __rest
     sq = 0.f;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-        int c = (threadIdx.x + i * WIDE_THREADS) * 4;
+        int c = (threadIdx.x + i * NT) * 4;
         v[i].x += s[i].x * rstd * post[i].x;
         v[i].y += s[i].y * rstd * post[i].y;
         v[i].z += s[i].z * rstd * post[i].z;
@@ -145,7 +146,7 @@ norm_add_wide_kernel(const float* __restrict__ y, int terms, const float* __rest
     rstd = 1.0f / sqrtf(total(sq, scratch[1]) / (float)hidden + eps_next);
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-        int c = (threadIdx.x + i * WIDE_THREADS) * 4;
+        int c = (threadIdx.x + i * NT) * 4;
         if (c < hidden)
             store4(h + t * hidden + c, make_float4(v[i].x * rstd * next[i].x, v[i].y * rstd * next[i].y,
                                                    v[i].z * rstd * next[i].z, v[i].w * rstd * next[i].w));
@@ -161,12 +162,17 @@ LLMB_EXPORT int llmb_norm_add(const float* y, int terms, const float* gain_post,
     size_t smem = sizeof(float) * (size_t)hidden;
     LLMB_REQUIRE(smem <= 200 * 1024, "norm_add: a row of %d values does not fit in shared memory", hidden);
     size_t addresses = (size_t)y | (size_t)gain_post | (size_t)x | (size_t)gain_next | (size_t)h;
-    int wide = hidden % 4 == 0 && addresses % 16 == 0 ? (hidden + 4 * WIDE_THREADS - 1) / (4 * WIDE_THREADS) : 0;
+    bool wide = hidden % 4 == 0 && hidden <= 16 * WIDE_THREADS && addresses % 16 == 0;
 #define LLMB_NORM_ADD(T)                                                                                           \
     do {                                                                                                           \
-        if (wide >= 1 && wide <= 4) {                                                                              \
-            auto kernel = wide == 1 ? norm_add_wide_kernel<T, 1> : wide == 2 ? norm_add_wide_kernel<T, 2> : norm_add_wide_kernel<T, 4>; \
-            LLMB_CUDA(llmb::launch(kernel, dim3(n_rows), dim3(WIDE_THREADS), 0, stream, true, y, terms, gain_post, \
+        if (wide) {                                                                                                \
+            /* as many threads as the row has groups of four, up to 512 */                                         \
+            int threads = hidden <= 128 ? 32 : hidden <= 256 ? 64 : hidden <= 512 ? 128 : hidden <= 1024 ? 256 : WIDE_THREADS; \
+            auto kernel = threads == 32 ? norm_add_wide_kernel<T, 1, 32> : threads == 64 ? norm_add_wide_kernel<T, 1, 64> \
+                          : threads == 128 ? norm_add_wide_kernel<T, 1, 128> : threads == 256 ? norm_add_wide_kernel<T, 1, 256> \
+                          : hidden <= 2048 ? norm_add_wide_kernel<T, 1, 512> : hidden <= 4096 ? norm_add_wide_kernel<T, 2, 512> \
+                          : norm_add_wide_kernel<T, 4, 512>;                                                       \
+            LLMB_CUDA(llmb::launch(kernel, dim3(n_rows), dim3(threads), 0, stream, true, y, terms, gain_post,      \
                                    eps_post, x, gain_next, eps_next, (T*)h, hidden));                              \
             break;                                                                                                 \
         }                                                                                                          \

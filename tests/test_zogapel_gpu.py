@@ -53,7 +53,7 @@ def test_norm_add(out_dtype, width):
             _close(got, want, out_dtype, (terms, n, "next"))
 
 
-@pytest.mark.parametrize("width", [4, 2048, 2052, 4096, 6148, 8192, 8196])
+@pytest.mark.parametrize("width", [4, 128, 132, 260, 512, 516, 1024, 1028, 2048, 2052, 4096, 6148, 8192, 8196])
 @pytest.mark.parametrize("terms", [1, 8])
 def test_norm_add_at_the_edges_of_rows_in_registers(width, terms):
     ops = _ops()
