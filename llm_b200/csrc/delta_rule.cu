@@ -141,7 +141,7 @@ delta_prepare_pieces_kernel(const T* __restrict__ proj, int ld, const float* __r
         // a lane's channels: EPL from `first` on, a q and k piece has k's behind q's
         bool keys = piece < G;
         int first = lane * EPL + (keys ? piece * D : 2 * GD + (piece - G) * PIECE), used = keys ? N : EPL;
-        if (first >= C) continue;                
+        if (first >= C) continue;
         float x[N][TOK + 3], tap[N][4];
 #pragma unroll
         for (int e = 0; e < N; ++e) {
@@ -509,7 +509,11 @@ LLMB_EXPORT int llmb_delta_rule(const void* proj, int ld, int dtype, const float
         if (n_taps > 1)                                                                                            \
             LLMB_CUDA(llmb::launch(delta_conv_state_kernel<T>, dim3((C + 127) / 128, n_seqs), dim3(128), 0, stream, \
                                    true, (const T*)proj, ld, n_taps, state, state_stride, cu_seqlens, slot_ids, C)); \
-        LLMB_CUDA(llmb::launch(scan, scan_grid, dim3(SCAN_THREADS), smem_scan, stream, true,                       \
+        /* launched plainly: few long blocks, which must find the SMs empty to be spread over them evenly. A dependent launch \
+           puts them down while the kernels in front drain, several on the SMs that are free (or set to enough shared memory) \
+           first, and those set the time: 2 x 777 tokens, 32 heads of 128 over 16, 552 us in all so and 403 plainly; 4,096 \
+           tokens 2,536 and 1,781; a decode step of one token 13.7 and 13.2 */                                     \
+        LLMB_CUDA(llmb::launch(scan, scan_grid, dim3(SCAN_THREADS), smem_scan, stream, false,                      \
                                (const float*)work, work_ld, state, state_stride, s_offset, cu_seqlens, slot_ids,  \
                                o, H * V, H, G, D, V, vectors));                                                    \
         LLMB_CUDA(llmb::launch(delta_finish_kernel<T>, dim3(n_tokens, (H + THREADS / 32 - 1) / (THREADS / 32)), dim3(THREADS), 0, stream, true,             \
