@@ -88,6 +88,7 @@ conv_kernel(ConvSource<T> source, const int* __restrict__ tok_seq, const int* __
 // The same for four taps where four neighbouring channels lie on a boundary: a thread takes them for TOK tokens that follow
 // each other, so that a row of x is read once for the TOK tokens, 8 or 16 bytes at a time, and the taps once. Every value is
 // the sum of the kernel above in its order. Bound by memory: 2,500 tokens of 4,096 channels (61 MB) 68 -> 19 us.
+// Shorter steps than four tokens an SM keep the kernel above: with one token a thread, 64 sequences took 9 us longer.
 template <typename T> struct alignas(4 * sizeof(T)) Four { T v[4]; };
 template <typename T, int TOK>
 __global__ void __launch_bounds__(256)
@@ -478,16 +479,16 @@ LLMB_EXPORT int llmb_gated_recurrence(const void* y, int y_stride, const void* x
 #define LLMB_RECURRENCE(T)                                                                                          \
     do {                                                                                                            \
         ConvSource<T> source{(const T*)x, x_stride, state, conv_w, conv_b, taps, channels};                         \
-        if (taps == 4 && channels % 4 == 0 && x_stride % 4 == 0 && ((size_t)x % (4 * sizeof(T))) == 0 &&            \
-            (((size_t)conv_w | (size_t)conv_b | (size_t)work) % 16) == 0) {                                         \
-            int tok = n_tokens >= 4 * 148 ? 4 : 1;                                                                  \
-            auto conv = tok == 4 ? conv_fours_kernel<T, 4> : conv_fours_kernel<T, 1>;                               \
-            LLMB_CUDA(llmb::launch(conv, dim3(ceil_div(n_tokens, tok), ceil_div(channels, 1024)), dim3(256), 0,     \
-                                   stream, true, source, tok_seq, cu_seqlens, slot_ids, u, n_tokens));              \
+        if (n_tokens >= 4 * 148 && taps == 4 && channels % 4 == 0 && x_stride % 4 == 0 &&                           \
+            ((size_t)x % (4 * sizeof(T))) == 0 && (((size_t)conv_w | (size_t)conv_b | (size_t)work) % 16) == 0) {   \
+            LLMB_CUDA(llmb::launch(conv_fours_kernel<T, 4>, dim3(ceil_div(n_tokens, 4), ceil_div(channels, 1024)),  \
+                                   dim3(256), 0, stream, true, source, tok_seq, cu_seqlens, slot_ids, u, n_tokens)); \
         } else                                                                                                      \
             LLMB_CUDA(llmb::launch(conv_kernel<T>, dim3(n_tokens, ceil_div(channels, 256)), dim3(256), 0, stream,   \
                                    true, source, tok_seq, cu_seqlens, slot_ids, u));                                \
-        LLMB_CUDA(llmb::launch(gates, grid_gates, dim3(256), 0, stream, true, (const float*)u, channels, gate_a,    \
+        /* launched plainly, so that its blocks find the SMs empty: put down while the convolution drains, several of them \
+           share an SM (64 sequences of one token, 4,096 channels: 49 us in all dependent, 26 plainly) */          \
+        LLMB_CUDA(llmb::launch(gates, grid_gates, dim3(256), 0, stream, false, (const float*)u, channels, gate_a,    \
                                gate_a_bias, gate_i, gate_i_bias, part, rate, decay, drive, n_tokens));              \
         if (n_tokens == n_seqs && single_tokens) {                                                                  \
             LLMB_CUDA(llmb::launch(scan_single_kernel<T>, dim3(ceil_div(channels, 256), n_seqs), dim3(256), 0, stream, \
