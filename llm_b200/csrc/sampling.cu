@@ -1,4 +1,4 @@
-// Token sampling on the device, one cluster of eight blocks per row of logits.
+// Token sampling on the device, one block or a cluster of blocks per row of logits.
 //
 // The chain and its order are those of MythEclipse/llm's sampler
 // (apps/engine/src/sampler.rs:54-96): repeat penalty over the recent window
@@ -16,11 +16,11 @@
 // uniform number picks differs from a walk in descending order).
 //
 // What bounds it: half a megabyte a row through the few SMs that a batch of rows keeps busy. With one block a row
-// (32 rows of 128,256: 32 of 148 SMs, the row read four times at some 100 GB/s an SM) a draw took 62 us; the eight
-// blocks of a cluster each read an eighth of the row (256 blocks for 32 rows), add their histograms into the first
-// block's shared memory and hand it their candidates, and the first block ranks them and draws. The select stops as
-// soon as the elements not below its bin fit the candidate buffer (after one digit for rows of logits), so the row is
-// read twice. Copying 32 rows of 128,256 logits and drawing from them with the default parameters: 76 -> 44 us.
+// (32 rows of 128,256: 32 of 148 SMs, the row read four times at some 100 GB/s an SM) a draw took 62 us. The blocks of a
+// cluster (up to eight: blocks_a_row) each read their share of the row, add their histograms into the first block's shared
+// memory and hand it their candidates, and the first block ranks them and draws. The select stops as soon as the elements
+// not below its bin fit the candidate buffer (after one digit for rows of logits), so the row is read twice. Copying 32
+// rows of 128,256 logits and drawing from them with the default parameters: 76 -> 44 us.
 #include <cooperative_groups.h>
 
 #include "common.cuh"
@@ -34,14 +34,28 @@ constexpr int MAX_TOP_K = 1024;
 constexpr int CANDIDATES = 2048;   // room for ties at the top-k threshold
 constexpr int RADIX_BINS = 2048;   // bins of the widest digit of the radix select
 constexpr int WINDOW = 1024;       // recent tokens the penalty handles in parallel (longer windows: one thread)
-constexpr int CLUSTER = 8;         // blocks a row (the portable cluster size)
+constexpr int CLUSTER = 8;         // most blocks a row (the portable cluster size)
+
+// The blocks of one row: a cluster, whose first block has the row's state and results in its shared memory, or one block.
+template <bool CLUSTERED> struct Team {
+    __device__ __forceinline__ int rank() const { return CLUSTERED ? (int)cooperative_groups::this_cluster().block_rank() : 0; }
+    __device__ __forceinline__ int blocks() const { return CLUSTERED ? (int)cooperative_groups::this_cluster().num_blocks() : 1; }
+    __device__ __forceinline__ void sync() const {
+        if constexpr (CLUSTERED) cooperative_groups::this_cluster().sync();
+        else __syncthreads();
+    }
+    template <typename T> __device__ __forceinline__ T* of(T* shared, int block) const {
+        if constexpr (CLUSTERED) return cooperative_groups::this_cluster().map_shared_rank(shared, block);
+        else return shared;
+    }
+};
 
 // The part of a row of n entries that block `rank` of its cluster reads: [begin, end), begins on multiples of four entries.
 struct Share {
     int begin, end;
 };
-__device__ __forceinline__ Share share_of(int n, int rank) {
-    int size = ((n + CLUSTER - 1) / CLUSTER + 3) / 4 * 4;
+__device__ __forceinline__ Share share_of(int n, int rank, int blocks) {
+    int size = ((n + blocks - 1) / blocks + 3) / 4 * 4;
     int begin = min(rank * size, n);
     return {begin, min(begin + size, n)};
 }
@@ -126,32 +140,62 @@ __device__ ArgMax block_argmax(const float* row, int n, ArgMax* scratch, float s
     return result;
 }
 
-// The same over a cluster: every block takes its share, block 0 has the result (the others' is their own share's).
-__device__ ArgMax cluster_argmax(const float* row, int n, ArgMax* scratch, ArgMax* gathered) {
-    namespace cg = cooperative_groups;
-    cg::cluster_group cluster = cg::this_cluster();
-    int rank = (int)cluster.block_rank();
-    Share share = share_of(n, rank);
+// The same over the blocks of a row: every block takes its share, block 0 has the result (the others' is their own share's).
+template <bool CLUSTERED>
+__device__ ArgMax team_argmax(const float* row, int n, ArgMax* scratch, ArgMax* gathered) {
+    Team<CLUSTERED> team;
+    if constexpr (!CLUSTERED) return block_argmax(row, n, scratch);
+    const int rank = team.rank(), blocks = team.blocks();
+    Share share = share_of(n, rank, blocks);
     ArgMax mine = block_argmax_open(row + share.begin, share.end - share.begin, scratch);
     if (mine.index != 0x7fffffff) mine.index += share.begin;
-    if (threadIdx.x == 0) cluster.map_shared_rank(gathered, 0)[rank] = mine;
-    cluster.sync();
+    if (threadIdx.x == 0) team.of(gathered, 0)[rank] = mine;
+    team.sync();
     ArgMax best = mine;
     if (rank == 0) {
-        for (int r = 0; r < CLUSTER; ++r) best = better(best, gathered[r]);
+        for (int r = 0; r < blocks; ++r) best = better(best, gathered[r]);
         if (best.index == 0x7fffffff) best.index = 0;
     }
     return best;
 }
 
-__global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(THREADS)
+template <bool CLUSTERED>
+__global__ void __launch_bounds__(THREADS)
 argmax_rows_kernel(const float* __restrict__ logits, int stride, int vocab, int* __restrict__ out) {
     __shared__ ArgMax scratch[32];
     __shared__ ArgMax gathered[CLUSTER];
-    cooperative_groups::this_cluster().sync();                // every block's shared memory exists from here on
-    int row = blockIdx.x / CLUSTER;
-    ArgMax best = cluster_argmax(logits + (size_t)row * stride, vocab, scratch, gathered);
-    if (blockIdx.x % CLUSTER == 0 && threadIdx.x == 0) out[row] = best.index;
+    Team<CLUSTERED> team;
+    if constexpr (CLUSTERED) team.sync();                     // every block's shared memory exists from here on
+    const int blocks = team.blocks();
+    int row = blockIdx.x / blocks;
+    ArgMax best = team_argmax<CLUSTERED>(logits + (size_t)row * stride, vocab, scratch, gathered);
+    if (blockIdx.x % blocks == 0 && threadIdx.x == 0) out[row] = best.index;
+}
+
+// How many blocks share a row. A row of a large vocabulary is long enough for several, as long as all rows' blocks find an
+// SM of their own; where they do not, blocks sit two on an SM (a walk over whole rows in index order, 16 rows of 128,256: 67 us
+// with one block a row or four, 79 with eight). What a cluster costs a short row is its barriers. The default chain, one
+// block -> as chosen here: 8 rows of 128,256 65 -> 31 us, 32 rows 68 -> 37, 64 rows 71 -> 45, 32 rows of 32,000 33 -> 25; and
+// eight blocks where one is chosen: 256 rows of 128,256 147 -> 258, 148 rows of 32,000 36 -> 81, 1,024 rows of 4,096 82 -> 406.
+static int blocks_a_row(int n_rows, int vocab) {
+    if (vocab < 16384) return 1;
+    if (n_rows <= 8) return 8;
+    if (n_rows <= 32) return 4;
+    return n_rows <= 64 && vocab >= 65536 ? 2 : 1;
+}
+template <typename... Params, typename... Args>
+static cudaError_t launch_rows(void (*kernel)(Params...), int blocks, int n_rows, cudaStream_t stream, Args... args) {
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(n_rows * blocks);
+    config.blockDim = dim3(THREADS);
+    config.stream = stream;
+    cudaLaunchAttribute attribute[1];
+    attribute[0].id = cudaLaunchAttributeClusterDimension;
+    attribute[0].val.clusterDim.x = blocks;
+    attribute[0].val.clusterDim.y = attribute[0].val.clusterDim.z = 1;
+    config.attrs = attribute;
+    config.numAttrs = blocks > 1 ? 1 : 0;
+    return cudaLaunchKernelEx(&config, kernel, Params(args)...);
 }
 
 LLMB_EXPORT int llmb_argmax_rows(const float* logits, int stride, int n_rows, int vocab, int* out,
@@ -159,7 +203,11 @@ LLMB_EXPORT int llmb_argmax_rows(const float* logits, int stride, int n_rows, in
     if (n_rows == 0) return LLMB_OK;
     LLMB_REQUIRE(n_rows > 0 && vocab > 0 && stride >= vocab, "argmax: bad sizes");
     LLMB_REQUIRE(n_rows <= 0x7fffffff / CLUSTER, "argmax: too many rows");
-    argmax_rows_kernel<<<n_rows * CLUSTER, THREADS, 0, stream>>>(logits, stride, vocab, out);
+    // (a maximum alone reads the row once: eight blocks pay from some 100,000 entries on, 16 rows of 128,256 6.0 -> 4.7 us,
+    // 8 rows of 32,000 3.0 -> 3.6)
+    int blocks = vocab >= 65536 && n_rows <= 32 ? blocks_a_row(n_rows, vocab) : 1;
+    LLMB_CUDA(launch_rows(blocks > 1 ? argmax_rows_kernel<true> : argmax_rows_kernel<false>, blocks, n_rows, stream, logits, stride,
+                          vocab, out));
     return check_launch("argmax_rows");
 }
 
@@ -200,7 +248,8 @@ __device__ unsigned block_exclusive_sum(unsigned value, unsigned* warp_totals) {
 //
 // Block 0 of a row's cluster owns the row's state and draws; the other blocks read their share of the row for the penalty,
 // the histogram and the candidates (and leave at once where the chain walks the whole row in index order).
-__global__ void __cluster_dims__(CLUSTER, 1, 1) __launch_bounds__(THREADS)
+template <bool CLUSTERED>
+__global__ void __launch_bounds__(THREADS)
 sample_rows_kernel(float* __restrict__ logits, int stride, int vocab,
                    const float4* __restrict__ params, const int2* __restrict__ iparams,
                    int* __restrict__ recent, int* __restrict__ recent_len,
@@ -215,13 +264,12 @@ sample_rows_kernel(float* __restrict__ logits, int stride, int vocab,
     __shared__ float block_sums[THREADS];
     __shared__ int window[WINDOW];
     __shared__ ArgMax gathered[CLUSTER];
-    namespace cg = cooperative_groups;
-    cg::cluster_group cluster = cg::this_cluster();
-    const int rank = (int)cluster.block_rank();
+    Team<CLUSTERED> team;
+    const int rank = team.rank(), blocks = team.blocks();
 
     // row of logits and of `out`; the sequence's parameters, window, generator and status are in
     // row state_rows[row] of their arrays (the same row if state_rows is null)
-    int logits_row = blockIdx.x / CLUSTER;
+    int logits_row = blockIdx.x / blocks;
     int row_id = state_rows ? state_rows[logits_row] : logits_row;
     LLMB_STAMP(0, 0);
     float* row = logits + (size_t)logits_row * stride;
@@ -229,7 +277,7 @@ sample_rows_kernel(float* __restrict__ logits, int stride, int vocab,
     float penalty = params[row_id].w;
     int top_k = iparams[row_id].x, last_n = iparams[row_id].y;
     int tid = threadIdx.x;
-    const Share share = share_of(vocab, rank);
+    const Share share = share_of(vocab, rank, blocks);
     // the chains without a ranking (whole row, or refused) run in block 0 alone
     const bool ranked = temperature > 0.f && (top_k > 0 || vocab <= MAX_TOP_K) && (top_k <= MAX_TOP_K || vocab <= MAX_TOP_K);
     const bool alone = temperature > 0.f && !ranked;
@@ -284,10 +332,10 @@ sample_rows_kernel(float* __restrict__ logits, int stride, int vocab,
     __syncthreads();
 
     // every block's shared memory exists, and every block has read the row's state (block 0's finish() changes it)
-    if (!alone) cluster.sync();
+    if (CLUSTERED && !alone) team.sync();
 
     if (!(temperature > 0.f)) {
-        ArgMax best = cluster_argmax(row, vocab, scratch, gathered);
+        ArgMax best = team_argmax<CLUSTERED>(row, vocab, scratch, gathered);
         if (rank == 0 && tid == 0) finish(best.index);
         return;
     }
@@ -387,7 +435,7 @@ sample_rows_kernel(float* __restrict__ logits, int stride, int vocab,
     for (; digit < 3;) {
         const int shift = bits(digit), n_bins = digit == 2 ? 1024 : 2048;
         for (int i = tid; i < RADIX_BINS; i += THREADS) histogram[i] = 0u;
-        cluster.sync();                        // (block 0's bins are zero before the others add to them)
+        team.sync();                        // (block 0's bins are zero before the others add to them)
         unsigned mask = digit == 0 ? 0u : (0xffffffffu << bits(digit - 1));
         for_each_of_row(row + share.begin, share.end - share.begin, [&](float v, int) {
             unsigned key = ordered_key(v * inverse);
@@ -395,30 +443,30 @@ sample_rows_kernel(float* __restrict__ logits, int stride, int vocab,
         });
         __syncthreads();
         if (rank != 0) {
-            unsigned* sums = cluster.map_shared_rank(histogram, 0);
+            unsigned* sums = team.of(histogram, 0);
             for (int i = tid; i < n_bins; i += THREADS)
                 if (histogram[i]) atomicAdd(&sums[i], histogram[i]);
         }
-        cluster.sync();
+        team.sync();
         if (rank == 0) {
             pick_bin(digit);
-            if (tid < CLUSTER && tid > 0) {
-                *cluster.map_shared_rank(&shared_prefix, tid) = shared_prefix;
-                *cluster.map_shared_rank(&shared_count, tid) = shared_count;
+            if (tid < blocks && tid > 0) {
+                *team.of(&shared_prefix, tid) = shared_prefix;
+                *team.of(&shared_count, tid) = shared_count;
             }
         }
-        cluster.sync();
+        team.sync();
         threshold = shared_prefix;
         ++digit;
         if (shared_count <= (unsigned)CANDIDATES) break;
     }
     LLMB_STAMP(2, 0);                                 // the radix select has its threshold
     if (rank == 0 && tid == 0) shared_gathered = 0u;     // now the number of candidates
-    cluster.sync();
+    team.sync();
     {
-        unsigned* at_ = cluster.map_shared_rank(&shared_gathered, 0);
-        float* values = cluster.map_shared_rank(cand_value, 0);
-        int* indices = cluster.map_shared_rank(cand_index, 0);
+        unsigned* at_ = team.of(&shared_gathered, 0);
+        float* values = team.of(cand_value, 0);
+        int* indices = team.of(cand_index, 0);
         for_each_of_row(row + share.begin, share.end - share.begin, [&](float v, int i) {
             v *= inverse;
             if (ordered_key(v) >= threshold) {
@@ -427,7 +475,7 @@ sample_rows_kernel(float* __restrict__ logits, int stride, int vocab,
             }
         });
     }
-    cluster.sync();
+    team.sync();
     if (rank != 0) return;
     LLMB_STAMP(3, 0);                                 // the candidates are gathered
     int count = (int)min(shared_gathered, (unsigned)CANDIDATES);
@@ -552,9 +600,10 @@ LLMB_EXPORT int llmb_sample_rows(float* logits, int stride, int n_rows, int voca
     LLMB_REQUIRE(n_rows > 0 && vocab > 0 && stride >= vocab, "sample: bad sizes");
     LLMB_REQUIRE(recent == nullptr || recent_cap > 0, "sample: recent window without capacity");
     LLMB_REQUIRE(n_rows <= 0x7fffffff / CLUSTER, "sample: too many rows");
-    sample_rows_kernel<<<n_rows * CLUSTER, THREADS, 0, stream>>>(
-        logits, stride, vocab, (const float4*)params, (const int2*)iparams, recent, recent_len,
-        recent_cap, rng, out, status, record, state_rows);
+    int blocks = blocks_a_row(n_rows, vocab);
+    LLMB_CUDA(launch_rows(blocks > 1 ? sample_rows_kernel<true> : sample_rows_kernel<false>, blocks, n_rows, stream, logits, stride,
+                          vocab, (const float4*)params, (const int2*)iparams, recent, recent_len, recent_cap, rng, out, status,
+                          record, state_rows));
     return check_launch("sample_rows");
 }
 
