@@ -1354,6 +1354,13 @@ def attention(qkv, k_cache, v_cache, block_table, ring_pages, tok_pos, tok_seq, 
     variant = tactics.choose_attention(decode, qkv.dtype, n_heads, n_kv_heads, head_dim, window,
                                        cu_seqlens is not None and seq_lens is not None,
                                        qkv.stride(0) % 8 == 0 and qkv.data_ptr() % 16 == 0)
+    if variant == "attention_prefill_window_tc":
+        # No bias, no soft cap, a positive scale, values of the keys' size, rows and pages on 16-byte boundaries.
+        # attention_prefill takes the others.
+        served = (bias is None and softcap <= 0.0 and scale > 0 and value_dim == head_dim and out.stride(0) % 8 == 0
+                  and not any(t.data_ptr() % 16 for t in (out, k_cache, v_cache)))
+        if not served:
+            variant = "attention_generic" if tactics.is_disabled("attention_prefill") else "attention_prefill"
     # the tcgen05 prefill takes a sink and a bias, none of the others
     sink_only = ((sinks is not None or bias is not None) and gate is None and out_scale == 1.0 and softcap <= 0.0 and value_dim == head_dim
                  and out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0)
@@ -1366,14 +1373,9 @@ def attention(qkv, k_cache, v_cache, block_table, ring_pages, tok_pos, tok_seq, 
             variant = "attention_prefill"
     if value_dim != head_dim:
         variant = "attention_generic"                 # the tile kernels take values of the keys' size
-    # With a window the choice is attention_prefill; its calls run on tcgen05 wherever that kernel is built for them (64 or 128
-    # elements a head, no bias, no soft cap, a positive scale, rows and pages on 16-byte boundaries).
-    windowed_tc = (variant == "attention_prefill" and window > 0 and head_dim in (64, 128) and bias is None and softcap <= 0.0
-                   and scale > 0 and not tactics.is_disabled("attention_prefill_tc") and qkv.stride(0) % 8 == 0
-                   and out.stride(0) % 8 == 0 and not any(t.data_ptr() % 16 for t in (qkv, out, k_cache, v_cache)))
     if variant == "attention_decode" and (qkv.stride(0) % 2 or qkv.data_ptr() % 4):
         variant = "attention_generic"
-    if variant == "attention_prefill_tc" or windowed_tc:
+    if variant in ("attention_prefill_tc", "attention_prefill_window_tc"):
         _call("attention_prefill_tc", "llmb_attention_prefill_tc", _ptr(qkv), _c_int(qkv.stride(0)),
               _c_int(n), _ptr(k_cache), _ptr(v_cache), _c_int(k_cache.shape[0]), _ptr(block_table),
               _c_int(block_table.shape[1]), _c_int(ring_pages), _ptr(cu_seqlens), _ptr(seq_lens),
@@ -1432,7 +1434,7 @@ def attention(qkv, k_cache, v_cache, block_table, ring_pages, tok_pos, tok_seq, 
 
 
 # the attention kernels that take a sink, a gate and a scale of the result
-_ATTENTION_WITH_EXTRAS = ("attention_generic", "attention_prefill", "attention_decode")
+_ATTENTION_WITH_EXTRAS = ("attention_generic", "attention_prefill", "attention_prefill_window_tc", "attention_decode")
 
 
 def attention_replay_key(step, n_heads: int, n_kv_heads: int, window: int = 0):
@@ -1682,9 +1684,10 @@ def sigmoid_attention(q, k_cache, v_cache, block_table, ring_pages, tok_pos, tok
         return out
     heads_at_once = 0
     if variant == "sigmoid_attention_tiles" and talk is not None and out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0 \
-            and k_cache.data_ptr() % 16 == 0 and v_cache.data_ptr() % 16 == 0:
+            and k_cache.data_ptr() % 16 == 0 and v_cache.data_ptr() % 16 == 0 and not tactics.is_disabled("sigmoid_attention_tc"):
         # With a mixing matrix the scores are a contraction over all key heads, a matrix product by size: tcgen05 wherever
-        # the kernel is built for the sizes. Without one they are one head long, and the tiles on mma.sync stay.
+        # the kernel is built for the sizes (unless "sigmoid_attention_tc" is switched off). Without one they are one head
+        # long, and the tiles on mma.sync stay.
         heads_at_once = sigmoid_mixed_heads(n, n_heads, n_kv_heads, dim, vdim)
     if heads_at_once:
         shape = (heads_at_once, n, n_kv_heads * dim)
@@ -1798,9 +1801,9 @@ def diff_attention(q, k_cache, v_cache, block_table, ring_pages, tok_pos, tok_se
     variant = tactics.choose_diff_attention(decode, q.dtype, n_heads, n_kv_heads, dim, vdim, window, keep_first,
                                             cu_seqlens is not None and seq_lens is not None,
                                             q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0)
-    # tcgen05 wherever it is built for the sizes (its tile of 128 queries is at no size slower than 64 on mma.sync)
+    # the prefill has two kernels: tcgen05 where it is built for the sizes (unless "diff_attention_tc" is switched off)
     if variant == "diff_attention_prefill" and diff_attention_tc_serves(dim, vdim) and scale > 0 and out.data_ptr() % 16 == 0 \
-            and k_cache.data_ptr() % 16 == 0 and v_cache.data_ptr() % 16 == 0:
+            and k_cache.data_ptr() % 16 == 0 and v_cache.data_ptr() % 16 == 0 and not tactics.is_disabled("diff_attention_tc"):
         _call("diff_attention_tc", "llmb_diff_attention_tc", _ptr(q), _c_int(q.stride(0)), _c_int(n), _ptr(k_cache),
               _ptr(v_cache), _c_int(k_cache.shape[0]), _ptr(block_table), _c_int(block_table.shape[1]), _c_int(ring_pages),
               _ptr(cu_seqlens), _ptr(seq_lens), _ptr(seq_order), _ptr(out), _c_int(out.stride(0)),

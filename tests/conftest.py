@@ -29,3 +29,16 @@ def plain_kernels(monkeypatch):
     import plain_ops
     plain_ops.install(monkeypatch)
     return plain_ops
+
+
+@pytest.fixture(params=["tcgen05", "mma.sync"])
+def prefill_form(request):
+    """Steps that either of two prefill kernels can serve all go to the one or the other: both are compared at every size."""
+    from llm_b200.ops import tactics
+    names = {"tcgen05": ("attention_prefill_window_mma", "diff_attention_mma", "sigmoid_attention_mma"),
+             "mma.sync": ("attention_prefill_window_tc", "diff_attention_tc", "sigmoid_attention_tc")}[request.param]
+    for name in names:
+        tactics.disable(name)
+    yield request.param
+    for name in names:
+        tactics.enable(name)

@@ -169,6 +169,7 @@ def test_diff_attention_any_sizes(dtype, sizes):
         _close(got, want, dtype, (window, keep_first))
 
 
+@pytest.mark.usefixtures("prefill_form")
 @pytest.mark.parametrize("shape", SHAPES)
 @pytest.mark.parametrize("window,keep_first", [(0, 0), (70, 3), (64, 0), (33, 65), (200, 1)])
 def test_diff_attention_prefill_kernel(shape, window, keep_first):
@@ -180,6 +181,7 @@ def test_diff_attention_prefill_kernel(shape, window, keep_first):
     _close(got, want, torch.bfloat16, (shape, window, keep_first))
 
 
+@pytest.mark.usefixtures("prefill_form")
 @pytest.mark.parametrize("shape", [(32, 64), (64, 64), (64, 128), (128, 128)])
 @pytest.mark.parametrize("window,keep_first", [(0, 0), (130, 0), (257, 70)])
 def test_diff_attention_prefill_at_the_edges_of_tiles(shape, window, keep_first):

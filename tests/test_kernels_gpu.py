@@ -493,6 +493,7 @@ def test_attention_finds_one_far_key(dtype):
     assert not torch.allclose(windowed[0], values[0][far, 0].to(dtype).float(), atol=0.1)
 
 
+@pytest.mark.usefixtures("prefill_form")
 @pytest.mark.parametrize("heads,kv_heads,dim", [(8, 2, 128), (4, 4, 64), (32, 1, 128)])
 @pytest.mark.parametrize("window", [1, 64, 130, 300])
 @pytest.mark.parametrize("extras", [False, True])

@@ -156,7 +156,8 @@ def _attention(fn, batch, heads, groups, dim, dtype, window, sinks, gated, share
 
 class only_generic:
     """Inside: the tensor-core attention kernels are switched off, so the generic ones run in bfloat16 too."""
-    NAMES = ("attention_prefill", "attention_decode", "sigmoid_attention_tiles", "sigmoid_attention_decode")
+    NAMES = ("attention_prefill", "attention_prefill_window_tc", "attention_decode", "sigmoid_attention_tiles",
+             "sigmoid_attention_decode")
 
     def __init__(self, on=True):
         self.on = on
@@ -174,6 +175,7 @@ class only_generic:
                 tactics.enable(name)
 
 
+@pytest.mark.usefixtures("prefill_form")
 @pytest.mark.parametrize("generic", [False, True])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("case", [
@@ -261,6 +263,7 @@ def _sigmoid(fn, batch, heads, groups, dim, vdim, dtype, window, talk, bias, see
     return out_wide
 
 
+@pytest.mark.usefixtures("prefill_form")
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("case", [
     # heads, kv heads, head size, value size, window, mixed, bias
@@ -283,6 +286,7 @@ def test_sigmoid_attention(dtype, case, generic):
         _close(got, want, dtype, (case, lengths))
 
 
+@pytest.mark.usefixtures("prefill_form")
 @pytest.mark.parametrize("case", [
     # heads, kv heads, head size, value size, window, bias: what the tcgen05 prefill serves
     (4, 4, 64, 64, 0, True), (8, 4, 64, 128, 257, False), (8, 1, 128, 64, 130, True), (16, 2, 128, 128, 0, True)])
@@ -304,6 +308,7 @@ def test_sigmoid_attention_prefill_at_the_edges_of_tiles(case, room, monkeypatch
         _close(got, want, torch.bfloat16, (case, lengths))
 
 
+@pytest.mark.usefixtures("prefill_form")
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, "generic"])
 @pytest.mark.parametrize("decode", [False, True])
 def test_sigmoid_attention_planted_keys_and_mixing(dtype, decode):

@@ -77,7 +77,7 @@ def test_refusals_name_the_assumption_that_fails():
     assert text.startswith("attention: attention_decode")               # a group of 16 heads: two blocks a key/value head
     text = tactics.explain("attention", decode=False, dtype=BF16, n_heads=32, n_kv_heads=2, head_dim=128,
                            window=100, packed=True)
-    assert text.startswith("attention: attention_prefill") and "no window" in text        # the tcgen05 kernel has none
+    assert text.startswith("attention: attention_prefill_window_tc") and "no window" in text      # the other form has none
     text = tactics.explain("attention", decode=False, dtype=BF16, n_heads=4, n_kv_heads=4, head_dim=80,
                            window=0, packed=True)
     assert text.startswith("attention: attention_generic") and "head_dim 80" in text
@@ -86,6 +86,26 @@ def test_refusals_name_the_assumption_that_fails():
     assert text.startswith("attention: attention_decode")               # the decode kernel takes windows
     text = tactics.explain("linear", m=2048, n=4096, k=4100, in_dtype=BF16, out_dtype=BF16, lda=4100)
     assert text.startswith("linear: gemm_simt") and "multiple of 8" in text and "exceed 64" in text
+
+
+def test_the_windowed_prefill_on_tcgen05_follows_its_switches():
+    """Choice and explanation name the kernel that runs; with either of its switches off the mma.sync kernel is chosen."""
+    args = dict(decode=False, dtype=BF16, n_heads=8, n_kv_heads=2, head_dim=64, window=100, packed=True)
+    assert tactics.choose_attention(**args) == "attention_prefill_window_tc"
+    assert tactics.choose_attention(**{**args, "head_dim": 96}) == "attention_prefill"
+    assert tactics.choose_attention(**args, aligned=False) == "attention_prefill"
+    for name, reason in (("attention_prefill_window_tc", "disabled"), ("attention_prefill_tc", "attention_prefill_tc is disabled")):
+        tactics.disable(name)
+        try:
+            assert tactics.choose_attention(**args) == "attention_prefill"
+            assert reason in tactics.explain("attention", **args)
+        finally:
+            tactics.enable(name)
+    tactics.disable("attention_prefill")
+    try:
+        assert tactics.choose_attention(**args) == "attention_prefill_window_tc"
+    finally:
+        tactics.enable("attention_prefill")
 
 
 def test_a_head_size_no_kernel_takes_is_refused_by_name():
