@@ -242,7 +242,8 @@ const std::vector<Row>& table(int family) {
          "at 8,192 (742 and 1,105 TFLOP/s of causal work); with heads of 64: 40.5 us at 2,048 tokens"},
         {"attention_prefill_window_tc", 12, prefill_window_tc_guard,
          "the kernel of attention_prefill_tc with a window (a tile starts at the first key block that a query of it sees), "
-         "a gate per head and a scale in the epilogue; no bias by distance and no soft cap, which go to attention_prefill. Measured: 69 us for 2,500 tokens, 32 heads "
+         "a gate per head and a scale in the epilogue; no bias by distance and no soft cap, which go to attention_prefill, as "
+         "do steps too short for its tiles of 128 queries (ops/prefill.py). Measured: 69 us for 2,500 tokens, 32 heads "
          "of 128 over one, window 2,048 (attention_prefill: 181 us)"},
         {"attention_prefill", 10, prefill_guard,
          "flash attention over the paged cache for steps with several new tokens a sequence: 64-query tiles, "

@@ -20,7 +20,7 @@ import torch
 
 from .. import native
 from ..errors import KernelError
-from . import tactics
+from . import prefill, tactics
 from .build import all_sources, ensure_built, load_library
 
 PAGE = native.plan_constant("page")              # positions per cache page (csrc/plan.h)
@@ -1355,12 +1355,17 @@ def attention(qkv, k_cache, v_cache, block_table, ring_pages, tok_pos, tok_seq, 
                                        cu_seqlens is not None and seq_lens is not None,
                                        qkv.stride(0) % 8 == 0 and qkv.data_ptr() % 16 == 0)
     if variant == "attention_prefill_window_tc":
-        # No bias, no soft cap, a positive scale, values of the keys' size, rows and pages on 16-byte boundaries.
+        # No bias, no soft cap, a positive scale, values of the keys' size, rows and pages on 16-byte boundaries; and not
+        # steps too short for it (ops/prefill.py; the switch "attention_prefill_window_mma" leaves them to it all the same).
         # attention_prefill takes the others.
         served = (bias is None and softcap <= 0.0 and scale > 0 and value_dim == head_dim and out.stride(0) % 8 == 0
                   and not any(t.data_ptr() % 16 for t in (out, k_cache, v_cache)))
+        mma = not tactics.is_disabled("attention_prefill")
         if not served:
-            variant = "attention_generic" if tactics.is_disabled("attention_prefill") else "attention_prefill"
+            variant = "attention_prefill" if mma else "attention_generic"
+        elif mma and not tactics.is_disabled("attention_prefill_window_mma") and not prefill.on_tcgen05(
+                ("window", head_dim), n_heads, n, cu_seqlens.numel() - 1, max_new, max_len, window):
+            variant = "attention_prefill"
     # the tcgen05 prefill takes a sink and a bias, none of the others
     sink_only = ((sinks is not None or bias is not None) and gate is None and out_scale == 1.0 and softcap <= 0.0 and value_dim == head_dim
                  and out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0)
@@ -1442,7 +1447,10 @@ def attention_replay_key(step, n_heads: int, n_kv_heads: int, window: int = 0):
     (Part.replay_key): the most new tokens of a sequence (prefill grids), the slices (decode)."""
     if step.decode:
         return (True, attention_decode_splits(step.n_seqs, n_heads, n_kv_heads, step.max_len, window))
-    return (False, max(step.new_counts))
+    newest = max(step.new_counts)
+    # which windowed kernel runs depends on how far the step reaches back
+    return (False, newest) + tuple(prefill.on_tcgen05(("window", d), n_heads, step.n_tokens, step.n_seqs, newest, step.max_len, window)
+                                   for d in ((64, 128) if window > 0 else ()))
 
 
 # ----------------------------------------------------------------------------- latent attention, shared rotated keys
@@ -1623,7 +1631,9 @@ def sigmoid_decode_splits(n_seqs: int, max_len: int, window: int, mixed_width: i
 def sigmoid_attention_replay_key(step, spec):
     if step.decode:
         return (True, sigmoid_decode_splits(step.n_seqs, step.max_len, spec.window, spec.n_kv_heads * spec.head_dim))
-    return (False, max(step.new_counts))
+    newest = max(step.new_counts)
+    return (False, newest, prefill.sigmoid_on_tcgen05(spec.n_heads, spec.n_kv_heads, spec.head_dim, step.n_tokens, step.n_seqs,
+                                                      newest, step.max_len, spec.window))
 
 
 SIGMOID_MIXED_BYTES = 256 << 20     # room for the mixed queries of a prefill; more heads than fit run one group after the other
@@ -1684,10 +1694,12 @@ def sigmoid_attention(q, k_cache, v_cache, block_table, ring_pages, tok_pos, tok
         return out
     heads_at_once = 0
     if variant == "sigmoid_attention_tiles" and talk is not None and out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0 \
-            and k_cache.data_ptr() % 16 == 0 and v_cache.data_ptr() % 16 == 0 and not tactics.is_disabled("sigmoid_attention_tc"):
-        # With a mixing matrix the scores are a contraction over all key heads, a matrix product by size: tcgen05 wherever
-        # the kernel is built for the sizes (unless "sigmoid_attention_tc" is switched off). Without one they are one head
-        # long, and the tiles on mma.sync stay.
+            and k_cache.data_ptr() % 16 == 0 and v_cache.data_ptr() % 16 == 0 and not tactics.is_disabled("sigmoid_attention_tc") \
+            and (tactics.is_disabled("sigmoid_attention_mma") or prefill.sigmoid_on_tcgen05(
+                n_heads, n_kv_heads, dim, n, cu_seqlens.numel() - 1, max_new, max_len, window)):
+        # With a mixing matrix the scores are a contraction over all key heads, a matrix product by size: tcgen05 where the
+        # kernel is built for the sizes and pays (ops/prefill.py). Without one they are one head long, and the tiles on
+        # mma.sync stay. The switches "sigmoid_attention_tc" and "sigmoid_attention_mma" take one of the two out.
         heads_at_once = sigmoid_mixed_heads(n, n_heads, n_kv_heads, dim, vdim)
     if heads_at_once:
         shape = (heads_at_once, n, n_kv_heads * dim)
@@ -1771,7 +1783,10 @@ def diff_attention_replay_key(step, spec):
     (Part.replay_key): the most new tokens of a sequence (prefill grids), the slices (decode)."""
     if step.decode:
         return (True, diff_decode_splits(step.n_seqs, spec.n_kv_heads, step.max_len, spec.window, spec.keep_first))
-    return (False, max(step.new_counts))
+    newest = max(step.new_counts)
+    return (False, newest, diff_attention_tc_serves(spec.head_dim, spec.value_dim) and prefill.on_tcgen05(
+        ("diff", spec.head_dim, spec.value_dim), spec.n_heads, step.n_tokens, step.n_seqs, newest, step.max_len, spec.window,
+        spec.keep_first))
 
 
 def diff_attention_tc_serves(dim: int, vdim: int) -> bool:
@@ -1801,9 +1816,12 @@ def diff_attention(q, k_cache, v_cache, block_table, ring_pages, tok_pos, tok_se
     variant = tactics.choose_diff_attention(decode, q.dtype, n_heads, n_kv_heads, dim, vdim, window, keep_first,
                                             cu_seqlens is not None and seq_lens is not None,
                                             q.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0)
-    # the prefill has two kernels: tcgen05 where it is built for the sizes (unless "diff_attention_tc" is switched off)
+    # the prefill has two kernels: tcgen05 where it is built for the sizes and pays (ops/prefill.py); the switches
+    # "diff_attention_tc" and "diff_attention_mma" take one of them out
     if variant == "diff_attention_prefill" and diff_attention_tc_serves(dim, vdim) and scale > 0 and out.data_ptr() % 16 == 0 \
-            and k_cache.data_ptr() % 16 == 0 and v_cache.data_ptr() % 16 == 0 and not tactics.is_disabled("diff_attention_tc"):
+            and k_cache.data_ptr() % 16 == 0 and v_cache.data_ptr() % 16 == 0 and not tactics.is_disabled("diff_attention_tc") \
+            and (tactics.is_disabled("diff_attention_mma")
+                 or prefill.on_tcgen05(("diff", dim, vdim), n_heads, n, cu_seqlens.numel() - 1, max_new, max_len, window, keep_first)):
         _call("diff_attention_tc", "llmb_diff_attention_tc", _ptr(q), _c_int(q.stride(0)), _c_int(n), _ptr(k_cache),
               _ptr(v_cache), _c_int(k_cache.shape[0]), _ptr(block_table), _c_int(block_table.shape[1]), _c_int(ring_pages),
               _ptr(cu_seqlens), _ptr(seq_lens), _ptr(seq_order), _ptr(out), _c_int(out.stride(0)),
