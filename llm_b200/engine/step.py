@@ -118,6 +118,7 @@ class Engine:
         self.vocab = model.spec.vocab
         self.steps_run = 0
         self.workspace = Workspace(self.device, model.scratch_requests)
+        self.scope = ops.StepScope()      # the kernels' own scratch: one for all steps, as they have one arena
         self.use_graphs = (use_graphs and self.device.type == "cuda"
                            and os.environ.get("LLMB_NO_GRAPHS", "0") in ("", "0")
                            and not ops.PROFILING
@@ -208,7 +209,10 @@ class Engine:
         return logits[torch.tensor(wanted, dtype=torch.long, device=self.device)]
 
     def _pass(self, entries, device_tokens=None, batch=None) -> torch.Tensor:
-        batch = batch or _Batch(entries)
+        with self.scope:
+            return self._pass_in_scope(entries, device_tokens, batch or _Batch(entries))
+
+    def _pass_in_scope(self, entries, device_tokens, batch) -> torch.Tensor:
         lib, cache = native.lib(), self.cache._handle
         n_sections = lib.llmh_step_sections(cache)
         offsets, sizes = (c_longlong * n_sections)(), (c_longlong * n_sections)()
@@ -269,7 +273,7 @@ class Engine:
         two passes of one key (tokens, positions, lengths, slots, pages, wanted rows) lies in the
         record's own device buffer, which is refreshed before the launches."""
         from ..ops import tactics
-        stamp = (ops.scratch_generation(), tactics.generation,
+        stamp = (self.scope.generation, tactics.generation,
                  self.workspace.arena.data_ptr() if self.workspace.arena is not None else 0)
         held = self._records.get(key)
         if held is not None and held[3] != stamp:
@@ -294,7 +298,7 @@ class Engine:
             finally:
                 ops.end_recording()
             # the arena may have grown while this pass was planned: the stamp is taken afterwards
-            stamp = (ops.scratch_generation(), tactics.generation, self.workspace.arena.data_ptr())
+            stamp = (self.scope.generation, tactics.generation, self.workspace.arena.data_ptr())
             if len(self._records) >= MAX_RECORDS:
                 self._records.pop(next(iter(self._records)))
             self._records[key] = (ops.RecordedPass(recording), meta, logits, stamp)

@@ -20,8 +20,9 @@ import torch
 
 from .. import native
 from ..errors import KernelError
-from . import prefill, tactics
+from . import prefill, scratch, tactics
 from .build import all_sources, ensure_built, load_library
+from .scratch import StepScope
 
 PAGE = native.plan_constant("page")              # positions per cache page (csrc/plan.h)
 BFLOAT16_ONLY = ("gemm_tc", "gemm_skinny", "attention_decode", "attention_decode_window", "attention_prefill",
@@ -120,7 +121,6 @@ if PROFILING:
 # ----------------------------------------------------------------------------- recorded passes
 
 _recording = None           # the Recording that launches are being entered into, or None
-_scratch_generation = 0     # grows when a scratch buffer that recorded passes point at is replaced
 
 
 class Recording:
@@ -146,9 +146,9 @@ def end_recording() -> None:
 class RecordedPass:
     """A Recording turned into a native plan (csrc/host/plan_run.cpp): `run()` makes the same
     launches with the same arguments on the current stream through the entry points' packed
-    doors, in one call of the native host library. The tensors the launches point at are kept
-    alive here. Valid while no scratch buffer of this module was replaced
-    (`scratch_generation`)."""
+    doors, in one call of the native host library. The tensors the launches point at, scratch
+    included, are kept alive here: a record made outside a StepScope runs on the stream it was
+    made on, or with nothing else running there. `scratch_generation`: of the time it was made."""
 
     def __init__(self, recording: Recording):
         doors, counts, stream_slots, slots = [], [], [], []
@@ -170,7 +170,7 @@ class RecordedPass:
         self._handle = handle
         self.kernels = recording.kernels
         self.launches = n
-        self.scratch_generation = _scratch_generation
+        self.scratch_generation = scratch_generation()
         self._libraries = [c[0] for c in recording.calls]
         self._failed = ctypes.c_int(-1)
 
@@ -209,7 +209,8 @@ class RecordedPass:
 
 
 def scratch_generation() -> int:
-    return _scratch_generation
+    """Grows when scratch that recorded passes point at is replaced."""
+    return scratch.generation
 
 
 def _call(lib_name: str, fn_name: str, *args, kernels: int = 1):
@@ -1037,35 +1038,16 @@ def conv_rope_cache_write(u, conv_w, state, tok_pos, tok_seq, cu_seqlens, seq_le
 
 # ----------------------------------------------------------------------------- matrix product
 
-_scratch: dict = {}
-_retired: list = []      # outgrown scratch buffers, kept alive for CUDA graphs that hold their address
+def _scratch(device, kind: str, floats: int, counters: int = 0) -> tuple:
+    """Scratch for a call on the current stream (scratch.py says whose): (float32 tensor, int32 tensor of zeros or None)."""
+    on_gpu = device.type == "cuda"
+    return scratch.of_call(device, (_stream().value or 0) if on_gpu else 0,
+                           on_gpu and torch.cuda.is_current_stream_capturing(), kind, floats, counters)
 
 
-_SCRATCH_FLOATS, _SCRATCH_COUNTERS = 148 * 2 * 128 * 256, 1 << 14      # what a product on pairs of SMs asks for at most
-_SCRATCH_STREAMS = 8                  # streams of a device that keep a pair of their own; any further ones share the first
-
-
-def _split_scratch(device, floats: int, counters: int):
-    """Partial sums and tile counters of the products that split K, one pair per device and stream (calls of a stream run
-    one after the other). It grows when a call needs more; an outgrown pair is kept alive because a captured step may
-    still hold its address. A step under capture takes a pair that the device has (a shape runs plainly before it is
-    captured, and what a capture allocates belongs to its graph)."""
-    capturing = device.type == "cuda" and torch.cuda.is_current_stream_capturing()
-    key = (device, 0 if device.type != "cuda" or capturing else _stream().value or 0)
-    if key not in _scratch and (capturing or sum(k[0] == device for k in _scratch) >= _SCRATCH_STREAMS):
-        key = next((k for k in _scratch if k[0] == device), key)
-    held = _scratch.get(key)
-    if held is None or held[0].numel() < floats or held[1].numel() < counters:
-        n_floats = max(floats, held[0].numel() if held else 0, _SCRATCH_FLOATS)
-        n_counters = max(counters, held[1].numel() if held else 0, _SCRATCH_COUNTERS)
-        global _scratch_generation
-        if held is not None:
-            _retired.append(held)
-            _scratch_generation += 1
-        held = (torch.empty(n_floats, dtype=torch.float32, device=device),
-                torch.zeros(n_counters, dtype=torch.int32, device=device))
-        _scratch[key] = held
-    return held
+def _split_scratch(device, floats: int, counters: int) -> tuple:
+    """Partial sums and tile counters of the products that split K or cut a tile along it."""
+    return _scratch(device, "products", floats, counters)
 
 
 def _skinny_scratch(device, m, n, k):
@@ -1085,9 +1067,18 @@ def _tc_needs(m: int, n: int, k: int) -> tuple:
             lib.llmb_gemm_tc_kernels(_c_int(m), _c_int(n), _c_int(k)))
 
 
-def _tc_scratch(device, m, n, k):
+def _tc_scratch(device, m, n, k) -> tuple:
+    """(partials, counters) of a tcgen05 product; a product in whole tiles has neither."""
     floats, counters, _ = _tc_needs(m, n, k)
-    return _split_scratch(device, floats, counters)
+    return _split_scratch(device, floats, counters) if floats else (None, None)
+
+
+def _scratch_arguments(partials, counters) -> tuple:
+    """Both tensors as a kernel takes them (the caller holds them until it has launched)."""
+    if partials is None:
+        return None, ctypes.c_longlong(0), None, _c_int(0)
+    return (_ptr(partials), ctypes.c_longlong(partials.numel()), _ptr(counters),
+            _c_int(counters.numel() if counters is not None else 0))
 
 
 def tensor_core_status() -> int:
@@ -1181,12 +1172,11 @@ def linear(a, w, bias=None, out_dtype=None, residual=None, out=None, glu=False, 
                               "K % 8 == 0, no bias and no residual")
         _check_out(out, (m, n // 2), a.dtype, "linear")
         result = out if out is not None else torch.empty((m, n // 2), dtype=a.dtype, device=a.device)
-        partials, counters = _tc_scratch(a.device, m, n, k)
+        parts = _tc_scratch(a.device, m, n, k)
         if emit is not None or rope is not None:
             raise KernelError("linear: the gated epilogue takes a folded norm only")
         _call("gemm_tc", "llmb_gemm_tc_ex", _ptr(a), _c_int(a.stride(0)), _ptr(w), None, _ptr(result),
-              _c_int(_code(a.dtype)), None, _ptr(partials), ctypes.c_longlong(partials.numel()),
-              _ptr(counters), _c_int(counters.numel()), _c_int(m), _c_int(n), _c_int(k),
+              _c_int(_code(a.dtype)), None, *_scratch_arguments(*parts), _c_int(m), _c_int(n), _c_int(k),
               _c_int(n // 2), _c_int(2 if glu == "gelu" else 1), _c_int(0 if tactics.is_disabled("gemm_tc_pair") else 1),
               ctypes.byref(_fusion_struct(norm, None, None)) if norm is not None else None, None,
               _stream(), kernels=_tc_kernels(m, n, k))
@@ -1208,12 +1198,11 @@ def linear(a, w, bias=None, out_dtype=None, residual=None, out=None, glu=False, 
     if fused and a.dtype != torch.bfloat16:
         raise KernelError("linear: norm, emit and rope ride only with bfloat16 products")
     if variant == "gemm_tc" and fused:
-        partials, counters = _tc_scratch(a.device, m, n, k)
+        parts = _tc_scratch(a.device, m, n, k)
         applied = _c_int(0)
         _call("gemm_tc", "llmb_gemm_tc_ex", _ptr(a), _c_int(a.stride(0)), _ptr(w), _ptr(bias),
               _ptr(result if residual is None else None), _c_int(_code(target_dtype)),
-              _ptr(residual), _ptr(partials), ctypes.c_longlong(partials.numel()),
-              _ptr(counters), _c_int(counters.numel()), _c_int(m), _c_int(n), _c_int(k), _c_int(n),
+              _ptr(residual), *_scratch_arguments(*parts), _c_int(m), _c_int(n), _c_int(k), _c_int(n),
               _c_int(0), _c_int(0 if tactics.is_disabled("gemm_tc_pair") else 1),
               ctypes.byref(_fusion_struct(norm, emit, rope)), ctypes.byref(applied), _stream(),
               kernels=_tc_kernels(m, n, k))
@@ -1244,11 +1233,10 @@ def linear(a, w, bias=None, out_dtype=None, residual=None, out=None, glu=False, 
                              rope.interleaved, rope.write_cache)
         return result
     if variant == "gemm_tc":
-        partials, counters = _tc_scratch(a.device, m, n, k)
+        parts = _tc_scratch(a.device, m, n, k)
         _call("gemm_tc", "llmb_gemm_tc", _ptr(a), _c_int(a.stride(0)), _ptr(w), _ptr(bias),
               _ptr(result if residual is None else None), _c_int(_code(target_dtype)),
-              _ptr(residual), _ptr(partials), ctypes.c_longlong(partials.numel()),
-              _ptr(counters), _c_int(counters.numel()), _c_int(m), _c_int(n), _c_int(k), _c_int(n),
+              _ptr(residual), *_scratch_arguments(*parts), _c_int(m), _c_int(n), _c_int(k), _c_int(n),
               _c_int(0), _c_int(0 if tactics.is_disabled("gemm_tc_pair") else 1), _stream(),
               kernels=_tc_kernels(m, n, k))
     elif variant == "gemm_skinny":
@@ -1269,9 +1257,6 @@ def linear(a, w, bias=None, out_dtype=None, residual=None, out=None, glu=False, 
 
 
 # ----------------------------------------------------------------------------- attention
-
-_attention_scratch: dict = {}      # outgrown buffers join `_retired` above
-
 
 def decode_splits(n_seqs: int, n_kv_heads: int, max_len: int, wave: int = 296) -> int:
     """Into how many slices the keys of every sequence are cut for decode
@@ -1407,17 +1392,10 @@ def attention(qkv, k_cache, v_cache, block_table, ring_pages, tok_pos, tok_seq, 
         sizer = getattr(lib, f"llmb_{name}_scratch_floats")
         sizer.restype = ctypes.c_longlong
         need = sizer(_c_int(n), _c_int(n_heads), _c_int(head_dim), _c_int(splits))
-        scratch = _attention_scratch.get(qkv.device)
-        if scratch is None or scratch.numel() < need:
-            if scratch is not None:
-                global _scratch_generation
-                _retired.append(scratch)
-                _scratch_generation += 1
-            scratch = torch.empty(max(need, 1 << 23), dtype=torch.float32, device=qkv.device)
-            _attention_scratch[qkv.device] = scratch
+        parts, _ = _scratch(qkv.device, "attention", need)
         head = (_ptr(qkv), _c_int(qkv.stride(0)), _ptr(k_cache), _ptr(v_cache), _ptr(block_table),
                 _c_int(block_table.shape[1]), _c_int(ring_pages), _ptr(seq_lens), _ptr(seq_order), _ptr(out),
-                _c_int(out.stride(0)), _ptr(scratch), ctypes.c_longlong(scratch.numel()), _c_int(n), _c_int(n_heads),
+                _c_int(out.stride(0)), _ptr(parts), ctypes.c_longlong(parts.numel()), _c_int(n), _c_int(n_heads),
                 _c_int(n_kv_heads), _c_int(head_dim), _c_float(scale), _c_int(window))
         if plain:
             _call(name, "llmb_attention_decode", *head, _c_int(splits), _stream(), kernels=2 if splits > 1 else 1)
@@ -1575,28 +1553,21 @@ def latent_attention(queries, cache, block_table, ring_pages, tok_pos, tok_seq, 
               _c_float(scale), _c_int(0), _ptr(sinks), None, _c_int(0), _c_float(1.0), _c_float(0.0), _c_int(rank), None, _c_int(0),
               _stream())
         return out
-    splits, scratch = 1, None
+    splits, parts = 1, None
     if decode:
         tensor = variant == "latent_decode_tc"
         splits = latent_decode_splits(n, n_heads, rank, rot, max_len, tensor)
         need = n * n_heads * splits * (rank + 2) if splits > 1 else 0
-        scratch = _attention_scratch.get(queries.device)
-        if scratch is None or scratch.numel() < need:
-            if scratch is not None:
-                global _scratch_generation
-                _retired.append(scratch)
-                _scratch_generation += 1
-            scratch = torch.empty(max(need, 1 << 23), dtype=torch.float32, device=queries.device)
-            _attention_scratch[queries.device] = scratch
+        parts, _ = _scratch(queries.device, "attention", need)
         if tensor:
             _call("latent_attention", "llmb_latent_decode_tc", _ptr(queries), _ptr(cache), _c_int(cache.shape[0]),
                   _ptr(block_table), _c_int(block_table.shape[1]), _c_int(ring_pages), _ptr(seq_lens), _ptr(seq_order), _ptr(out),
-                  _ptr(scratch), ctypes.c_longlong(scratch.numel()), _c_int(n), _c_int(n_heads), _c_int(rank), _c_int(rot),
+                  _ptr(parts), ctypes.c_longlong(parts.numel()), _c_int(n), _c_int(n_heads), _c_int(rank), _c_int(rot),
                   _c_float(scale), _ptr(sinks), _c_int(splits), _stream(), kernels=2 if splits > 1 else 1)
             return out
     _call("latent_attention", "llmb_latent_attention", _ptr(queries), _ptr(cache), _ptr(block_table), _c_int(block_table.shape[1]),
-          _c_int(ring_pages), _ptr(cu_seqlens), _ptr(seq_lens), _ptr(seq_order), _ptr(out), _ptr(scratch),
-          ctypes.c_longlong(scratch.numel() if scratch is not None else 0), _c_int(n), _c_int(cu_seqlens.numel() - 1),
+          _c_int(ring_pages), _ptr(cu_seqlens), _ptr(seq_lens), _ptr(seq_order), _ptr(out), _ptr(parts),
+          ctypes.c_longlong(parts.numel() if parts is not None else 0), _c_int(n), _c_int(cu_seqlens.numel() - 1),
           _c_int(1 if decode else max_new), _c_int(n_heads), _c_int(rank), _c_int(rot), _c_float(scale), _ptr(sinks), _c_int(splits), _stream(),
           kernels=2 if splits > 1 else 1)
     return out
@@ -1678,17 +1649,10 @@ def sigmoid_attention(q, k_cache, v_cache, block_table, ring_pages, tok_pos, tok
     if variant == "sigmoid_attention_decode":
         splits = sigmoid_decode_splits(n, max_len, window, n_kv_heads * dim)
         need = (n * (16 if n_heads <= 16 else 32) * n_kv_heads * dim + 1) // 2 + (n * splits * n_heads * vdim if splits > 1 else 0)
-        scratch = _attention_scratch.get(q.device)
-        if scratch is None or scratch.numel() < need:
-            if scratch is not None:
-                global _scratch_generation
-                _retired.append(scratch)
-                _scratch_generation += 1
-            scratch = torch.empty(max(need, 1 << 23), dtype=torch.float32, device=q.device)
-            _attention_scratch[q.device] = scratch
+        parts, _ = _scratch(q.device, "attention", need)
         _call("sigmoid_attention", "llmb_sigmoid_attention_decode", _ptr(q), _c_int(q.stride(0)), _ptr(k_cache),
               _ptr(v_cache), _ptr(block_table), _c_int(block_table.shape[1]), _c_int(ring_pages), _ptr(seq_lens),
-              _ptr(out), _c_int(out.stride(0)), _ptr(scratch), ctypes.c_longlong(scratch.numel()), _c_int(n),
+              _ptr(out), _c_int(out.stride(0)), _ptr(parts), ctypes.c_longlong(parts.numel()), _c_int(n),
               _c_int(n_heads), _c_int(n_kv_heads), _c_int(dim), _c_int(vdim), _c_float(scale), _c_int(window),
               _ptr(talk), _ptr(head_bias), _c_float(out_scale), _c_int(splits), _stream(), kernels=3 if splits > 1 else 2)
         return out
@@ -1838,17 +1802,10 @@ def diff_attention(q, k_cache, v_cache, block_table, ring_pages, tok_pos, tok_se
     elif variant == "diff_attention_decode":
         splits = diff_decode_splits(n, n_kv_heads, max_len, window, keep_first)
         need = n * n_heads * 2 * splits * (vdim + 2)
-        scratch = _attention_scratch.get(q.device)
-        if scratch is None or scratch.numel() < need:
-            if scratch is not None:
-                global _scratch_generation
-                _retired.append(scratch)
-                _scratch_generation += 1
-            scratch = torch.empty(max(need, 1 << 23), dtype=torch.float32, device=q.device)
-            _attention_scratch[q.device] = scratch
+        parts, _ = _scratch(q.device, "attention", need)
         _call("diff_attention", "llmb_diff_attention_decode", _ptr(q), _c_int(q.stride(0)), _ptr(k_cache),
               _ptr(v_cache), _ptr(block_table), _c_int(block_table.shape[1]), _c_int(ring_pages), _ptr(seq_lens),
-              _ptr(seq_order), _ptr(out), _c_int(out.stride(0)), _ptr(scratch), ctypes.c_longlong(scratch.numel()),
+              _ptr(seq_order), _ptr(out), _c_int(out.stride(0)), _ptr(parts), ctypes.c_longlong(parts.numel()),
               _c_int(n), _c_int(n_heads), _c_int(n_kv_heads), _c_int(dim), _c_int(vdim), _c_float(scale),
               _c_int(window), _c_int(keep_first), _c_float(lam), _c_float(eps), _c_float(out_scale),
               _c_int(1 if head_norm else 0), _c_int(splits), _stream(), kernels=2 if splits > 1 else 1)
@@ -1900,7 +1857,7 @@ def required_libraries() -> list:
             "attention_decode", "attention_prefill", "attention_prefill_tc", "sampling"]
 
 
-__all__ = ["PAGE", "GLU_BLOCK", "glu_fusable", "embed", "scale_", "random_normal_", "begin_recording", "end_recording", "RecordedPass", "scratch_generation", "Emit", "FoldedNorm", "RopeWrite", "cast_sumsq", "SUMSQ_LD", "rmsnorm", "swiglu", "rope_cache_write", "linear", "attention",
+__all__ = ["PAGE", "GLU_BLOCK", "glu_fusable", "embed", "scale_", "random_normal_", "begin_recording", "end_recording", "RecordedPass", "StepScope", "scratch_generation", "Emit", "FoldedNorm", "RopeWrite", "cast_sumsq", "SUMSQ_LD", "rmsnorm", "swiglu", "rope_cache_write", "linear", "attention",
            "softcap_", "add_rows_", "conv_rope_cache_write", "diff_attention", "tanh_norm", "norm_rope_cache_write",
            "sigmoid_attention", "gated_recurrence", "state_space", "attention_replay_key", "layernorm", "input_conv", "output_norm_add_", "forget_recurrence",
            "latent_write", "head_products", "latent_attention", "latent_prefill", "attention_decode_splits", "sigmoid_attention_replay_key", "sigmoid_decode_splits", "sigmoid_mixed_heads",

@@ -42,20 +42,22 @@ import torch
 
 sys.path.insert(0, str(Path(__file__).resolve().parent))
 
-from llm_b200.ops import attention, linear, rmsnorm, rope_cache_write, swiglu, tactics  # noqa: E402
+from llm_b200.ops import StepScope, attention, linear, rmsnorm, rope_cache_write, swiglu, tactics  # noqa: E402
 
 DEV = "cuda:0"
 
 
 def time_in_graph(fn, reps: int, rounds: int = 10) -> float:
-    """Microseconds per call of fn, from `rounds` replays of a graph of `reps` calls."""
-    fn()
-    fn()
-    torch.cuda.synchronize()
-    graph = torch.cuda.CUDAGraph()
-    with torch.cuda.graph(graph):
-        for _ in range(reps):
-            fn()
+    """Microseconds per call of fn, from `rounds` replays of a graph of `reps` calls (one line of work, as an engine's steps)."""
+    scope = StepScope()
+    with scope:
+        fn()
+        fn()
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            for _ in range(reps):
+                fn()
     graph.replay()
     torch.cuda.synchronize()
     begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)

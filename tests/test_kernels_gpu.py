@@ -213,6 +213,84 @@ def test_linear_on_two_streams_at_once():
     assert all(torch.equal(g, want[i]) for i in range(2) for g in got[i])
 
 
+@pytest.mark.parametrize("m,n,k", [(350, 4096, 4096), (64, 4096, 4096)])      # parts of tiles; K split over blocks
+def test_products_on_many_streams_and_in_a_graph_at_once(m, n, k):
+    """More streams than keep scratch, and a captured product replayed on one more, with nothing between them: the bits of
+    single calls."""
+    a = randn(m, k, dtype=torch.bfloat16, seed=211)
+    ws = [randn(n, k, dtype=torch.bfloat16, seed=212 + i, scale=0.05) for i in range(3)]
+    want = [ops().linear(a, w) for w in ws]
+    streams = [torch.cuda.Stream() for _ in range(11)]
+    graphs, captured = [], []
+    for w in ws[:2]:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            captured.append([ops().linear(a, w), ops().linear(a, ws[2])])
+        graphs.append(graph)
+    torch.cuda.synchronize()
+    got = []
+    for turn in range(5):
+        for i, stream in enumerate(streams):
+            with torch.cuda.stream(stream):
+                if i in (3, 7):
+                    graphs[i == 7].replay()
+                else:
+                    got.append((i % 3, ops().linear(a, ws[i % 3])))
+        if turn < 4:
+            continue
+        torch.cuda.synchronize()
+    assert all(torch.equal(g, want[w]) for w, g in got)
+    assert all(torch.equal(c[0], want[i]) and torch.equal(c[1], want[2]) for i, c in enumerate(captured))
+    assert ops().tensor_core_status() == 0
+
+
+def test_two_engines_on_two_streams_at_once():
+    """Prompts, recorded passes and replayed decode steps of two engines, each on its stream with nothing between them: the
+    logits of the same steps alone."""
+    from llm_b200.config import config_from_dict
+    from llm_b200.engine import DecoderModel, Engine, Entry
+    from llm_b200.shapes import shape
+    config = config_from_dict(shape("llama-3.2-1b", 2))
+
+    def engine(seed):
+        gen = torch.Generator(device=DEV).manual_seed(seed)
+        model = DecoderModel(config.model_spec())
+        weights = {name: torch.empty(spec.shape, dtype=torch.bfloat16, device=DEV).normal_(generator=gen).mul_(0.02)
+                   for name, spec in model.parameters().items()}
+        model.bind(weights, torch.bfloat16, DEV)
+        return Engine(model, max_tokens=2048, max_seq_len=512, max_slots=4)
+
+    def steps(e, seed):
+        """A generator of logits: three prompts of one size (plain, recorded, run from the record), then decode steps."""
+        gen = torch.Generator().manual_seed(seed)
+        ids = lambda n: torch.randint(0, 1000, (n,), generator=gen).tolist()      # noqa: E731
+        for _ in range(3):
+            slots = e.acquire(1)
+            yield e.step([Entry(slots[0], ids(300), [299])])
+            e.release(slots)
+        slots = e.acquire(2)
+        yield e.step([Entry(s, ids(200), [199]) for s in slots])
+        for _ in range(6):
+            yield e.step([Entry(s, ids(1), [0]) for s in slots])
+
+    engines = [engine(seed) for seed in (1, 2)]
+    alone = []
+    for i in (0, 1):
+        alone.append([logits.clone() for logits in steps(engine(i + 1), 7 + i)])
+        torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in engines]
+    torch.cuda.synchronize()
+    runs, both = [steps(e, 7 + i) for i, e in enumerate(engines)], [[], []]
+    for _ in alone[0]:
+        for i in (0, 1):
+            with torch.cuda.stream(streams[i]):
+                both[i].append(next(runs[i]))
+    torch.cuda.synchronize()
+    assert all(e.records_run >= 1 and e.graph_replays >= 1 for e in engines)
+    for i in (0, 1):
+        assert all(torch.equal(x, y) for x, y in zip(alone[i], both[i])), i
+
+
 def test_linear_rows_do_not_depend_on_the_batch():
     """32-bit: a row's product is bit-equal whether it is computed alone or among 200 rows."""
     a = randn(200, 172, seed=8)
