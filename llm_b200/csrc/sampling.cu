@@ -172,17 +172,16 @@ argmax_rows_kernel(const float* __restrict__ logits, int stride, int vocab, int*
     if (blockIdx.x % blocks == 0 && threadIdx.x == 0) out[row] = best.index;
 }
 
-// How many blocks share a row. A row of a large vocabulary is long enough for several, as long as all rows' blocks find an
-// SM of their own; where they do not, blocks sit two on an SM (a walk over whole rows in index order, 16 rows of 128,256: 67 us
-// with one block a row or four, 79 with eight). What a cluster costs a short row is its barriers. The default chain, one
-// block -> as chosen here: 8 rows of 128,256 65 -> 31 us, 32 rows 68 -> 37, 64 rows 71 -> 45, 32 rows of 32,000 33 -> 25; and
-// eight blocks where one is chosen: 256 rows of 128,256 147 -> 258, 148 rows of 32,000 36 -> 81, 1,024 rows of 4,096 82 -> 406.
+// How many blocks share a row. A row of a large vocabulary is long enough for several, as long as they fill no more than the
+// GPU. What a cluster costs a short row is its barriers. The default chain, one block -> as chosen here: 8 rows of 128,256
+// 65 -> 31 us, 32 rows 68 -> 36, 64 rows 71 -> 45, 32 rows of 32,000 33 -> 24; and eight blocks where one is chosen: 256 rows
+// of 128,256 147 -> 258, 148 rows of 32,000 36 -> 81, 1,024 rows of 4,096 82 -> 406.
 static int blocks_a_row(int n_rows, int vocab) {
     if (vocab < 16384) return 1;
-    if (n_rows <= 8) return 8;
-    if (n_rows <= 32) return 4;
+    if (n_rows <= 32) return 8;
     return n_rows <= 64 && vocab >= 65536 ? 2 : 1;
 }
+
 template <typename... Params, typename... Args>
 static cudaError_t launch_rows(void (*kernel)(Params...), int blocks, int n_rows, cudaStream_t stream, Args... args) {
     cudaLaunchConfig_t config = {};
@@ -247,7 +246,7 @@ __device__ unsigned block_exclusive_sum(unsigned value, unsigned* warp_totals) {
 // never clears it, so a refusal in any step stays visible until the host has read and cleared it.
 //
 // Block 0 of a row's cluster owns the row's state and draws; the other blocks read their share of the row for the penalty,
-// the histogram and the candidates (and leave at once where the chain walks the whole row in index order).
+// the histogram and the candidates. Where the chain walks the whole row in index order, one block does and the others leave.
 template <bool CLUSTERED>
 __global__ void __launch_bounds__(THREADS)
 sample_rows_kernel(float* __restrict__ logits, int stride, int vocab,
@@ -278,10 +277,11 @@ sample_rows_kernel(float* __restrict__ logits, int stride, int vocab,
     int top_k = iparams[row_id].x, last_n = iparams[row_id].y;
     int tid = threadIdx.x;
     const Share share = share_of(vocab, rank, blocks);
-    // the chains without a ranking (whole row, or refused) run in block 0 alone
+    // the chains without a ranking (whole row, or refused) run in one block alone, each row in another: where the
+    // clusters of several rows share SMs, their walking blocks do not (32 rows of 128,256: 67 us, and 88 in block 0 of each)
     const bool ranked = temperature > 0.f && (top_k > 0 || vocab <= MAX_TOP_K) && (top_k <= MAX_TOP_K || vocab <= MAX_TOP_K);
     const bool alone = temperature > 0.f && !ranked;
-    if (alone && rank != 0) return;
+    if (alone && rank != logits_row % blocks) return;
     // the entries this block applies the penalty to: those that it reads
     const int own_begin = alone ? 0 : share.begin, own_end = alone ? vocab : share.end;
     // block 0's thread 0 calls this once: the token is the row's result and, with `record`, the newest entry
