@@ -209,10 +209,7 @@ class Engine:
         return logits[torch.tensor(wanted, dtype=torch.long, device=self.device)]
 
     def _pass(self, entries, device_tokens=None, batch=None) -> torch.Tensor:
-        with self.scope:
-            return self._pass_in_scope(entries, device_tokens, batch or _Batch(entries))
-
-    def _pass_in_scope(self, entries, device_tokens, batch) -> torch.Tensor:
+        batch = batch or _Batch(entries)
         lib, cache = native.lib(), self.cache._handle
         n_sections = lib.llmh_step_sections(cache)
         offsets, sizes = (c_longlong * n_sections)(), (c_longlong * n_sections)()
@@ -257,7 +254,8 @@ class Engine:
             ctx, tokens_dev, rows_dev = context(dev)
             if device_tokens is not None:
                 tokens_dev.copy_(device_tokens)
-            logits = self.model.forward(tokens_dev, ctx, rows_dev)
+            with self.scope:
+                logits = self.model.forward(tokens_dev, ctx, rows_dev)
         native.check(lib.llmh_step_commit(cache, batch.n, batch.slots, batch.counts))
         self.steps_run += 1
         return logits
@@ -294,7 +292,8 @@ class Engine:
                 tokens_dev.copy_(device_tokens)
             recording = ops.begin_recording()
             try:
-                logits = self.model.forward(tokens_dev, ctx, rows_dev)
+                with self.scope:
+                    logits = self.model.forward(tokens_dev, ctx, rows_dev)
             finally:
                 ops.end_recording()
             # the arena may have grown while this pass was planned: the stamp is taken afterwards
@@ -359,7 +358,7 @@ class Engine:
             before = ops.launch_count()
             torch.cuda.synchronize(self.device)
             cuda_graph = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(cuda_graph, pool=self._graph_pool):
+            with self.scope, torch.cuda.graph(cuda_graph, pool=self._graph_pool):
                 out = self.model.forward(tokens_dev, ctx, rows_dev)
             if self._graph_pool is None:
                 self._graph_pool = cuda_graph.pool()
