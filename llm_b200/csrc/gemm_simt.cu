@@ -117,7 +117,8 @@ gemm_simt_kernel(const TIn* __restrict__ a, const TIn* __restrict__ w,
 // Up to 8 rows of 32-bit operands with 16-byte rows (a decode step of the 32-bit path). Such a product streams the weights
 // once, and what bounds the tiled kernel there is the chain load - park - barrier - multiply of its one tile in flight, and
 // blocks that multiply 32 rows of which 29 are padding. Here a block is one warp with a ring of FEW_STAGES tiles of the
-// weights in flight (cp.async, requested before the wait for the kernel in front: no kernel writes weights); a lane owns a
+// weights in flight (cp.async; requested before the wait for the kernel in front where the caller says that w was complete
+// before that kernel was launched, as a model's weights are: w_bound); a lane owns a
 // weight row (32 / GROUPS rows a block, the lanes' groups take RPT of the token rows each) and adds k = 0, 1, 2, ... as the
 // tiled kernel does, so the bits are the same. A decode step of a 2-layer model of width 64 (9 such products among 23
 // launches, with all of the path's kernels chained by programmatic dependent launch): 73 -> 62 us.
@@ -125,8 +126,8 @@ constexpr int FEW_BK = 64, FEW_STAGES = 4, FEW_LD = FEW_BK + 4, FEW_ROWS = 8;   
 
 template <int GROUPS, int RPT>
 __global__ void __launch_bounds__(32)
-gemm_simt_few_kernel(const float* a, const float* __restrict__ w, const float* __restrict__ bias, float* __restrict__ out,
-                     float* __restrict__ residual, int M, int N, int K, int lda, int ldc) {
+gemm_simt_few_kernel(const float* a, const float* w, const float* bias, float* __restrict__ out,
+                     float* __restrict__ residual, int M, int N, int K, int lda, int ldc, int w_bound) {
     constexpr int COLS = 32 / GROUPS, ROWS = GROUPS * RPT;
     __shared__ __align__(16) float w_tile[FEW_STAGES][COLS][FEW_LD];
     __shared__ __align__(16) float a_tile[FEW_STAGES][ROWS][FEW_BK];
@@ -152,10 +153,18 @@ gemm_simt_few_kernel(const float* a, const float* __restrict__ w, const float* _
         for (int i = lane; i < FEW_STAGES * COLS * FEW_LD; i += 32) (&w_tile[0][0][0])[i] = 0.f;
     __syncwarp();
     griddep_launch();
+    if (w_bound) {
 #pragma unroll
-    for (int s = 0; s < FEW_STAGES - 1; ++s) if (s < n_k) request_w(s);
+        for (int s = 0; s < FEW_STAGES - 1; ++s) if (s < n_k) request_w(s);
+    }
     griddep_wait();
     a = behind_wait(a);
+    w = behind_wait(w);
+    bias = behind_wait(bias);
+    if (!w_bound) {
+#pragma unroll
+        for (int s = 0; s < FEW_STAGES - 1; ++s) if (s < n_k) request_w(s);
+    }
 #pragma unroll
     for (int s = 0; s < FEW_STAGES - 1; ++s) {
         if (s < n_k) request_a(s);
@@ -204,7 +213,7 @@ gemm_simt_few_kernel(const float* a, const float* __restrict__ w, const float* _
 
 template <typename TIn, typename TOut>
 static int launch(const void* a, const void* w, const float* bias, void* out, float* residual,
-                  int M, int N, int K, int lda, int ldc, cudaStream_t stream) {
+                  int M, int N, int K, int lda, int ldc, int w_bound, cudaStream_t stream) {
     // 16-byte loads: 32-bit elements, every row of both operands on a 16-byte boundary
     int vector = sizeof(TIn) == 4 && K % 4 == 0 && lda % 4 == 0 && (reinterpret_cast<uintptr_t>(a) & 15) == 0 &&
                  (reinterpret_cast<uintptr_t>(w) & 15) == 0;
@@ -213,7 +222,7 @@ static int launch(const void* a, const void* w, const float* bias, void* out, fl
             // (two rows a lane up to 4 rows: the more blocks, the more of the weights in flight)
             auto kernel = M <= 2 ? gemm_simt_few_kernel<1, 2> : M <= 4 ? gemm_simt_few_kernel<2, 2> : gemm_simt_few_kernel<2, 4>;
             LLMB_CUDA(llmb::launch(kernel, dim3(ceil_div(N, M <= 2 ? 32 : 16)), dim3(32), 0, stream, true, (const float*)a,
-                                   (const float*)w, bias, (float*)out, residual, M, N, K, lda, ldc));
+                                   (const float*)w, bias, (float*)out, residual, M, N, K, lda, ldc, w_bound));
             return check_launch("gemm_simt (few rows)");
         }
     }
@@ -231,23 +240,24 @@ static int launch(const void* a, const void* w, const float* bias, void* out, fl
 
 // in_dtype: element type of a and w. out_dtype: element type of `out` (ignored
 // when `residual` is given: then the product is added to residual[M, N], 32-bit).
+// w_bound: w was complete before the kernel in front of this call was launched (it may then be read before that one ends).
 LLMB_EXPORT int llmb_gemm_simt(const void* a, const void* w, const float* bias, void* out,
                                float* residual, int in_dtype, int out_dtype, int M, int N, int K,
-                               int lda, int ldc, cudaStream_t stream) {
+                               int lda, int ldc, int w_bound, cudaStream_t stream) {
     if (M == 0 || N == 0) return LLMB_OK;
     LLMB_REQUIRE(M > 0 && N > 0 && K > 0 && lda >= K && ldc >= N, "gemm_simt: bad sizes");
     LLMB_REQUIRE((out != nullptr) != (residual != nullptr), "gemm_simt: give out or residual");
     LLMB_REQUIRE(ceil_div(M, 32) <= 65535, "gemm_simt: too many rows");
     if (in_dtype == LLMB_DTYPE_F32) {
         if (residual || out_dtype == LLMB_DTYPE_F32)
-            return launch<float, float>(a, w, bias, out, residual, M, N, K, lda, ldc, stream);
+            return launch<float, float>(a, w, bias, out, residual, M, N, K, lda, ldc, w_bound, stream);
         return fail(LLMB_ERR_ARGUMENT, "gemm_simt: 32-bit inputs need a 32-bit output");
     }
     if (in_dtype == LLMB_DTYPE_BF16) {
         if (residual || out_dtype == LLMB_DTYPE_F32)
-            return launch<__nv_bfloat16, float>(a, w, bias, out, residual, M, N, K, lda, ldc, stream);
+            return launch<__nv_bfloat16, float>(a, w, bias, out, residual, M, N, K, lda, ldc, w_bound, stream);
         if (out_dtype == LLMB_DTYPE_BF16)
-            return launch<__nv_bfloat16, __nv_bfloat16>(a, w, bias, out, residual, M, N, K, lda, ldc, stream);
+            return launch<__nv_bfloat16, __nv_bfloat16>(a, w, bias, out, residual, M, N, K, lda, ldc, w_bound, stream);
     }
     return fail(LLMB_ERR_ARGUMENT, "gemm_simt: unknown dtypes %d -> %d", in_dtype, out_dtype);
 }

@@ -1156,7 +1156,11 @@ def linear(a, w, bias=None, out_dtype=None, residual=None, out=None, glu=False, 
     rows of the result are scaled by the norm's 1 / sqrt(mean square + eps) before the bias.
     `emit` (Emit, with `residual`): the updated residual rows as bfloat16 and the partial sums
     of their squares, for the next norm. `rope` (RopeWrite): the result is the q/k/v projection;
-    queries and keys are rotated, queries stay in the result, keys and values go to the cache."""
+    queries and keys are rotated, queries stay in the result, keys and values go to the cache.
+
+    When w may be written last: 32-bit products read w behind the kernel in front of them; inside a StepScope, and as
+    bfloat16 everywhere, a product may read w while that kernel still runs, so w must be complete before it was launched
+    (a model's weights are)."""
     _require_cuda(a, w, bias, residual)
     (m, k), (n, k2) = a.shape, w.shape
     if norm is not None:
@@ -1250,7 +1254,7 @@ def linear(a, w, bias=None, out_dtype=None, residual=None, out=None, glu=False, 
         _call("gemm_simt", "llmb_gemm_simt", _ptr(a), _ptr(w), _ptr(bias),
               _ptr(result if residual is None else None), _ptr(residual),
               _c_int(_code(a.dtype)), _c_int(_code(target_dtype)), _c_int(m), _c_int(n), _c_int(k),
-              _c_int(a.stride(0)), _c_int(n), _stream())
+              _c_int(a.stride(0)), _c_int(n), _c_int(1 if scratch.inside() else 0), _stream())
     else:
         raise KernelError(f"linear: no kernel named {variant}")
     return result

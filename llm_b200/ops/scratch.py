@@ -31,7 +31,8 @@ def _new(device, floats: int, counters: int) -> tuple:
 
 class StepScope:
     """The scratch of one line of work, an engine's steps for instance. Inside `with scope:` the calls of this thread use it,
-    on any stream and under capture. It grows when a call needs more; what was outgrown is kept, because captured and
+    on any stream and under capture, and products and norms take the matrices and gains that they are given for weights, which
+    no kernel inside the scope writes (ops.linear, ops.norm_add_). It grows when a call needs more; what was outgrown is kept, because captured and
     recorded steps may hold its address. `generation` counts that."""
 
     def __init__(self):
@@ -62,6 +63,11 @@ class StepScope:
             generation += 1
         self._held[(device, kind)] = grown
         return grown
+
+
+def inside() -> bool:
+    """Whether this thread is inside a StepScope."""
+    return bool(getattr(_line, "entered", None))
 
 
 def of_call(device, stream: int, capturing: bool, kind: str, floats: int, counters: int = 0) -> tuple:

@@ -782,6 +782,23 @@ def test_linear_of_few_rows_in_32_bit(n, k, residual):
     assert torch.allclose(whole, want, atol=k * 2.0 ** -24 * float((x.abs() @ w.abs().T).max()), rtol=1e-6)
 
 
+@pytest.mark.parametrize("m,n,k", [(1, 512, 4096), (3, 4096, 512), (8, 64, 64)])
+def test_linear_of_few_rows_reads_a_matrix_written_just_before(m, n, k):
+    """The matrix is the result of the launch in front, into the same memory each time."""
+    x, w = randn(m, k, seed=330), torch.empty(n, k, device=DEV)
+    rows = [randn(n, k, seed=331 + i) for i in range(8)]
+    gain = torch.ones(k, device=DEV)
+    got = []
+    for r in rows:
+        ops().rmsnorm(r, gain, 1e-5, torch.float32, out=w)
+        got.append(ops().linear(x, w, out_dtype=torch.float32))
+    torch.cuda.synchronize()
+    for r, g in zip(rows, got):
+        ops().rmsnorm(r, gain, 1e-5, torch.float32, out=w)
+        torch.cuda.synchronize()
+        assert torch.equal(g, ops().linear(x, w, out_dtype=torch.float32))
+
+
 # ----------------------------------------------------------------------------- what rides in a product's epilogue
 
 def _sums_in_parts(x, parts, seed):
