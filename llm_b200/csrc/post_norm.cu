@@ -65,11 +65,12 @@ norm_add_kernel(const float* __restrict__ y, int terms, const float* __restrict_
 
 // The same for rows of a multiple of four values up to 8,192, all arrays on 16-byte boundaries: NT threads (as many as the row
 // has groups of four, up to 512) hold a row in registers, NV groups of four values each, and every load that does not wait
-// for a sum is requested before the first one is needed (the gains even before the kernel in front has ended). A row is one
-// chain of load, sum, sum; the kernel above walks it element by element, with a chain of `terms` loads for each. Rows of
-// 4,096, some of them with eight terms: 24 rows 14.7 -> 4.2 us, 2,077 rows 44.7 -> 37.0 us. Short rows, 4,096 of them with one
-// term: of 64 values 8.3 us by the kernel above, 19.3 with 512 threads a row, 4.7 so; of 1,024 values 17.6, 20.6 and 9.3. The
-// choice depends on the row's width and the addresses' alignment only, so that a row's sums have one order in every step.
+// for a sum is requested before the first one is needed (the gains even before the kernel in front has ended, where the
+// caller says that they were complete before that one was launched: gains_bound). A row is one chain of load, sum, sum; the
+// kernel above walks it element by element, with a chain of `terms` loads for each. Rows of 4,096, some of them with eight
+// terms: 24 rows 14.7 -> 4.2 us, 2,077 rows 44.7 -> 37.0 us. Short rows, 4,096 of them with one term: of 64 values 8.3 us by the kernel above,
+// 19.3 with 512 threads a row, 4.7 so; of 1,024 values 17.6, 20.6 and 9.3. The choice depends on the row's width and the
+// addresses' alignment only, so that a row's sums have one order in every step.
 constexpr int WIDE_THREADS = 512;      // most threads a row
 template <typename TOut> __device__ __forceinline__ void store4(TOut* p, float4 v);
 template <> __device__ __forceinline__ void store4<float>(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
@@ -81,7 +82,7 @@ __device__ __forceinline__ float square4(float4 v, float sum) {
     return fmaf(v.w, v.w, fmaf(v.z, v.z, fmaf(v.y, v.y, fmaf(v.x, v.x, sum))));
 }
 
-template <typename TOut, int NV, int NT>
+template <typename TOut, int NV, int NT, bool BOUND>
 __global__ void __launch_bounds__(NT)
 norm_add_wide_kernel(const float* __restrict__ y, int terms, const float* __restrict__ gain_post, float eps_post,
                      float* __restrict__ x, const float* __restrict__ gain_next, float eps_next, TOut* __restrict__ h,
@@ -89,6 +90,11 @@ norm_add_wide_kernel(const float* __restrict__ y, int terms, const float* __rest
     __shared__ float scratch[2][NT / 32];
     int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     griddep_launch();
+    if constexpr (!BOUND) {
+        griddep_wait();
+        gain_post = behind_wait(gain_post);
+        gain_next = behind_wait(gain_next);
+    }
     float4 post[NV], next[NV];
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
@@ -99,7 +105,7 @@ norm_add_wide_kernel(const float* __restrict__ y, int terms, const float* __rest
             if (gain_next) next[i] = *reinterpret_cast<const float4*>(gain_next + c);
         }
     }
-    griddep_wait();
+    if constexpr (BOUND) griddep_wait();
     y = behind_wait(y);
     size_t t = blockIdx.x;
     float* x_row = x + t * hidden;
@@ -153,9 +159,23 @@ norm_add_wide_kernel(const float* __restrict__ y, int terms, const float* __rest
     }
 }
 
+// The instance for a row: as many threads as it has groups of four, up to 512.
+template <typename T, bool BOUND>
+static auto norm_add_wide(int hidden, int* threads) {
+    *threads = hidden <= 128 ? 32 : hidden <= 256 ? 64 : hidden <= 512 ? 128 : hidden <= 1024 ? 256 : WIDE_THREADS;
+    return hidden <= 128    ? norm_add_wide_kernel<T, 1, 32, BOUND>
+           : hidden <= 256  ? norm_add_wide_kernel<T, 1, 64, BOUND>
+           : hidden <= 512  ? norm_add_wide_kernel<T, 1, 128, BOUND>
+           : hidden <= 1024 ? norm_add_wide_kernel<T, 1, 256, BOUND>
+           : hidden <= 2048 ? norm_add_wide_kernel<T, 1, 512, BOUND>
+           : hidden <= 4096 ? norm_add_wide_kernel<T, 2, 512, BOUND>
+                            : norm_add_wide_kernel<T, 4, 512, BOUND>;
+}
+
+// gains_bound: the gains were complete before the kernel in front of this call was launched.
 LLMB_EXPORT int llmb_norm_add(const float* y, int terms, const float* gain_post, float eps_post, float* x,
                               const float* gain_next, float eps_next, void* h, int h_dtype, int n_rows, int hidden,
-                              cudaStream_t stream) {
+                              int gains_bound, cudaStream_t stream) {
     if (n_rows == 0) return LLMB_OK;
     LLMB_REQUIRE(hidden > 0 && terms > 0 && y && x && gain_post, "norm_add: bad sizes or a missing array");
     LLMB_REQUIRE(!gain_next || h, "norm_add: the next norm has no output");
@@ -166,12 +186,8 @@ LLMB_EXPORT int llmb_norm_add(const float* y, int terms, const float* gain_post,
 #define LLMB_NORM_ADD(T)                                                                                           \
     do {                                                                                                           \
         if (wide) {                                                                                                \
-            /* as many threads as the row has groups of four, up to 512 */                                         \
-            int threads = hidden <= 128 ? 32 : hidden <= 256 ? 64 : hidden <= 512 ? 128 : hidden <= 1024 ? 256 : WIDE_THREADS; \
-            auto kernel = threads == 32 ? norm_add_wide_kernel<T, 1, 32> : threads == 64 ? norm_add_wide_kernel<T, 1, 64> \
-                          : threads == 128 ? norm_add_wide_kernel<T, 1, 128> : threads == 256 ? norm_add_wide_kernel<T, 1, 256> \
-                          : hidden <= 2048 ? norm_add_wide_kernel<T, 1, 512> : hidden <= 4096 ? norm_add_wide_kernel<T, 2, 512> \
-                          : norm_add_wide_kernel<T, 4, 512>;                                                       \
+            int threads = 0;                                                                                       \
+            auto kernel = gains_bound ? norm_add_wide<T, true>(hidden, &threads) : norm_add_wide<T, false>(hidden, &threads); \
             LLMB_CUDA(llmb::launch(kernel, dim3(n_rows), dim3(threads), 0, stream, true, y, terms, gain_post,      \
                                    eps_post, x, gain_next, eps_next, (T*)h, hidden));                              \
             break;                                                                                                 \

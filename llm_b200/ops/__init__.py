@@ -492,7 +492,8 @@ def norm_add_(x, y, gain_post, eps_post, terms: int = 1, gain_next=None, eps_nex
     """x[t] += s / sqrt(mean(s^2) + eps_post) * gain_post with s = sum_k y[t * terms + k] (y float32
     [T * terms, hidden]): the norm behind a part and the residual sum. With `gain_next` also
     out[t] = x[t] / sqrt(mean(x[t]^2) + eps_next) * gain_next in `out_dtype`: the norm in front of the
-    next part, of the updated rows. Returns `out` (or None)."""
+    next part, of the updated rows. Returns `out` (or None). Inside a StepScope the gains may be read while the
+    kernel in front still runs: they must be complete before it was launched."""
     _require_cuda(x, y, gain_post, gain_next, out)
     n, hidden = x.shape
     if (x.dtype != torch.float32 or y.dtype != torch.float32 or not x.is_contiguous() or not y.is_contiguous()
@@ -510,7 +511,7 @@ def norm_add_(x, y, gain_post, eps_post, terms: int = 1, gain_next=None, eps_nex
         out = None
     _call("post_norm", "llmb_norm_add", _ptr(y), _c_int(terms), _ptr(gain_post), _c_float(eps_post), _ptr(x),
           _ptr(gain_next), _c_float(eps_next), _ptr(out), _c_int(_code(out.dtype) if out is not None else 0),
-          _c_int(n), _c_int(hidden), _stream())
+          _c_int(n), _c_int(hidden), _c_int(1 if scratch.inside() else 0), _stream())
     return out
 
 

@@ -70,6 +70,28 @@ def test_norm_add_at_the_edges_of_rows_in_registers(width, terms):
         _close(got, want, torch.bfloat16, (terms, n, "next"))
 
 
+def test_norm_add_reads_gains_written_just_before():
+    """The gains are the result of the launch in front, into the same memory each time."""
+    ops = _ops()
+    gen = torch.Generator().manual_seed(12)
+    n, width = 300, 4096
+    x, y = (torch.randn((n, width), generator=gen).to(DEV) for _ in range(2))
+    rows = [torch.randn((2, width), generator=gen).to(DEV) for _ in range(8)]
+    gains, ones = torch.empty((2, width), device=DEV), torch.ones(width, device=DEV)
+    got = []
+    for r in rows:
+        after = x.clone()
+        ops.rmsnorm(r, ones, 1e-5, torch.float32, out=gains)
+        got.append((after, ops.norm_add_(after, y, gains[0], 1e-5, 1, gains[1], 1e-5, out_dtype=torch.float32)))
+    torch.cuda.synchronize()
+    for r, (after, h) in zip(rows, got):
+        ops.rmsnorm(r, ones, 1e-5, torch.float32, out=gains)
+        want = x.clone()
+        torch.cuda.synchronize()
+        assert torch.equal(h, ops.norm_add_(want, y, gains[0], 1e-5, 1, gains[1], 1e-5, out_dtype=torch.float32))
+        assert torch.equal(after, want)
+
+
 def test_norm_add_sums_a_token_s_rows_in_their_order():
     """Three rows a token whose sum in another order would round differently: 1e8 - 1e8 + 1 is 1, not 0."""
     ops = _ops()
