@@ -97,15 +97,17 @@ conv_fours_kernel(ConvSource<T> source, const int* __restrict__ tok_seq, const i
     griddep_launch();
     int c = (blockIdx.y * 256 + threadIdx.x) * 4;
     if (c >= source.channels) return;
+    griddep_wait();
+    const float* conv_w = behind_wait(source.conv_w);
+    const float* conv_b = behind_wait(source.conv_b);
     float taps[4][4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-        float4 w = *reinterpret_cast<const float4*>(source.conv_w + (size_t)(c + e) * 4);
+        float4 w = *reinterpret_cast<const float4*>(conv_w + (size_t)(c + e) * 4);
         taps[e][0] = w.x; taps[e][1] = w.y; taps[e][2] = w.z; taps[e][3] = w.w;
     }
-    float4 bias4 = *reinterpret_cast<const float4*>(source.conv_b + c);
+    float4 bias4 = *reinterpret_cast<const float4*>(conv_b + c);
     const float bias[4] = {bias4.x, bias4.y, bias4.z, bias4.w};
-    griddep_wait();
     const T* x = behind_wait(source.x) + c;
     int t0 = blockIdx.x * TOK, count = min(TOK, n_tokens - t0);
     int seq0 = tok_seq[t0];

@@ -411,6 +411,27 @@ def test_gated_recurrence_of_aligned_rows(dtype, channels, blocks):
         _close(states[0], states[1], torch.float32, (channels, lengths, "state"))
 
 
+def test_gated_recurrence_reads_taps_written_just_before():
+    """The taps are the result of the launch in front, into the same memory each time."""
+    ops = _ops()
+    channels, n = 1024, 700
+    batch = Batch([n], [n])
+    _, params, state = _recurrence_inputs(channels, 4, 4, n, 2, torch.float32, seed=5)
+    wide = torch.randn((n, 2 * channels), generator=torch.Generator().manual_seed(8)).to(DEV)
+    raw = [torch.randn((channels, 4), generator=torch.Generator().manual_seed(20 + i)).to(DEV) for i in range(6)]
+    ones, got = torch.ones(4, device=DEV), []
+    for r in raw:
+        held = state.clone()
+        ops.rmsnorm(r, ones, 1e-5, torch.float32, out=params["conv_w"])
+        got.append(_recurrence(ops.gated_recurrence, wide, params, held, batch, channels, torch.float32, at=0))
+    torch.cuda.synchronize()
+    for r, g in zip(raw, got):
+        held = state.clone()
+        ops.rmsnorm(r, ones, 1e-5, torch.float32, out=params["conv_w"])
+        torch.cuda.synchronize()
+        assert torch.equal(g, _recurrence(ops.gated_recurrence, wide, params, held, batch, channels, torch.float32, at=0))
+
+
 def test_gated_recurrence_carries_its_state_across_any_cut():
     """A sequence in one step, and the same cut at every place into two steps (the second also token by
     token): the same results to the last bit in 32-bit, and the state that the cuts leave is the same."""
