@@ -125,7 +125,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                             const int* __restrict__ seq_lens, const int* __restrict__ seq_order,
                             __nv_bfloat16* __restrict__ out, int out_stride,
                             int n_heads, int n_kv_heads, float scale_log2, const float* __restrict__ sinks,
-                            const float* __restrict__ bias, int span, int window, const __nv_bfloat16* __restrict__ gate,
+                            const float* __restrict__ bias, int span, int window, const __nv_bfloat16* gate,
                             int gate_stride, float out_scale, int* status) {
     constexpr int PIECES = HD / 64;
     constexpr int Q_BYTES = PIECES * Q_PIECE;         // the block's queries
@@ -150,6 +150,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
 
     griddep_launch();            // the next kernel may set itself up; this one needs the one before it whole
     griddep_wait();
+    if constexpr (WINDOW) gate = behind_wait(gate);
     // seq_order (optional): sequences by falling length, so that the longest start first
     int seq = seq_order ? seq_order[blockIdx.z] : (int)blockIdx.z, head = blockIdx.x;
     int first_token = cu_seqlens[seq];
