@@ -1626,6 +1626,13 @@ def sigmoid_mixed_heads(n_tokens: int, n_heads: int, n_kv_heads: int, dim: int, 
     return (n_heads + groups - 1) // groups             # groups of equal size
 
 
+def sigmoid_mixed_elements(n_tokens: int, n_heads: int, n_kv_heads: int, dim: int) -> int:
+    """Elements of the buffer that the mixed queries of a step are kept in: never fewer than a shorter step asks for
+    (the number of heads that fit into them jumps), so that no step outgrows what a longer one planned."""
+    one = n_tokens * n_kv_heads * dim
+    return min(n_heads * one, max(SIGMOID_MIXED_BYTES // 2, one))
+
+
 def sigmoid_attention(q, k_cache, v_cache, block_table, ring_pages, tok_pos, tok_seq, n_heads, n_kv_heads, dim, vdim,
                       scale, window, talk, head_bias, out_scale, out, decode=False, seq_lens=None, max_len=0,
                       cu_seqlens=None, max_new=0, seq_order=None, mixed=None):
@@ -1865,6 +1872,6 @@ def required_libraries() -> list:
 __all__ = ["PAGE", "GLU_BLOCK", "glu_fusable", "embed", "scale_", "random_normal_", "begin_recording", "end_recording", "RecordedPass", "StepScope", "scratch_generation", "Emit", "FoldedNorm", "RopeWrite", "cast_sumsq", "SUMSQ_LD", "rmsnorm", "swiglu", "rope_cache_write", "linear", "attention",
            "softcap_", "add_rows_", "conv_rope_cache_write", "diff_attention", "tanh_norm", "norm_rope_cache_write",
            "sigmoid_attention", "gated_recurrence", "state_space", "attention_replay_key", "layernorm", "input_conv", "output_norm_add_", "forget_recurrence",
-           "latent_write", "head_products", "latent_attention", "latent_prefill", "attention_decode_splits", "sigmoid_attention_replay_key", "sigmoid_decode_splits", "sigmoid_mixed_heads",
+           "latent_write", "head_products", "latent_attention", "latent_prefill", "attention_decode_splits", "sigmoid_attention_replay_key", "sigmoid_decode_splits", "sigmoid_mixed_heads", "sigmoid_mixed_elements",
            "argmax_rows", "sample_rows", "launch_count", "count_launches", "tensor_core_status", "check_device_status", "ensure_built", "load_library", "all_sources",
            "required_libraries", "tactics"]

@@ -88,9 +88,10 @@ class SigmoidAttentionMixer(ProjectedMixer):
         from ..engine.workspace import BufferRequest
         # phases: 0 norm + rotation + cache write, 1 attention
         out = [BufferRequest("queries", (n_tokens, self.q_width), dtype, 0, 1)]
-        mixed = self._mixed_shape(n_tokens, dtype)
-        if mixed is not None:
-            out.append(BufferRequest("mixed_queries", mixed, dtype, 1, 1))
+        if self._mixed_shape(n_tokens, dtype) is not None:
+            s = self.spec
+            out.append(BufferRequest("mixed_queries", (ops.sigmoid_mixed_elements(n_tokens, s.n_heads, s.n_kv_heads, s.head_dim),),
+                                     dtype, 1, 1))
         return out
 
     def _mixed_shape(self, n_tokens, dtype):

@@ -215,3 +215,16 @@ def test_inspect_and_random_commands(tmp_path, capsys):
     assert main(["inspect", str(tmp_path / "m")]) == 0
     text = capsys.readouterr().out
     assert "Mefolorn" in text and "sigmoid attention" in text
+
+
+def test_the_room_for_mixed_queries_never_shrinks_as_steps_grow():
+    """A step's mixed queries fit into what its plan asks for, and a shorter step never asks for more than a longer one."""
+    from llm_b200 import ops
+    for heads, groups, dim in ((32, 8, 128), (8, 1, 64), (128, 16, 64), (4, 4, 128)):
+        last = 0
+        for n in list(range(1, 200)) + [511, 512, 2500, 4095, 4096, 4097, 4100, 4300, 8192, 8193, 20000, 65536, 140000, 300000]:
+            room = ops.sigmoid_mixed_elements(n, heads, groups, dim)
+            at_once = ops.sigmoid_mixed_heads(n, heads, groups, dim, 64)
+            assert room >= last and at_once >= 1 and at_once * n * groups * dim <= room, (heads, n)
+            assert 2 * room <= max(ops.SIGMOID_MIXED_BYTES, 2 * n * groups * dim)
+            last = room
