@@ -1749,11 +1749,11 @@ LLMB_EXPORT int llmb_gemm_tc_counters(int M, int N, int K) {
     return p.tiles_a * p.tiles_b;
 }
 
-// Kernels a call launches (1, or 2 where the split-K sum is a kernel of its own).
-LLMB_EXPORT int llmb_gemm_tc_kernels(int M, int N, int K) {
+// Kernels a call launches (1, or 2 where the sum of parts is a kernel of its own).
+LLMB_EXPORT int llmb_gemm_tc_kernels(int M, int N, int K, int allow_pair) {
     Plan p = make_plan(M, N, K);
     int n_pairs;
-    if (on_pairs(p, M, N)) return plan_pairs(M, N, K, &n_pairs).tail_tiles > 0 ? 2 : 1;
+    if (allow_pair && on_pairs(p, M, N)) return plan_pairs(M, N, K, &n_pairs).tail_tiles > 0 ? 2 : 1;
     return 1 + sums_later(p.swap, p.splits, p.bn);
 }
 

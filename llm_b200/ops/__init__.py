@@ -1059,13 +1059,14 @@ def _skinny_scratch(device, m, n, k):
 
 
 @functools.lru_cache(maxsize=4096)
-def _tc_needs(m: int, n: int, k: int) -> tuple:
-    """(floats of partial sums, tile counters, kernels launched) of a tcgen05 product of this shape."""
+def _tc_needs(m: int, n: int, k: int, pairs: bool = True) -> tuple:
+    """(floats of partial sums, tile counters, kernels launched) of a tcgen05 product of this shape; `pairs`: on pairs of SMs
+    where its tiles fit them."""
     lib = load_library("gemm_tc")
     lib.llmb_gemm_tc_scratch_floats.restype = ctypes.c_longlong
     return (lib.llmb_gemm_tc_scratch_floats(_c_int(m), _c_int(n), _c_int(k)),
             lib.llmb_gemm_tc_counters(_c_int(m), _c_int(n), _c_int(k)),
-            lib.llmb_gemm_tc_kernels(_c_int(m), _c_int(n), _c_int(k)))
+            lib.llmb_gemm_tc_kernels(_c_int(m), _c_int(n), _c_int(k), _c_int(1 if pairs else 0)))
 
 
 def _tc_scratch(device, m, n, k) -> tuple:
@@ -1111,7 +1112,7 @@ def glu_fusable(n_rows: int, k: int, dtype) -> bool:
 
 def _tc_kernels(m: int, n: int, k: int) -> int:
     """Kernels one call of the tcgen05 product launches (2 where the split-K sum is its own kernel)."""
-    return _tc_needs(m, n, k)[2]
+    return _tc_needs(m, n, k, not tactics.is_disabled("gemm_tc_pair"))[2]
 
 
 def _fusion_struct(norm, emit, rope):
