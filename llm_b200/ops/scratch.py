@@ -78,11 +78,12 @@ def of_call(device, stream: int, capturing: bool, kind: str, floats: int, counte
     if capturing:
         return _new(device, floats, counters)
     with _lock:
-        scope = _of_stream.pop((device, stream), None) or StepScope()
+        scope = _of_stream.pop((device, stream), None)
+        if scope is None:
+            scope = StepScope()
+            for key in [key for key in _of_stream if key[0] == device][:1 - STREAMS]:
+                del _of_stream[key]
         _of_stream[(device, stream)] = scope
-        mine = [key for key in _of_stream if key[0] == device]
-        for key in mine[:-STREAMS]:
-            del _of_stream[key]
         found = scope.room(device, kind, floats, counters, False)
         scope._outgrown.clear()           # nothing but records points at it, and those keep it themselves
         return found
