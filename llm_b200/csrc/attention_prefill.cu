@@ -47,12 +47,6 @@ constexpr int STAGES = 2;
 constexpr int PAD = 8;
 
 // 2^x by the hardware approximation (relative error about 2^-22; 2^-inf = 0)
-__device__ __forceinline__ float fast_exp2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
 template <int D, bool BIAS>
 __global__ void __launch_bounds__(WARPS * 32, 3)          // three blocks per SM: at most 170 registers
 attention_prefill_kernel(const __nv_bfloat16* __restrict__ q, int q_stride,

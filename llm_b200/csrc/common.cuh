@@ -92,6 +92,13 @@ __device__ __forceinline__ float warp_max(float v) {
     return v;
 }
 
+// 2^x by the special-function unit
+__device__ __forceinline__ float fast_exp2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
 inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
 
 // Programmatic dependent launch: a kernel launched with `dependent` may begin while the kernel

@@ -177,12 +177,6 @@ LLMB_PACKED(llmb_diff_attention_generic)
 
 constexpr int PAD = 8;                       // bf16 elements of row padding in shared memory
 
-__device__ __forceinline__ float fast_exp2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
 // ----------------------------------------------------------------------------- prefill
 // grid (heads, query tiles, sequences); tile 0 of the grid is a sequence's last 64 queries. Eight
 // warps: warps 0-3 compute map 1 of the tile's 64 queries (16 rows a warp), warps 4-7 map 2, over

@@ -42,15 +42,6 @@ constexpr int Q_PIECE = BQ * 64 * 2;              // 128 query rows, 64 columns 
 constexpr int KV_PIECE = LLMB_PAGE * 64 * 2;      // one page, 64 columns
 constexpr uint32_t O_COL = 256, TMEM_COLS = 512;  // scores: (map * 2 + buffer) * 64
 
-__device__ __forceinline__ float fast_exp2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
-    __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&v);
-}
 __device__ __forceinline__ void softmax_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(SOFTMAX_THREADS) : "memory"); }
 
 template <int DK, int DV>

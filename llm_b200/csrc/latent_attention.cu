@@ -300,12 +300,6 @@ LLMB_PACKED(llmb_head_products)
 
 // ---------------------------------------------------------------------------------------------- attention
 
-__device__ __forceinline__ float fast_exp2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
 // What a sink adds to a denominator in units of 2^m (m: the row's reference, base 2). A sink far above every score makes it
 // infinite and the row's result zero, as it should be.
 __device__ __forceinline__ float sink_share(float sink, float m) { return exp2f(fmaf(sink, 1.4426950408889634f, -m)); }

@@ -40,15 +40,6 @@ constexpr int Q_PIECE = BQ * 64 * 2, KV_PIECE = BKV * 64 * 2;
 // tensor memory of a tile: two buffers of scores (64 columns each), then O
 constexpr uint32_t S_COL = 0, O_COL = 128, TILE_COLS = 256, TMEM_COLS = TILES * TILE_COLS;
 
-__device__ __forceinline__ float fast_exp2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
-    __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&v);
-}
 
 // D and V: 64 or 128 (one or two 64-column pieces); the rotated part is one piece of up to 64.
 template <int D, int V>

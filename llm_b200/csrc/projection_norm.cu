@@ -327,11 +327,10 @@ LLMB_EXPORT int llmb_norm_rope_cache_write(const void* u, int u_stride, int dtyp
     if (eights && norm_unit > 0) smem += sizeof(float) * (size_t)((q_width + k_width) / norm_unit);
 #define LLMB_NORM_ROPE(T)                                                                                            \
     do {                                                                                                             \
-        auto norm_rope_cache_write_kernel = eights ? norm_rope_cache_write_eights_kernel<T> : ::norm_rope_cache_write_kernel<T>; \
+        auto kernel = eights ? norm_rope_cache_write_eights_kernel<T> : norm_rope_cache_write_kernel<T>;             \
         if (smem > 48 * 1024)                                                                                        \
-            LLMB_CUDA(cudaFuncSetAttribute(norm_rope_cache_write_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                           (int)smem));                                                              \
-        LLMB_CUDA(llmb::launch(norm_rope_cache_write_kernel, dim3(n_tokens), dim3(THREADS), smem, stream, true,    \
+            LLMB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));          \
+        LLMB_CUDA(llmb::launch(kernel, dim3(n_tokens), dim3(THREADS), smem, stream, true,                            \
                                (const T*)u, u_stride, q_width, k_width, v_width, q_gain, k_gain, eps, rope_table,   \
                                rope_table ? n_rot : 0, rot_unit > 0 ? rot_unit : 1, interleaved, tok_pos, tok_seq,   \
                                (T*)q_out, q_out_stride, block_table, table_stride, ring_pages, (T*)k_cache, k_heads, \

@@ -534,8 +534,8 @@ using namespace llmb::tc;
 constexpr int GM = 128, GK = 64, G_THREADS = 192;
 constexpr int A_BYTES = GM * GK * 2;
 // tiles of 128 columns: a ring of three stages, two blocks an SM
-__host__ __device__ constexpr int stages_of(int) { return 3; }
-__host__ __device__ constexpr size_t smem_of(int gn) { return 1024 + (size_t)stages_of(gn) * (A_BYTES + gn * GK * 2) + (2 * stages_of(gn) + 1) * 8 + 16; }
+constexpr int GN = 128, G_STAGES = 3;
+constexpr size_t WIDE_SMEM = 1024 + (size_t)G_STAGES * (A_BYTES + GN * GK * 2) + (2 * G_STAGES + 1) * 8 + 16;
 
 // Xs[s, :] = h[sorted[s] / top, :]: the rows of h in the order of the plan (16 bytes a thread a time).
 __global__ void __launch_bounds__(256)
@@ -552,9 +552,9 @@ gather_rows_kernel(const __nv_bfloat16* __restrict__ h, int ld, int top, const i
     }
 }
 
-// The epilogue of one tile by one thread: row `row` of the tile's rows [first, first + rows) of the list, the GN accumulator
-// columns at taddr, the output columns from n0 on.
-template <bool GLU, int GN>
+// The epilogue of one tile by one thread: row `row` of the tile's rows [first, first + rows) of the list, the COLUMNS
+// accumulator columns at taddr, the output columns from n0 on.
+template <bool GLU, int COLUMNS>
 __device__ __forceinline__ void store_row(uint32_t taddr, int row, int rows, int first, int n0, int N, __nv_bfloat16* act, float* y,
                                           const int* sorted, const float* weights, Activation activation) {
     bool live = row < rows;
@@ -563,10 +563,10 @@ __device__ __forceinline__ void store_row(uint32_t taddr, int row, int rows, int
         __nv_bfloat16* out = act + (long long)(first + row) * N + n0;
         bool vector = N % 8 == 0;
 #pragma unroll 1
-        for (int c = 0; c < GN / 2; c += 16) {
+        for (int c = 0; c < COLUMNS / 2; c += 16) {
             uint32_t g[16], u[16];
             tmem_ld16(taddr + c, g);
-            tmem_ld16(taddr + GN / 2 + c, u);
+            tmem_ld16(taddr + COLUMNS / 2 + c, u);
             if (!live || n0 + c >= N) continue;
             float v[16];
 #pragma unroll
@@ -596,7 +596,7 @@ __device__ __forceinline__ void store_row(uint32_t taddr, int row, int rows, int
         float* out = y + (long long)assignment * N + n0;
         bool vector = N % 4 == 0;
 #pragma unroll 1
-        for (int c = 0; c < GN; c += 16) {
+        for (int c = 0; c < COLUMNS; c += 16) {
             uint32_t r[16];
             tmem_ld16(taddr + c, r);
             if (!live || n0 + c >= N) continue;
@@ -621,13 +621,13 @@ __device__ __forceinline__ void store_row(uint32_t taddr, int row, int rows, int
 // gate rows, then N up rows, and a stage holds GN / 2 gate rows and the GN / 2 up rows of the same features, so that the
 // accumulator's first half are gates and its second half the ups. Warp 0: TMA producer. Warp 1: tensor memory and the
 // products. Warps 2..5: epilogue, a thread a row. Every wait is bounded and reports through `status`.
-template <bool GLU, int GN>
+template <bool GLU>
 __global__ void __launch_bounds__(G_THREADS, 2)
 expert_product_wide_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                            const int* __restrict__ plan, int E, int max_tiles, int b_rows, int N, int n_kblocks,
                            __nv_bfloat16* __restrict__ act, float* __restrict__ y, const int* __restrict__ sorted,
                            const float* __restrict__ weights, Activation activation, int* status) {
-    constexpr int G_STAGES = stages_of(GN), B_BYTES = GN * GK * 2;
+    constexpr int B_BYTES = GN * GK * 2;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     unsigned char* a_tiles = base;
@@ -944,15 +944,15 @@ LLMB_EXPORT int llmb_routed_experts(const void* h, int ld, int dtype, const floa
     if (wide_tiles) {
         typedef __nv_bfloat16 B;
         using namespace wide;
-        // tiles of 256 columns wherever the products are wide enough for them (ahead at every length of the lists that comes
-        // here, 128 to 8,192 tokens, and at all four shapes that were measured)
+        // Tiles of 256 columns wherever the products are wide enough for them. The whole feed-forward with them over that with
+        // tiles of 128, from 128 (or the first that comes here) to 8,192 tokens: 8 of 32 experts of 1,792 at width 4,096 0.95 to
+        // 0.70, 2 of 8 of 14,336 0.96 to 0.73; at width 2,048 8 of 64 of 1,024 0.94 to 0.76, 6 of 64 of 1,408 0.88 to 0.74; at
+        // width 1,024 4 of 128 of 512 0.89 to 0.92; only 256 experts of 512 at width 4,096 gain little, 0.93 to 1.04.
         bool wide256 = tensor_cores >= 3 && F >= 128 && hidden >= 256;
-        constexpr int GN = 128;
-        size_t smem = smem_of(GN);
         static bool configured = false;
         if (!configured) {
-            LLMB_CUDA(cudaFuncSetAttribute(expert_product_wide_kernel<true, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_of(128)));
-            LLMB_CUDA(cudaFuncSetAttribute(expert_product_wide_kernel<false, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_of(128)));
+            LLMB_CUDA(cudaFuncSetAttribute(expert_product_wide_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WIDE_SMEM));
+            LLMB_CUDA(cudaFuncSetAttribute(expert_product_wide_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WIDE_SMEM));
             LLMB_CUDA(cudaFuncSetAttribute(expert_product_stream_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)STREAM_SMEM));
             LLMB_CUDA(cudaFuncSetAttribute(expert_product_stream_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)STREAM_SMEM));
             configured = true;
@@ -982,12 +982,12 @@ LLMB_EXPORT int llmb_routed_experts(const void* h, int ld, int dtype, const floa
                                    (F + GK - 1) / GK, (B*)nullptr, y, (const int*)sorted, down_weights, activation, status_dev));
             return check_launch("routed_experts");
         }
-        auto up = expert_product_wide_kernel<true, 128>;
-        auto down = expert_product_wide_kernel<false, 128>;
-        LLMB_CUDA(llmb::launch(up, dim3((F + GN / 2 - 1) / (GN / 2), tiles), dim3(G_THREADS), smem, stream, true, map_x, map_up,
+        auto up = expert_product_wide_kernel<true>;
+        auto down = expert_product_wide_kernel<false>;
+        LLMB_CUDA(llmb::launch(up, dim3((F + GN / 2 - 1) / (GN / 2), tiles), dim3(G_THREADS), WIDE_SMEM, stream, true, map_x, map_up,
                                (const int*)plan, E, max_tiles, 2 * F, F, (hidden + GK - 1) / GK, (B*)act, (float*)nullptr,
                                (const int*)sorted, up_weights, activation, status_dev));
-        LLMB_CUDA(llmb::launch(down, dim3((hidden + GN - 1) / GN, tiles), dim3(G_THREADS), smem, stream, true, map_act, map_down,
+        LLMB_CUDA(llmb::launch(down, dim3((hidden + GN - 1) / GN, tiles), dim3(G_THREADS), WIDE_SMEM, stream, true, map_act, map_down,
                                (const int*)plan, E, max_tiles, hidden, hidden, (F + GK - 1) / GK, (B*)nullptr, y,
                                (const int*)sorted, down_weights, activation, status_dev));
     } else if (tc) {

@@ -162,12 +162,6 @@ constexpr int TILE_WARPS = 2 * WARPS;        // two warps share 16 query rows an
 constexpr int STAGES = 3;
 constexpr int PAD = 8;
 
-__device__ __forceinline__ float fast_exp2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
 template <int D, int DV>
 __global__ void __launch_bounds__(TILE_WARPS * 32)
 sigmoid_attention_tiles_kernel(const __nv_bfloat16* __restrict__ q, int q_stride, const __nv_bfloat16* __restrict__ k_cache,

@@ -49,15 +49,6 @@ constexpr int STAGE_BYTES = A_BYTES + STEP_PAGES * PAGE_PIECE;
 constexpr int VALUE_PAGES = 2;               // pages whose values a stage takes
 constexpr uint32_t S_COL = 0, W_COL = 256, O_COL = 384, TMEM_COLS = 512;
 
-__device__ __forceinline__ float fast_exp2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
-    __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&v);
-}
 
 // mixed[h][t][g * D + d] = sum over the heads b of group g of talk[first_head + h, b] * q[t][b][d]
 constexpr int MIX_THREADS = 256;
