@@ -120,8 +120,8 @@ gemm_simt_kernel(const TIn* __restrict__ a, const TIn* __restrict__ w,
 // weights in flight (cp.async; requested before the wait for the kernel in front where the caller says that w was complete
 // before that kernel was launched, as a model's weights are: w_bound); a lane owns a
 // weight row (32 / GROUPS rows a block, the lanes' groups take RPT of the token rows each) and adds k = 0, 1, 2, ... as the
-// tiled kernel does, so the bits are the same. A decode step of a 2-layer model of width 64 (9 such products among 23
-// launches, with all of the path's kernels chained by programmatic dependent launch): 73 -> 62 us.
+// tiled kernel does, so the bits are the same. A decode step of a 2-layer model of width 64 (9 such products among 21
+// kernels, all of the path's chained by programmatic dependent launch): 73 -> 63 us, the host's time; the kernels take 41.
 constexpr int FEW_BK = 64, FEW_STAGES = 4, FEW_LD = FEW_BK + 4, FEW_ROWS = 8;      // (rows of 68 floats: 8 lanes' 16-byte reads meet all 32 banks)
 
 template <int GROUPS, int RPT>
