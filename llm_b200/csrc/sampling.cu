@@ -17,10 +17,12 @@
 //
 // What bounds it: half a megabyte a row through the few SMs that a batch of rows keeps busy. With one block a row
 // (32 rows of 128,256: 32 of 148 SMs, the row read four times at some 100 GB/s an SM) a draw took 62 us. The blocks of a
-// cluster (up to eight: blocks_a_row) each read their share of the row, add their histograms into the first block's shared
-// memory and hand it their candidates, and the first block ranks them and draws. The select stops as soon as the elements
-// not below its bin fit the candidate buffer (after one digit for rows of logits), so the row is read twice. Copying 32
-// rows of 128,256 logits and drawing from them with the default parameters: 76 -> 44 us.
+// cluster (up to eight: blocks_a_row) each read their share of the row, tell each other how many elements they have from
+// their own cut on, gather what can be among the row's top_k and hand it to the first block, which ranks it and draws. The
+// row is read twice (the second time from L1), and two blocks an SM (64 registers a thread) keep the clusters of 32 rows in
+// one wave: with one, 42 us. Copying 32 rows of 128,256 logits and drawing from them with the default parameters: 76 us
+// with one block a row, 44 with the row's histograms summed over the cluster digit by digit, 36 now, of which the copy takes
+// 4.4, the penalty's four dependent reads 3.4, the cuts 4.4, the candidates 4.7, their sort 3.9 and the draw 2.2.
 #include <cooperative_groups.h>
 
 #include "common.cuh"
@@ -34,6 +36,7 @@ constexpr int MAX_TOP_K = 1024;
 constexpr int CANDIDATES = 2048;   // room for ties at the top-k threshold
 constexpr int RADIX_BINS = 2048;   // bins of the widest digit of the radix select
 constexpr int WINDOW = 1024;       // recent tokens the penalty handles in parallel (longer windows: one thread)
+constexpr int WINDOW_BINS = 32;    // bins from a share's cut on whose counts the blocks of a row exchange
 constexpr int CLUSTER = 8;         // most blocks a row (the portable cluster size)
 
 // The blocks of one row: a cluster, whose first block has the row's state and results in its shared memory, or one block.
@@ -88,15 +91,15 @@ __device__ __forceinline__ void for_each_of_row(const float* row, int n, Visit v
         visit(v.z, 4 * q + 2);
         visit(v.w, 4 * q + 3);
     };
-    int q = threadIdx.x;
-    for (; q + 7 * THREADS < quads; q += 8 * THREADS) {
+    for (int q = threadIdx.x; q < quads; q += 8 * THREADS) {
         float4 v[8];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) v[u] = row4[q + u * THREADS];          // eight loads in flight
+        for (int u = 0; u < 8; ++u)
+            if (q + u * THREADS < quads) v[u] = row4[q + u * THREADS];     // eight loads in flight, the last round's too
 #pragma unroll
-        for (int u = 0; u < 8; ++u) visit4(v[u], q + u * THREADS);
+        for (int u = 0; u < 8; ++u)
+            if (q + u * THREADS < quads) visit4(v[u], q + u * THREADS);
     }
-    for (; q < quads; q += THREADS) visit4(row4[q], q);
     for (int i = 4 * quads + threadIdx.x; i < n; i += THREADS) visit(row[i], i);
 }
 
@@ -164,6 +167,8 @@ __global__ void __launch_bounds__(THREADS)
 argmax_rows_kernel(const float* __restrict__ logits, int stride, int vocab, int* __restrict__ out) {
     __shared__ ArgMax scratch[32];
     __shared__ ArgMax gathered[CLUSTER];
+    griddep_wait();
+    logits = behind_wait(logits);
     Team<CLUSTERED> team;
     if constexpr (CLUSTERED) team.sync();                     // every block's shared memory exists from here on
     const int blocks = team.blocks();
@@ -173,9 +178,10 @@ argmax_rows_kernel(const float* __restrict__ logits, int stride, int vocab, int*
 }
 
 // How many blocks share a row. A row of a large vocabulary is long enough for several, as long as they fill no more than the
-// GPU. What a cluster costs a short row is its barriers. The default chain, one block -> as chosen here: 8 rows of 128,256
-// 65 -> 31 us, 32 rows 68 -> 36, 64 rows 71 -> 45, 32 rows of 32,000 33 -> 24; and eight blocks where one is chosen: 256 rows
-// of 128,256 147 -> 258, 148 rows of 32,000 36 -> 81, 1,024 rows of 4,096 82 -> 406.
+// GPU. What a cluster costs a short row is its barriers. The default chain behind a copy of the logits, with the row's
+// histograms summed over the cluster -> as it is now: 8 rows of 128,256 35 -> 25 us, 32 rows 41 -> 31, 64 rows 49 -> 39, 32 rows
+// of 32,000 30 -> 23 (one block a row took 30 more at 8 rows of 128,256). Eight blocks where one is chosen, when that was
+// decided: 256 rows of 128,256 147 -> 258, 148 rows of 32,000 36 -> 81, 1,024 rows of 4,096 82 -> 406.
 static int blocks_a_row(int n_rows, int vocab) {
     if (vocab < 16384) return 1;
     if (n_rows <= 32) return 8;
@@ -188,12 +194,20 @@ static cudaError_t launch_rows(void (*kernel)(Params...), int blocks, int n_rows
     config.gridDim = dim3(n_rows * blocks);
     config.blockDim = dim3(THREADS);
     config.stream = stream;
-    cudaLaunchAttribute attribute[1];
-    attribute[0].id = cudaLaunchAttributeClusterDimension;
-    attribute[0].val.clusterDim.x = blocks;
-    attribute[0].val.clusterDim.y = attribute[0].val.clusterDim.z = 1;
+    cudaLaunchAttribute attribute[2];
+    int n = 0;
+    if (pdl_enabled()) {
+        attribute[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attribute[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (blocks > 1) {
+        attribute[n].id = cudaLaunchAttributeClusterDimension;
+        attribute[n].val.clusterDim.x = blocks;
+        attribute[n].val.clusterDim.y = attribute[n].val.clusterDim.z = 1;
+        ++n;
+    }
     config.attrs = attribute;
-    config.numAttrs = blocks > 1 ? 1 : 0;
+    config.numAttrs = n;
     return cudaLaunchKernelEx(&config, kernel, Params(args)...);
 }
 
@@ -237,6 +251,134 @@ __device__ unsigned block_exclusive_sum(unsigned value, unsigned* warp_totals) {
     return before + inclusive - value;
 }
 
+// The candidates in order: descending by value, ascending by index among equals (a bitonic sort). Up to one a thread they are
+// sorted in registers, and shared memory carries only the exchanges between warps (10 of the 45 steps of 512 candidates).
+__device__ void sort_candidates(float* value, int* index, int count) {
+    const int tid = threadIdx.x;
+    // whether the pair (a at the lower place, b) is in order
+    auto in_order = [](float va, int ia, float vb, int ib) { return va > vb || (va == vb && ia < ib); };
+    int padded = 1;
+    while (padded < count) padded <<= 1;
+    if (padded <= THREADS) {
+        // the warps that have candidates; the others wait at the end
+        const int threads = padded < 32 ? 32 : padded;
+        if (tid < threads) {
+            auto meet = [&]() { asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory"); };
+            float v = tid < count ? value[tid] : -INFINITY;
+            int i = tid < count ? index[tid] : 0x7fffffff;
+            for (int size = 2; size <= padded; size <<= 1) {
+                for (int step = size >> 1; step > 0; step >>= 1) {
+                    float pv;
+                    int pi;
+                    if (step < 32) {
+                        pv = __shfl_xor_sync(0xffffffffu, v, step);
+                        pi = __shfl_xor_sync(0xffffffffu, i, step);
+                    } else {
+                        meet();
+                        value[tid] = v;
+                        index[tid] = i;
+                        meet();
+                        pv = value[tid ^ step];
+                        pi = index[tid ^ step];
+                    }
+                    bool lower = (tid & step) == 0, descending = (tid & size) == 0;
+                    bool ordered = lower ? in_order(v, i, pv, pi) : in_order(pv, pi, v, i);
+                    if (ordered != descending) { v = pv; i = pi; }
+                }
+            }
+            meet();
+            value[tid] = v;
+            index[tid] = i;
+        }
+        __syncthreads();
+        return;
+    }
+    for (int i = count + tid; i < padded; i += THREADS) { value[i] = -INFINITY; index[i] = 0x7fffffff; }
+    __syncthreads();
+    for (int size = 2; size <= padded; size <<= 1) {
+        for (int step = size >> 1; step > 0; step >>= 1) {
+            for (int i = tid; i < padded; i += THREADS) {
+                int partner = i ^ step;
+                if (partner > i) {
+                    bool descending = (i & size) == 0;
+                    float va = value[i], vb = value[partner];
+                    int ia = index[i], ib = index[partner];
+                    if (in_order(va, ia, vb, ib) != descending) {
+                        value[i] = vb; value[partner] = va;
+                        index[i] = ib; index[partner] = ia;
+                    }
+                }
+            }
+            __syncthreads();
+        }
+    }
+}
+
+// The draw among the `kept` sorted candidates, by one warp: softmax, top-p, min-p and the walk. Every sum runs over the
+// candidates one after the other, all lanes alike; the values come 32 at a time from the lanes, so that a step of a chain
+// waits for an addition and not for shared memory. (Places past the end hold zero, which leaves a sum as it is.)
+__device__ int draw(float* value, const int* index, int kept, float top_p, float min_p, unsigned long long* rng) {
+    const int lane = threadIdx.x & 31;
+    auto part = [&](int base, int n) { return base + lane < n ? value[base + lane] : 0.f; };
+    auto sum_of = [&](int n) {
+        float sum = 0.f;
+        for (int base = 0; base < n; base += 32) {
+            float v = part(base, n);
+#pragma unroll
+            for (int j = 0; j < 32; ++j) sum += __shfl_sync(0xffffffffu, v, j);
+        }
+        return sum;
+    };
+    unsigned long long state = *rng;                       // (requested before the sums)
+    float top_value = value[0];
+    __syncwarp();
+    for (int i = lane; i < kept; i += 32) value[i] = expf(value[i] - top_value);
+    __syncwarp();
+    float sum = sum_of(kept);
+    if (sum > 0.f)
+        for (int i = lane; i < kept; i += 32) value[i] /= sum;
+    __syncwarp();
+    if (top_p >= 0.f && top_p < 1.f) {
+        float cumulative = 0.f;
+        int last = -1;
+        for (int base = 0; base < kept && last < 0; base += 32) {
+            float v = part(base, kept);
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+                cumulative += __shfl_sync(0xffffffffu, v, j);
+                if (last < 0 && cumulative > top_p) last = base + j;
+            }
+        }
+        if (last >= 0) kept = min(kept, last + 1);
+    }
+    if (min_p > 0.f) {
+        float cut = value[0] * min_p;
+        int keep = kept;
+        for (int base = 0; base < kept; base += 32) {
+            unsigned below = __ballot_sync(0xffffffffu, base + lane < kept && !(value[base + lane] >= cut));
+            if (below) { keep = base + __ffs(below) - 1; break; }
+        }
+        kept = keep;
+    }
+    float total = sum_of(kept);
+    int pick = 0;
+    if (total > 0.f) {
+        float target = next_uniform(&state) * total;
+        if (lane == 0) *rng = state;
+        int found = -1;
+        for (int base = 0; base < kept && found < 0; base += 32) {
+            float v = part(base, kept);
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+                target -= __shfl_sync(0xffffffffu, v, j);
+                if (found < 0 && base + j < kept && target <= 0.f) found = base + j;
+            }
+        }
+        if (found >= 0) pick = found;
+    }
+    return index[pick];
+}
+
 // params[row] = {temperature, top_p, min_p, repeat_penalty}; iparams[row] =
 // {top_k, repeat_last_n}. recent[row, 0..recent_cap) holds the row's generated
 // tokens as a ring: token number i (counted from 0) is at recent[row, i % cap],
@@ -248,7 +390,7 @@ __device__ unsigned block_exclusive_sum(unsigned value, unsigned* warp_totals) {
 // Block 0 of a row's cluster owns the row's state and draws; the other blocks read their share of the row for the penalty,
 // the histogram and the candidates. Where the chain walks the whole row in index order, one block does and the others leave.
 template <bool CLUSTERED>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(THREADS, 2)
 sample_rows_kernel(float* __restrict__ logits, int stride, int vocab,
                    const float4* __restrict__ params, const int2* __restrict__ iparams,
                    int* __restrict__ recent, int* __restrict__ recent_len,
@@ -260,9 +402,15 @@ sample_rows_kernel(float* __restrict__ logits, int stride, int vocab,
     __shared__ float cand_value[CANDIDATES];
     __shared__ int cand_index[CANDIDATES];
     __shared__ unsigned shared_prefix, shared_need, shared_count, shared_gathered;
+    __shared__ unsigned shared_counts[CLUSTER], window_counts[WINDOW_BINS], shared_windows[CLUSTER * WINDOW_BINS];
+    __shared__ int shared_bins[CLUSTER];       // of the row's blocks: the bin of the first digit that holds a share's top_k-th largest
     __shared__ float block_sums[THREADS];
     __shared__ int window[WINDOW];
     __shared__ ArgMax gathered[CLUSTER];
+    griddep_wait();
+    params = behind_wait(params);
+    iparams = behind_wait(iparams);
+    state_rows = behind_wait(state_rows);
     Team<CLUSTERED> team;
     const int rank = team.rank(), blocks = team.blocks();
 
@@ -275,6 +423,7 @@ sample_rows_kernel(float* __restrict__ logits, int stride, int vocab,
     float temperature = params[row_id].x, top_p = params[row_id].y, min_p = params[row_id].z;
     float penalty = params[row_id].w;
     int top_k = iparams[row_id].x, last_n = iparams[row_id].y;
+    const int held = recent != nullptr && recent_len != nullptr ? recent_len[row_id] : 0;      // (requested together with the parameters)
     int tid = threadIdx.x;
     const Share share = share_of(vocab, rank, blocks);
     // the chains without a ranking (whole row, or refused) run in one block alone, each row in another: where the
@@ -289,9 +438,8 @@ sample_rows_kernel(float* __restrict__ logits, int stride, int vocab,
     auto finish = [&](int token) {
         out[logits_row] = token;
         if (record && recent != nullptr) {
-            int total = recent_len[row_id];
-            recent[(size_t)row_id * recent_cap + (total % recent_cap)] = token;
-            recent_len[row_id] = total + 1;
+            recent[(size_t)row_id * recent_cap + (held % recent_cap)] = token;
+            recent_len[row_id] = held + 1;
         }
     };
 
@@ -299,7 +447,7 @@ sample_rows_kernel(float* __restrict__ logits, int stride, int vocab,
         // A token that occurs c times in the window is penalised c times, one after the other
         // (apps/engine/src/sampler.rs:115-127). One thread per window place; the first place of a
         // token applies all of its c steps, so the arithmetic is that of the serial loop.
-        int total = recent_len[row_id];
+        const int total = held;
         int span = min(min(total, last_n), recent_cap);
         if (span <= WINDOW) {
             for (int t = tid; t < span; t += THREADS)
@@ -331,6 +479,7 @@ sample_rows_kernel(float* __restrict__ logits, int stride, int vocab,
     }
     __syncthreads();
 
+    if (tid == 0) shared_gathered = 0u;
     // every block's shared memory exists, and every block has read the row's state (block 0's finish() changes it)
     if (CLUSTERED && !alone) team.sync();
 
@@ -429,54 +578,144 @@ sample_rows_kernel(float* __restrict__ logits, int stride, int vocab,
         }
         __syncthreads();
     };
-    if (tid == 0) { shared_prefix = 0u; shared_need = (unsigned)top_k; shared_count = 0u; }
     unsigned threshold = 0u;                   // keys of the gathered elements are not below it
     int digit = 0;                             // digits the threshold has
-    for (; digit < 3;) {
-        const int shift = bits(digit), n_bins = digit == 2 ? 1024 : 2048;
+    bool gathered_all = false;
+    if constexpr (CLUSTERED) {
+        // Each block alone: the bin of the first digit down to which its own share has top_k elements, its cut. The row's cut is
+        // no lower than any share's. Every block tells the others its cut and how many elements it has from there on and
+        // from each of the bins above; all then know a bin down to which the row has top_k elements (counts past the window are
+        // taken for zero, which lowers it at most), and everything down to it holds all that the row's select would keep,
+        // ties included: some eighty elements of a row of logits. Three exchanges between the blocks instead of the six of
+        // the row's select, which follows where they do not fit the buffer (rows that are mostly one value).
         for (int i = tid; i < RADIX_BINS; i += THREADS) histogram[i] = 0u;
-        team.sync();                        // (block 0's bins are zero before the others add to them)
-        unsigned mask = digit == 0 ? 0u : (0xffffffffu << bits(digit - 1));
+        if (tid == 0) shared_prefix = 0u;
+        __syncthreads();
         for_each_of_row(row + share.begin, share.end - share.begin, [&](float v, int) {
-            unsigned key = ordered_key(v * inverse);
-            if ((key & mask) == threshold) atomicAdd(&histogram[(key >> shift) & (unsigned)(n_bins - 1)], 1u);
+            atomicAdd(&histogram[ordered_key(v * inverse) >> 21], 1u);
         });
         __syncthreads();
-        if (rank != 0) {
-            unsigned* sums = team.of(histogram, 0);
-            for (int i = tid; i < n_bins; i += THREADS)
-                if (histogram[i]) atomicAdd(&sums[i], histogram[i]);
+        int top_bin = RADIX_BINS - 1 - 4 * tid;                   // as in pick_bin
+        unsigned mine = histogram[top_bin] + histogram[top_bin - 1] + histogram[top_bin - 2] + histogram[top_bin - 3];
+        unsigned before = block_exclusive_sum(mine, block_sums_u);
+        if (before < (unsigned)top_k && before + mine >= (unsigned)top_k) {
+            int bin = top_bin;
+            for (unsigned have = before + histogram[bin]; have < (unsigned)top_k; have += histogram[bin]) --bin;
+            shared_prefix = (unsigned)bin;
         }
-        team.sync();
-        if (rank == 0) {
-            pick_bin(digit);
-            if (tid < blocks && tid > 0) {
-                *team.of(&shared_prefix, tid) = shared_prefix;
-                *team.of(&shared_count, tid) = shared_count;
+        __syncthreads();
+        // the number of elements from each bin of this thread's four on, into the window behind the cut
+        const int cut = (int)shared_prefix;
+        if (tid < WINDOW_BINS) window_counts[tid] = 0u;
+        __syncthreads();
+        if (top_bin >= cut) {
+            unsigned from = before;
+            for (int bin = top_bin; bin > top_bin - 4; --bin) {
+                from += histogram[bin];
+                if (bin >= cut && bin < cut + WINDOW_BINS) window_counts[bin - cut] = from;
             }
         }
+        __syncthreads();
+        if (tid < blocks * WINDOW_BINS) {
+            const int to = tid / WINDOW_BINS, at = tid % WINDOW_BINS;
+            team.of(shared_windows, to)[rank * WINDOW_BINS + at] = window_counts[at];
+            if (at == 0) team.of(shared_bins, to)[rank] = cut;
+        }
         team.sync();
-        threshold = shared_prefix;
-        ++digit;
-        if (shared_count <= (unsigned)CANDIDATES) break;
-    }
-    LLMB_STAMP(2, 0);                                 // the radix select has its threshold
-    if (rank == 0 && tid == 0) shared_gathered = 0u;     // now the number of candidates
-    team.sync();
-    {
-        unsigned* at_ = team.of(&shared_gathered, 0);
-        float* values = team.of(cand_value, 0);
-        int* indices = team.of(cand_index, 0);
+        LLMB_STAMP(2, 0);                             // the shares have their cuts
+        int bin = 0;
+        for (int r = 0; r < blocks; ++r) bin = max(bin, shared_bins[r]);
+        if ((tid & 31) < WINDOW_BINS) {               // a lane a bin from there on: the highest that has top_k elements
+            unsigned have = 0u;
+            for (int r = 0; r < blocks; ++r) {
+                int at = bin + (tid & 31) - shared_bins[r];
+                if (at < WINDOW_BINS) have += shared_windows[r * WINDOW_BINS + at];
+            }
+            unsigned enough = __ballot_sync(0xffffffffu, have >= (unsigned)top_k);
+            if (enough) bin += 31 - __clz(enough);
+        }
+        threshold = (unsigned)bin << 21;
+        // each block gathers its own, and the first block fetches what the others have (a counter and a buffer in the first
+        // block's memory that all blocks write to took some 10 us for 450 candidates)
         for_each_of_row(row + share.begin, share.end - share.begin, [&](float v, int i) {
             v *= inverse;
             if (ordered_key(v) >= threshold) {
-                unsigned at = atomicAdd(at_, 1u);
-                if (at < CANDIDATES) { values[at] = v; indices[at] = share.begin + i; }
+                unsigned at = atomicAdd(&shared_gathered, 1u);
+                if (at < CANDIDATES) { cand_value[at] = v; cand_index[at] = share.begin + i; }
             }
         });
+        __syncthreads();
+        if (tid < blocks) team.of(shared_counts, tid)[rank] = shared_gathered;
+        team.sync();
+        unsigned total = 0u;
+        for (int r = 0; r < blocks; ++r) total += shared_counts[r];
+        gathered_all = total <= (unsigned)CANDIDATES;
+        if (gathered_all) {
+            if (rank == 0) {
+                unsigned own = shared_counts[0];
+                for (unsigned i = own + tid; i < total; i += THREADS) {
+                    unsigned at = i - own;
+                    int r = 1;
+                    while (at >= shared_counts[r]) at -= shared_counts[r++];
+                    cand_value[i] = team.of(cand_value, r)[at];
+                    cand_index[i] = team.of(cand_index, r)[at];
+                }
+            }
+            team.sync();                       // the others' memory has been read
+            if (rank != 0) return;
+            if (tid == 0) shared_gathered = total;
+            __syncthreads();
+        }
+        threshold = 0u;
     }
-    team.sync();
-    if (rank != 0) return;
+    if (tid == 0) { shared_prefix = 0u; shared_need = (unsigned)top_k; shared_count = 0u; }
+    if (!gathered_all) {
+        for (; digit < 3;) {
+            const int shift = bits(digit), n_bins = digit == 2 ? 1024 : 2048;
+            for (int i = tid; i < RADIX_BINS; i += THREADS) histogram[i] = 0u;
+            team.sync();                        // (block 0's bins are zero before the others add to them)
+            unsigned mask = digit == 0 ? 0u : (0xffffffffu << bits(digit - 1));
+            for_each_of_row(row + share.begin, share.end - share.begin, [&](float v, int) {
+                unsigned key = ordered_key(v * inverse);
+                if ((key & mask) == threshold) atomicAdd(&histogram[(key >> shift) & (unsigned)(n_bins - 1)], 1u);
+            });
+            __syncthreads();
+            if (rank != 0) {
+                unsigned* sums = team.of(histogram, 0);
+                for (int i = tid; i < n_bins; i += THREADS)
+                    if (histogram[i]) atomicAdd(&sums[i], histogram[i]);
+            }
+            team.sync();
+            if (rank == 0) {
+                pick_bin(digit);
+                if (tid < blocks && tid > 0) {
+                    *team.of(&shared_prefix, tid) = shared_prefix;
+                    *team.of(&shared_count, tid) = shared_count;
+                }
+            }
+            team.sync();
+            threshold = shared_prefix;
+            ++digit;
+            if (shared_count <= (unsigned)CANDIDATES) break;
+        }
+        LLMB_STAMP(2, 0);                                 // the radix select has its threshold
+        if (rank == 0 && tid == 0) shared_gathered = 0u;     // now the number of candidates
+        team.sync();
+        {
+            unsigned* at_ = team.of(&shared_gathered, 0);
+            float* values = team.of(cand_value, 0);
+            int* indices = team.of(cand_index, 0);
+            for_each_of_row(row + share.begin, share.end - share.begin, [&](float v, int i) {
+                v *= inverse;
+                if (ordered_key(v) >= threshold) {
+                    unsigned at = atomicAdd(at_, 1u);
+                    if (at < CANDIDATES) { values[at] = v; indices[at] = share.begin + i; }
+                }
+            });
+        }
+        team.sync();
+        if (rank != 0) return;
+    }
     LLMB_STAMP(3, 0);                                 // the candidates are gathered
     int count = (int)min(shared_gathered, (unsigned)CANDIDATES);
     if (shared_gathered > (unsigned)CANDIDATES) {
@@ -484,13 +723,14 @@ sample_rows_kernel(float* __restrict__ logits, int stride, int vocab,
         if (tid == 0) { status[row_id] = 1; finish(0); }
         return;
     }
-    if (digit < 3) {
-        // the digits that are left, among the candidates; then those below the whole threshold go
+    if (digit < 3 && count > THREADS) {
+        // more than a sort in registers takes: the digits that are left, among the candidates; then those below the whole
+        // threshold go
         for (; digit < 3; ++digit) {
             const int shift = bits(digit), n_bins = digit == 2 ? 1024 : 2048;
             for (int i = tid; i < RADIX_BINS; i += THREADS) histogram[i] = 0u;
             __syncthreads();
-            unsigned prefix = shared_prefix, mask = 0xffffffffu << bits(digit - 1);
+            unsigned prefix = shared_prefix, mask = digit == 0 ? 0u : (0xffffffffu << bits(digit - 1));
             for (int i = tid; i < count; i += THREADS) {
                 unsigned key = ordered_key(cand_value[i]);
                 if ((key & mask) == prefix) atomicAdd(&histogram[(key >> shift) & (unsigned)(n_bins - 1)], 1u);
@@ -520,72 +760,12 @@ sample_rows_kernel(float* __restrict__ logits, int stride, int vocab,
         __syncthreads();
         count = (int)shared_count;
     }
-    // bitonic sort, descending by value, ascending by index among equals
-    int padded = 1;
-    while (padded < count) padded <<= 1;
-    for (int i = count + tid; i < padded; i += THREADS) { cand_value[i] = -INFINITY; cand_index[i] = 0x7fffffff; }
-    __syncthreads();
-    for (int size = 2; size <= padded; size <<= 1) {
-        for (int step = size >> 1; step > 0; step >>= 1) {
-            for (int i = tid; i < padded; i += THREADS) {
-                int partner = i ^ step;
-                if (partner > i) {
-                    bool descending = (i & size) == 0;
-                    float va = cand_value[i], vb = cand_value[partner];
-                    int ia = cand_index[i], ib = cand_index[partner];
-                    bool a_first = va > vb || (va == vb && ia < ib);
-                    if (a_first != descending) {
-                        cand_value[i] = vb; cand_value[partner] = va;
-                        cand_index[i] = ib; cand_index[partner] = ia;
-                    }
-                }
-            }
-            __syncthreads();
-        }
-    }
+    sort_candidates(cand_value, cand_index, count);
     LLMB_STAMP(4, 0);                                 // the candidates are sorted
-    int kept = min(count, top_k);
-    float top_value = cand_value[0];
-    for (int i = tid; i < kept; i += THREADS) cand_value[i] = expf(cand_value[i] - top_value);
-    __syncthreads();
-    if (tid == 0) {
-        float sum = 0.f;
-        for (int i = 0; i < kept; ++i) sum += cand_value[i];
-        block_sums[0] = sum;
-    }
-    __syncthreads();
-    if (float sum = block_sums[0]; sum > 0.f)
-        for (int i = tid; i < kept; i += THREADS) cand_value[i] /= sum;
-    __syncthreads();
-    if (tid == 0) {
-        if (top_p >= 0.f && top_p < 1.f) {
-            float cumulative = 0.f;
-            for (int i = 0; i < kept; ++i) {
-                cumulative += cand_value[i];
-                if (cumulative > top_p) { kept = i + 1; break; }
-            }
-        }
-        if (min_p > 0.f) {
-            float cut = cand_value[0] * min_p;
-            int keep = 0;
-            while (keep < kept && cand_value[keep] >= cut) ++keep;
-            kept = keep;
-        }
-        float total = 0.f;
-        for (int i = 0; i < kept; ++i) total += cand_value[i];
-        int pick = cand_index[0];
-        if (total > 0.f) {
-            unsigned long long state = rng[row_id];
-            float target = next_uniform(&state) * total;
-            rng[row_id] = state;
-            for (int i = 0; i < kept; ++i) {
-                target -= cand_value[i];
-                if (target <= 0.f) { pick = cand_index[i]; break; }
-            }
-        }
-        finish(pick);
-        LLMB_STAMP(5, 0);                             // the token is drawn
-    }
+    if (tid >= 32) return;
+    int token = draw(cand_value, cand_index, min(count, top_k), top_p, min_p, rng + row_id);
+    if (tid == 0) finish(token);
+    LLMB_STAMP(5, 0);                                 // the token is drawn
 }
 
 // The stamps of the last sampling launch in a build with -DLLMB_TRACE (see common.cuh); 1 otherwise.

@@ -746,6 +746,30 @@ def test_sample_rows_over_a_cluster(vocab, steps):
             assert state_gpu[4][r] == state_cpu[4][r].to(DEV) and state_gpu[2][r].tolist() == state_cpu[2][r].tolist()
 
 
+@pytest.mark.parametrize("allowed", [3, 39, 41, 700, 5000])
+def test_sample_rows_of_mostly_masked_logits(allowed):
+    """Rows that are -inf but for a few entries, all of them in one block's share or spread: the shares' own cuts then lie at
+    -inf, and where that is all a row has, its select runs over the whole row (or is refused for its ties, as before)."""
+    vocab, n = 128256, 4
+    params = [[0.7, 0.75, 0.25, 1.1], [1.0, 0.9, 0.0, 1.0], [1.3, 2.0, 0.1, 1.0], [0.8, 0.95, 0.0, 1.0]]
+    state_gpu = _sampler_state(n, params, [[40, 8], [1, 0], [600, 0], [40, 8]], [3, 4, 5, 6])
+    state_cpu = [t.cpu().clone() for t in state_gpu]
+    full = randn(n, vocab, seed=320, scale=2.0)
+    places = torch.randperm(vocab, generator=torch.Generator().manual_seed(allowed))[:allowed]
+    logits = torch.full_like(full, float("-inf"))
+    logits[:2, :allowed] = full[:2, :allowed]
+    logits[2:, places.to(DEV)] = full[2:, :allowed]
+    cpu_logits = logits.cpu().clone()
+    ops().sample_rows(logits, *state_gpu, record=True)
+    plain_ops.sample_rows(cpu_logits, *state_cpu, record=True)
+    for r, k in enumerate((40, 1, 600, 40)):
+        if k > allowed:
+            assert int(state_gpu[6][r]) == 1, r              # more than 2,048 equal ones at the cut
+        else:
+            assert int(state_gpu[6][r]) == 0 and int(state_gpu[5][r]) == int(state_cpu[5][r]), r
+            assert state_gpu[4][r] == state_cpu[4][r].to(DEV), r
+
+
 @pytest.mark.parametrize("rows,vocab", [(1, 1), (3, 7), (2, 33), (5, 4099), (33, 128256)])
 def test_argmax_over_a_cluster(rows, vocab):
     """First maximum over the blocks' shares, also with equal maxima in several shares and rows of -inf and NaN."""
