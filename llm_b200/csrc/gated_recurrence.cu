@@ -9,8 +9,9 @@
 //     out[t, c] = out_scale * S[t, c] * gelu(y[t, c])                              (tanh form of gelu)
 //
 // x and y are the two branches' projections (with their biases) in the run's dtype. Everything between
-// reading them and rounding `out` is 32-bit: the convolution's sum, both gates' matrix products (on the
-// CUDA cores, fixed order of summation per output), the decay, the recurrence and S.
+// reading them and rounding `out` is 32-bit: the convolution's sum, both gates' matrix products (fixed order of
+// summation per output; where the matrices are bfloat16 numbers on the tensor cores, of exact products), the decay, the
+// recurrence and S.
 //
 // Per sequence the cache holds state[slot] = [taps, C] float32: rows 0 .. taps - 2 are the last taps - 1
 // inputs x (oldest first), the last row is S. A slot's state is zeroed when the slot is taken, which is
@@ -34,9 +35,10 @@
 // new S of sequences that end in it and their convolution rows. The sums are the same up to rounding
 // (a chunk's start value is formed from the chunk before it as a whole); short steps, and so every decode
 // step, keep the token order exactly.
-#include "common.cuh"
+#include "tc.cuh"
 
 using namespace llmb;
+using namespace llmb::tc;
 
 LLMB_DEFINE_LAST_ERROR(llmb_gated_recurrence)
 
@@ -245,6 +247,225 @@ gates_kernel(const float* __restrict__ u, int channels, const float* __restrict_
             decay[(size_t)t * channels + c] = a;
             drive[(size_t)t * channels + c] = sqrtf(1.0f - a * a) * g * uc;
         }
+    }
+}
+
+// ------------------------------------------------------------------------- both gates on the tensor cores
+// For matrices whose values are bfloat16 (a checkpoint in bfloat16, held in 32 bits): the 32-bit inputs u are taken apart
+// instead of rounded. u = hi + mid + lo with bfloat16 parts of 8 bits each is exact (each part is cut off, not rounded),
+// every product of a part with a weight is exact in 32 bits, and the tensor core adds them in 32 bits, hi's products in one
+// accumulator and those of mid and lo, which are 2^-8 of them, in another, so that hi's chain stays short. One block an SM
+// takes units of 128 tokens x 64 channels of one part, both gates of a channel side by side (128 columns):
+//
+// * warps 0-7: epilogue. A warp reads 32 tokens of 32 channels from tensor memory, forms the gates, a and the driving term.
+// * warps 8-11: take u apart, a k-block of 64 at a time, into three swizzled tiles of 128 x 64.
+// * warp 12, one lane: TMA loads of the weights' tile (128 rows x 64). Warp 13, one lane: the products.
+//
+// Bound by the epilogue's exponentials, divisions and roots (8 warps an SM) and the taking apart of u, which every group of 64
+// channels of a part does again. 4,096 channels in 16 parts, the gates_kernel of the CUDA cores -> here, whole calls: 2,500 tokens
+// 411 -> 202 us, 600 151 -> 76, 129 70 -> 41, 64 sequences of one token 27 -> 23, one token 22 -> 18; a is 5.0e-8 away from 64
+// bits (5.3e-8 there), the driving term 9.3e-8 (9.9e-8).
+//
+// gate_rows: bfloat16 [2 C, P]: per group of 64 channels of a part, its 64 rows of gate_a, then its 64 rows of gate_i.
+constexpr int TC_TOKENS = 128, TC_CHANNELS = 64, TC_K = 64, TC_STAGES = 3;
+constexpr int TC_EPILOGUE_WARPS = 8, TC_SPLIT_WARPS = 4, TC_THREADS = (TC_EPILOGUE_WARPS + TC_SPLIT_WARPS + 2) * 32;
+constexpr int TC_TILE = 128 * TC_K * 2;                           // bytes of a tile of bfloat16, of u's parts or of weights
+constexpr int TC_STAGE = 4 * TC_TILE;                             // hi | mid | lo | weights
+constexpr int TC_COLS = 2 * TC_CHANNELS;                          // columns of an accumulator: both gates
+
+__device__ __forceinline__ uint32_t high_halves(float a, float b) {      // the top 16 bits of both, a's in the low half
+    return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
+}
+// v minus its top 16 bits: exact. An infinity has no rest.
+__device__ __forceinline__ float below_high(float v) {
+    float rest = v - __uint_as_float(__float_as_uint(v) & 0xffff0000u);
+    return fabsf(v) == INFINITY ? 0.f : rest;
+}
+
+__global__ void __launch_bounds__(TC_THREADS, 1)
+gates_tc_kernel(const __grid_constant__ CUtensorMap map_rows, const float* __restrict__ u, int channels,
+                const float* __restrict__ gate_a_bias, const float* __restrict__ gate_i_bias, int part,
+                const float* __restrict__ rate, float* __restrict__ decay, float* __restrict__ drive, int n_tokens,
+                int n_units, int* status) {
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    unsigned char* tiles = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    __shared__ uint64_t full_bar[TC_STAGES], empty_bar[TC_STAGES], acc_full_bar[2], acc_empty_bar[2];
+    __shared__ uint32_t tmem_slot;
+    __shared__ volatile int abort_flag;
+    int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    griddep_launch();
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < TC_STAGES; ++s) {
+            mbar_init(smem_u32(&full_bar[s]), TC_SPLIT_WARPS + 1);
+            mbar_init(smem_u32(&empty_bar[s]), 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(smem_u32(&acc_full_bar[b]), 1);
+            mbar_init(smem_u32(&acc_empty_bar[b]), TC_EPILOGUE_WARPS);
+        }
+        abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        fence_async_shared();
+    }
+    if (warp == 13) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&tmem_slot)) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tcgen05_fence_before();
+    __syncthreads();
+    tcgen05_fence_after();
+    const uint32_t tmem = tmem_slot;
+    griddep_wait();
+    u = behind_wait(u);
+    gate_a_bias = behind_wait(gate_a_bias);
+    gate_i_bias = behind_wait(gate_i_bias);
+    rate = behind_wait(rate);
+
+    // units: the groups of 64 channels run fastest, so that the blocks at work share the tokens' rows in L2
+    const int groups = channels / TC_CHANNELS, kblocks = part / TC_K;
+    if (warp < TC_EPILOGUE_WARPS) {
+        const int quarter = warp & 3, half = warp >> 2;
+        uint32_t n_done = 0;
+        for (int unit = blockIdx.x; unit < n_units; unit += gridDim.x, ++n_done) {
+            uint32_t buffer = n_done & 1, use = n_done >> 1;
+            int t = unit / groups * TC_TOKENS + quarter * 32 + lane, c0 = unit % groups * TC_CHANNELS + half * 32;
+            if (!mbar_wait(smem_u32(&acc_full_bar[buffer]), use & 1, &abort_flag, status, 3)) break;
+            tcgen05_fence_after();
+            uint32_t at = tmem + ((uint32_t)(quarter * 32) << 16) + buffer * (2 * TC_COLS) + half * 32;
+#pragma unroll 1
+            for (int c = 0; c < 32; c += 16) {
+                uint32_t a_hi[16], a_low[16], i_hi[16], i_low[16];
+                tmem_ld16(at + c, a_hi);
+                tmem_ld16(at + TC_CHANNELS + c, i_hi);
+                tmem_ld16(at + TC_COLS + c, a_low);
+                tmem_ld16(at + TC_COLS + TC_CHANNELS + c, i_low);
+                if (t < n_tokens) {
+                    size_t place = (size_t)t * channels + c0 + c;
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        float4 uc = *reinterpret_cast<const float4*>(u + place + 4 * q);
+                        float4 ba = *reinterpret_cast<const float4*>(gate_a_bias + c0 + c + 4 * q);
+                        float4 bi = *reinterpret_cast<const float4*>(gate_i_bias + c0 + c + 4 * q);
+                        float4 r4 = *reinterpret_cast<const float4*>(rate + c0 + c + 4 * q);
+                        const float us[4] = {uc.x, uc.y, uc.z, uc.w}, bas[4] = {ba.x, ba.y, ba.z, ba.w};
+                        const float bis[4] = {bi.x, bi.y, bi.z, bi.w}, rates[4] = {r4.x, r4.y, r4.z, r4.w};
+                        float as[4], ds[4];
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            float sa = __uint_as_float(a_hi[4 * q + e]) + __uint_as_float(a_low[4 * q + e]);
+                            float si = __uint_as_float(i_hi[4 * q + e]) + __uint_as_float(i_low[4 * q + e]);
+                            float r = 1.0f / (1.0f + expf(-(sa + bas[e])));
+                            float g = 1.0f / (1.0f + expf(-(si + bis[e])));
+                            as[e] = expf(rates[e] * r);
+                            ds[e] = sqrtf(1.0f - as[e] * as[e]) * g * us[e];
+                        }
+                        *reinterpret_cast<float4*>(decay + place + 4 * q) = make_float4(as[0], as[1], as[2], as[3]);
+                        *reinterpret_cast<float4*>(drive + place + 4 * q) = make_float4(ds[0], ds[1], ds[2], ds[3]);
+                    }
+                }
+                __syncwarp();
+            }
+            tcgen05_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&acc_empty_bar[buffer]));
+        }
+    } else if (warp < TC_EPILOGUE_WARPS + TC_SPLIT_WARPS) {
+        // a thread takes 8 neighbouring values of 8 tokens (16 apart) a k-block, requested before the stage is free
+        const int thread = (int)threadIdx.x - TC_EPILOGUE_WARPS * 32, piece = thread & 7, row0 = thread >> 3;
+        int s = 0;
+        uint32_t phase = 0;
+        bool ok = true;
+        for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x) {
+            int t0 = unit / groups * TC_TOKENS, first = unit % groups * TC_CHANNELS / part * part;
+            for (int kb = 0; kb < kblocks; ++kb) {
+                float4 v[8][2];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    int t = t0 + row0 + 16 * i;
+                    const float4* from = reinterpret_cast<const float4*>(u + (size_t)t * channels + first + kb * TC_K + piece * 8);
+                    v[i][0] = t < n_tokens ? from[0] : make_float4(0.f, 0.f, 0.f, 0.f);
+                    v[i][1] = t < n_tokens ? from[1] : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+                ok = mbar_wait(smem_u32(&empty_bar[s]), phase ^ 1, &abort_flag, status, 1);
+                if (!ok) break;
+                unsigned char* to = tiles + s * TC_STAGE;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    int row = row0 + 16 * i;
+                    float x[8] = {v[i][0].x, v[i][0].y, v[i][0].z, v[i][0].w, v[i][1].x, v[i][1].y, v[i][1].z, v[i][1].w};
+#pragma unroll
+                    for (int p = 0; p < 3; ++p) {
+                        uint4 packed = make_uint4(high_halves(x[0], x[1]), high_halves(x[2], x[3]),
+                                                  high_halves(x[4], x[5]), high_halves(x[6], x[7]));
+                        // rows of 128 bytes, the 16-byte piece at place piece ^ (row % 8): the 128-byte swizzle
+                        *reinterpret_cast<uint4*>(to + p * TC_TILE + row * 128 + ((piece ^ (row & 7)) << 4)) = packed;
+                        if (p < 2) {
+#pragma unroll
+                            for (int e = 0; e < 8; ++e) x[e] = below_high(x[e]);
+                        }
+                    }
+                }
+                fence_async_shared();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&full_bar[s]));
+                if (++s == TC_STAGES) { s = 0; phase ^= 1; }
+            }
+        }
+    } else if (warp == 12) {
+        if (lane == 0) {
+            int s = 0;
+            uint32_t phase = 0;
+            bool ok = true;
+            for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x) {
+                int row = unit % groups * TC_COLS;
+                for (int kb = 0; kb < kblocks; ++kb) {
+                    ok = mbar_wait(smem_u32(&empty_bar[s]), phase ^ 1, &abort_flag, status, 1);
+                    if (!ok) break;
+                    mbar_expect_tx(smem_u32(&full_bar[s]), TC_TILE);
+                    tma_load_2d(smem_u32(tiles + s * TC_STAGE + 3 * TC_TILE), &map_rows, smem_u32(&full_bar[s]), kb * TC_K, row);
+                    if (++s == TC_STAGES) { s = 0; phase ^= 1; }
+                }
+            }
+        }
+    } else if (lane == 0) {
+        // D 32-bit, A and B bfloat16, both K-major, M = 128, N = 128
+        constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TC_COLS >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+        int s = 0;
+        uint32_t phase = 0, n_done = 0;
+        bool ok = true;
+        for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x, ++n_done) {
+            uint32_t buffer = n_done & 1, use = n_done >> 1, hi = tmem + buffer * (2 * TC_COLS), low = hi + TC_COLS;
+            ok = mbar_wait(smem_u32(&acc_empty_bar[buffer]), (use & 1) ^ 1, &abort_flag, status, 4);
+            if (!ok) break;
+            tcgen05_fence_after();
+            for (int kb = 0; kb < kblocks; ++kb) {
+                ok = mbar_wait(smem_u32(&full_bar[s]), phase, &abort_flag, status, 2);
+                if (!ok) break;
+                tcgen05_fence_after();
+                uint64_t x = smem_desc(smem_u32(tiles + s * TC_STAGE)), w = x + (uint64_t)(3 * (TC_TILE >> 4));
+#pragma unroll
+                for (int k = 0; k < TC_K / 16; ++k) {
+                    tcgen05_mma(low, x + (uint64_t)(2 * (TC_TILE >> 4)) + 2 * k, w + 2 * k, idesc, kb > 0 || k > 0);
+                    tcgen05_mma(low, x + (uint64_t)(TC_TILE >> 4) + 2 * k, w + 2 * k, idesc, 1u);
+                    tcgen05_mma(hi, x + 2 * k, w + 2 * k, idesc, kb > 0 || k > 0);
+                }
+                tcgen05_commit(smem_u32(&empty_bar[s]));
+                if (++s == TC_STAGES) { s = 0; phase ^= 1; }
+            }
+            if (ok) tcgen05_commit(smem_u32(&acc_full_bar[buffer]));
+        }
+    }
+    __syncwarp();
+    tcgen05_fence_before();
+    __syncthreads();
+    if (abort_flag) {
+        // let copies that are still in flight land before shared memory is given up
+        for (int i = 0; i < 100; ++i) __nanosleep(10000);
+        __syncthreads();
+    }
+    if (warp == 13) {
+        tcgen05_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
     }
 }
 
@@ -457,14 +678,24 @@ scan_apply_kernel(const T* __restrict__ y, int y_stride, const T* __restrict__ x
     }
 }
 
-// work [3, T, C] float32: u, a, the driving term.
+// 0 if nothing went wrong since the last call of this function; else the code of the wait that ran out (1 operands, 2 products,
+// 3 epilogue, 4 accumulator). Call after a synchronisation.
+LLMB_EXPORT int llmb_gated_recurrence_status() {
+    int* s = status_word();
+    if (!s) return -1;
+    int v = *s;
+    *s = 0;
+    return v;
+}
+
+// work [3, T, C] float32: u, a, the driving term. gate_rows: both gates' rows in bfloat16 as gates_tc_kernel reads them, or nullptr.
 LLMB_EXPORT int llmb_gated_recurrence(const void* y, int y_stride, const void* x, int x_stride, int dtype,
                                       const float* conv_w, const float* conv_b, int taps, const float* gate_a,
                                       const float* gate_a_bias, const float* gate_i, const float* gate_i_bias,
                                       int blocks, const float* rate, float* state, const int* tok_seq,
                                       const int* cu_seqlens, const int* slot_ids, void* out, int out_stride,
                                       float out_scale, float* work, int n_tokens, int channels, int n_seqs,
-                                      int single_tokens, cudaStream_t stream) {
+                                      int single_tokens, const void* gate_rows, cudaStream_t stream) {
     if (n_tokens == 0) return LLMB_OK;
     LLMB_REQUIRE(taps >= 1 && taps <= MAX_TAPS, "gated_recurrence: %d taps (1 to %d are built)", taps, MAX_TAPS);
     LLMB_REQUIRE(channels > 0 && blocks > 0 && channels % blocks == 0 && n_seqs > 0,
@@ -478,6 +709,25 @@ LLMB_EXPORT int llmb_gated_recurrence(const void* y, int y_stride, const void* x
     float* decay = work + (size_t)n_tokens * channels;
     float* drive = decay + (size_t)n_tokens * channels;
     auto gates = long_step ? gates_kernel<8> : gates_kernel<2>;
+    bool on_tensor_cores = gate_rows && part % TC_CHANNELS == 0 &&
+                           (((size_t)gate_rows | (size_t)work | (size_t)gate_a_bias | (size_t)gate_i_bias | (size_t)rate) % 16) == 0;
+    const size_t tc_smem = 1024 + (size_t)TC_STAGES * TC_STAGE;
+    int n_units = ceil_div(n_tokens, TC_TOKENS) * (channels / TC_CHANNELS);
+    static int n_sms = 0;
+    CUtensorMap map_rows;
+    int* status_dev = nullptr;
+    if (on_tensor_cores) {
+        if (n_sms == 0) {
+            int device = 0, count = 0;
+            LLMB_CUDA(cudaGetDevice(&device));
+            LLMB_CUDA(cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, device));
+            LLMB_CUDA(cudaFuncSetAttribute(gates_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc_smem));
+            n_sms = count;
+        }
+        int code = make_map_2d(&map_rows, gate_rows, 2LL * channels, part, part, TC_K, 128);
+        if (code) return code;
+        if (int* word = status_word()) cudaHostGetDevicePointer((void**)&status_dev, word, 0);
+    }
 #define LLMB_RECURRENCE(T)                                                                                          \
     do {                                                                                                            \
         ConvSource<T> source{(const T*)x, x_stride, state, conv_w, conv_b, taps, channels};                         \
@@ -488,6 +738,11 @@ LLMB_EXPORT int llmb_gated_recurrence(const void* y, int y_stride, const void* x
         } else                                                                                                      \
             LLMB_CUDA(llmb::launch(conv_kernel<T>, dim3(n_tokens, ceil_div(channels, 256)), dim3(256), 0, stream,   \
                                    true, source, tok_seq, cu_seqlens, slot_ids, u));                                \
+        if (on_tensor_cores)                                                                                        \
+            LLMB_CUDA(llmb::launch(gates_tc_kernel, dim3(n_units < n_sms ? n_units : n_sms), dim3(TC_THREADS), tc_smem, stream, \
+                                   true, map_rows, (const float*)u, channels, gate_a_bias, gate_i_bias, part, rate, \
+                                   decay, drive, n_tokens, n_units, status_dev));                                   \
+        else                                                                                                        \
         /* launched plainly, so that its blocks find the SMs empty: put down while the convolution drains, several of them \
            share an SM (64 sequences of one token, 4,096 channels: 49 us in all dependent, 26 plainly) */          \
         LLMB_CUDA(llmb::launch(gates, grid_gates, dim3(256), 0, stream, false, (const float*)u, channels, gate_a,    \

@@ -1094,7 +1094,7 @@ def check_device_status() -> None:
     reads a word of host memory); meaningful after the stream was synchronised."""
     from .build import _loaded
     for name in ("gemm_tc", "attention_prefill_tc", "routed_experts", "latent_prefill_tc", "latent_attention",
-                 "sigmoid_attention_tc", "diff_attention_tc"):
+                 "sigmoid_attention_tc", "diff_attention_tc", "gated_recurrence"):
         if name in _loaded:
             code = getattr(_loaded[name], f"llmb_{name}_status")()
             if code != 0:
@@ -1705,8 +1705,22 @@ def sigmoid_attention(q, k_cache, v_cache, block_table, ring_pages, tok_pos, tok
     return out
 
 
+GATE_GROUP = 64                                 # channels whose rows of both gates lie together in gate_rows
+
+
+def gate_rows_of(gate_a, gate_i):
+    """Both gate matrices (float32 [blocks, P, P]) as gated_recurrence's tensor-core kernel reads them: bfloat16
+    [2 blocks P, P], per 64 channels their rows of gate_a and then of gate_i. None where P is no multiple of 64 or a value is
+    not a bfloat16 number (then the gates are summed from the 32-bit matrices)."""
+    blocks, part, _ = gate_a.shape
+    rows = torch.stack([g.to(torch.bfloat16) for g in (gate_a, gate_i)], dim=1)                # [blocks, 2, P, P]
+    if part % GATE_GROUP or not torch.equal(rows.float(), torch.stack([gate_a, gate_i], dim=1)):
+        return None
+    return rows.view(blocks, 2, part // GATE_GROUP, GATE_GROUP, part).transpose(1, 2).reshape(2 * blocks * part, part).contiguous()
+
+
 def gated_recurrence(y, x, conv_w, conv_b, gate_a, gate_a_bias, gate_i, gate_i_bias, rate, state, tok_seq,
-                     cu_seqlens, slot_ids, out, out_scale, work, single_tokens=False):
+                     cu_seqlens, slot_ids, out, out_scale, work, single_tokens=False, gate_rows=None):
     """A real-gated linear recurrence behind a short causal convolution, on C channels. `y`, `x`
     [T, C] (the run's dtype; rows contiguous, may be column ranges): the two branches' projections
     with their biases. u = conv_b + sum_j conv_w[:, j] * x[t - (taps - 1) + j] over the tokens of
@@ -1718,9 +1732,11 @@ def gated_recurrence(y, x, conv_w, conv_b, gate_a, gate_a_bias, gate_i, gate_i_b
     [slots, taps, C]: rows 0 .. taps - 2 the convolution's last inputs (oldest first), the last row
     S; it is read at the slot of each sequence and brought up to date. `work` float32 [3, T, C]:
     u, a and the driving term of every token, between the three kernels. Everything but the rounding of
-    `out` is 32-bit. `single_tokens`: every sequence brings exactly one token (token b is sequence b's)."""
+    `out` is 32-bit. `single_tokens`: every sequence brings exactly one token (token b is sequence b's).
+    `gate_rows` (gate_rows_of): the same two matrices for the tensor cores, where their values are bfloat16; the gates' sums are
+    then formed there, of the same exact products."""
     _require_cuda(y, x, conv_w, conv_b, gate_a, gate_a_bias, gate_i, gate_i_bias, rate, state, tok_seq, cu_seqlens,
-                  slot_ids, out, work)
+                  slot_ids, out, work, gate_rows)
     n, channels = y.shape
     taps, blocks = conv_w.shape[1], gate_a.shape[0]
     _check_rows(y, n, channels, y.dtype, "gated_recurrence: y")
@@ -1736,11 +1752,14 @@ def gated_recurrence(y, x, conv_w, conv_b, gate_a, gate_a_bias, gate_i, gate_i_b
         raise KernelError(f"gated_recurrence: the state must be contiguous float32 [slots, {taps}, {channels}]")
     if work.dtype != torch.float32 or tuple(work.shape) != (3, n, channels) or not work.is_contiguous():
         raise KernelError(f"gated_recurrence: work must be contiguous float32 [3, {n}, {channels}]")
+    if gate_rows is not None and (gate_rows.dtype != torch.bfloat16 or tuple(gate_rows.shape) != (2 * channels, part)
+                                  or not gate_rows.is_contiguous()):
+        raise KernelError(f"gated_recurrence: gate_rows must be contiguous bfloat16 [{2 * channels}, {part}]")
     _call("gated_recurrence", "llmb_gated_recurrence", _ptr(y), _c_int(y.stride(0)), _ptr(x), _c_int(x.stride(0)),
           _c_int(_code(y.dtype)), _ptr(conv_w), _ptr(conv_b), _c_int(taps), _ptr(gate_a), _ptr(gate_a_bias),
           _ptr(gate_i), _ptr(gate_i_bias), _c_int(blocks), _ptr(rate), _ptr(state), _ptr(tok_seq), _ptr(cu_seqlens),
           _ptr(slot_ids), _ptr(out), _c_int(out.stride(0)), _c_float(out_scale), _ptr(work), _c_int(n),
-          _c_int(channels), _c_int(cu_seqlens.numel() - 1), _c_int(1 if single_tokens else 0), _stream(),
+          _c_int(channels), _c_int(cu_seqlens.numel() - 1), _c_int(1 if single_tokens else 0), _ptr(gate_rows), _stream(),
           kernels=3 if n <= 256 else 5)
     return out
 

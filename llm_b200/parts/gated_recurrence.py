@@ -34,6 +34,7 @@ class GatedRecurrenceMixer(ProjectedMixer):
                               f"(or has no taps: {s.conv_taps})")
         self.spec = spec
         self.conv = self.conv_bias = self.gate_a = self.gate_a_bias = self.gate_i = self.gate_i_bias = self.rate = None
+        self.gate_rows = None
 
     @property
     def in_width(self):
@@ -62,6 +63,9 @@ class GatedRecurrenceMixer(ProjectedMixer):
         self.conv_bias = to_float32(tensors[t["conv_bias"]], device)
         # the gates are 32-bit in every run: their matrices are held so
         self.gate_a, self.gate_i = to_float32(tensors[t["ra"]], device), to_float32(tensors[t["ri"]], device)
+        # in bfloat16 runs the tensor cores form their sums where the matrices are bfloat16 numbers
+        on_gpu = dtype == torch.bfloat16 and torch.device(device).type == "cuda"
+        self.gate_rows = ops.gate_rows_of(self.gate_a, self.gate_i) if on_gpu else None
         self.gate_a_bias = to_float32(tensors[t["ra_bias"]], device).reshape(-1).contiguous()
         self.gate_i_bias = to_float32(tensors[t["ri_bias"]], device).reshape(-1).contiguous()
         # log a = rate * r with rate = -decay * softplus(lam), once, in 32-bit
@@ -91,7 +95,7 @@ class GatedRecurrenceMixer(ProjectedMixer):
         ops.gated_recurrence(proj[:, :s.width], proj[:, s.width:], self.conv, self.conv_bias, self.gate_a,
                              self.gate_a_bias, self.gate_i, self.gate_i_bias, self.rate, ctx.cache.state_view(entry),
                              ctx.tok_seq, ctx.cu_seqlens, ctx.slot_ids, out, s.out_scale, work,
-                             single_tokens=ctx.decode)
+                             single_tokens=ctx.decode, **({} if self.gate_rows is None else {"gate_rows": self.gate_rows}))
 
 
 register_mixer("gated_recurrence", GatedRecurrenceMixer)

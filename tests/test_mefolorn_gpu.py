@@ -392,6 +392,57 @@ def test_gated_recurrence(dtype, case):
         _close(states[0], states[1], torch.float32, (case, lengths, "state"))
 
 
+@pytest.mark.parametrize("channels,blocks", [(64, 1), (256, 2), (768, 3), (1024, 4)])
+@pytest.mark.parametrize("new", [[1], [1, 1, 1], [127], [128], [64, 65], [300, 20, 5]])
+def test_gates_on_the_tensor_cores(channels, blocks, new):
+    """Gate matrices of bfloat16 values: the sums of the tensor cores beside those of the 32-bit kernel, both against 64 bits, for
+    tiles that are empty in part, one or several k-blocks and groups. A gate's sum of P exact products in 32 bits is off by
+    P 2^-24 of its magnitudes (some 3) at most, 5e-5 at P = 256; a sigmoid passes a quarter of that on, and the exponent's
+    rate (30 at most here) times a (e^-x x <= 0.37) what is left: 2e-5 in a; the driving term's root has the slope
+    a / sqrt(1 - a^2), some 25 where a comes nearest to one."""
+    ops = _ops()
+    batch = Batch([n + 2 for n in new], new, seed=1)
+    _, params, state = _recurrence_inputs(channels, blocks, 4, batch.n_tokens, len(new) + 2, torch.bfloat16, seed=channels)
+    wide = torch.randn((batch.n_tokens, 2 * channels), generator=torch.Generator().manual_seed(5)).bfloat16().to(DEV)
+    for name in ("gate_a", "gate_i"):
+        params[name] = params[name].bfloat16().float()
+    rows = ops.gate_rows_of(params["gate_a"], params["gate_i"])
+    assert rows.shape == (2 * channels, channels // blocks)
+    p = params
+    u, a, drive, out = [], [], [], []
+    for gate_rows in (None, rows):
+        work, held = torch.empty((3, batch.n_tokens, channels), device=DEV), state.clone()
+        out.append(torch.empty((batch.n_tokens, channels), dtype=torch.bfloat16, device=DEV))
+        ops.gated_recurrence(wide[:, :channels], wide[:, channels:], p["conv_w"], p["conv_b"], p["gate_a"], p["gate_a_bias"],
+                             p["gate_i"], p["gate_i_bias"], p["rate"], held, batch.tok_seq, batch.cu, batch.slots, out[-1], 0.9,
+                             work, single_tokens=all(k == 1 for k in new), gate_rows=gate_rows)
+        for kept, t in zip((u, a, drive), work.double()):
+            kept.append(t.clone())
+    torch.cuda.synchronize()
+    ops.check_device_status()
+    assert torch.allclose(out[0].float(), out[1].float(), atol=2 ** -7 * float(out[0].abs().max()))
+    if batch.n_tokens > 256:                     # (long steps reuse u's place and rewrite a sequence's first token)
+        return
+    assert torch.equal(u[0], u[1])
+    parts = u[0].view(-1, blocks, channels // blocks)
+    r, i = (torch.sigmoid(torch.einsum("tbi,boi->tbo", parts, p[g].double()).reshape(u[0].shape) + p[g + "_bias"].double())
+            for g in ("gate_a", "gate_i"))
+    want_a = torch.exp(p["rate"].double() * r)
+    want_drive = torch.sqrt(1.0 - want_a * want_a) * i * u[0]
+    for got_a, got_drive in zip(a, drive):
+        assert float((got_a - want_a).abs().max()) <= 2e-5
+        assert float((got_drive - want_drive).abs().max()) <= 5e-4 * float(want_drive.abs().max())
+
+
+def test_gate_rows_need_bfloat16_values():
+    ops = _ops()
+    gate = torch.randn((2, 64, 64), generator=torch.Generator().manual_seed(3)).to(DEV)
+    exact = gate.bfloat16().float()
+    assert ops.gate_rows_of(exact, exact) is not None
+    assert ops.gate_rows_of(exact, gate) is None and ops.gate_rows_of(gate, exact) is None
+    assert ops.gate_rows_of(exact[:, :48, :48].contiguous(), exact[:, :48, :48].contiguous()) is None
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("channels,blocks", [(32, 2), (1028, 4)])
 def test_gated_recurrence_of_aligned_rows(dtype, channels, blocks):
