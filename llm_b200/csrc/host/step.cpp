@@ -50,50 +50,62 @@ void layout(const Cache& cache, int n, const int* counts, const int* want_counts
     *total = std::max<long long>(at, 4);
 }
 
+void check_batch(const Cache& cache, int n, const int* slots, const int* counts, const int* tokens, const int* want_counts,
+                 const int* wants, int vocab, int max_seq_len) {
+    std::vector<char> seen(cache.max_slots, 0);
+    long long token_at = 0, want_at = 0;
+    for (int i = 0; i < n; ++i) {
+        int slot = slots[i];
+        cache.require_held(slot);
+        if (seen[slot]) throw Failure{LLMH_FORMAT, "slot " + std::to_string(slot) + " appears twice in one step"};
+        seen[slot] = 1;
+        if (counts[i] <= 0) throw Failure{LLMH_FORMAT, "slot " + std::to_string(slot) + " brings no token"};
+        for (int t = 0; t < counts[i]; ++t) {
+            int id = tokens[token_at + t];
+            if (id < 0 || id >= vocab)
+                throw Failure{LLMH_FORMAT, "token id " + std::to_string(id) + " is outside the vocabulary of " + std::to_string(vocab)};
+        }
+        for (int w = 0; w < want_counts[i]; ++w) {
+            int place = wants[want_at + w];
+            if (place < 0 || place >= counts[i])
+                throw Failure{LLMH_FORMAT, "wanted place " + std::to_string(place) + " is outside the " +
+                                               std::to_string(counts[i]) + " tokens of slot " + std::to_string(slot)};
+        }
+        long long new_length = (long long)cache.length(slot) + counts[i];
+        if (new_length > max_seq_len) throw Failure{LLMH_CONTEXT_FULL, "", new_length, max_seq_len};
+        token_at += counts[i];
+        want_at += want_counts[i];
+    }
+}
+
+void reserve_batch(Cache& cache, int n, const int* slots, const int* counts) {
+    std::vector<long long> lengths(n);
+    for (int i = 0; i < n; ++i) {
+        cache.require_held(slots[i]);
+        lengths[i] = (long long)cache.length(slots[i]) + counts[i];
+    }
+    cache.reserve_many(n, slots, lengths.data());
+}
+
 }  // namespace
 
 // Everything that can be wrong with a batch, found before anything is launched or changed.
-LLMH_EXPORT int llmh_step_check(void* cache_, int n, const int* slots, const int* counts, const int* tokens,
+LLMH_EXPORT int llmh_step_check(void* cache, int n, const int* slots, const int* counts, const int* tokens,
                                 const int* want_counts, const int* wants, int vocab, int max_seq_len) {
-    return guarded([&] {
-        const Cache& cache = *static_cast<Cache*>(cache_);
-        std::vector<char> seen(cache.max_slots, 0);
-        long long token_at = 0, want_at = 0;
-        for (int i = 0; i < n; ++i) {
-            int slot = slots[i];
-            cache.require_held(slot);
-            if (seen[slot]) throw Failure{LLMH_FORMAT, "slot " + std::to_string(slot) + " appears twice in one step"};
-            seen[slot] = 1;
-            if (counts[i] <= 0) throw Failure{LLMH_FORMAT, "slot " + std::to_string(slot) + " brings no token"};
-            for (int t = 0; t < counts[i]; ++t) {
-                int id = tokens[token_at + t];
-                if (id < 0 || id >= vocab)
-                    throw Failure{LLMH_FORMAT, "token id " + std::to_string(id) + " is outside the vocabulary of " + std::to_string(vocab)};
-            }
-            for (int w = 0; w < want_counts[i]; ++w) {
-                int place = wants[want_at + w];
-                if (place < 0 || place >= counts[i])
-                    throw Failure{LLMH_FORMAT, "wanted place " + std::to_string(place) + " is outside the " +
-                                                   std::to_string(counts[i]) + " tokens of slot " + std::to_string(slot)};
-            }
-            long long new_length = (long long)cache.length(slot) + counts[i];
-            if (new_length > max_seq_len) throw Failure{LLMH_CONTEXT_FULL, "", new_length, max_seq_len};
-            token_at += counts[i];
-            want_at += want_counts[i];
-        }
-    });
+    return guarded([&] { check_batch(*static_cast<Cache*>(cache), n, slots, counts, tokens, want_counts, wants, vocab, max_seq_len); });
 }
 
 // Pages for every entry's new length, all or nothing.
-LLMH_EXPORT int llmh_step_reserve(void* cache_, int n, const int* slots, const int* counts) {
+LLMH_EXPORT int llmh_step_reserve(void* cache, int n, const int* slots, const int* counts) {
+    return guarded([&] { reserve_batch(*static_cast<Cache*>(cache), n, slots, counts); });
+}
+
+// Both, one after the other.
+LLMH_EXPORT int llmh_step_begin(void* cache, int n, const int* slots, const int* counts, const int* tokens,
+                                const int* want_counts, const int* wants, int vocab, int max_seq_len) {
     return guarded([&] {
-        Cache& cache = *static_cast<Cache*>(cache_);
-        std::vector<long long> lengths(n);
-        for (int i = 0; i < n; ++i) {
-            cache.require_held(slots[i]);
-            lengths[i] = (long long)cache.length(slots[i]) + counts[i];
-        }
-        cache.reserve_many(n, slots, lengths.data());
+        check_batch(*static_cast<Cache*>(cache), n, slots, counts, tokens, want_counts, wants, vocab, max_seq_len);
+        reserve_batch(*static_cast<Cache*>(cache), n, slots, counts);
     });
 }
 

@@ -30,6 +30,7 @@ GRAPH_AFTER_STEPS = 2      # plain steps of a shape before it is captured
 MAX_GRAPHS = 128           # captured shapes (batch size, bucket of pages) an engine keeps
 RECORD_AFTER_PASSES = 1    # plain passes of a shape before the next one is recorded
 MAX_RECORDS = 32           # recorded passes an engine keeps
+MAX_LAYOUTS = 4096         # shapes whose sections an engine knows
 MAX_RECORDED_LOGITS = 1 << 25   # a recorded pass holds its logits buffer: none for more values than this
 
 
@@ -132,6 +133,7 @@ class Engine:
         self._records, self._record_seen = {}, {}
         self.records_run = 0
         self._ring, self._ring_at = [(None, None)] * 4, 0
+        self._layouts = {}                # of step buffers, by numbers of entries, tokens and wanted rows
 
     # ------------------------------------------------------------------ sequences
 
@@ -174,8 +176,7 @@ class Engine:
         # checked, and pages taken for the whole step (all or nothing), by the native host library
         batch = _Batch(entries)
         lib, cache = native.lib(), self.cache._handle
-        native.check(lib.llmh_step_check(cache, *batch.arguments(), self.vocab, self.max_seq_len))
-        native.check(lib.llmh_step_reserve(cache, batch.n, batch.slots, batch.counts))
+        native.check(lib.llmh_step_begin(cache, *batch.arguments(), self.vocab, self.max_seq_len))
         longest = max(len(e.tokens) for e in entries)
         total = sum(len(e.tokens) for e in entries)
         if longest <= self.step_tokens and total <= self.pass_tokens:
@@ -211,25 +212,35 @@ class Engine:
     def _pass(self, entries, device_tokens=None, batch=None) -> torch.Tensor:
         batch = batch or _Batch(entries)
         lib, cache = native.lib(), self.cache._handle
-        n_sections = lib.llmh_step_sections(cache)
-        offsets, sizes = (c_longlong * n_sections)(), (c_longlong * n_sections)()
-        total, summary = c_longlong(), (c_longlong * 5)()
-        native.check(lib.llmh_step_layout(cache, batch.n, batch.counts, batch.want_counts, offsets, sizes, byref(total)))
-        total = total.value
+        # where the sections lie follows from the numbers of entries, tokens and wanted rows
+        shape = (batch.n, len(batch.tokens), len(batch.wants))
+        plan = self._layouts.get(shape)
+        if plan is None:
+            n_sections = lib.llmh_step_sections(cache)
+            offsets, sizes, total = (c_longlong * n_sections)(), (c_longlong * n_sections)(), c_longlong()
+            native.check(lib.llmh_step_layout(cache, batch.n, batch.counts, batch.want_counts, offsets, sizes, byref(total)))
+            if len(self._layouts) >= MAX_LAYOUTS:
+                self._layouts.clear()
+            plan = self._layouts[shape] = (offsets, sizes, list(offsets), list(sizes), total.value)
+        c_offsets, c_sizes, offsets, sizes, total = plan
         host = self._host_buffer(total)
+        summary = (c_longlong * 5)()
         native.check(lib.llmh_step_pack(cache, *batch.arguments(), host.data_ptr(), host.numel(),
-                                        offsets, sizes, summary))
-        offsets, sizes = list(offsets), list(sizes)
+                                        c_offsets, c_sizes, summary))
         n_tokens, decode, max_len = summary[0], bool(summary[2]), summary[3]
-        counts = list(batch.counts)
-        seq_lens = host[offsets[4]:offsets[4] + batch.n].tolist()
-        starts = [after - c for after, c in zip(seq_lens, counts)]
-        n_groups = n_sections - 8
+        n_groups = len(offsets) - 8
+
+        def lengths():
+            """New tokens and the length before the step, per entry (a replayed step does not ask)."""
+            counts = list(batch.counts)
+            seq_lens = host[offsets[4]:offsets[4] + batch.n].tolist()
+            return counts, [after - c for after, c in zip(seq_lens, counts)]
 
         def context(dev):
             def view(i):
                 return dev[offsets[i]:offsets[i] + sizes[i]]
             n_seqs = batch.n
+            counts, starts = lengths()
             ctx = StepContext(
                 n_tokens=n_tokens, n_seqs=n_seqs, dtype=self.dtype, device=self.device,
                 tok_pos=view(1), tok_seq=view(2), cu_seqlens=view(3), seq_lens=view(4),
@@ -244,7 +255,7 @@ class Engine:
         if graphable:
             logits = self._replay(len(entries), max_len, host, total, context, device_tokens)
         if logits is None and self.use_records and not graphable:
-            step = _HostStep(n_tokens, batch.n, decode, counts, starts, max_len)
+            step = _HostStep(n_tokens, batch.n, decode, *lengths(), max_len)
             key = self.model.replay_key(step, sizes[6])
             if key is not None and sizes[6] * self.vocab <= MAX_RECORDED_LOGITS:
                 logits = self._run_recorded(key, batch.n, host, total, context, device_tokens)

@@ -55,6 +55,7 @@ _SIGNATURES = {
     "llmh_cache_check": (c_int, [_P]),
     "llmh_step_check": (c_int, [_P, *_BATCH, c_int, c_int]),
     "llmh_step_reserve": (c_int, [_P, c_int, _INTS, _INTS]),
+    "llmh_step_begin": (c_int, [_P, *_BATCH, c_int, c_int]),
     "llmh_step_sections": (c_int, [_P]),
     "llmh_step_layout": (c_int, [_P, c_int, _INTS, _INTS, _LONGS, _LONGS, _LONGS]),
     "llmh_step_pack": (c_int, [_P, *_BATCH, _P, c_longlong, _LONGS, _LONGS, _LONGS]),
