@@ -55,6 +55,29 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     }
     return true;
 }
+// Loops that issue copies or products are run by a whole warp, and one elected lane issues: with a loop of one lane alone the
+// compiler keeps stages, phases and descriptors in the lanes' registers and moves each operand to the uniform ones in front
+// of every instruction. Four products of a k-block took 277 cycles of issue so and take some 50 run by the warp.
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+__device__ __forceinline__ bool elect_one() {
+    uint32_t elected;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(elected));
+    return elected != 0;
+}
+// mbar_wait by a whole warp: every lane gets the same answer.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    long long start = clock64();
+    while (!__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) {
+        bool late = clock64() - start > WAIT_CYCLES;
+        if (late) {
+            *abort_flag = 1;
+            if (status) atomicCAS(status, 0, code);
+        }
+        if (__any_sync(0xffffffffu, late || *abort_flag)) return false;
+    }
+    return true;
+}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar,
                                             int x, int y) {
     asm volatile(
