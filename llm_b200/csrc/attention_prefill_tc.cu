@@ -153,7 +153,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     int tile = n_tiles - 1 - blockIdx.y;
     int start = seq_lens[seq] - n_new;
     int kv_head = head / (n_heads / n_kv_heads);
-    int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     int tile_last_pos = start + min(tile * BQ + BQ - 1, n_new - 1);
     int first_block = WINDOW ? max(start + tile * BQ - window + 1, 0) / BKV : 0;      // the first key block that a query of the tile sees
     int n_blocks = tile_last_pos / BKV + 1 - first_block;
@@ -176,49 +176,50 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
 
     if (warp == 0 || warp == 6) {
         // warp 0 brings Q and the keys, warp 6 the values: each waits only for its own buffers
-        if (lane == 0) {
-            bool keys = warp == 0;
-            if (keys) {
-                uint32_t bar = smem_u32(q_full);
-                mbar_expect_tx(bar, Q_BYTES);
-                for (int h = 0; h < PIECES; ++h)
-                    tma_load_2d(smem_u32(q_tile + h * Q_PIECE), &map_q, bar, head * HD + h * 64,
-                                first_token + tile * BQ);
-            }
-            const CUtensorMap* map = keys ? &map_k : &map_v;
-            unsigned char* tiles = keys ? k_tile : v_tile;
-            uint64_t* full = keys ? k_full : v_full;
-            uint64_t* empty = keys ? k_empty : v_empty;
-            for (int kb = 0; kb < n_blocks; ++kb) {
-                int b = kb & 1;
-                if (kb >= 2 && !mbar_wait(smem_u32(&empty[b]), ((kb >> 1) - 1) & 1, abort_flag, status, keys ? 11 : 12))
-                    break;
+        const bool keys = warp == 0;
+        if (keys && elect_one()) {
+            uint32_t bar = smem_u32(q_full);
+            mbar_expect_tx(bar, Q_BYTES);
+            for (int h = 0; h < PIECES; ++h)
+                tma_load_2d(smem_u32(q_tile + h * Q_PIECE), &map_q, bar, head * HD + h * 64,
+                            first_token + tile * BQ);
+        }
+        __syncwarp();
+        const CUtensorMap* map = keys ? &map_k : &map_v;
+        unsigned char* tiles = keys ? k_tile : v_tile;
+        uint64_t* full = keys ? k_full : v_full;
+        uint64_t* empty = keys ? k_empty : v_empty;
+        for (int kb = 0; kb < n_blocks; ++kb) {
+            int b = kb & 1;
+            int page = pages[(first_block + kb) % ring_pages];
+            if (kb >= 2 && !mbar_wait_warp(smem_u32(&empty[b]), ((kb >> 1) - 1) & 1, abort_flag, status, keys ? 11 : 12)) break;
+            if (elect_one()) {
                 uint32_t bar = smem_u32(&full[b]);
                 mbar_expect_tx(bar, KV_BYTES);
-                int page = pages[(first_block + kb) % ring_pages];
                 int row = (page * n_kv_heads + kv_head) * LLMB_PAGE;
                 for (int h = 0; h < PIECES; ++h)
                     tma_load_2d(smem_u32(tiles + b * KV_BYTES + h * KV_PIECE), map, bar, h * 64, row);
             }
+            __syncwarp();
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            // D 32-bit, A and B bfloat16, M = 128; S has N = 64 keys, O has N = HD with B MN-major
-            constexpr uint32_t idesc_qk = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BKV >> 3) << 17) |
-                                          ((uint32_t)(BQ >> 4) << 24);
-            constexpr uint32_t idesc_pv = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) |
-                                          ((uint32_t)(HD >> 3) << 17) | ((uint32_t)(BQ >> 4) << 24);
-            // the descriptors of the tiles' first bytes are made once; a step inside a tile adds a constant
-            // to the address field (this thread's instructions set the pace of the products)
-            const uint64_t q_desc = smem_desc(smem_u32(q_tile));
-            const uint64_t k_desc0 = smem_desc(smem_u32(k_tile)), v_desc0 = smem_desc_mn(smem_u32(v_tile), KV_PIECE);
-            constexpr uint64_t BUFFER = (uint64_t)(KV_BYTES >> 4);       // the second buffer, in the address field
-            // S[buffer kb & 1] = Q K(kb)^T; the buffer's last probabilities have been consumed by a
-            // product that this thread issued earlier (products run in the order of their issue)
-            auto issue_qk = [&](int kb) -> bool {
-                int b = kb & 1;
-                if (!mbar_wait(smem_u32(&k_full[b]), (kb >> 1) & 1, abort_flag, status, 14)) return false;
-                tcgen05_fence_after();
+        // D 32-bit, A and B bfloat16, M = 128; S has N = 64 keys, O has N = HD with B MN-major
+        constexpr uint32_t idesc_qk = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BKV >> 3) << 17) |
+                                      ((uint32_t)(BQ >> 4) << 24);
+        constexpr uint32_t idesc_pv = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) |
+                                      ((uint32_t)(HD >> 3) << 17) | ((uint32_t)(BQ >> 4) << 24);
+        // the descriptors of the tiles' first bytes are made once; a step inside a tile adds a constant
+        // to the address field (this warp's instructions set the pace of the products)
+        const uint64_t q_desc = smem_desc(smem_u32(q_tile));
+        const uint64_t k_desc0 = smem_desc(smem_u32(k_tile)), v_desc0 = smem_desc_mn(smem_u32(v_tile), KV_PIECE);
+        constexpr uint64_t BUFFER = (uint64_t)(KV_BYTES >> 4);       // the second buffer, in the address field
+        // S[buffer kb & 1] = Q K(kb)^T; the buffer's last probabilities have been consumed by a
+        // product that this warp issued earlier (products run in the order of their issue)
+        auto issue_qk = [&](int kb) -> bool {
+            int b = kb & 1;
+            if (!mbar_wait_warp(smem_u32(&k_full[b]), (kb >> 1) & 1, abort_flag, status, 14)) return false;
+            tcgen05_fence_after();
+            if (elect_one()) {
 #pragma unroll
                 for (int j = 0; j < HD / 16; ++j) {
                     uint64_t q_off = (uint64_t)(((j >> 2) * Q_PIECE + (j & 3) * 32) >> 4);
@@ -228,35 +229,39 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 }
                 tcgen05_commit(smem_u32(&s_full[b]));
                 tcgen05_commit(smem_u32(&k_empty[b]));
-                return true;
-            };
-            LAPS_BEGIN
-            bool ok = mbar_wait(smem_u32(q_full), 0, abort_flag, status, 13) && issue_qk(0);
-            if (ok && n_blocks > 1) ok = issue_qk(1);
-            LAP(4);
-            for (int kb = 0; kb < n_blocks && ok; ++kb) {
-                int b = kb & 1, phase = (kb >> 1) & 1;
-                ok = mbar_wait(smem_u32(&p_full[b]), phase, abort_flag, status, 15);
-                LAP(0);
-                ok = ok && mbar_wait(smem_u32(&v_full[b]), phase, abort_flag, status, 16);
-                LAP(1);
-                if (!ok) break;
-                tcgen05_fence_after();
+            }
+            __syncwarp();
+            return true;
+        };
+        LAPS_BEGIN
+        bool ok = mbar_wait_warp(smem_u32(q_full), 0, abort_flag, status, 13) && issue_qk(0);
+        if (ok && n_blocks > 1) ok = issue_qk(1);
+        LAP(4);
+        for (int kb = 0; kb < n_blocks && ok; ++kb) {
+            int b = kb & 1, phase = (kb >> 1) & 1;
+            ok = mbar_wait_warp(smem_u32(&p_full[b]), phase, abort_flag, status, 15);
+            LAP(0);
+            ok = ok && mbar_wait_warp(smem_u32(&v_full[b]), phase, abort_flag, status, 16);
+            LAP(1);
+            if (!ok) break;
+            tcgen05_fence_after();
+            if (elect_one()) {
 #pragma unroll
-                for (int j = 0; j < BKV / 16; ++j)        // 16 keys a step: 8 columns of P, 2048 bytes of V rows
+                for (int j = 0; j < BKV / 16; ++j)    // 16 keys a step: 8 columns of P, 2048 bytes of V rows
                     tcgen05_mma_ts(tmem_base + O_COL, tmem_base + S_COL + b * BKV + j * 8,
                                    v_desc0 + b * BUFFER + (uint64_t)((j * 2048) >> 4), idesc_pv,
                                    (kb > 0 || j > 0) ? 1u : 0u);
                 tcgen05_commit(smem_u32(o_full));
                 tcgen05_commit(smem_u32(&v_empty[b]));
-                LAP(2);
-                // the scores of the key block after the next go where these probabilities were: the
-                // softmax of the next key block runs meanwhile on the other buffer
-                if (kb + 2 < n_blocks) ok = issue_qk(kb + 2);
-                LAP(3);
             }
-            LAPS_END(6, 5, n_blocks);
+            __syncwarp();
+            LAP(2);
+            // the scores of the key block after the next go where these probabilities were: the
+            // softmax of the next key block runs meanwhile on the other buffer
+            if (kb + 2 < n_blocks) ok = issue_qk(kb + 2);
+            LAP(3);
         }
+        LAPS_END(6, 5, n_blocks);
     } else {
         int quarter = warp & 3;
         int row = quarter * 32 + lane;                       // query row of the tile = lane of tensor memory

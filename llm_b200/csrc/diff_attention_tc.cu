@@ -88,7 +88,7 @@ diff_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     int tile = n_tiles - 1 - blockIdx.y;                     // the heaviest tile of every head first
     int start = seq_lens[seq] - n_new;
     int kv_head = head / (n_heads / n_kv_heads);
-    int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     PageWalk walk = page_walk(start + tile * BQ, start + min(tile * BQ + BQ - 1, n_new - 1), window, keep_first);
     const int* pages = block_table + (size_t)seq * table_stride;
 
@@ -109,45 +109,47 @@ diff_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     griddep_launch();            // behind the allocation: no block of the next kernel can hold this one's tensor memory
 
     if (warp == 8 || warp == 10) {
-        if (lane == 0) {
-            bool keys = warp == 8;
-            if (keys) {
-                uint32_t bar = smem_u32(q_full);
-                mbar_expect_tx(bar, T::Q_BYTES);
-                for (int h = 0; h < T::K_PIECES; ++h)
-                    tma_load_2d(smem_u32(q_tile + h * Q_PIECE), &map_q, bar, head * 2 * DK + h * 64, first_token + tile * BQ);
-            }
-            const CUtensorMap* map = keys ? &map_k : &map_v;
-            unsigned char* tiles = keys ? k_tile : v_tile;
-            uint64_t* full = keys ? k_full : v_full;
-            uint64_t* empty = keys ? k_empty : v_empty;
-            int bytes = keys ? T::K_BYTES : T::V_BYTES, pieces = keys ? T::K_PIECES : T::V_PIECES;
-            for (int n = 0; n < walk.count; ++n) {
-                int stage = n % STAGES, turn = n / STAGES;
-                if (turn > 0 && !mbar_wait(smem_u32(&empty[stage]), (turn - 1) & 1, abort_flag, status, keys ? 1 : 2)) break;
+        const bool keys = warp == 8;
+        if (keys && elect_one()) {
+            uint32_t bar = smem_u32(q_full);
+            mbar_expect_tx(bar, T::Q_BYTES);
+            for (int h = 0; h < T::K_PIECES; ++h)
+                tma_load_2d(smem_u32(q_tile + h * Q_PIECE), &map_q, bar, head * 2 * DK + h * 64, first_token + tile * BQ);
+        }
+        __syncwarp();
+        const CUtensorMap* map = keys ? &map_k : &map_v;
+        unsigned char* tiles = keys ? k_tile : v_tile;
+        uint64_t* full = keys ? k_full : v_full;
+        uint64_t* empty = keys ? k_empty : v_empty;
+        const int bytes = keys ? T::K_BYTES : T::V_BYTES, pieces = keys ? T::K_PIECES : T::V_PIECES;
+        for (int n = 0; n < walk.count; ++n) {
+            int stage = n % STAGES, turn = n / STAGES;
+            int row = (pages[walk.logical(n) % ring_pages] * n_kv_heads + kv_head) * LLMB_PAGE;
+            if (turn > 0 && !mbar_wait_warp(smem_u32(&empty[stage]), (turn - 1) & 1, abort_flag, status, keys ? 1 : 2)) break;
+            if (elect_one()) {
                 uint32_t bar = smem_u32(&full[stage]);
                 mbar_expect_tx(bar, bytes);
-                int row = (pages[walk.logical(n) % ring_pages] * n_kv_heads + kv_head) * LLMB_PAGE;
                 for (int h = 0; h < pieces; ++h)
                     tma_load_2d(smem_u32(tiles + stage * bytes + h * KV_PIECE), map, bar, h * 64, row);
             }
+            __syncwarp();
         }
     } else if (warp == 9) {
-        if (lane == 0) {
-            // D 32-bit, A and B bfloat16, M = 128; S has N = 64 keys, O has N = DV with B MN-major
-            constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BQ >> 4) << 24);
-            constexpr uint32_t idesc_s = idesc | ((uint32_t)(LLMB_PAGE >> 3) << 17);
-            constexpr uint32_t idesc_o = idesc | (1u << 16) | ((uint32_t)(DV >> 3) << 17);
-            const uint64_t q_desc = smem_desc(smem_u32(q_tile)), k_desc = smem_desc(smem_u32(k_tile));
-            const uint64_t v_desc = smem_desc_mn(smem_u32(v_tile), KV_PIECE);
-            // scores of page n, map m (map 2's columns follow map 1's in a row of the tiles); a page's keys are free behind map 2
-            auto issue_scores = [&](int n, int m) -> bool {
-                int stage = n % STAGES;
-                if (m == 0) {
-                    if (!mbar_wait(smem_u32(&k_full[stage]), (n / STAGES) & 1, abort_flag, status, 3)) return false;
-                    tcgen05_fence_after();
-                }
-                uint64_t k_at = k_desc + (uint64_t)((stage * T::K_BYTES) >> 4);
+        // D 32-bit, A and B bfloat16, M = 128; S has N = 64 keys, O has N = DV with B MN-major
+        constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BQ >> 4) << 24);
+        constexpr uint32_t idesc_s = idesc | ((uint32_t)(LLMB_PAGE >> 3) << 17);
+        constexpr uint32_t idesc_o = idesc | (1u << 16) | ((uint32_t)(DV >> 3) << 17);
+        const uint64_t q_desc = smem_desc(smem_u32(q_tile)), k_desc = smem_desc(smem_u32(k_tile));
+        const uint64_t v_desc = smem_desc_mn(smem_u32(v_tile), KV_PIECE);
+        // scores of page n, map m (map 2's columns follow map 1's in a row of the tiles); a page's keys are free behind map 2
+        auto issue_scores = [&](int n, int m) -> bool {
+            int stage = n % STAGES;
+            if (m == 0) {
+                if (!mbar_wait_warp(smem_u32(&k_full[stage]), (n / STAGES) & 1, abort_flag, status, 3)) return false;
+                tcgen05_fence_after();
+            }
+            uint64_t k_at = k_desc + (uint64_t)((stage * T::K_BYTES) >> 4);
+            if (elect_one()) {
 #pragma unroll
                 for (int j = 0; j < DK / 16; ++j) {
                     int c = m * DK + j * 16;
@@ -156,28 +158,32 @@ diff_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                 }
                 tcgen05_commit(smem_u32(&s_full[m * 2 + (n & 1)]));
                 if (m == 1) tcgen05_commit(smem_u32(&k_empty[stage]));
-                return true;
-            };
-            bool ok = mbar_wait(smem_u32(q_full), 0, abort_flag, status, 4);
-            for (int n = 0; n < 2 && n < walk.count && ok; ++n) ok = issue_scores(n, 0) && issue_scores(n, 1);
-            for (int n = 0; n < walk.count && ok; ++n) {
-                int stage = n % STAGES;
-                uint64_t v_at = v_desc + (uint64_t)((stage * T::V_BYTES) >> 4);
+            }
+            __syncwarp();
+            return true;
+        };
+        bool ok = mbar_wait_warp(smem_u32(q_full), 0, abort_flag, status, 4);
+        for (int n = 0; n < 2 && n < walk.count && ok; ++n) ok = issue_scores(n, 0) && issue_scores(n, 1);
+        for (int n = 0; n < walk.count && ok; ++n) {
+            int stage = n % STAGES;
+            uint64_t v_at = v_desc + (uint64_t)((stage * T::V_BYTES) >> 4);
 #pragma unroll
-                for (int m = 0; m < 2; ++m) {
-                    ok = mbar_wait(smem_u32(&p_full[m * 2 + (n & 1)]), (n >> 1) & 1, abort_flag, status, 5);
-                    if (ok && m == 0) ok = mbar_wait(smem_u32(&v_full[stage]), (n / STAGES) & 1, abort_flag, status, 6);
-                    if (!ok) break;
-                    tcgen05_fence_after();
+            for (int m = 0; m < 2; ++m) {
+                ok = mbar_wait_warp(smem_u32(&p_full[m * 2 + (n & 1)]), (n >> 1) & 1, abort_flag, status, 5);
+                if (ok && m == 0) ok = mbar_wait_warp(smem_u32(&v_full[stage]), (n / STAGES) & 1, abort_flag, status, 6);
+                if (!ok) break;
+                tcgen05_fence_after();
+                if (elect_one()) {
 #pragma unroll
-                    for (int j = 0; j < LLMB_PAGE / 16; ++j)          // 16 keys: 8 columns of P, 2048 bytes of value rows
+                    for (int j = 0; j < LLMB_PAGE / 16; ++j)      // 16 keys: 8 columns of P, 2048 bytes of value rows
                         tcgen05_mma_ts(tmem_base + O_COL + m * DV, tmem_base + (m * 2 + (n & 1)) * LLMB_PAGE + j * 8,
                                        v_at + (uint64_t)((j * 2048) >> 4), idesc_o, (n > 0 || j > 0) ? 1u : 0u);
                     tcgen05_commit(smem_u32(&o_full[m]));
                     if (m == 1) tcgen05_commit(smem_u32(&v_empty[stage]));
-                    if (n + 2 < walk.count) ok = issue_scores(n + 2, m);
-                    if (!ok) break;
                 }
+                __syncwarp();
+                if (n + 2 < walk.count) ok = issue_scores(n + 2, m);
+                if (!ok) break;
             }
         }
     } else {

@@ -259,7 +259,7 @@ gates_kernel(const float* __restrict__ u, int channels, const float* __restrict_
 //
 // * warps 0-7: epilogue. A warp reads 32 tokens of 32 channels from tensor memory, forms the gates, a and the driving term.
 // * warps 8-11: take u apart, a k-block of 64 at a time, into three swizzled tiles of 128 x 64.
-// * warp 12, one lane: TMA loads of the weights' tile (128 rows x 64). Warp 13, one lane: the products.
+// * warp 12: TMA loads of the weights' tile (128 rows x 64). Warp 13: the products. One elected lane of either issues.
 //
 // Bound by the epilogue's exponentials, divisions and roots (8 warps an SM) and the taking apart of u, which every group of 64
 // channels of a part does again. 4,096 channels in 16 parts, the gates_kernel of the CUDA cores -> here, whole calls: 2,500 tokens
@@ -292,7 +292,7 @@ gates_tc_kernel(const __grid_constant__ CUtensorMap map_rows, const float* __res
     __shared__ uint64_t full_bar[TC_STAGES], empty_bar[TC_STAGES], acc_full_bar[2], acc_empty_bar[2];
     __shared__ uint32_t tmem_slot;
     __shared__ volatile int abort_flag;
-    int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     griddep_launch();
     if (threadIdx.x == 0) {
         for (int s = 0; s < TC_STAGES; ++s) {
@@ -412,47 +412,52 @@ gates_tc_kernel(const __grid_constant__ CUtensorMap map_rows, const float* __res
             }
         }
     } else if (warp == 12) {
-        if (lane == 0) {
-            int s = 0;
-            uint32_t phase = 0;
-            bool ok = true;
-            for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x) {
-                int row = unit % groups * TC_COLS;
-                for (int kb = 0; kb < kblocks; ++kb) {
-                    ok = mbar_wait(smem_u32(&empty_bar[s]), phase ^ 1, &abort_flag, status, 1);
-                    if (!ok) break;
+        int s = 0;
+        uint32_t phase = 0;
+        bool ok = true;
+        for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x) {
+            int row = unit % groups * TC_COLS;
+            for (int kb = 0; kb < kblocks; ++kb) {
+                ok = mbar_wait_warp(smem_u32(&empty_bar[s]), phase ^ 1, &abort_flag, status, 1);
+                if (!ok) break;
+                if (elect_one()) {
                     mbar_expect_tx(smem_u32(&full_bar[s]), TC_TILE);
                     tma_load_2d(smem_u32(tiles + s * TC_STAGE + 3 * TC_TILE), &map_rows, smem_u32(&full_bar[s]), kb * TC_K, row);
-                    if (++s == TC_STAGES) { s = 0; phase ^= 1; }
                 }
+                __syncwarp();
+                if (++s == TC_STAGES) { s = 0; phase ^= 1; }
             }
         }
-    } else if (lane == 0) {
+    } else {
         // D 32-bit, A and B bfloat16, both K-major, M = 128, N = 128
         constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TC_COLS >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+        const uint64_t x0 = smem_desc(smem_u32(tiles));
         int s = 0;
         uint32_t phase = 0, n_done = 0;
         bool ok = true;
         for (int unit = blockIdx.x; unit < n_units && ok; unit += gridDim.x, ++n_done) {
             uint32_t buffer = n_done & 1, use = n_done >> 1, hi = tmem + buffer * (2 * TC_COLS), low = hi + TC_COLS;
-            ok = mbar_wait(smem_u32(&acc_empty_bar[buffer]), (use & 1) ^ 1, &abort_flag, status, 4);
+            ok = mbar_wait_warp(smem_u32(&acc_empty_bar[buffer]), (use & 1) ^ 1, &abort_flag, status, 4);
             if (!ok) break;
             tcgen05_fence_after();
             for (int kb = 0; kb < kblocks; ++kb) {
-                ok = mbar_wait(smem_u32(&full_bar[s]), phase, &abort_flag, status, 2);
+                ok = mbar_wait_warp(smem_u32(&full_bar[s]), phase, &abort_flag, status, 2);
                 if (!ok) break;
                 tcgen05_fence_after();
-                uint64_t x = smem_desc(smem_u32(tiles + s * TC_STAGE)), w = x + (uint64_t)(3 * (TC_TILE >> 4));
+                uint64_t x = x0 + (uint64_t)(s * (TC_STAGE >> 4)), w = x + (uint64_t)(3 * (TC_TILE >> 4));
+                if (elect_one()) {
 #pragma unroll
-                for (int k = 0; k < TC_K / 16; ++k) {
-                    tcgen05_mma(low, x + (uint64_t)(2 * (TC_TILE >> 4)) + 2 * k, w + 2 * k, idesc, kb > 0 || k > 0);
-                    tcgen05_mma(low, x + (uint64_t)(TC_TILE >> 4) + 2 * k, w + 2 * k, idesc, 1u);
-                    tcgen05_mma(hi, x + 2 * k, w + 2 * k, idesc, kb > 0 || k > 0);
+                    for (int k = 0; k < TC_K / 16; ++k) {
+                        tcgen05_mma(low, x + (uint64_t)(2 * (TC_TILE >> 4)) + 2 * k, w + 2 * k, idesc, kb > 0 || k > 0);
+                        tcgen05_mma(low, x + (uint64_t)(TC_TILE >> 4) + 2 * k, w + 2 * k, idesc, 1u);
+                        tcgen05_mma(hi, x + 2 * k, w + 2 * k, idesc, kb > 0 || k > 0);
+                    }
+                    tcgen05_commit(smem_u32(&empty_bar[s]));
+                    if (kb + 1 == kblocks) tcgen05_commit(smem_u32(&acc_full_bar[buffer]));
                 }
-                tcgen05_commit(smem_u32(&empty_bar[s]));
+                __syncwarp();
                 if (++s == TC_STAGES) { s = 0; phase ^= 1; }
             }
-            if (ok) tcgen05_commit(smem_u32(&acc_full_bar[buffer]));
         }
     }
     __syncwarp();

@@ -645,7 +645,7 @@ expert_product_wide_kernel(const __grid_constant__ CUtensorMap map_a, const __gr
     const int* tile_expert = plan + E + 2;
     int e = tile_expert[tile], first = tile_expert[max_tiles + tile], rows = tile_expert[2 * max_tiles + tile];
     int n0 = blockIdx.x * (GLU ? GN / 2 : GN);
-    int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
@@ -670,12 +670,12 @@ expert_product_wide_kernel(const __grid_constant__ CUtensorMap map_a, const __gr
     uint32_t tmem_base = *tmem_slot;
 
     if (warp == 0) {
-        if (lane == 0) {
-            int s = 0;
-            uint32_t round = 0;
-            int b_row = e * b_rows + n0;
-            for (int kb = 0; kb < n_kblocks; ++kb) {
-                if (!mbar_wait(smem_u32(&empty_bar[s]), (round & 1) ^ 1, abort_flag, status, 1)) break;
+        int s = 0;
+        uint32_t round = 0;
+        int b_row = e * b_rows + n0;
+        for (int kb = 0; kb < n_kblocks; ++kb) {
+            if (!mbar_wait_warp(smem_u32(&empty_bar[s]), (round & 1) ^ 1, abort_flag, status, 1)) break;
+            if (elect_one()) {
                 uint32_t bar = smem_u32(&full_bar[s]);
                 mbar_expect_tx(bar, A_BYTES + B_BYTES);
                 tma_load_2d(smem_u32(a_tiles + (size_t)s * A_BYTES), &map_a, bar, kb * GK, first);
@@ -685,30 +685,30 @@ expert_product_wide_kernel(const __grid_constant__ CUtensorMap map_a, const __gr
                 } else {
                     tma_load_2d(smem_u32(b_tiles + (size_t)s * B_BYTES), &map_b, bar, kb * GK, b_row);
                 }
-                if (++s == G_STAGES) { s = 0; ++round; }
             }
+            __syncwarp();
+            if (++s == G_STAGES) { s = 0; ++round; }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            // instruction descriptor: D 32-bit, A and B bfloat16, both K-major, N = GN, M = 128
-            constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(GN >> 3) << 17) | ((uint32_t)(GM >> 4) << 24);
-            const uint64_t a_desc0 = smem_desc(smem_u32(a_tiles)), b_desc0 = smem_desc(smem_u32(b_tiles));
-            int s = 0;
-            uint32_t phase = 0;
-            bool ok = true;
-            for (int kb = 0; kb < n_kblocks; ++kb) {
-                ok = mbar_wait(smem_u32(&full_bar[s]), phase, abort_flag, status, 2);
-                if (!ok) break;
-                tcgen05_fence_after();
-                uint64_t a_desc = a_desc0 + (uint64_t)(s * (A_BYTES >> 4));
-                uint64_t b_desc = b_desc0 + (uint64_t)(s * (B_BYTES >> 4));
+        // instruction descriptor: D 32-bit, A and B bfloat16, both K-major, N = GN, M = 128
+        constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(GN >> 3) << 17) | ((uint32_t)(GM >> 4) << 24);
+        const uint64_t a_desc0 = smem_desc(smem_u32(a_tiles)), b_desc0 = smem_desc(smem_u32(b_tiles));
+        int s = 0;
+        uint32_t phase = 0;
+        for (int kb = 0; kb < n_kblocks; ++kb) {
+            if (!mbar_wait_warp(smem_u32(&full_bar[s]), phase, abort_flag, status, 2)) break;
+            tcgen05_fence_after();
+            uint64_t a_desc = a_desc0 + (uint64_t)(s * (A_BYTES >> 4));
+            uint64_t b_desc = b_desc0 + (uint64_t)(s * (B_BYTES >> 4));
+            if (elect_one()) {
 #pragma unroll
                 for (int k = 0; k < GK / 16; ++k)               // 16 k-values = 32 bytes inside the swizzled row
                     tcgen05_mma(tmem_base, a_desc + 2 * k, b_desc + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
                 tcgen05_commit(smem_u32(&empty_bar[s]));
-                if (++s == G_STAGES) { s = 0; phase ^= 1; }
+                if (kb + 1 == n_kblocks) tcgen05_commit(smem_u32(acc_bar));
             }
-            if (ok) tcgen05_commit(smem_u32(acc_bar));
+            __syncwarp();
+            if (++s == G_STAGES) { s = 0; phase ^= 1; }
         }
     } else {
         int quarter = warp & 3;                                  // the 32 lanes of tensor memory this warp may read
@@ -759,7 +759,7 @@ expert_product_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __
     uint64_t* acc_empty = acc_full + 2;                    // [2]
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 4);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-    int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
@@ -791,51 +791,53 @@ expert_product_stream_kernel(const __grid_constant__ CUtensorMap map_a, const __
     int columns = (N + STEP - 1) / STEP, total = plan[E + 1] * columns;
 
     if (warp == 0) {
-        if (lane == 0) {
-            int s = 0;
-            uint32_t round = 0;
-            bool ok = true;
-            for (int u = blockIdx.x; u < total && ok; u += gridDim.x) {
-                int tile = u / columns, n0 = (u - tile * columns) * STEP;
-                int first = tile_expert[max_tiles + tile], b_row = tile_expert[tile] * b_rows + n0;
-                for (int kb = 0; kb < n_kblocks; ++kb) {
-                    ok = mbar_wait(smem_u32(&empty_bar[s]), (round & 1) ^ 1, abort_flag, status, 1);
-                    if (!ok) break;
+        int s = 0;
+        uint32_t round = 0;
+        bool ok = true;
+        for (int u = blockIdx.x; u < total && ok; u += gridDim.x) {
+            int tile = u / columns, n0 = (u - tile * columns) * STEP;
+            int first = tile_expert[max_tiles + tile], b_row = tile_expert[tile] * b_rows + n0;
+            for (int kb = 0; kb < n_kblocks; ++kb) {
+                ok = mbar_wait_warp(smem_u32(&empty_bar[s]), (round & 1) ^ 1, abort_flag, status, 1);
+                if (!ok) break;
+                if (elect_one()) {
                     uint32_t bar = smem_u32(&full_bar[s]);
                     mbar_expect_tx(bar, A_BYTES + B_BYTES);
                     tma_load_2d(smem_u32(a_tiles + (size_t)s * A_BYTES), &map_a, bar, kb * GK, first);
                     // boxes of 128 rows: the gate rows and the up rows of the same features, or 256 rows on end
                     tma_load_2d(smem_u32(b_tiles + (size_t)s * B_BYTES), &map_b, bar, kb * GK, b_row);
                     tma_load_2d(smem_u32(b_tiles + (size_t)s * B_BYTES + B_BYTES / 2), &map_b, bar, kb * GK, b_row + (GLU ? N : SN / 2));
-                    if (++s == STAGES) { s = 0; ++round; }
                 }
+                __syncwarp();
+                if (++s == STAGES) { s = 0; ++round; }
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            // instruction descriptor: D 32-bit, A and B bfloat16, both K-major, N = 256, M = 128
-            constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(SN >> 3) << 17) | ((uint32_t)(GM >> 4) << 24);
-            const uint64_t a_desc0 = smem_desc(smem_u32(a_tiles)), b_desc0 = smem_desc(smem_u32(b_tiles));
-            int s = 0;
-            uint32_t phase = 0, done = 0;
-            bool ok = true;
-            for (int u = blockIdx.x; u < total && ok; u += gridDim.x, ++done) {
-                uint32_t buffer = done & 1, use = done >> 1;
-                ok = mbar_wait(smem_u32(&acc_empty[buffer]), (use & 1) ^ 1, abort_flag, status, 4);
+        // instruction descriptor: D 32-bit, A and B bfloat16, both K-major, N = 256, M = 128
+        constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(SN >> 3) << 17) | ((uint32_t)(GM >> 4) << 24);
+        const uint64_t a_desc0 = smem_desc(smem_u32(a_tiles)), b_desc0 = smem_desc(smem_u32(b_tiles));
+        int s = 0;
+        uint32_t phase = 0, done = 0;
+        bool ok = true;
+        for (int u = blockIdx.x; u < total && ok; u += gridDim.x, ++done) {
+            uint32_t buffer = done & 1, use = done >> 1;
+            ok = mbar_wait_warp(smem_u32(&acc_empty[buffer]), (use & 1) ^ 1, abort_flag, status, 4);
+            if (!ok) break;
+            tcgen05_fence_after();
+            for (int kb = 0; kb < n_kblocks; ++kb) {
+                ok = mbar_wait_warp(smem_u32(&full_bar[s]), phase, abort_flag, status, 2);
                 if (!ok) break;
                 tcgen05_fence_after();
-                for (int kb = 0; kb < n_kblocks; ++kb) {
-                    ok = mbar_wait(smem_u32(&full_bar[s]), phase, abort_flag, status, 2);
-                    if (!ok) break;
-                    tcgen05_fence_after();
-                    uint64_t a_desc = a_desc0 + (uint64_t)(s * (A_BYTES >> 4)), b_desc = b_desc0 + (uint64_t)(s * (B_BYTES >> 4));
+                uint64_t a_desc = a_desc0 + (uint64_t)(s * (A_BYTES >> 4)), b_desc = b_desc0 + (uint64_t)(s * (B_BYTES >> 4));
+                if (elect_one()) {
 #pragma unroll
                     for (int k = 0; k < GK / 16; ++k)
                         tcgen05_mma(tmem_base + buffer * SN, a_desc + 2 * k, b_desc + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
                     tcgen05_commit(smem_u32(&empty_bar[s]));
-                    if (++s == STAGES) { s = 0; phase ^= 1; }
+                    if (kb + 1 == n_kblocks) tcgen05_commit(smem_u32(&acc_full[buffer]));
                 }
-                if (ok) tcgen05_commit(smem_u32(&acc_full[buffer]));
+                __syncwarp();
+                if (++s == STAGES) { s = 0; phase ^= 1; }
             }
         }
     } else {

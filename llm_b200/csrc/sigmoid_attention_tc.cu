@@ -131,7 +131,7 @@ sigmoid_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     int tile = n_tiles - 1 - blockIdx.y;                     // the heaviest tile of every head first
     int start = seq_lens[seq] - n_new;
     int kv_head = head / (n_heads / n_kv_heads);
-    int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     int tile_last_pos = start + min(tile * BQ + BQ - 1, n_new - 1);
     int n_pages = tile_last_pos / LLMB_PAGE + 1;
     int first_page = window > 0 ? max(start + tile * BQ - window + 1, 0) / LLMB_PAGE : 0;
@@ -156,110 +156,119 @@ sigmoid_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     griddep_launch();            // behind the allocation: no block of the next kernel can hold this one's tensor memory
 
     if (warp == EPILOGUE_WARPS) {
-        if (lane == 0) {
-            // the ring's order is the products' order: the k-blocks of step n, then the values of step n - 1
-            int unit = 0;
-            bool ok = true;
-            auto next = [&](uint32_t bytes, uint32_t& bar, unsigned char*& to) {
-                int stage = unit % STAGES, turn = unit / STAGES;
-                if (turn > 0 && !mbar_wait(smem_u32(&empty[stage]), (turn - 1) & 1, abort_flag, status, 1)) return false;
-                bar = smem_u32(&full[stage]);
-                to = ring + stage * STAGE_BYTES;
-                mbar_expect_tx(bar, bytes);
-                ++unit;
-                return true;
-            };
-            int q_row = (head - first_head) * n_tokens + first_token + tile * BQ;
-            for (int n = 0; n <= n_steps && ok; ++n) {
-                if (n < n_steps) {
-                    int p0 = first_page + n * STEP_PAGES, count = min(STEP_PAGES, n_pages - p0);
-                    int row[STEP_PAGES];
+        // the ring's order is the products' order: the k-blocks of step n, then the values of step n - 1
+        int unit = 0;
+        bool ok = true;
+        auto next = [&](uint32_t bytes, uint32_t& bar, unsigned char*& to) {
+            int stage = unit % STAGES, turn = unit / STAGES;
+            if (turn > 0 && !mbar_wait_warp(smem_u32(&empty[stage]), (turn - 1) & 1, abort_flag, status, 1)) return false;
+            bar = smem_u32(&full[stage]);
+            to = ring + stage * STAGE_BYTES;
+            if (elect_one()) mbar_expect_tx(bar, bytes);
+            __syncwarp();
+            ++unit;
+            return true;
+        };
+        int q_row = (head - first_head) * n_tokens + first_token + tile * BQ;
+        for (int n = 0; n <= n_steps && ok; ++n) {
+            if (n < n_steps) {
+                int p0 = first_page + n * STEP_PAGES, count = min(STEP_PAGES, n_pages - p0);
+                int row[STEP_PAGES];
 #pragma unroll
-                    for (int p = 0; p < STEP_PAGES; ++p)
-                        row[p] = p < count ? pages[(p0 + p) % ring_pages] * n_kv_heads * LLMB_PAGE : 0;
-                    for (int j = 0; j < n_kblocks && ok; ++j) {
-                        uint32_t bar;
-                        unsigned char* to;
-                        ok = next(A_BYTES + count * PAGE_PIECE, bar, to);
-                        if (!ok) break;
+                for (int p = 0; p < STEP_PAGES; ++p)
+                    row[p] = p < count ? pages[(p0 + p) % ring_pages] * n_kv_heads * LLMB_PAGE : 0;
+                for (int j = 0; j < n_kblocks && ok; ++j) {
+                    uint32_t bar;
+                    unsigned char* to;
+                    ok = next(A_BYTES + count * PAGE_PIECE, bar, to);
+                    if (!ok) break;
+                    int g = j / PIECES, x = (j % PIECES) * 64;
+                    if (elect_one()) {
                         tma_load_2d(smem_u32(to), &map_q, bar, j * 64, q_row);
-                        int g = j / PIECES, x = (j % PIECES) * 64;
 #pragma unroll
                         for (int p = 0; p < STEP_PAGES; ++p)
                             if (p < count) tma_load_2d(smem_u32(to + A_BYTES + p * PAGE_PIECE), &map_k, bar, x, row[p] + g * LLMB_PAGE);
                     }
+                    __syncwarp();
                 }
-                if (n > 0) {
-                    int p0 = first_page + (n - 1) * STEP_PAGES, count = min(STEP_PAGES, n_pages - p0);
-                    for (int v = 0; v < count && ok; v += VALUE_PAGES) {
-                        uint32_t bar;
-                        unsigned char* to;
-                        int here = min(VALUE_PAGES, count - v);
-                        ok = next(here * V_PAGE, bar, to);
-                        if (!ok) break;
-                        for (int p = 0; p < here; ++p) {
-                            int row = (pages[(p0 + v + p) % ring_pages] * n_kv_heads + kv_head) * LLMB_PAGE;
+            }
+            if (n > 0) {
+                int p0 = first_page + (n - 1) * STEP_PAGES, count = min(STEP_PAGES, n_pages - p0);
+                for (int v = 0; v < count && ok; v += VALUE_PAGES) {
+                    uint32_t bar;
+                    unsigned char* to;
+                    int here = min(VALUE_PAGES, count - v);
+                    ok = next(here * V_PAGE, bar, to);
+                    if (!ok) break;
+                    for (int p = 0; p < here; ++p) {
+                        int row = (pages[(p0 + v + p) % ring_pages] * n_kv_heads + kv_head) * LLMB_PAGE;
+                        if (elect_one()) {
                             for (int h = 0; h < V_PIECES; ++h)
                                 tma_load_2d(smem_u32(to + p * V_PAGE + h * PAGE_PIECE), &map_v, bar, h * 64, row);
                         }
+                        __syncwarp();
                     }
                 }
             }
         }
     } else if (warp == EPILOGUE_WARPS + 1) {
-        if (lane == 0) {
-            // D 32-bit, A and B bfloat16, M = 128; S has N = the step's keys, O has N = DV with B MN-major
-            constexpr uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BQ >> 4) << 24);
-            constexpr uint32_t idesc_o = idesc_s | (1u << 16) | ((uint32_t)(DV >> 3) << 17);
-            const uint64_t a_desc = smem_desc(smem_u32(ring)), b_desc = smem_desc(smem_u32(ring + A_BYTES));
-            const uint64_t v_desc = smem_desc_mn(smem_u32(ring), PAGE_PIECE);
-            constexpr uint64_t STAGE = (uint64_t)(STAGE_BYTES >> 4);
-            int stage = 0, phase = 0;
-            auto advance = [&]() { if (++stage == STAGES) { stage = 0; phase ^= 1; } };
-            bool ok = true;
-            for (int n = 0; n <= n_steps && ok; ++n) {
-                if (n < n_steps) {
-                    int count = min(STEP_PAGES, n_pages - (first_page + n * STEP_PAGES));
-                    uint32_t idesc = idesc_s | ((uint32_t)((count * LLMB_PAGE) >> 3) << 17);
-                    if (n > 0) ok = mbar_wait(smem_u32(s_empty), (n - 1) & 1, abort_flag, status, 2);
+        // D 32-bit, A and B bfloat16, M = 128; S has N = the step's keys, O has N = DV with B MN-major
+        constexpr uint32_t idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BQ >> 4) << 24);
+        constexpr uint32_t idesc_o = idesc_s | (1u << 16) | ((uint32_t)(DV >> 3) << 17);
+        const uint64_t a_desc = smem_desc(smem_u32(ring)), b_desc = smem_desc(smem_u32(ring + A_BYTES));
+        const uint64_t v_desc = smem_desc_mn(smem_u32(ring), PAGE_PIECE);
+        constexpr uint64_t STAGE = (uint64_t)(STAGE_BYTES >> 4);
+        int stage = 0, phase = 0;
+        auto advance = [&]() { if (++stage == STAGES) { stage = 0; phase ^= 1; } };
+        bool ok = true;
+        for (int n = 0; n <= n_steps && ok; ++n) {
+            if (n < n_steps) {
+                int count = min(STEP_PAGES, n_pages - (first_page + n * STEP_PAGES));
+                uint32_t idesc = idesc_s | ((uint32_t)((count * LLMB_PAGE) >> 3) << 17);
+                if (n > 0) ok = mbar_wait_warp(smem_u32(s_empty), (n - 1) & 1, abort_flag, status, 2);
+                if (!ok) break;
+                tcgen05_fence_after();
+                for (int j = 0; j < n_kblocks && ok; ++j) {
+                    ok = mbar_wait_warp(smem_u32(&full[stage]), phase, abort_flag, status, 3);
                     if (!ok) break;
                     tcgen05_fence_after();
-                    for (int j = 0; j < n_kblocks && ok; ++j) {
-                        ok = mbar_wait(smem_u32(&full[stage]), phase, abort_flag, status, 3);
-                        if (!ok) break;
-                        tcgen05_fence_after();
+                    if (elect_one()) {
 #pragma unroll
                         for (int k = 0; k < 4; ++k)
                             tcgen05_mma(tmem_base + S_COL, a_desc + stage * STAGE + k * 2, b_desc + stage * STAGE + k * 2, idesc,
                                         (j > 0 || k > 0) ? 1u : 0u);
                         tcgen05_commit(smem_u32(&empty[stage]));
-                        advance();
+                        if (j + 1 == n_kblocks) tcgen05_commit(smem_u32(s_full));
                     }
-                    if (!ok) break;
-                    tcgen05_commit(smem_u32(s_full));
+                    __syncwarp();
+                    advance();
                 }
-                if (n > 0) {
-                    int count = min(STEP_PAGES, n_pages - (first_page + (n - 1) * STEP_PAGES));
-                    ok = mbar_wait(smem_u32(w_full), (n - 1) & 1, abort_flag, status, 4);
+                if (!ok) break;
+            }
+            if (n > 0) {
+                int count = min(STEP_PAGES, n_pages - (first_page + (n - 1) * STEP_PAGES));
+                ok = mbar_wait_warp(smem_u32(w_full), (n - 1) & 1, abort_flag, status, 4);
+                if (!ok) break;
+                tcgen05_fence_after();
+                for (int v = 0; v < count && ok; v += VALUE_PAGES) {
+                    ok = mbar_wait_warp(smem_u32(&full[stage]), phase, abort_flag, status, 5);
                     if (!ok) break;
                     tcgen05_fence_after();
-                    for (int v = 0; v < count && ok; v += VALUE_PAGES) {
-                        ok = mbar_wait(smem_u32(&full[stage]), phase, abort_flag, status, 5);
-                        if (!ok) break;
-                        tcgen05_fence_after();
-                        int here = min(VALUE_PAGES, count - v);
+                    int here = min(VALUE_PAGES, count - v);
+                    if (elect_one()) {
                         for (int p = 0; p < here; ++p)
 #pragma unroll
-                            for (int k = 0; k < LLMB_PAGE / 16; ++k)          // 16 keys: 8 columns of W, 2048 bytes of value rows
+                            for (int k = 0; k < LLMB_PAGE / 16; ++k)      // 16 keys: 8 columns of W, 2048 bytes of value rows
                                 tcgen05_mma_ts(tmem_base + O_COL, tmem_base + W_COL + (v + p) * (LLMB_PAGE / 2) + k * 8,
                                                v_desc + stage * STAGE + (uint64_t)((p * V_PAGE + k * 2048) >> 4), idesc_o,
                                                (n > 1 || v + p > 0 || k > 0) ? 1u : 0u);
                         tcgen05_commit(smem_u32(&empty[stage]));
-                        advance();
+                        if (v + VALUE_PAGES >= count) tcgen05_commit(smem_u32(o_full));
                     }
-                    if (!ok) break;
-                    tcgen05_commit(smem_u32(o_full));
+                    __syncwarp();
+                    advance();
                 }
+                if (!ok) break;
             }
         }
     } else {
