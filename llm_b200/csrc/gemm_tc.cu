@@ -1102,10 +1102,11 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
         "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
         ::"r"(dst), "l"(map), "r"(cluster_bar), "r"(x), "r"(y) : "memory");
 }
-__device__ __forceinline__ void tcgen05_commit_pair(uint32_t bar) {
+// `mask`: the blocks of the cluster whose barrier at this place is signalled
+__device__ __forceinline__ void tcgen05_commit_pair(uint32_t bar, uint16_t mask = 3) {
     asm volatile(
         "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-        ::"r"(bar), "h"((uint16_t)3) : "memory");
+        ::"r"(bar), "h"(mask) : "memory");
 }
 __device__ __forceinline__ void tcgen05_mma_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
                                                  uint32_t idesc, uint32_t accumulate) {
@@ -1117,6 +1118,7 @@ __device__ __forceinline__ void tcgen05_mma_pair(uint32_t d_tmem, uint64_t a_des
           "r"(0u), "r"(0u), "r"(0u), "r"(0u), "r"(0u), "r"(0u), "r"(0u), "r"(0u) : "memory");
 }
 
+constexpr int PAIRS = 74;           // of SMs
 constexpr int PAIR_BN = 256;        // columns of the pair's tile; each block loads half of them
 
 // The order in which the pairs take the tiles. The 74 tiles that run at the same time read their
@@ -1547,6 +1549,325 @@ pair_tail_sum_kernel(float* partials, Epilogue ep, PairWork work) {
     }
 }
 
+// ------------------------------------------------------------------------- weights on the pair's row side
+// From some tokens to some thousand, 256 x 256 tiles with the tokens as rows are too coarse: 350 tokens fill 512 rows, a
+// 4,096-wide output has 32 tiles for 74 pairs, and a tile takes its 26 us (64 k-blocks) whatever the other pairs do. Here the
+// weights are the 256 rows of a pair's tile and the tokens its N side, whose width (32 to 256, a multiple of 32) is chosen
+// so that the tokens fill it; and where the tiles are too few, `splits` pairs of one cluster share a tile, each with a
+// slice of its k-blocks. Their accumulators meet in shared memory: when every pair of the cluster is done, each block
+// writes the columns that another one finishes into that block's (now empty) operand ring, and after one cluster barrier
+// every block adds its share of the columns in the order of k and runs the epilogue on it. (Partial tiles through global
+// memory and a second kernel cost some 12 us a product.)
+//
+// The epilogue turns the tile around: a thread holds one output column (weight row) of 16 tokens at a time and writes
+// them to a staging buffer [16 tokens][128 outputs], from which the copy engine stores (or adds, 32-bit residual) whole rows;
+// tokens and outputs beyond the matrix are dropped by its bounds. Targets that a tensor map cannot describe are stored directly.
+struct WideWork {
+    int n_kblocks, tiles_t, tiles_w, bn, splits;      // token tiles of bn, weight tiles of 256
+};
+
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, uint32_t src, int x, int y) {
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%2, %3}], [%1];"
+                 ::"l"(map), "r"(src), "r"(x), "r"(y) : "memory");
+}
+
+__global__ void __launch_bounds__(THREADS, 1)
+gemm_tc_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
+                    const __grid_constant__ CUtensorMap map_out, Epilogue ep, WideWork work, int* status, int stages,
+                    int out_by_tma) {
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    constexpr int A_BYTES = BM * BK * 2;
+    const int bn = work.bn, B_BYTES = (bn / 2) * BK * 2;
+    unsigned char* base = reinterpret_cast<unsigned char*>(
+        (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    unsigned char* a_tiles = base;
+    unsigned char* b_tiles = base + (size_t)stages * A_BYTES;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(b_tiles + (size_t)stages * B_BYTES);
+    uint64_t* full_bar = bars;
+    uint64_t* empty_bar = bars + stages;
+    uint64_t* acc_full_bar = bars + 2 * stages;
+    uint64_t* acc_empty_bar = bars + 2 * stages + 2;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * stages + 4);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    unsigned char* staging = base + (size_t)stages * (A_BYTES + B_BYTES) + 1024;       // two buffers of [16][128] values
+    __shared__ float rstd_s[2][PAIR_BN];                // scales of a tile's tokens (a folded norm)
+
+    const int warp = warp_index(), lane = threadIdx.x & 31;
+    const uint32_t cluster = cluster_rank(), rank = cluster & 1, lead = cluster & ~1u;
+    const int split = (int)(cluster >> 1), splits = work.splits;
+    const int n_units = work.tiles_t * work.tiles_w;
+    const int n_teams = (int)gridDim.x / (2 * splits), team = (int)blockIdx.x / (2 * splits);
+    const int k_begin = work.n_kblocks * split / splits, k_end = work.n_kblocks * (split + 1) / splits;
+    int tmem_cols = 32;
+    while (tmem_cols < (splits > 1 ? bn : 2 * bn)) tmem_cols *= 2;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < stages; ++s) {
+            mbar_init(smem_u32(&full_bar[s]), 1);
+            mbar_init(smem_u32(&empty_bar[s]), 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(smem_u32(&acc_full_bar[b]), 1);
+            mbar_init(smem_u32(&acc_empty_bar[b]), 8);          // four epilogue warps in each block of the pair
+        }
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;"
+                     ::"r"(smem_u32(tmem_slot)), "r"(tmem_cols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    tcgen05_fence_before();
+    __syncthreads();
+    cluster_sync();                                   // the partner's barriers exist from here on
+    tcgen05_fence_after();
+    uint32_t tmem_base = *tmem_slot;
+
+    // As in gemm_tc_kernel: the first weight tiles (operand A here) are fetched while the kernel before this one may still be
+    // running; the tokens only after griddep_wait().
+    griddep_launch();
+    uint32_t early = 0;
+    if (warp == 0 && team < n_units) {
+        Unit w = pair_unit_of(team, work.tiles_t, work.tiles_w);
+        early = (uint32_t)min(stages, k_end - k_begin);
+        if (elect_one()) {
+            for (uint32_t i = 0; i < early; ++i) {
+                if (rank == 0) mbar_expect_tx(smem_u32(&full_bar[i]), 2 * (A_BYTES + B_BYTES));
+                tma_load_2d_pair(smem_u32(a_tiles + (size_t)i * A_BYTES), &map_w, map_to_rank(smem_u32(&full_bar[i]), lead),
+                                 (k_begin + (int)i) * BK, w.tile_b * 2 * BM + (int)rank * BM);
+            }
+        }
+        __syncwarp();
+    }
+    griddep_wait();
+
+    if (warp == 0) {
+        const uint32_t full_of_lead = map_to_rank(smem_u32(&full_bar[0]), lead);     // both blocks' bytes are counted there
+        uint32_t it = 0;
+        int s = 0;
+        uint32_t round = 0;                                     // how often the ring has been walked through
+        bool ok = true;
+        for (int u = team; u < n_units && ok; u += n_teams) {
+            Unit w = pair_unit_of(u, work.tiles_t, work.tiles_w);
+            const int x_row = w.tile_a * bn + (int)rank * (bn / 2), w_row = w.tile_b * 2 * BM + (int)rank * BM;
+            for (int kb = k_begin; kb < k_end; ++kb, ++it, s = (s + 1 == stages ? 0 : s + 1), round += (s == 0)) {
+                const bool armed = it < early;                  // above, and the weight tile is in flight
+                if (!armed) {
+                    ok = mbar_wait_warp(smem_u32(&empty_bar[s]), (round & 1) ^ 1, abort_flag, status, 1);
+                    if (!ok) break;
+                }
+                if (elect_one()) {
+                    const uint32_t bar = full_of_lead + 8 * s;
+                    if (!armed && rank == 0) mbar_expect_tx(smem_u32(&full_bar[s]), 2 * (A_BYTES + B_BYTES));
+                    if (!armed) tma_load_2d_pair(smem_u32(a_tiles + (size_t)s * A_BYTES), &map_w, bar, kb * BK, w_row);
+                    tma_load_2d_pair(smem_u32(b_tiles + (size_t)s * B_BYTES), &map_x, bar, kb * BK, x_row);
+                }
+                __syncwarp();
+            }
+        }
+    } else if (warp == 1) {
+        if (rank == 0) {
+            // D 32-bit, A and B bfloat16, both K-major, N = bn, M = 256 over the pair (the loop as in gemm_tc_pair_kernel)
+            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) |
+                                   ((uint32_t)(bn >> 3) << 17) | ((uint32_t)((2 * BM) >> 4) << 24);
+            const uint16_t mask = (uint16_t)(3u << lead);
+            uint32_t n_done = 0;
+            int s = 0;
+            uint32_t phase = 0;
+            const uint64_t a_desc0 = smem_desc(smem_u32(a_tiles)), b_desc0 = smem_desc(smem_u32(b_tiles));
+            const uint32_t full0 = smem_u32(&full_bar[0]), empty0 = smem_u32(&empty_bar[0]);
+            const uint32_t b_step = (uint32_t)B_BYTES >> 4;
+            bool ok = true;
+            for (int u = team; u < n_units && ok; u += n_teams, ++n_done) {
+                uint32_t buffer = n_done & 1, use = n_done >> 1;
+                ok = mbar_wait_warp(smem_u32(&acc_empty_bar[buffer]), (use & 1) ^ 1, abort_flag, status, 4);
+                if (!ok) break;
+                tcgen05_fence_after();
+                uint32_t d_tmem = tmem_base + buffer * bn;
+                for (int kb = k_begin; kb < k_end; ++kb) {
+                    ok = mbar_wait_warp(full0 + 8 * s, phase, abort_flag, status, 2);
+                    if (!ok) break;
+                    tcgen05_fence_after();
+                    uint64_t a_desc = a_desc0 + (uint64_t)(s * (A_BYTES >> 4));
+                    uint64_t b_desc = b_desc0 + (uint64_t)(s * b_step);
+                    if (elect_one()) {
+#pragma unroll
+                        for (int k = 0; k < BK / UMMA_K; ++k)
+                            tcgen05_mma_pair(d_tmem, a_desc + 2 * k, b_desc + 2 * k, idesc, k > 0 || kb > k_begin);
+                        tcgen05_commit_pair(empty0 + 8 * s, mask);     // frees the stage in both blocks
+                        if (kb + 1 == k_end) tcgen05_commit_pair(smem_u32(&acc_full_bar[buffer]), mask);
+                    }
+                    __syncwarp();
+                    if (++s == stages) { s = 0; phase ^= 1; }
+                }
+            }
+        }
+        __syncwarp();
+    }
+
+    const int quarter = warp & 3, row = quarter * 32 + lane, n_chunks = bn / 16;
+    // Sixteen tokens of this thread's output column: scale, bias, then out. c: the first token's column in the tile.
+    uint32_t turn = 0;                                  // which staging buffer is next
+    auto finish = [&](const Unit& w, int c, float (&v)[16], const float* rstd) {
+        int token0 = w.tile_a * bn + c, n0 = w.tile_b * 2 * BM + (int)rank * BM, n = n0 + row;
+        if (rstd) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] *= rstd[c + j];
+        }
+        if (!out_by_tma) {
+            store_columns<16>(ep, 1, n, 0, token0, v);
+            return;
+        }
+        unsigned char* buffer = staging + (turn & 1) * (16 * BM * 4);
+        ++turn;
+        if (threadIdx.x == 64) bulk_wait_read<1>();     // the copy that last read this buffer is done with it
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        if (ep.glu) {
+            // lanes 0-15 hold 16 gate rows, lanes 16-31 the up rows of the same features: the halves exchange so that a
+            // gate lane gets the even tokens of its feature and an up lane the odd ones
+            __nv_bfloat16* to = reinterpret_cast<__nv_bfloat16*>(buffer) + quarter * 16 + (lane & 15);
+#pragma unroll
+            for (int j = 0; j < 16; j += 2) {
+                float other = __shfl_xor_sync(0xffffffffu, lane < 16 ? v[j + 1] : v[j], 16);
+                float a = lane < 16 ? gated(ep, v[j], other) : gated(ep, other, v[j + 1]);
+                to[(j + (lane >> 4)) * (BM / 2)] = __float2bfloat16_rn(a);
+            }
+        } else {
+            float b = ep.bias && n < ep.outs ? ep.bias[n] : 0.f;
+            if (ep.residual || !ep.out_is_bf16) {
+                float* to = reinterpret_cast<float*>(buffer) + row;
+#pragma unroll
+                for (int j = 0; j < 16; ++j) to[j * BM] = v[j] + b;
+            } else {
+                __nv_bfloat16* to = reinterpret_cast<__nv_bfloat16*>(buffer) + row;
+#pragma unroll
+                for (int j = 0; j < 16; ++j) to[j * BM] = __float2bfloat16_rn(v[j] + b);
+            }
+        }
+        fence_async_shared();
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        if (threadIdx.x == 64) {
+            if (n0 < ep.outs && token0 < ep.tokens) {
+                if (ep.residual) tma_reduce_add_2d(&map_out, smem_u32(buffer), n0, token0);
+                else tma_store_2d(&map_out, smem_u32(buffer), ep.glu ? n0 / 2 : n0, token0);
+            }
+            bulk_commit();
+        }
+    };
+    auto scales = [&](const Unit& w, uint32_t n_done) -> const float* {
+        if (!ep.f.norm_sumsq) return nullptr;           // as in gemm_tc_kernel: while the products run
+        tile_rstd(ep, rstd_s[n_done & 1], quarter, w.tile_a * bn, bn);
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        return rstd_s[n_done & 1];
+    };
+
+    if (splits == 1) {
+        if (warp >= 2) {
+            uint32_t n_done = 0;
+            bool ok = true;
+            for (int u = team; u < n_units && ok; u += n_teams, ++n_done) {
+                Unit w = pair_unit_of(u, work.tiles_t, work.tiles_w);
+                uint32_t buffer = n_done & 1, use = n_done >> 1;
+                const float* rstd = scales(w, n_done);
+                ok = mbar_wait(smem_u32(&acc_full_bar[buffer]), use & 1, abort_flag, status, 3);
+                if (!ok) break;
+                tcgen05_fence_after();
+                uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + buffer * bn;
+#pragma unroll 1
+                for (int chunk = 0; chunk < n_chunks; ++chunk) {
+                    uint32_t r[16];
+                    float v[16];
+                    tmem_ld16(taddr + chunk * 16, r);
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
+                    finish(w, chunk * 16, v, rstd);
+                }
+                tcgen05_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_remote(map_to_rank(smem_u32(&acc_empty_bar[buffer]), lead));
+            }
+        }
+    } else {
+        // one tile a cluster (n_units == n_teams). Block `split` of either half finishes the chunks [first, last).
+        Unit w = pair_unit_of(team, work.tiles_t, work.tiles_w);
+        const int first = n_chunks * split / splits, last = n_chunks * (split + 1) / splits;
+        const float* rstd = nullptr;
+        bool ok = true;
+        if (warp >= 2) {
+            rstd = scales(w, 0);
+            ok = mbar_wait(smem_u32(&acc_full_bar[0]), 0, abort_flag, status, 3);
+            tcgen05_fence_after();
+        }
+        __syncwarp();
+        cluster_sync();                                 // every pair's products are done: the rings may be written over
+        uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16);
+        // a chunk's values from one pair: [4][128 rows] of four neighbouring columns
+        const int slot = (n_chunks + splits - 1) / splits * 16 * BM;     // floats a pair sends to one block at most
+        const uint32_t ring = smem_u32(base);
+        if (warp >= 2 && ok) {
+            for (int to = 0; to < splits; ++to) {
+                if (to == split) continue;
+                int its_first = n_chunks * to / splits, its_last = n_chunks * (to + 1) / splits;
+                uint32_t there = map_to_rank(ring, (uint32_t)(2 * to) + rank) + (uint32_t)(split * slot + row * 4) * 4;
+#pragma unroll 1
+                for (int chunk = its_first; chunk < its_last; ++chunk) {
+                    uint32_t r[16];
+                    tmem_ld16(taddr + chunk * 16, r);
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};"
+                                     ::"r"(there + (uint32_t)((((chunk - its_first) * 4 + q) * BM) * 16)),
+                                       "r"(r[4 * q]), "r"(r[4 * q + 1]), "r"(r[4 * q + 2]), "r"(r[4 * q + 3]) : "memory");
+                }
+            }
+        }
+        __syncwarp();
+        cluster_sync();
+        if (warp >= 2 && ok) {
+            const float4* mine = reinterpret_cast<const float4*>(base) + row;
+#pragma unroll 1
+            for (int chunk = first; chunk < last; ++chunk) {
+                uint32_t r[16];
+                float v[16];
+                tmem_ld16(taddr + chunk * 16, r);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) v[j] = 0.f;
+                for (int from = 0; from < splits; ++from) {              // in the order of k
+                    if (from == split) {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) v[j] += __uint_as_float(r[j]);
+                        continue;
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        float4 p = mine[from * (slot / 4) + ((chunk - first) * 4 + q) * BM];
+                        v[4 * q] += p.x;
+                        v[4 * q + 1] += p.y;
+                        v[4 * q + 2] += p.z;
+                        v[4 * q + 3] += p.w;
+                    }
+                }
+                finish(w, chunk * 16, v, rstd);
+            }
+        }
+        __syncwarp();
+    }
+
+    if (threadIdx.x == 64) bulk_wait<0>();            // the copy engine is done with the staging buffers
+    tcgen05_fence_before();
+    __syncthreads();
+    if (*abort_flag) {
+        for (int i = 0; i < 100; ++i) __nanosleep(10000);
+        __syncthreads();
+    }
+    cluster_sync();                                   // nobody leaves while the partner may still signal it
+    if (warp == 1) {
+        tcgen05_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
+    }
+}
+
 // ------------------------------------------------------------------------- host side
 
 // rows x K bfloat16, K contiguous with `ld` elements between rows; box 64 x box_rows, 128-byte swizzle
@@ -1656,6 +1977,52 @@ int launch_pair(const CUtensorMap& map_a, const CUtensorMap& map_b, const Epilog
     return check_launch("gemm_tc_pair (the sums of the last round)");
 }
 
+int launch_wide(const void* x, int ldx, const void* w, const Epilogue& ep, const WideWork& work, int M, int N, int K,
+                cudaStream_t stream) {
+    CUtensorMap map_w, map_x, map_out;
+    int code;
+    if ((code = make_map(&map_w, w, N, K, K, BM))) return code;
+    if ((code = make_map(&map_x, x, M, K, ldx, work.bn / 2))) return code;
+    // ring | 1 KB: barriers and control words | two staging buffers of 16 tokens x 128 outputs
+    const size_t stage_bytes = (size_t)BM * BK * 2 + (size_t)(work.bn / 2) * BK * 2, staging = 2 * 16 * BM * 4;
+    int stages = (int)(204 * 1024 / stage_bytes);
+    if (stages > 10) stages = 10;
+    size_t smem = 1024 + stages * stage_bytes + 1024 + staging;
+    static bool configured = false;
+    if (!configured) {                                  // (every width's ring fits into what the widest takes and 227 KB hold)
+        LLMB_CUDA(cudaFuncSetAttribute(gemm_tc_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 1024 + 204 * 1024 + 1024 + (int)staging));
+        configured = true;
+    }
+    // the target as a tensor map, where one can describe it (boxes of one block's outputs x 16 tokens, no swizzle)
+    map_out = map_w;
+    bool wide = ep.residual || !ep.out_is_bf16;
+    void* target = ep.residual ? (void*)ep.residual : ep.out;
+    int columns = ep.glu ? N / 2 : N, out_by_tma = 0;
+    if (ep.ldo % (wide ? 4 : 8) == 0 && (reinterpret_cast<uintptr_t>(target) & 15) == 0) {
+        if ((code = make_map_plain(&map_out, target, wide, M, columns, ep.ldo, ep.glu ? BM / 2 : BM, 16))) return code;
+        out_by_tma = 1;
+    }
+    int* status = status_word();
+    int* status_dev = nullptr;
+    if (status) cudaHostGetDevicePointer((void**)&status_dev, status, 0);
+    int units = work.tiles_t * work.tiles_w, teams = work.splits > 1 || units < PAIRS ? units : PAIRS;
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(teams * 2 * work.splits);
+    config.blockDim = dim3(THREADS);
+    config.dynamicSmemBytes = smem;
+    config.stream = stream;
+    cudaLaunchAttribute attributes[2];
+    attributes[0].id = cudaLaunchAttributeClusterDimension;
+    attributes[0].val.clusterDim.x = 2 * work.splits;
+    attributes[0].val.clusterDim.y = attributes[0].val.clusterDim.z = 1;
+    attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attributes[1].val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = attributes;
+    config.numAttrs = pdl_enabled() ? 2 : 1;
+    LLMB_CUDA(cudaLaunchKernelEx(&config, gemm_tc_wide_kernel, map_w, map_x, map_out, ep, work, status_dev, stages, out_by_tma));
+    return check_launch("gemm_tc_wide");
+}
+
 struct Plan {
     int swap, bn, tiles_a, tiles_b, n_kblocks, per_split, splits;
 };
@@ -1664,7 +2031,7 @@ struct Plan {
 // 128 tokens, and up to 1,024 tokens where 256 x 256 tiles are too few for the pairs of SMs even when cut along K. (With the
 // tokens on the 128-row side a 128 x 4096 x 4096 product has 16 tiles and took 38 us; this way it takes 16. At 512 x 6144 x
 // 4096 the 48 pair tiles are faster again: 28 against 34 us.)
-constexpr int SWAP_TOKENS = 128, SWAP_TOKENS_MOST = 1024, PAIRS = 74;
+constexpr int SWAP_TOKENS = 128, SWAP_TOKENS_MOST = 1024;
 
 // How the pairs share the tiles (PairWork). A tile takes 0.4 us a k-block whatever the other pairs do, so a last round of R of
 // 74 tiles wastes (74 - R) / 74 of it. Cut into pieces (multiples of four k-blocks, at least an eighth of a tile) it takes
@@ -1730,6 +2097,60 @@ Plan make_plan(int M, int N, int K) {
     return p;
 }
 
+// Whether a product runs with its weights on the pairs' row side, and how: the width of the token tiles and the pairs a tile, if any,
+// whose estimate is below the other kernels' by 4 %. Estimates in us, from the measured times of 160 products of 17 to 3,001
+// tokens with 2,048 to 28,672 outputs and K from 2,048 to 14,336, which they meet within some 10 %:
+// * here, a round of 74 pairs takes 0.2 us a k-block up to 128 tokens a tile (the loads' pace) and 0.00151 us a token above, a call 4 us
+//   more, or 8 where pairs share a tile; a gated tile's activations take 0.06 us a token, under the next round's products and
+//   behind the last one's;
+// * 256 x 256 tiles on pairs: 0.35 us a k-block and round, or, with the last round cut along K, 0.38 of the rounds' exact number (0.48
+//   where there is no full one) and 12, and 6 for the last tiles' activations;
+// * weights on one block's row side, tokens in tiles of 128: the weights at 6.5 TB/s, 1.4 ns a tile and k-block, 4.5 a call; it
+//   leaves a norm's input or rotates in its sum, which takes a kernel of some 4 us behind this one;
+// none faster than its weights at 5.5 TB/s.
+// Others -> here: 350 x 6144 x 4096 27.7 -> 19.7, 350 x 4096 x 4096 25.5 -> 16.9, 350 x 28672 x 4096 89.5 -> 80.8, 350 x 4096 x 14336 46.8 ->
+// 39.9, 512 x 4096 x 14336 62.1 -> 49.9, 160 x 6144 x 4096 22.0 -> 17.6, 1300 x 4096 x 4096 45.3 -> 37.0; and not taken: 512 x 28672 x
+// 4096 94.8 (99.6 here), 1024 x 4096 x 4096 27.6 (29.5), 2048 x 6144 x 4096 72.8 (78).
+// Up to 128 tokens the sums' fused epilogues are worth more, except behind a gated product, which has none: 64 x 28672 x 4096 47.9 ->
+// 43.9, 128 x 28672 x 4096 57.6 -> 49.6, 64 x 16384 x 2048 19.0 -> 17.0 (17 tokens 41.4 -> 43.5: from 33 on).
+bool plan_wide(int M, int N, int K, int glu, WideWork* best) {
+    if (M > 2048 || N < 256 || (M <= SWAP_TOKENS && !(glu && M > 32 && N >= 8192))) return false;
+    Plan p = make_plan(M, N, K);
+    const int kblocks = p.n_kblocks, tiles_w = (N + 2 * BM - 1) / (2 * BM);
+    const double weights = 2.0 * N * K * 1e-6, epilogue = glu ? 6.0 : 0.0, least = weights / 5.5 + 4.0 + epilogue;      // (bytes in MB, us)
+    double others;
+    if (on_pairs(p, M, N)) {
+        int n_pairs;
+        PairWork w = plan_pairs(M, N, K, &n_pairs);
+        const int units = w.tiles_a * w.tiles_b;
+        others = epilogue + (w.tail_tiles > 0 ? (double)units / PAIRS * kblocks * (units < PAIRS ? 0.48 : 0.38) + 12.0 : (double)((units + PAIRS - 1) / PAIRS) * kblocks * 0.35 + 4.0);
+    } else {
+        others = weights / 6.5 + 4.5 + epilogue + 0.0014 * p.tiles_a * p.tiles_b * kblocks;
+    }
+    if (others < least) others = least;
+    double lowest = others / 1.04;
+    bool found = false;
+    const double behind = p.swap && p.splits > 1 && !glu ? 4.0 : 0.0;
+    for (int bn = 64; bn <= PAIR_BN; bn += 32) {
+        const int tiles_t = (M + bn - 1) / bn, units = tiles_t * tiles_w;
+        for (int splits = 1; splits <= 3; ++splits) {
+            // (clusters of four blocks fit 34 times beside each other, of six 18 times; more would wait for a second wave)
+            if (splits > 1 && (units > (splits == 2 ? 34 : 18) || kblocks < 8 * splits)) continue;
+            const int rounds = splits > 1 ? 1 : (units + PAIRS - 1) / PAIRS;
+            const double last = glu ? 0.06 * bn : 0.0, round = ((kblocks + splits - 1) / splits) * (bn <= 128 ? 0.2 : 0.00151 * bn);
+            double t = rounds * (round > last ? round : last) + (splits > 1 ? 8.0 : 4.0) + last;
+            if (t < least) t = least;
+            t += behind;
+            if (t < lowest) {
+                lowest = t;
+                *best = WideWork{kblocks, tiles_t, tiles_w, bn, splits};
+                found = true;
+            }
+        }
+    }
+    return found;
+}
+
 }  // namespace
 
 // 0 if nothing went wrong since the last call of this function; else the code of the
@@ -1762,7 +2183,9 @@ LLMB_EXPORT int llmb_gemm_tc_counters(int M, int N, int K) {
 }
 
 // Kernels a call launches (1, or 2 where the sum of parts is a kernel of its own).
-LLMB_EXPORT int llmb_gemm_tc_kernels(int M, int N, int K, int allow_pair) {
+LLMB_EXPORT int llmb_gemm_tc_kernels(int M, int N, int K, int glu, int allow_pair) {
+    WideWork w;
+    if (allow_pair && plan_wide(M, N, K, glu, &w)) return 1;
     Plan p = make_plan(M, N, K);
     int n_pairs;
     if (allow_pair && on_pairs(p, M, N)) return plan_pairs(M, N, K, &n_pairs).tail_tiles > 0 ? 2 : 1;
@@ -1786,7 +2209,7 @@ LLMB_EXPORT int llmb_gemm_tc_fuses_rope(int M, int N, int K, int n_heads, int n_
 }
 
 // out[M, N] = x[M, K] . w[N, K]^T (+ bias[N]); or residual[M, N] += the same.
-// allow_pair != 0: products with more than 128 rows run 256 x 256 tiles on pairs of SMs.
+// allow_pair != 0: products with more than 128 rows run on pairs of SMs, as 256 x 256 tiles or with the weights on the row side.
 // glu != 0: w holds gate and up rows alternating in blocks of 16 (N = 2 F rows, N % 32 == 0) and
 // out is bfloat16 [M, ldo] with F columns act(gate) * up (1: silu, 2: the tanh form of gelu); no bias, no residual.
 // fusion (optional): see fusion.h. *applied (optional) tells which parts ran inside the kernels:
@@ -1822,6 +2245,8 @@ LLMB_EXPORT int llmb_gemm_tc_ex(const void* x, int ldx, const void* w, const flo
     }
     Epilogue ep{bias, out, residual, out_dtype == LLMB_DTYPE_BF16, ldo, M, N, glu != 0, {},
                 glu == 2 ? 1.5957691216057308f : 1.0f, glu == 2 ? 0.0713548162726009f : 0.0f};
+    WideWork wide_work;
+    const bool wide = allow_pair && plan_wide(M, N, K, glu, &wide_work);
     int did = 0;
     if (fusion) {
         llmb_gemm_fusion f = *fusion;
@@ -1832,7 +2257,7 @@ LLMB_EXPORT int llmb_gemm_tc_ex(const void* x, int ldx, const void* w, const flo
         } else {
             f.norm_parts = 0;
         }
-        if (f.emit_rows && f.emit_sumsq && residual && llmb_gemm_tc_emit_parts(M, N, K) > 0) {
+        if (f.emit_rows && f.emit_sumsq && residual && !wide && llmb_gemm_tc_emit_parts(M, N, K) > 0) {
             did |= LLMB_FUSED_EMIT;
         } else {
             f.emit_rows = nullptr;
@@ -1842,12 +2267,13 @@ LLMB_EXPORT int llmb_gemm_tc_ex(const void* x, int ldx, const void* w, const flo
             LLMB_REQUIRE(out && out_dtype == LLMB_DTYPE_BF16 && !glu && !residual && f.tok_pos && f.tok_seq &&
                          f.block_table && f.k_cache && f.v_cache && f.ring_pages > 0,
                          "gemm_tc: the rotation needs a bfloat16 output, positions, a page table and the cache");
-            if (llmb_gemm_tc_fuses_rope(M, N, K, f.n_heads, f.n_kv_heads, f.head_dim)) did |= LLMB_FUSED_ROPE;
+            if (!wide && llmb_gemm_tc_fuses_rope(M, N, K, f.n_heads, f.n_kv_heads, f.head_dim)) did |= LLMB_FUSED_ROPE;
             else f.rope = 0;
         }
         ep.f = f;
     }
     if (applied) *applied = did;
+    if (wide) return launch_wide(x, ldx, w, ep, wide_work, M, N, K, stream);
     CUtensorMap map_a, map_b;
     int code;
     if (allow_pair && on_pairs(p, M, N)) {

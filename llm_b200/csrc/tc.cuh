@@ -261,6 +261,22 @@ inline int make_map_2d_f32(CUtensorMap* map, const void* ptr, long long rows, lo
     return LLMB_OK;
 }
 
+// float32 (`wide`) or bfloat16 [rows, cols] with `ld` elements between rows; boxes of box_cols x box_rows as they are (no swizzle)
+inline int make_map_plain(CUtensorMap* map, const void* ptr, bool wide, long long rows, long long cols, long long ld,
+                          int box_cols, int box_rows) {
+    EncodeTiled encode = encode_fn();
+    if (!encode) return fail(LLMB_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
+    cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+    cuuint64_t strides[1] = {(cuuint64_t)ld * (wide ? 4 : 2)};
+    cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
+    cuuint32_t elem[2] = {1, 1};
+    CUresult r = encode(map, wide ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr),
+                        dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(LLMB_ERR_CUDA, "cuTensorMapEncodeTiled (plain) failed with %d", (int)r);
+    return LLMB_OK;
+}
+
 // out[box at (x, y)] += the box in shared memory (element-wise 32-bit add done by the copy engine;
 // rows and columns beyond the tensor are dropped). x must be a multiple of 4 elements.
 __device__ __forceinline__ void tma_reduce_add_2d(const CUtensorMap* map, uint32_t src, int x, int y) {

@@ -1059,14 +1059,14 @@ def _skinny_scratch(device, m, n, k):
 
 
 @functools.lru_cache(maxsize=4096)
-def _tc_needs(m: int, n: int, k: int, pairs: bool = True) -> tuple:
+def _tc_needs(m: int, n: int, k: int, pairs: bool = True, glu: bool = False) -> tuple:
     """(floats of partial sums, tile counters, kernels launched) of a tcgen05 product of this shape; `pairs`: on pairs of SMs
-    where its tiles fit them."""
+    where its tiles fit them; `glu`: with the gated epilogue."""
     lib = load_library("gemm_tc")
     lib.llmb_gemm_tc_scratch_floats.restype = ctypes.c_longlong
     return (lib.llmb_gemm_tc_scratch_floats(_c_int(m), _c_int(n), _c_int(k)),
             lib.llmb_gemm_tc_counters(_c_int(m), _c_int(n), _c_int(k)),
-            lib.llmb_gemm_tc_kernels(_c_int(m), _c_int(n), _c_int(k), _c_int(1 if pairs else 0)))
+            lib.llmb_gemm_tc_kernels(_c_int(m), _c_int(n), _c_int(k), _c_int(1 if glu else 0), _c_int(1 if pairs else 0)))
 
 
 def _tc_scratch(device, m, n, k) -> tuple:
@@ -1110,9 +1110,9 @@ def glu_fusable(n_rows: int, k: int, dtype) -> bool:
     return dtype == torch.bfloat16 and n_rows % (2 * GLU_BLOCK) == 0 and k % 8 == 0
 
 
-def _tc_kernels(m: int, n: int, k: int) -> int:
+def _tc_kernels(m: int, n: int, k: int, glu: bool = False) -> int:
     """Kernels one call of the tcgen05 product launches (2 where the split-K sum is its own kernel)."""
-    return _tc_needs(m, n, k, not tactics.is_disabled("gemm_tc_pair"))[2]
+    return _tc_needs(m, n, k, not tactics.is_disabled("gemm_tc_pair"), glu)[2]
 
 
 def _fusion_struct(norm, emit, rope):
@@ -1185,7 +1185,7 @@ def linear(a, w, bias=None, out_dtype=None, residual=None, out=None, glu=False, 
               _c_int(_code(a.dtype)), None, *_scratch_arguments(*parts), _c_int(m), _c_int(n), _c_int(k),
               _c_int(n // 2), _c_int(2 if glu == "gelu" else 1), _c_int(0 if tactics.is_disabled("gemm_tc_pair") else 1),
               ctypes.byref(_fusion_struct(norm, None, None)) if norm is not None else None, None,
-              _stream(), kernels=_tc_kernels(m, n, k))
+              _stream(), kernels=_tc_kernels(m, n, k, True))
         return result
     if k != k2 or a.dtype != w.dtype:
         raise KernelError(f"linear: a {tuple(a.shape)} {a.dtype} does not fit w {tuple(w.shape)} {w.dtype}")

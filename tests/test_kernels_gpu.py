@@ -197,6 +197,40 @@ def test_linear_cuts_the_last_round_of_tiles(m, n, k):
     assert ops().tensor_core_status() == 0
 
 
+@pytest.mark.parametrize("m,n,k", [(353, 6152, 1032), (350, 4102, 2056), (511, 4104, 4096), (256, 4104, 8192), (300, 4096, 4096),
+                                   (190, 4096, 8192), (129, 6144, 4096), (1300, 4096, 1536), (64, 8224, 520), (100, 16416, 1032),
+                                   (37, 8192, 1024), (350, 12320, 2056)])
+def test_linear_with_the_weights_on_the_row_side(m, n, k):
+    """Products whose weights are the rows of the pairs' tiles: token tiles of several widths that end inside a tile and inside 16
+    tokens, outputs that end inside a tile and a block, rows no tensor map can describe (4,102), K that ends inside a
+    k-block, one pair a tile and two or three in a cluster; every epilogue, with a folded norm and without, one order of the
+    sums (two runs give the same bits). Up to 128 tokens only gated products come here. Errors as in the test above."""
+    a = randn(m, k, dtype=torch.bfloat16, seed=231)
+    w = randn(n, k, dtype=torch.bfloat16, seed=232, scale=0.05)
+    bias = randn(n, seed=233)
+    plain = a.double() @ w.double().T
+    want = plain + bias.double()
+    scale = float(want.abs().max())
+    got = ops().linear(a, w, bias, out_dtype=torch.float32)
+    assert float((got - want).abs().max()) <= 2e-3 * scale
+    assert torch.equal(got, ops().linear(a, w, bias, out_dtype=torch.float32))
+    assert float((ops().linear(a, w, bias).double() - want).abs().max()) <= 1e-2 * scale
+    residual = randn(m, n, seed=234)
+    expect = residual.double() + want
+    ops().linear(a, w, bias, residual=residual)
+    assert float((residual - expect).abs().max()) <= 2e-3 * scale
+    norm = ops().FoldedNorm(a, _sums_in_parts(a, 5, 235), 5, 1e-5, k)
+    rstd = 1.0 / torch.sqrt((a.double() ** 2).mean(dim=1, keepdim=True) + 1e-5)
+    assert float((ops().linear(a, w, bias, norm=norm).double() - (plain * rstd + bias.double())).abs().max()) <= 1e-2 * scale
+    if n % 32 == 0:
+        for scaled, kind, extra in ((plain, True, {}), (plain * rstd, "gelu", {"norm": norm})):
+            gate, up = scaled.view(m, n // 32, 2, 16).unbind(2)
+            act = gate / (1 + torch.exp(-gate)) if kind is True else torch.nn.functional.gelu(gate, approximate="tanh")
+            act = (act * up).reshape(m, n // 2)
+            assert float((ops().linear(a, w, glu=kind, **extra).double() - act).abs().max()) <= 1e-2 * float(act.abs().max())
+    assert ops().tensor_core_status() == 0
+
+
 def test_linear_on_two_streams_at_once():
     """Products that leave parts in scratch, on two streams with nothing between them: each stream has its own."""
     a = randn(350, 4096, dtype=torch.bfloat16, seed=205)
