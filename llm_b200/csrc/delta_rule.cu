@@ -98,6 +98,9 @@ template <typename T, int N> struct alignas(N * sizeof(T)) Wide { T v[N]; };
 // through shared memory. Pieces: key head g's q and k (2 D channels), 32 * EPL channels of v, the gates of all heads.
 // A lane has EPL neighbouring channels, so that its loads and stores are EPL values wide. 8,192 channels: 24 tokens 32.5 -> 6.2 us (one token a
 // warp, all pieces side by side), 2,077 tokens 117 -> 83 us (four tokens, the pieces one after the other).
+// Four tokens' pieces are shared by three blocks: with one, 592 tokens were 148 blocks for 296 places and 2,077 tokens two waves. Whole
+// calls: 592 tokens 292 -> 266 us, four sequences of 300 to 900 624 -> 601, 777 + 1,300 613 -> 610, 4,096 1,782 -> 1,772.
+constexpr int PIECE_BLOCKS = 3;
 template <typename T, int EPL, int TOK>
 __global__ void __launch_bounds__(THREADS, 2)
 delta_prepare_pieces_kernel(const T* __restrict__ proj, int ld, const float* __restrict__ taps,
@@ -494,7 +497,7 @@ LLMB_EXPORT int llmb_delta_rule(const void* proj, int ld, int dtype, const float
             int tok = n_tokens >= 4 * 148 ? 4 : 1;                                                                 \
             auto kernel = D == 128 ? (tok == 4 ? delta_prepare_pieces_kernel<T, 4, 4> : delta_prepare_pieces_kernel<T, 4, 1>) \
                                    : (tok == 4 ? delta_prepare_pieces_kernel<T, 2, 4> : delta_prepare_pieces_kernel<T, 2, 1>); \
-            dim3 grid((n_tokens + tok - 1) / tok, tok == 4 ? 1 : (G + (H * V + D - 1) / D + THREADS / 32) / (THREADS / 32)); \
+            dim3 grid((n_tokens + tok - 1) / tok, tok == 4 ? PIECE_BLOCKS : (G + (H * V + D - 1) / D + THREADS / 32) / (THREADS / 32)); \
             LLMB_CUDA(llmb::launch(kernel, grid, dim3(THREADS), 0, stream, true, (const T*)proj, ld, taps,         \
                                    (const float*)state, state_stride, tok_seq, cu_seqlens, slot_ids, rate, dt_bias, \
                                    unit_eps, work, work_ld, n_tokens, H, G, V));                                   \

@@ -1552,7 +1552,7 @@ pair_tail_sum_kernel(float* partials, Epilogue ep, PairWork work) {
 // ------------------------------------------------------------------------- weights on the pair's row side
 // From some tokens to some thousand, 256 x 256 tiles with the tokens as rows are too coarse: 350 tokens fill 512 rows, a
 // 4,096-wide output has 32 tiles for 74 pairs, and a tile takes its 26 us (64 k-blocks) whatever the other pairs do. Here the
-// weights are the 256 rows of a pair's tile and the tokens its N side, whose width (32 to 256, a multiple of 32) is chosen
+// weights are the 256 rows of a pair's tile and the tokens its N side, whose width (64 to 256, a multiple of 32) is chosen
 // so that the tokens fill it; and where the tiles are too few, `splits` pairs of one cluster share a tile, each with a
 // slice of its k-blocks. Their accumulators meet in shared memory: when every pair of the cluster is done, each block
 // writes the columns that another one finishes into that block's (now empty) operand ring, and after one cluster barrier
@@ -2111,10 +2111,10 @@ Plan make_plan(int M, int N, int K) {
 // Others -> here: 350 x 6144 x 4096 27.7 -> 19.7, 350 x 4096 x 4096 25.5 -> 16.9, 350 x 28672 x 4096 89.5 -> 80.8, 350 x 4096 x 14336 46.8 ->
 // 39.9, 512 x 4096 x 14336 62.1 -> 49.9, 160 x 6144 x 4096 22.0 -> 17.6, 1300 x 4096 x 4096 45.3 -> 37.0; and not taken: 512 x 28672 x
 // 4096 94.8 (99.6 here), 1024 x 4096 x 4096 27.6 (29.5), 2048 x 6144 x 4096 72.8 (78).
-// Up to 128 tokens the sums' fused epilogues are worth more, except behind a gated product, which has none: 64 x 28672 x 4096 47.9 ->
-// 43.9, 128 x 28672 x 4096 57.6 -> 49.6, 64 x 16384 x 2048 19.0 -> 17.0 (17 tokens 41.4 -> 43.5: from 33 on).
+// Up to 128 tokens the sums' fused epilogues are worth more; a gated product, which has none, is faster here alone (64 x 16384 x
+// 2048 18.5 -> 17.3), and a decode step of 64 sequences with it is not (2,558 -> 2,574 us): the kernel in front has its SMs longer.
 bool plan_wide(int M, int N, int K, int glu, WideWork* best) {
-    if (M > 2048 || N < 256 || (M <= SWAP_TOKENS && !(glu && M > 32 && N >= 8192))) return false;
+    if (M <= SWAP_TOKENS || M > 2048 || N < 256) return false;
     Plan p = make_plan(M, N, K);
     const int kblocks = p.n_kblocks, tiles_w = (N + 2 * BM - 1) / (2 * BM);
     const double weights = 2.0 * N * K * 1e-6, epilogue = glu ? 6.0 : 0.0, least = weights / 5.5 + 4.0 + epilogue;      // (bytes in MB, us)

@@ -198,13 +198,13 @@ def test_linear_cuts_the_last_round_of_tiles(m, n, k):
 
 
 @pytest.mark.parametrize("m,n,k", [(353, 6152, 1032), (350, 4102, 2056), (511, 4104, 4096), (256, 4104, 8192), (300, 4096, 4096),
-                                   (190, 4096, 8192), (129, 6144, 4096), (1300, 4096, 1536), (64, 8224, 520), (100, 16416, 1032),
-                                   (37, 8192, 1024), (350, 12320, 2056)])
+                                   (190, 4096, 8192), (129, 6144, 4096), (1300, 4096, 1536), (140, 8224, 4104), (511, 4128, 4096),
+                                   (300, 8224, 4104), (350, 12320, 2056)])
 def test_linear_with_the_weights_on_the_row_side(m, n, k):
     """Products whose weights are the rows of the pairs' tiles: token tiles of several widths that end inside a tile and inside 16
     tokens, outputs that end inside a tile and a block, rows no tensor map can describe (4,102), K that ends inside a
     k-block, one pair a tile and two or three in a cluster; every epilogue, with a folded norm and without, one order of the
-    sums (two runs give the same bits). Up to 128 tokens only gated products come here. Errors as in the test above."""
+    sums (two runs give the same bits). Errors as in the test above."""
     a = randn(m, k, dtype=torch.bfloat16, seed=231)
     w = randn(n, k, dtype=torch.bfloat16, seed=232, scale=0.05)
     bias = randn(n, seed=233)
