@@ -329,7 +329,7 @@ gates_tc_kernel(const __grid_constant__ CUtensorMap map_rows, const float* __res
         for (int unit = blockIdx.x; unit < n_units; unit += gridDim.x, ++n_done) {
             uint32_t buffer = n_done & 1, use = n_done >> 1;
             int t = unit / groups * TC_TOKENS + quarter * 32 + lane, c0 = unit % groups * TC_CHANNELS + half * 32;
-            if (!mbar_wait(smem_u32(&acc_full_bar[buffer]), use & 1, &abort_flag, status, 3)) break;
+            if (!mbar_wait_warp(smem_u32(&acc_full_bar[buffer]), use & 1, &abort_flag, status, 3)) break;
             tcgen05_fence_after();
             uint32_t at = tmem + ((uint32_t)(quarter * 32) << 16) + buffer * (2 * TC_COLS) + half * 32;
 #pragma unroll 1
@@ -386,7 +386,7 @@ gates_tc_kernel(const __grid_constant__ CUtensorMap map_rows, const float* __res
                     v[i][0] = t < n_tokens ? from[0] : make_float4(0.f, 0.f, 0.f, 0.f);
                     v[i][1] = t < n_tokens ? from[1] : make_float4(0.f, 0.f, 0.f, 0.f);
                 }
-                ok = mbar_wait(smem_u32(&empty_bar[s]), phase ^ 1, &abort_flag, status, 1);
+                ok = mbar_wait_warp(smem_u32(&empty_bar[s]), phase ^ 1, &abort_flag, status, 1);
                 if (!ok) break;
                 unsigned char* to = tiles + s * TC_STAGE;
 #pragma unroll

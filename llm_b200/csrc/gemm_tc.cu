@@ -36,8 +36,9 @@
 // products of the next unit run under the epilogue of the last.
 //
 // Every wait on an mbarrier is bounded by a clock limit. A wait that runs out
-// sets a status word that the host can read, raises the block's abort flag so
-// that every role leaves its loop, and the block still frees its tensor memory.
+// sets a status word that the host can read, raises the block's abort flag so that
+// the roles that load and multiply leave their loops (the epilogue runs through
+// its own, see accumulator_wait), and the block still frees its tensor memory.
 #include <cuda.h>
 
 #include "common.cuh"
@@ -392,6 +393,15 @@ __device__ __forceinline__ void finish_rope(const Epilogue& ep, int a_row, int t
     asm volatile("bar.sync 1, 128;" ::: "memory");      // the staged values are free for the block's next unit
 }
 
+// The epilogue's wait for an accumulator. Whether it ran out is each thread's own finding, and what follows has barriers of the
+// epilogue warps and loads of whole warps: a thread that left its loop here would leave the others waiting for good. So all
+// go on, with sums that are not valid (the status word says so), through every barrier of their units; the waits that are
+// left end as soon as they see the abort flag.
+__device__ __forceinline__ void accumulator_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status) {
+    mbar_wait(bar, parity, abort_flag, status, 3);
+    __syncwarp();
+}
+
 // Persistent: the grid has at most as many blocks as fit on the GPU at once, and block b
 // takes the units b, b + gridDim.x, ... . The shared-memory ring and the two accumulator
 // buffers in tensor memory run on across units, so the loads and products of the next unit
@@ -562,8 +572,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         int quarter = warp & 3;                          // the 32 lanes of tensor memory this warp may read
         int row = quarter * 32 + lane;                   // row of the tile = row of A
         uint32_t n_done = 0;
-        bool ok = true;
-        for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x, ++n_done) {
+        for (int u = blockIdx.x; u < n_units; u += gridDim.x, ++n_done) {
             Unit w = unit_of(u, tiles_a, splits);
             uint32_t buffer = n_done & 1, use = n_done >> 1;
             // a folded norm: the scales of this tile's token rows, computed while the products run
@@ -578,8 +587,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             // a fused rotation: positions, pages and angles of the tile's tokens into shared memory
             // (read again only after this unit's epilogue, which ends with a barrier of these warps)
             if (BN == 16 && swap && splits > 1 && ep.f.rope) stage_rope(ep, rope_stage, w.tile_b * BN);
-            ok = mbar_wait(smem_u32(&acc_full_bar[buffer]), use & 1, abort_flag, status, 3);
-            if (!ok) break;
+            accumulator_wait(smem_u32(&acc_full_bar[buffer]), use & 1, abort_flag, status);
             tcgen05_fence_after();
             uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + buffer * BN;
             int a_row = w.tile_a * BM + row;             // swap: output column; else: token
@@ -1331,8 +1339,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         int quarter = warp & 3;
         int row = quarter * 32 + lane;
         uint32_t n_done = 0;
-        bool ok = true;
-        for (; ok && pair_piece(work, pair, n_pairs, (int)n_done, p); ++n_done) {
+        for (; pair_piece(work, pair, n_pairs, (int)n_done, p); ++n_done) {
             uint32_t buffer = n_done & 1, use = n_done >> 1;
             const float* rstd = nullptr;
             if (ep.f.norm_sumsq) {                    // as in gemm_tc_kernel: while the products run
@@ -1340,8 +1347,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 asm volatile("bar.sync 1, 128;" ::: "memory");
                 rstd = rstd_s[n_done & 1];
             }
-            ok = mbar_wait(smem_u32(&acc_full_bar[buffer]), use & 1, abort_flag, status, 3);
-            if (!ok) break;
+            accumulator_wait(smem_u32(&acc_full_bar[buffer]), use & 1, abort_flag, status);
             tcgen05_fence_after();
             uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + buffer * PAIR_BN;
             int a_row = p.tile_a * 2 * BM + (int)rank * BM + row;
@@ -1765,13 +1771,11 @@ gemm_tc_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     if (splits == 1) {
         if (warp >= 2) {
             uint32_t n_done = 0;
-            bool ok = true;
-            for (int u = team; u < n_units && ok; u += n_teams, ++n_done) {
+            for (int u = team; u < n_units; u += n_teams, ++n_done) {
                 Unit w = pair_unit_of(u, work.tiles_t, work.tiles_w);
                 uint32_t buffer = n_done & 1, use = n_done >> 1;
                 const float* rstd = scales(w, n_done);
-                ok = mbar_wait(smem_u32(&acc_full_bar[buffer]), use & 1, abort_flag, status, 3);
-                if (!ok) break;
+                accumulator_wait(smem_u32(&acc_full_bar[buffer]), use & 1, abort_flag, status);
                 tcgen05_fence_after();
                 uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + buffer * bn;
 #pragma unroll 1
@@ -1793,10 +1797,9 @@ gemm_tc_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         Unit w = pair_unit_of(team, work.tiles_t, work.tiles_w);
         const int first = n_chunks * split / splits, last = n_chunks * (split + 1) / splits;
         const float* rstd = nullptr;
-        bool ok = true;
         if (warp >= 2) {
             rstd = scales(w, 0);
-            ok = mbar_wait(smem_u32(&acc_full_bar[0]), 0, abort_flag, status, 3);
+            accumulator_wait(smem_u32(&acc_full_bar[0]), 0, abort_flag, status);
             tcgen05_fence_after();
         }
         __syncwarp();
@@ -1805,7 +1808,7 @@ gemm_tc_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         // a chunk's values from one pair: [4][128 rows] of four neighbouring columns
         const int slot = (n_chunks + splits - 1) / splits * 16 * BM;     // floats a pair sends to one block at most
         const uint32_t ring = smem_u32(base);
-        if (warp >= 2 && ok) {
+        if (warp >= 2) {
             for (int to = 0; to < splits; ++to) {
                 if (to == split) continue;
                 int its_first = n_chunks * to / splits, its_last = n_chunks * (to + 1) / splits;
@@ -1824,7 +1827,7 @@ gemm_tc_wide_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
         }
         __syncwarp();
         cluster_sync();
-        if (warp >= 2 && ok) {
+        if (warp >= 2) {
             const float4* mine = reinterpret_cast<const float4*>(base) + row;
 #pragma unroll 1
             for (int chunk = first; chunk < last; ++chunk) {
