@@ -818,6 +818,19 @@ def test_argmax_over_a_cluster(rows, vocab):
     assert ops().argmax_rows(x).tolist() == want
 
 
+@pytest.mark.parametrize("vocab", [2048, 14336, 16380, 16384, 18436, 30720, 32772])
+def test_argmax_at_the_ends_of_rounds(vocab):
+    """A block reads 16,384 entries a round, the last round's in pieces of 2,048: maxima at the first and last entry of either,
+    alone and with an equal one behind."""
+    ends = sorted({i for edge in range(0, vocab + 2048, 2048) for i in (edge - 1, edge, vocab - 1) if 0 <= i < vocab})
+    x = randn(len(ends), vocab, seed=312).clamp_(max=5.0)
+    for r, i in enumerate(ends):
+        x[r, i] = 7.0
+        if r % 2:
+            x[r, ends[r:]] = 7.0
+    assert ops().argmax_rows(x).tolist() == ends
+
+
 @pytest.mark.parametrize("n,k", [(16, 4), (17, 64), (64, 172), (344, 64), (1000, 68), (100, 4096), (4099, 260)])
 @pytest.mark.parametrize("residual", [False, True])
 def test_linear_of_few_rows_in_32_bit(n, k, residual):
