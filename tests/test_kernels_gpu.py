@@ -831,6 +831,31 @@ def test_argmax_at_the_ends_of_rounds(vocab):
     assert ops().argmax_rows(x).tolist() == ends
 
 
+@pytest.mark.parametrize("vocab,rows", [(384, 3), (5000, 3), (20000, 3), (20000, 40)])
+def test_sample_the_first_of_equal_logits(vocab, rows):
+    """top_k of one: the first of 1 to 1,500 equal maxima is drawn (fewer and more than a warp, than the threads of a block), the
+    generator moves on as in the plain chain, and more equal ones than the candidates' room are refused."""
+    state_gpu = _sampler_state(rows, [[0.7, 0.95, 0.05, 1.0]] * rows, [[1, 0]] * rows, list(range(3, 3 + rows)))
+    state_cpu = [t.cpu().clone() for t in state_gpu]
+    for equal in (1, 2, 33, 300, 1500, 2500):
+        if equal >= vocab:
+            continue
+        logits = randn(rows, vocab, seed=340 + equal).clamp_(max=3.0)
+        for r in range(rows):
+            places = torch.randperm(vocab, generator=torch.Generator().manual_seed(equal + r))[:equal]
+            logits[r, places.to(DEV)] = 4.0
+        cpu_logits = logits.cpu().clone()
+        before = state_gpu[4].clone()
+        ops().sample_rows(logits, *state_gpu)
+        if equal > 2048:
+            assert state_gpu[6].tolist() == [1] * rows and torch.equal(state_gpu[4], before)
+            continue
+        plain_ops.sample_rows(cpu_logits, *state_cpu)
+        assert state_gpu[5].tolist() == state_cpu[5].tolist(), equal
+        assert state_gpu[4].tolist() == state_cpu[4].tolist()
+        assert state_gpu[6].tolist() == [0] * rows
+
+
 @pytest.mark.parametrize("n,k", [(16, 4), (17, 64), (64, 172), (344, 64), (1000, 68), (100, 4096), (4099, 260)])
 @pytest.mark.parametrize("residual", [False, True])
 def test_linear_of_few_rows_in_32_bit(n, k, residual):
