@@ -11,7 +11,7 @@
 // * emit_rows / emit_sumsq (products that add into the residual): the updated residual rows are also
 //   written as bfloat16 [tokens, ldo] and their squares are summed per row into emit_sumsq
 //   [tokens, LLMB_SUMSQ_LD], one partial sum per block of output columns: the next norm's input.
-//   How many partials a call writes per row is told by llmb_gemm_tc_emit_parts().
+//   How many partials a call writes per row is told by llmb_gemm_tc_plan().
 // * rope (the q/k/v product): output columns are heads of head_dim values: n_heads query heads,
 //   n_kv_heads key heads, n_kv_heads value heads. Query and key heads are rotated by the angles of
 //   rope_table[position] (cos in the first half of a row of head_dim values, sin in the second;

@@ -2154,6 +2154,50 @@ bool plan_wide(int M, int N, int K, int glu, WideWork* best) {
     return found;
 }
 
+// Which kernel a product takes and what that kernel needs: the one answer that the launch and all questions about it share.
+struct Choice {
+    enum Kernel { BLOCKS, PAIRS_OF_SMS, ROW_SIDE } kernel;
+    Plan plan;                          // BLOCKS
+    PairWork pairs;                     // PAIRS_OF_SMS
+    int n_pairs;
+    WideWork wide;                      // ROW_SIDE
+    long long scratch_floats;           // partial sums
+    int counters, kernels;              // tile counters; kernels launched
+    int emit_parts;                     // partial sums of squares a row (0: the kernels do not emit)
+    bool can_rotate;                    // the q/k/v product's rotation, where its heads fit the tiles
+};
+
+Choice choose(int M, int N, int K, int glu, int allow_pair) {
+    Choice c = {};
+    c.kernels = 1;
+    if (allow_pair && plan_wide(M, N, K, glu, &c.wide)) {
+        c.kernel = Choice::ROW_SIDE;
+        return c;
+    }
+    const Plan p = c.plan = make_plan(M, N, K);
+    if (allow_pair && on_pairs(p, M, N)) {
+        c.kernel = Choice::PAIRS_OF_SMS;
+        c.pairs = plan_pairs(M, N, K, &c.n_pairs);
+        if (c.pairs.tail_tiles > 0) {
+            c.scratch_floats = 2LL * c.n_pairs * PIECE_FLOATS;
+            c.kernels = 2;
+        }
+        return c;
+    }
+    c.kernel = Choice::BLOCKS;
+    if (p.splits > 1) {
+        c.scratch_floats = (long long)p.tiles_a * p.tiles_b * p.splits * p.bn * BM;
+        c.counters = p.tiles_a * p.tiles_b;
+        c.kernels = 1 + sums_later(p.swap, p.splits, p.bn);
+        if (p.swap) {
+            const int parts = sums_later(p.swap, p.splits, p.bn) ? (N + 255) / 256 : p.tiles_a;
+            c.emit_parts = parts <= LLMB_SUMSQ_LD ? parts : 0;
+            c.can_rotate = true;
+        }
+    }
+    return c;
+}
+
 }  // namespace
 
 // 0 if nothing went wrong since the last call of this function; else the code of the
@@ -2170,45 +2214,18 @@ LLMB_EXPORT int llmb_gemm_tc_status() {
     return v;
 }
 
-// Floats of partial-sum scratch and counters a call needs (0 when it does not split K).
-LLMB_EXPORT long long llmb_gemm_tc_scratch_floats(int M, int N, int K) {
-    Plan p = make_plan(M, N, K);
-    if (on_pairs(p, M, N)) {
-        int n_pairs;
-        return plan_pairs(M, N, K, &n_pairs).tail_tiles > 0 ? 2LL * n_pairs * PIECE_FLOATS : 0;
-    }
-    return p.splits > 1 ? (long long)p.tiles_a * p.tiles_b * p.splits * p.bn * BM : 0;
-}
-LLMB_EXPORT int llmb_gemm_tc_counters(int M, int N, int K) {
-    Plan p = make_plan(M, N, K);
-    if (on_pairs(p, M, N)) return 0;
-    return p.tiles_a * p.tiles_b;
-}
-
-// Kernels a call launches (1, or 2 where the sum of parts is a kernel of its own).
-LLMB_EXPORT int llmb_gemm_tc_kernels(int M, int N, int K, int glu, int allow_pair) {
-    WideWork w;
-    if (allow_pair && plan_wide(M, N, K, glu, &w)) return 1;
-    Plan p = make_plan(M, N, K);
-    int n_pairs;
-    if (allow_pair && on_pairs(p, M, N)) return plan_pairs(M, N, K, &n_pairs).tail_tiles > 0 ? 2 : 1;
-    return 1 + sums_later(p.swap, p.splits, p.bn);
-}
-
-// Partial sums of squares per row that a call with emit_rows / emit_sumsq writes inside its kernels
-// (0: the shape's kernels do not, and the caller runs llmb_cast_sumsq behind the product).
-LLMB_EXPORT int llmb_gemm_tc_emit_parts(int M, int N, int K) {
-    Plan p = make_plan(M, N, K);
-    if (!p.swap || p.splits <= 1) return 0;
-    int parts = sums_later(p.swap, p.splits, p.bn) ? (N + 255) / 256 : p.tiles_a;
-    return parts <= LLMB_SUMSQ_LD ? parts : 0;
-}
-
-// Whether a call with `rope` rotates and writes the cache inside its kernels.
-LLMB_EXPORT int llmb_gemm_tc_fuses_rope(int M, int N, int K, int n_heads, int n_kv_heads, int head_dim) {
-    Plan p = make_plan(M, N, K);
-    return p.swap && p.splits > 1 && head_dim >= 2 && head_dim % 2 == 0 && BM % head_dim == 0 &&
-           (long long)(n_heads + 2 * n_kv_heads) * head_dim == N;
+// What a call of these sizes does and needs: {kernel (0 blocks, 1 pairs, 2 row side), token or column width of its tiles, blocks
+// or pairs that share a tile's K, tiles cut along K in the last round, floats of partial sums, tile counters, kernels launched,
+// partial sums of squares a row that emit_rows / emit_sumsq leave (0: the caller runs llmb_cast_sumsq behind the product)}.
+LLMB_EXPORT int llmb_gemm_tc_plan(int M, int N, int K, int glu, int allow_pair, long long* out) {
+    Choice c = choose(M, N, K, glu, allow_pair);
+    const bool blocks = c.kernel == Choice::BLOCKS, row_side = c.kernel == Choice::ROW_SIDE;
+    const long long values[8] = {(long long)c.kernel, row_side ? c.wide.bn : blocks ? c.plan.bn : PAIR_BN,
+                                 row_side ? c.wide.splits : blocks ? c.plan.splits : 1,
+                                 c.kernel == Choice::PAIRS_OF_SMS ? c.pairs.tail_tiles : 0,
+                                 c.scratch_floats, c.counters, c.kernels, c.emit_parts};
+    for (int i = 0; i < 8; ++i) out[i] = values[i];
+    return LLMB_OK;
 }
 
 // out[M, N] = x[M, K] . w[N, K]^T (+ bias[N]); or residual[M, N] += the same.
@@ -2240,16 +2257,15 @@ LLMB_EXPORT int llmb_gemm_tc_ex(const void* x, int ldx, const void* w, const flo
     } else {
         LLMB_REQUIRE(ldo >= N, "gemm_tc: bad output stride");
     }
-    Plan p = make_plan(M, N, K);
+    const Choice choice = choose(M, N, K, glu, allow_pair);
+    const Plan& p = choice.plan;
     LLMB_REQUIRE((long long)p.tiles_a * p.tiles_b * p.splits < (1ll << 30), "gemm_tc: too many tiles");
-    if (p.splits > 1) {
-        LLMB_REQUIRE(partials && counters && partial_floats >= llmb_gemm_tc_scratch_floats(M, N, K) &&
-                     n_counters >= p.tiles_a * p.tiles_b, "gemm_tc: scratch is missing or too small");
+    if (choice.counters > 0) {
+        LLMB_REQUIRE(partials && counters && partial_floats >= choice.scratch_floats && n_counters >= choice.counters,
+                     "gemm_tc: scratch is missing or too small");
     }
     Epilogue ep{bias, out, residual, out_dtype == LLMB_DTYPE_BF16, ldo, M, N, glu != 0, {},
                 glu == 2 ? 1.5957691216057308f : 1.0f, glu == 2 ? 0.0713548162726009f : 0.0f};
-    WideWork wide_work;
-    const bool wide = allow_pair && plan_wide(M, N, K, glu, &wide_work);
     int did = 0;
     if (fusion) {
         llmb_gemm_fusion f = *fusion;
@@ -2260,7 +2276,7 @@ LLMB_EXPORT int llmb_gemm_tc_ex(const void* x, int ldx, const void* w, const flo
         } else {
             f.norm_parts = 0;
         }
-        if (f.emit_rows && f.emit_sumsq && residual && !wide && llmb_gemm_tc_emit_parts(M, N, K) > 0) {
+        if (f.emit_rows && f.emit_sumsq && residual && choice.emit_parts > 0) {
             did |= LLMB_FUSED_EMIT;
         } else {
             f.emit_rows = nullptr;
@@ -2270,20 +2286,21 @@ LLMB_EXPORT int llmb_gemm_tc_ex(const void* x, int ldx, const void* w, const flo
             LLMB_REQUIRE(out && out_dtype == LLMB_DTYPE_BF16 && !glu && !residual && f.tok_pos && f.tok_seq &&
                          f.block_table && f.k_cache && f.v_cache && f.ring_pages > 0,
                          "gemm_tc: the rotation needs a bfloat16 output, positions, a page table and the cache");
-            if (!wide && llmb_gemm_tc_fuses_rope(M, N, K, f.n_heads, f.n_kv_heads, f.head_dim)) did |= LLMB_FUSED_ROPE;
+            if (choice.can_rotate && f.head_dim >= 2 && f.head_dim % 2 == 0 && BM % f.head_dim == 0 &&
+                (long long)(f.n_heads + 2 * f.n_kv_heads) * f.head_dim == N) did |= LLMB_FUSED_ROPE;
             else f.rope = 0;
         }
         ep.f = f;
     }
     if (applied) *applied = did;
-    if (wide) return launch_wide(x, ldx, w, ep, wide_work, M, N, K, stream);
+    if (choice.kernel == Choice::ROW_SIDE) return launch_wide(x, ldx, w, ep, choice.wide, M, N, K, stream);
     CUtensorMap map_a, map_b;
     int code;
-    if (allow_pair && on_pairs(p, M, N)) {
+    if (choice.kernel == Choice::PAIRS_OF_SMS) {
         // 256 x 256 tiles over pairs of SMs; each block's boxes are 128 rows
-        int n_pairs;
-        PairWork work = plan_pairs(M, N, K, &n_pairs);
-        if (work.tail_tiles > 0 && (!partials || partial_floats < 2LL * n_pairs * PIECE_FLOATS)) {      // no room for parts: whole tiles only
+        int n_pairs = choice.n_pairs;
+        PairWork work = choice.pairs;
+        if (work.tail_tiles > 0 && (!partials || partial_floats < choice.scratch_floats)) {      // no room for parts: whole tiles only
             work.n_full = work.tiles_a * work.tiles_b;
             work.tail_tiles = 0;
             n_pairs = work.n_full < PAIRS ? work.n_full : PAIRS;

@@ -11,6 +11,7 @@ The parts call these functions as attributes of this module
 from __future__ import annotations
 
 import atexit
+import collections
 import ctypes
 import functools
 import os
@@ -1058,21 +1059,27 @@ def _skinny_scratch(device, m, n, k):
     return _split_scratch(device, need // 4, (n + 15) // 16)
 
 
+ProductPlan = collections.namedtuple("ProductPlan", "kernel width splits tail scratch_floats counters kernels emit_parts")
+
+
 @functools.lru_cache(maxsize=4096)
-def _tc_needs(m: int, n: int, k: int, pairs: bool = True, glu: bool = False) -> tuple:
-    """(floats of partial sums, tile counters, kernels launched) of a tcgen05 product of this shape; `pairs`: on pairs of SMs
-    where its tiles fit them; `glu`: with the gated epilogue."""
-    lib = load_library("gemm_tc")
-    lib.llmb_gemm_tc_scratch_floats.restype = ctypes.c_longlong
-    return (lib.llmb_gemm_tc_scratch_floats(_c_int(m), _c_int(n), _c_int(k)),
-            lib.llmb_gemm_tc_counters(_c_int(m), _c_int(n), _c_int(k)),
-            lib.llmb_gemm_tc_kernels(_c_int(m), _c_int(n), _c_int(k), _c_int(1 if glu else 0), _c_int(1 if pairs else 0)))
+def _tc_plan(m: int, n: int, k: int, glu: bool, pairs: bool) -> ProductPlan:
+    out = (ctypes.c_longlong * 8)()
+    load_library("gemm_tc").llmb_gemm_tc_plan(_c_int(m), _c_int(n), _c_int(k), _c_int(1 if glu else 0), _c_int(1 if pairs else 0), out)
+    return ProductPlan(("blocks", "pairs", "row_side")[out[0]], *out[1:])
 
 
-def _tc_scratch(device, m, n, k) -> tuple:
+def product_plan(m: int, n: int, k: int, glu: bool = False) -> ProductPlan:
+    """What a tcgen05 product of these sizes runs as, with `glu` in its epilogue or not: `kernel` ("blocks": single SMs, "pairs":
+    256 x 256 tiles on pairs of SMs, "row_side": pairs with the weights on the row side), the `width` of its tiles, how many
+    share a tile's K (`splits`), tiles cut along K in the last round (`tail`), floats of partial sums and tile counters it
+    needs, kernels it launches, and the partial sums of squares a row that it leaves for the next norm (0: none)."""
+    return _tc_plan(m, n, k, bool(glu), not tactics.is_disabled("gemm_tc_pair"))
+
+
+def _tc_scratch(device, plan) -> tuple:
     """(partials, counters) of a tcgen05 product; a product in whole tiles has neither."""
-    floats, counters, _ = _tc_needs(m, n, k)
-    return _split_scratch(device, floats, counters) if floats else (None, None)
+    return _split_scratch(device, plan.scratch_floats, plan.counters) if plan.scratch_floats else (None, None)
 
 
 def _scratch_arguments(partials, counters) -> tuple:
@@ -1110,11 +1117,6 @@ def glu_fusable(n_rows: int, k: int, dtype) -> bool:
     return dtype == torch.bfloat16 and n_rows % (2 * GLU_BLOCK) == 0 and k % 8 == 0
 
 
-def _tc_kernels(m: int, n: int, k: int, glu: bool = False) -> int:
-    """Kernels one call of the tcgen05 product launches (2 where the split-K sum is its own kernel)."""
-    return _tc_needs(m, n, k, not tactics.is_disabled("gemm_tc_pair"), glu)[2]
-
-
 def _fusion_struct(norm, emit, rope):
     f = _Fusion()
     if norm is not None:
@@ -1130,11 +1132,6 @@ def _fusion_struct(norm, emit, rope):
         f.block_table, f.table_stride = rope.block_table.data_ptr(), rope.block_table.shape[1]
         f.ring_pages, f.k_cache, f.v_cache = rope.ring_pages, rope.k_cache.data_ptr(), rope.v_cache.data_ptr()
     return f
-
-
-@functools.lru_cache(maxsize=4096)
-def _tc_emit_parts(m: int, n: int, k: int) -> int:
-    return load_library("gemm_tc").llmb_gemm_tc_emit_parts(_c_int(m), _c_int(n), _c_int(k))
 
 
 def _check_norm(norm, m, k):
@@ -1178,14 +1175,15 @@ def linear(a, w, bias=None, out_dtype=None, residual=None, out=None, glu=False, 
                               "K % 8 == 0, no bias and no residual")
         _check_out(out, (m, n // 2), a.dtype, "linear")
         result = out if out is not None else torch.empty((m, n // 2), dtype=a.dtype, device=a.device)
-        parts = _tc_scratch(a.device, m, n, k)
+        plan = product_plan(m, n, k, True)
+        parts = _tc_scratch(a.device, plan)
         if emit is not None or rope is not None:
             raise KernelError("linear: the gated epilogue takes a folded norm only")
         _call("gemm_tc", "llmb_gemm_tc_ex", _ptr(a), _c_int(a.stride(0)), _ptr(w), None, _ptr(result),
               _c_int(_code(a.dtype)), None, *_scratch_arguments(*parts), _c_int(m), _c_int(n), _c_int(k),
               _c_int(n // 2), _c_int(2 if glu == "gelu" else 1), _c_int(0 if tactics.is_disabled("gemm_tc_pair") else 1),
               ctypes.byref(_fusion_struct(norm, None, None)) if norm is not None else None, None,
-              _stream(), kernels=_tc_kernels(m, n, k, True))
+              _stream(), kernels=plan.kernels)
         return result
     if k != k2 or a.dtype != w.dtype:
         raise KernelError(f"linear: a {tuple(a.shape)} {a.dtype} does not fit w {tuple(w.shape)} {w.dtype}")
@@ -1203,18 +1201,20 @@ def linear(a, w, bias=None, out_dtype=None, residual=None, out=None, glu=False, 
                                     a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
     if fused and a.dtype != torch.bfloat16:
         raise KernelError("linear: norm, emit and rope ride only with bfloat16 products")
+    if variant == "gemm_tc":
+        plan = product_plan(m, n, k)
     if variant == "gemm_tc" and fused:
-        parts = _tc_scratch(a.device, m, n, k)
+        parts = _tc_scratch(a.device, plan)
         applied = _c_int(0)
         _call("gemm_tc", "llmb_gemm_tc_ex", _ptr(a), _c_int(a.stride(0)), _ptr(w), _ptr(bias),
               _ptr(result if residual is None else None), _c_int(_code(target_dtype)),
               _ptr(residual), *_scratch_arguments(*parts), _c_int(m), _c_int(n), _c_int(k), _c_int(n),
               _c_int(0), _c_int(0 if tactics.is_disabled("gemm_tc_pair") else 1),
               ctypes.byref(_fusion_struct(norm, emit, rope)), ctypes.byref(applied), _stream(),
-              kernels=_tc_kernels(m, n, k))
+              kernels=plan.kernels)
         if emit is not None:
             if applied.value & FUSED_EMIT:
-                emit.parts = _tc_emit_parts(m, n, k)
+                emit.parts = plan.emit_parts
             else:
                 cast_sumsq(residual, emit)
         if rope is not None and not applied.value & FUSED_ROPE:
@@ -1239,12 +1239,12 @@ def linear(a, w, bias=None, out_dtype=None, residual=None, out=None, glu=False, 
                              rope.interleaved, rope.write_cache)
         return result
     if variant == "gemm_tc":
-        parts = _tc_scratch(a.device, m, n, k)
+        parts = _tc_scratch(a.device, plan)
         _call("gemm_tc", "llmb_gemm_tc", _ptr(a), _c_int(a.stride(0)), _ptr(w), _ptr(bias),
               _ptr(result if residual is None else None), _c_int(_code(target_dtype)),
               _ptr(residual), *_scratch_arguments(*parts), _c_int(m), _c_int(n), _c_int(k), _c_int(n),
               _c_int(0), _c_int(0 if tactics.is_disabled("gemm_tc_pair") else 1), _stream(),
-              kernels=_tc_kernels(m, n, k))
+              kernels=plan.kernels)
     elif variant == "gemm_skinny":
         partials, counters = _skinny_scratch(a.device, m, n, k)
         _call("gemm_skinny", "llmb_gemm_skinny", _ptr(a), _c_int(a.stride(0)), _ptr(w), _ptr(bias),
