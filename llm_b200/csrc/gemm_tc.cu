@@ -2100,9 +2100,12 @@ Plan make_plan(int M, int N, int K) {
     return p;
 }
 
+// Where a product's results go: what an epilogue costs depends on it.
+enum Target { TO_BF16, TO_F32, TO_RESIDUAL, TO_GATED };
+
 // Whether a product runs with its weights on the pairs' row side, and how: the width of the token tiles and the pairs a tile, if any,
-// whose estimate is below the other kernels' by 4 %. Estimates in us, from the measured times of 160 products of 17 to 3,001
-// tokens with 2,048 to 28,672 outputs and K from 2,048 to 14,336, which they meet within some 10 %:
+// whose estimate is below the other kernels' by 4 %, provided that it stays so when what leaves the tiles is counted. Estimates in us,
+// from the measured times of 1,700 products of 129 to 2,100 tokens with 256 to 131,000 outputs and K from 64 to 16,384:
 // * here, a round of 74 pairs takes 0.2 us a k-block up to 128 tokens a tile (the loads' pace) and 0.00151 us a token above, a call 4 us
 //   more, or 8 where pairs share a tile; a gated tile's activations take 0.06 us a token, under the next round's products and
 //   behind the last one's;
@@ -2110,40 +2113,54 @@ Plan make_plan(int M, int N, int K) {
 //   where there is no full one) and 12, and 6 for the last tiles' activations;
 // * weights on one block's row side, tokens in tiles of 128: the weights at 6.5 TB/s, 1.4 ns a tile and k-block, 4.5 a call; it
 //   leaves a norm's input or rotates in its sum, which takes a kernel of some 4 us behind this one;
-// none faster than its weights at 5.5 TB/s.
-// Others -> here: 350 x 6144 x 4096 27.7 -> 19.7, 350 x 4096 x 4096 25.5 -> 16.9, 350 x 28672 x 4096 89.5 -> 80.8, 350 x 4096 x 14336 46.8 ->
-// 39.9, 512 x 4096 x 14336 62.1 -> 49.9, 160 x 6144 x 4096 22.0 -> 17.6, 1300 x 4096 x 4096 45.3 -> 37.0; and not taken: 512 x 28672 x
-// 4096 94.8 (99.6 here), 1024 x 4096 x 4096 27.6 (29.5), 2048 x 6144 x 4096 72.8 (78).
+// none faster than its weights at 5.5 TB/s. With a short K a round takes what its tiles need to leave: bfloat16 rows 1.8 us and 0.023 a
+// token here and 5 there (9 the call), additions to the residual 1.25 and 0.022 (in a single round they are in its 4 us) and
+// 5.5; 32-bit results are always faster here. Additions of more than 200 us stay there unless 12 % are in it, since at the power
+// cap both ways end up together, and a gated round of more than 64 k-blocks against tiles on pairs took a third longer.
+// Others -> here: 350 x 6144 x 4096 27.0 -> 19.3, 350 x 4096 x 4096 28.0 -> 18.4, 350 x 28672 x 4096 gated 101 -> 86, 350 x 4096 x 14336 47.5 ->
+// 41.1, 600 x 4096 x 14336 85.9 -> 64.1, 1300 x 4096 x 4096 49.6 -> 39.1. Before what leaves was counted, short products of many
+// outputs came here that are slower: 598 x 113152 x 128 107 -> 150, 855 x 24448 x 320 38 -> 51, 1365 x 16000 x 512 41 -> 51.
 // Up to 128 tokens the sums' fused epilogues are worth more; a gated product, which has none, is faster here alone (64 x 16384 x
 // 2048 18.5 -> 17.3), and a decode step of 64 sequences with it is not (2,558 -> 2,574 us): the kernel in front has its SMs longer.
-bool plan_wide(int M, int N, int K, int glu, WideWork* best) {
+bool plan_wide(int M, int N, int K, Target target, WideWork* best) {
     if (M <= SWAP_TOKENS || M > 2048 || N < 256) return false;
     Plan p = make_plan(M, N, K);
+    const bool glu = target == TO_GATED;
     const int kblocks = p.n_kblocks, tiles_w = (N + 2 * BM - 1) / (2 * BM);
     const double weights = 2.0 * N * K * 1e-6, epilogue = glu ? 6.0 : 0.0, least = weights / 5.5 + 4.0 + epilogue;      // (bytes in MB, us)
-    double others;
-    if (on_pairs(p, M, N)) {
-        int n_pairs;
-        PairWork w = plan_pairs(M, N, K, &n_pairs);
-        const int units = w.tiles_a * w.tiles_b;
-        others = epilogue + (w.tail_tiles > 0 ? (double)units / PAIRS * kblocks * (units < PAIRS ? 0.48 : 0.38) + 12.0 : (double)((units + PAIRS - 1) / PAIRS) * kblocks * 0.35 + 4.0);
-    } else {
-        others = weights / 6.5 + 4.5 + epilogue + 0.0014 * p.tiles_a * p.tiles_b * kblocks;
-    }
-    if (others < least) others = least;
-    double lowest = others / 1.04;
-    bool found = false;
     const double behind = p.swap && p.splits > 1 && !glu ? 4.0 : 0.0;
+    // the other kernels, a round of whose 256 x 256 tiles takes `leave` at least
+    auto others = [&](double leave) {
+        double t;
+        if (on_pairs(p, M, N)) {
+            int n_pairs;
+            PairWork w = plan_pairs(M, N, K, &n_pairs);
+            const int units = w.tiles_a * w.tiles_b, rounds = (units + PAIRS - 1) / PAIRS;
+            const double round = kblocks * 0.35;
+            t = epilogue + (w.tail_tiles > 0 ? (double)units / PAIRS * kblocks * (units < PAIRS ? 0.48 : 0.38) + 12.0
+                                             : rounds * (round > leave ? round : leave) + 4.0);
+        } else {
+            t = weights / 6.5 + 4.5 + epilogue + 0.0014 * p.tiles_a * p.tiles_b * kblocks;
+        }
+        return t > least ? t : least;
+    };
+    // this kernel, with tiles of bn tokens and `splits` pairs a tile
+    auto here = [&](int bn, int splits, double leave, double slower) {
+        const int units = (M + bn - 1) / bn * tiles_w, rounds = splits > 1 ? 1 : (units + PAIRS - 1) / PAIRS;
+        const double last = glu ? 0.06 * bn : 0.0;
+        double round = ((kblocks + splits - 1) / splits) * (bn <= 128 ? 0.2 : 0.00151 * bn) * slower;
+        if (round < last) round = last;
+        const double t = rounds * (round > leave ? round : leave) + (splits > 1 ? 8.0 : 4.0) + last;
+        return (t > least ? t : least) + behind;
+    };
+    double lowest = others(0.0) / 1.04;
+    bool found = false;
     for (int bn = 64; bn <= PAIR_BN; bn += 32) {
         const int tiles_t = (M + bn - 1) / bn, units = tiles_t * tiles_w;
         for (int splits = 1; splits <= 3; ++splits) {
             // (clusters of four blocks fit 34 times beside each other, of six 18 times; more would wait for a second wave)
             if (splits > 1 && (units > (splits == 2 ? 34 : 18) || kblocks < 8 * splits)) continue;
-            const int rounds = splits > 1 ? 1 : (units + PAIRS - 1) / PAIRS;
-            const double last = glu ? 0.06 * bn : 0.0, round = ((kblocks + splits - 1) / splits) * (bn <= 128 ? 0.2 : 0.00151 * bn);
-            double t = rounds * (round > last ? round : last) + (splits > 1 ? 8.0 : 4.0) + last;
-            if (t < least) t = least;
-            t += behind;
+            const double t = here(bn, splits, 0.0, 1.0);
             if (t < lowest) {
                 lowest = t;
                 *best = WideWork{kblocks, tiles_t, tiles_w, bn, splits};
@@ -2151,7 +2168,13 @@ bool plan_wide(int M, int N, int K, int glu, WideWork* best) {
             }
         }
     }
-    return found;
+    if (!found || target == TO_F32) return found;
+    const bool one_round = best->splits > 1 || best->tiles_t * best->tiles_w <= PAIRS;
+    const double leave = target == TO_BF16 ? 1.8 + 0.023 * best->bn : target == TO_RESIDUAL && !one_round ? 1.25 + 0.022 * best->bn : 0.0;
+    double there = others(target == TO_BF16 ? 5.0 : target == TO_RESIDUAL ? 5.5 : 0.0);
+    if (target == TO_BF16 && there < 9.0) there = 9.0;
+    const double t = here(best->bn, best->splits, leave, glu && !p.swap && one_round && kblocks > 64 ? 1.3 : 1.0);
+    return t * (target == TO_RESIDUAL && there > 200.0 ? 1.12 : 1.0) < there;
 }
 
 // Which kernel a product takes and what that kernel needs: the one answer that the launch and all questions about it share.
@@ -2167,10 +2190,10 @@ struct Choice {
     bool can_rotate;                    // the q/k/v product's rotation, where its heads fit the tiles
 };
 
-Choice choose(int M, int N, int K, int glu, int allow_pair) {
+Choice choose(int M, int N, int K, Target target, int allow_pair) {
     Choice c = {};
     c.kernels = 1;
-    if (allow_pair && plan_wide(M, N, K, glu, &c.wide)) {
+    if (allow_pair && plan_wide(M, N, K, target, &c.wide)) {
         c.kernel = Choice::ROW_SIDE;
         return c;
     }
@@ -2214,11 +2237,12 @@ LLMB_EXPORT int llmb_gemm_tc_status() {
     return v;
 }
 
-// What a call of these sizes does and needs: {kernel (0 blocks, 1 pairs, 2 row side), token or column width of its tiles, blocks
+// What a call of these sizes does and needs, its results going to `target` (0 bfloat16, 1 float32, 2 the residual, 3 the gated
+// activation in bfloat16): {kernel (0 blocks, 1 pairs, 2 row side), token or column width of its tiles, blocks
 // or pairs that share a tile's K, tiles cut along K in the last round, floats of partial sums, tile counters, kernels launched,
 // partial sums of squares a row that emit_rows / emit_sumsq leave (0: the caller runs llmb_cast_sumsq behind the product)}.
-LLMB_EXPORT int llmb_gemm_tc_plan(int M, int N, int K, int glu, int allow_pair, long long* out) {
-    Choice c = choose(M, N, K, glu, allow_pair);
+LLMB_EXPORT int llmb_gemm_tc_plan(int M, int N, int K, int target, int allow_pair, long long* out) {
+    Choice c = choose(M, N, K, (Target)target, allow_pair);
     const bool blocks = c.kernel == Choice::BLOCKS, row_side = c.kernel == Choice::ROW_SIDE;
     const long long values[8] = {(long long)c.kernel, row_side ? c.wide.bn : blocks ? c.plan.bn : PAIR_BN,
                                  row_side ? c.wide.splits : blocks ? c.plan.splits : 1,
@@ -2257,7 +2281,8 @@ LLMB_EXPORT int llmb_gemm_tc_ex(const void* x, int ldx, const void* w, const flo
     } else {
         LLMB_REQUIRE(ldo >= N, "gemm_tc: bad output stride");
     }
-    const Choice choice = choose(M, N, K, glu, allow_pair);
+    const Target target = glu ? TO_GATED : residual ? TO_RESIDUAL : out_dtype == LLMB_DTYPE_BF16 ? TO_BF16 : TO_F32;
+    const Choice choice = choose(M, N, K, target, allow_pair);
     const Plan& p = choice.plan;
     LLMB_REQUIRE((long long)p.tiles_a * p.tiles_b * p.splits < (1ll << 30), "gemm_tc: too many tiles");
     if (choice.counters > 0) {

@@ -1062,19 +1062,22 @@ def _skinny_scratch(device, m, n, k):
 ProductPlan = collections.namedtuple("ProductPlan", "kernel width splits tail scratch_floats counters kernels emit_parts")
 
 
+TARGETS = ("bfloat16", "float32", "residual", "gated")       # where a product's results go (enum Target of csrc/gemm_tc.cu)
+
+
 @functools.lru_cache(maxsize=4096)
-def _tc_plan(m: int, n: int, k: int, glu: bool, pairs: bool) -> ProductPlan:
+def _tc_plan(m: int, n: int, k: int, target: int, pairs: bool) -> ProductPlan:
     out = (ctypes.c_longlong * 8)()
-    load_library("gemm_tc").llmb_gemm_tc_plan(_c_int(m), _c_int(n), _c_int(k), _c_int(1 if glu else 0), _c_int(1 if pairs else 0), out)
+    load_library("gemm_tc").llmb_gemm_tc_plan(_c_int(m), _c_int(n), _c_int(k), _c_int(target), _c_int(1 if pairs else 0), out)
     return ProductPlan(("blocks", "pairs", "row_side")[out[0]], *out[1:])
 
 
-def product_plan(m: int, n: int, k: int, glu: bool = False) -> ProductPlan:
-    """What a tcgen05 product of these sizes runs as, with `glu` in its epilogue or not: `kernel` ("blocks": single SMs, "pairs":
-    256 x 256 tiles on pairs of SMs, "row_side": pairs with the weights on the row side), the `width` of its tiles, how many
-    share a tile's K (`splits`), tiles cut along K in the last round (`tail`), floats of partial sums and tile counters it
-    needs, kernels it launches, and the partial sums of squares a row that it leaves for the next norm (0: none)."""
-    return _tc_plan(m, n, k, bool(glu), not tactics.is_disabled("gemm_tc_pair"))
+def product_plan(m: int, n: int, k: int, target: str = "bfloat16") -> ProductPlan:
+    """What a tcgen05 product of these sizes runs as, its results going to `target` (one of TARGETS): `kernel` ("blocks": single
+    SMs, "pairs": 256 x 256 tiles on pairs of SMs, "row_side": pairs with the weights on the row side), the `width` of its
+    tiles, how many share a tile's K (`splits`), tiles cut along K in the last round (`tail`), floats of partial sums and tile
+    counters it needs, kernels it launches, and the partial sums of squares a row that it leaves for the next norm (0: none)."""
+    return _tc_plan(m, n, k, TARGETS.index(target), not tactics.is_disabled("gemm_tc_pair"))
 
 
 def _tc_scratch(device, plan) -> tuple:
@@ -1175,7 +1178,7 @@ def linear(a, w, bias=None, out_dtype=None, residual=None, out=None, glu=False, 
                               "K % 8 == 0, no bias and no residual")
         _check_out(out, (m, n // 2), a.dtype, "linear")
         result = out if out is not None else torch.empty((m, n // 2), dtype=a.dtype, device=a.device)
-        plan = product_plan(m, n, k, True)
+        plan = product_plan(m, n, k, "gated")
         parts = _tc_scratch(a.device, plan)
         if emit is not None or rope is not None:
             raise KernelError("linear: the gated epilogue takes a folded norm only")
@@ -1202,7 +1205,8 @@ def linear(a, w, bias=None, out_dtype=None, residual=None, out=None, glu=False, 
     if fused and a.dtype != torch.bfloat16:
         raise KernelError("linear: norm, emit and rope ride only with bfloat16 products")
     if variant == "gemm_tc":
-        plan = product_plan(m, n, k)
+        plan = product_plan(m, n, k, "residual" if residual is not None else
+                            "bfloat16" if target_dtype == torch.bfloat16 else "float32")
     if variant == "gemm_tc" and fused:
         parts = _tc_scratch(a.device, plan)
         applied = _c_int(0)
