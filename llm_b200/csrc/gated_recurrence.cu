@@ -714,7 +714,10 @@ LLMB_EXPORT int llmb_gated_recurrence(const void* y, int y_stride, const void* x
     float* decay = work + (size_t)n_tokens * channels;
     float* drive = decay + (size_t)n_tokens * channels;
     auto gates = long_step ? gates_kernel<8> : gates_kernel<2>;
-    bool on_tensor_cores = gate_rows && part % TC_CHANNELS == 0 &&
+    // Up to 64 tokens a part of 64 or 128 channels is over on the CUDA cores before the tensor cores are set up: one token of 1,024
+    // channels in 16 parts 10.1 us, 14.2 there, 64 tokens of 4,096 in 64 parts 14.8, 18.7; in 32 parts 18.7, 19.8. From 65
+    // tokens (96 in 64 parts 28.7, 21.0) or parts of 192 channels (one token of 1,152 in 6 parts 17.7, 16.1) on it is not.
+    bool on_tensor_cores = gate_rows && part % TC_CHANNELS == 0 && (long_step || part > 128) &&
                            (((size_t)gate_rows | (size_t)work | (size_t)gate_a_bias | (size_t)gate_i_bias | (size_t)rate) % 16) == 0;
     const size_t tc_smem = 1024 + (size_t)TC_STAGES * TC_STAGE;
     int n_units = ceil_div(n_tokens, TC_TOKENS) * (channels / TC_CHANNELS);

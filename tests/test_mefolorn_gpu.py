@@ -434,6 +434,25 @@ def test_gates_on_the_tensor_cores(channels, blocks, new):
         assert float((got_drive - want_drive).abs().max()) <= 5e-4 * float(want_drive.abs().max())
 
 
+@pytest.mark.parametrize("channels,blocks,tokens,tensor_cores", [(64, 1, 1, False), (256, 2, 64, False), (1024, 16, 17, False),
+                                                                 (64, 1, 65, True), (256, 2, 65, True), (192, 1, 1, True)])
+def test_short_steps_of_small_parts_stay_on_the_cuda_cores(channels, blocks, tokens, tensor_cores):
+    """Parts of up to 128 channels: the bits of the 32-bit kernel up to 64 tokens, other sums behind them."""
+    ops = _ops()
+    batch = Batch([3], [tokens], seed=2)
+    wide, p, state = _recurrence_inputs(channels, blocks, 4, tokens, 3, torch.bfloat16, seed=channels + tokens)
+    for name in ("gate_a", "gate_i"):
+        p[name] = p[name].bfloat16().float()
+    work = [torch.empty((3, tokens, channels), device=DEV) for _ in range(2)]
+    for w, rows in zip(work, (None, ops.gate_rows_of(p["gate_a"], p["gate_i"]))):
+        out = torch.empty((tokens, channels), dtype=torch.bfloat16, device=DEV)
+        ops.gated_recurrence(wide[:, :channels], wide[:, channels:2 * channels], p["conv_w"], p["conv_b"], p["gate_a"], p["gate_a_bias"],
+                             p["gate_i"], p["gate_i_bias"], p["rate"], state.clone(), batch.tok_seq, batch.cu, batch.slots, out, 0.9, w,
+                             gate_rows=rows)
+    torch.cuda.synchronize()
+    assert torch.equal(work[0][:2], work[1][:2]) != tensor_cores
+
+
 def test_gate_rows_need_bfloat16_values():
     ops = _ops()
     gate = torch.randn((2, 64, 64), generator=torch.Generator().manual_seed(3)).to(DEV)
