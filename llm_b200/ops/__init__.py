@@ -1715,10 +1715,11 @@ GATE_GROUP = 64                                 # channels whose rows of both ga
 def gate_rows_of(gate_a, gate_i):
     """Both gate matrices (float32 [blocks, P, P]) as gated_recurrence's tensor-core kernel reads them: bfloat16
     [2 blocks P, P], per 64 channels their rows of gate_a and then of gate_i. None where P is no multiple of 64 or a value is
-    not a bfloat16 number (then the gates are summed from the 32-bit matrices)."""
+    not a finite bfloat16 number (then the gates are summed from the 32-bit matrices: the tensor cores multiply every weight
+    with parts of the input that may be zero, and zero times infinity is not a number)."""
     blocks, part, _ = gate_a.shape
     rows = torch.stack([g.to(torch.bfloat16) for g in (gate_a, gate_i)], dim=1)                # [blocks, 2, P, P]
-    if part % GATE_GROUP or not torch.equal(rows.float(), torch.stack([gate_a, gate_i], dim=1)):
+    if part % GATE_GROUP or not torch.equal(rows.float(), torch.stack([gate_a, gate_i], dim=1)) or not rows.isfinite().all():
         return None
     return rows.view(blocks, 2, part // GATE_GROUP, GATE_GROUP, part).transpose(1, 2).reshape(2 * blocks * part, part).contiguous()
 

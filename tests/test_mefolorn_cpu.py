@@ -228,3 +228,14 @@ def test_the_room_for_mixed_queries_never_shrinks_as_steps_grow():
             assert room >= last and at_once >= 1 and at_once * n * groups * dim <= room, (heads, n)
             assert 2 * room <= max(ops.SIGMOID_MIXED_BYTES, 2 * n * groups * dim)
             last = room
+
+
+def test_gate_matrices_with_infinities_stay_in_32_bits():
+    """A weight of infinity times the zero part of an input would not be a number; the 32-bit sums keep their infinity."""
+    from llm_b200 import ops
+    gate = torch.randn((2, 64, 64), generator=torch.Generator().manual_seed(3)).bfloat16().float()
+    assert ops.gate_rows_of(gate, gate) is not None
+    for value in (float("inf"), float("-inf"), float("nan")):
+        other = gate.clone()
+        other[1, 5, 7] = value
+        assert ops.gate_rows_of(gate, other) is None and ops.gate_rows_of(other, gate) is None
