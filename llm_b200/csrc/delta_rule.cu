@@ -497,7 +497,8 @@ LLMB_EXPORT int llmb_delta_rule(const void* proj, int ld, int dtype, const float
             int tok = n_tokens >= 4 * 148 ? 4 : 1;                                                                 \
             auto kernel = D == 128 ? (tok == 4 ? delta_prepare_pieces_kernel<T, 4, 4> : delta_prepare_pieces_kernel<T, 4, 1>) \
                                    : (tok == 4 ? delta_prepare_pieces_kernel<T, 2, 4> : delta_prepare_pieces_kernel<T, 2, 1>); \
-            dim3 grid((n_tokens + tok - 1) / tok, tok == 4 ? PIECE_BLOCKS : (G + (H * V + D - 1) / D + THREADS / 32) / (THREADS / 32)); \
+            int pieces = G + (H * V + D - 1) / D + 1, full = (pieces + THREADS / 32 - 1) / (THREADS / 32);                      \
+            dim3 grid((n_tokens + tok - 1) / tok, tok == 4 && full > PIECE_BLOCKS ? PIECE_BLOCKS : full);                        \
             LLMB_CUDA(llmb::launch(kernel, grid, dim3(THREADS), 0, stream, true, (const T*)proj, ld, taps,         \
                                    (const float*)state, state_stride, tok_seq, cu_seqlens, slot_ids, rate, dt_bias, \
                                    unit_eps, work, work_ld, n_tokens, H, G, V));                                   \
