@@ -10,10 +10,10 @@
 // One block serves 128 queries of one head of one sequence and walks the visible keys in
 // blocks of 64 (one cache page):
 //
-// * warp 0, one lane: TMA for Q (once) and for the keys; warp 6, one lane: TMA for the values. 64 x 64
+// * warp 0: TMA for Q (once) and for the keys; warp 6: TMA for the values; one elected lane of each issues. 64 x 64
 //   boxes, two buffers each for K and V with barriers of their own, so that a buffer is requested
 //   again as soon as the product that read it is complete.
-// * warp 1, one lane: issues the products. S[128 q, 64 keys] = Q K^T (K=16 steps over the head
+// * warp 1, one elected lane: issues the products. S[128 q, 64 keys] = Q K^T (K=16 steps over the head
 //   dimension, both operands K-major in shared memory) into one of TWO score buffers in tensor memory
 //   (columns 0-63 and 64-127); then O[128 q, d] += P V with P read from tensor memory and V from shared
 //   memory as an MN-major operand (its rows are keys, the contiguous direction is d), accumulating in

@@ -5,9 +5,9 @@
 // is a softmax attention of its own over its half of the key rows and the same values, so a block holds two
 // pipelines that share the keys' and values' tiles:
 //
-// * warp 8, one lane: TMA for the queries (once) and the key pages; warp 10, one lane: TMA for the value pages.
-//   64 x 64 boxes, STAGES pages of each in flight.
-// * warp 9, one lane: issues the products. Per map S[128, 64 keys] = Q K^T into one of two score buffers, and
+// * warp 8: TMA for the queries (once) and the key pages; warp 10: TMA for the value pages; one elected lane of each
+//   issues. 64 x 64 boxes, STAGES pages of each in flight.
+// * warp 9, one elected lane: issues the products. Per map S[128, 64 keys] = Q K^T into one of two score buffers, and
 //   O[128, DV] += P V with P read from tensor memory (over the buffer's first 32 columns) and V an MN-major
 //   operand. The scores of page n + 2 of a map are issued right behind P V of page n, as in attention_prefill_tc.
 // * warps 0-3 are the softmax of map 1, warps 4-7 that of map 2; a thread owns a query row. While one map's

@@ -1557,7 +1557,7 @@ pair_tail_sum_kernel(float* partials, Epilogue ep, PairWork work) {
 
 // ------------------------------------------------------------------------- weights on the pair's row side
 // From some tokens to some thousand, 256 x 256 tiles with the tokens as rows are too coarse: 350 tokens fill 512 rows, a
-// 4,096-wide output has 32 tiles for 74 pairs, and a tile takes its 26 us (64 k-blocks) whatever the other pairs do. Here the
+// 4,096-wide output has 32 tiles for 74 pairs, and a tile takes its 18 us (64 k-blocks) whatever the other pairs do. Here the
 // weights are the 256 rows of a pair's tile and the tokens its N side, whose width (64 to 256, a multiple of 32) is chosen
 // so that the tokens fill it; and where the tiles are too few, `splits` pairs of one cluster share a tile, each with a
 // slice of its k-blocks. Their accumulators meet in shared memory: when every pair of the cluster is done, each block
@@ -2032,17 +2032,18 @@ struct Plan {
 
 // The weights take the 128-row side of the tiles (tokens in tiles of up to 128 on the other) and K is split over blocks up to
 // 128 tokens, and up to 1,024 tokens where 256 x 256 tiles are too few for the pairs of SMs even when cut along K. (With the
-// tokens on the 128-row side a 128 x 4096 x 4096 product has 16 tiles and took 38 us; this way it takes 16. At 512 x 6144 x
-// 4096 the 48 pair tiles are faster again: 28 against 34 us.)
+// tokens on the 128-row side a 128 x 4096 x 4096 product has 16 tiles and took 38 us; this way it takes 14. At 512 x 6144 x
+// 4096 the 48 pair tiles are faster again: 27 against 32 us.)
 constexpr int SWAP_TOKENS = 128, SWAP_TOKENS_MOST = 1024;
 
-// How the pairs share the tiles (PairWork). A tile takes 0.4 us a k-block whatever the other pairs do, so a last round of R of
+// How the pairs share the tiles (PairWork). A tile takes 0.35 us a k-block whatever the other pairs do, so a last round of R of
 // 74 tiles wastes (74 - R) / 74 of it. Cut into pieces (multiples of four k-blocks, at least an eighth of a tile) it takes
-// R / 74 of a tile's time, but leaving the parts and adding them in a kernel behind takes about 12 us, 30 k-blocks, and the
-// pairs, each at another k, no longer share what they read, about a third of a piece. The cut is made where it saves
-// more than that. Measured, whole tiles -> cut: 350 x 28672 x 4096 (224 tiles) 98.7 -> 93.4 us, 3001 x 28672 x 4096 (1,344)
-// 531 -> 494, 1300 x 4096 x 14336 (96) 150 -> 127, 256 x 6144 x 4096 (24) 26.4 -> 22.6; and not cut because slower:
-// 512 x 4096 x 4096 (32) 26.2 -> 29.2, 2048 x 4096 x 14336 (128) 174 -> 182.
+// R / 74 of a tile's time, but leaving the parts and adding them in a kernel behind takes about 12 us, 34 k-blocks (30 when the line
+// was drawn, at 0.4 us a k-block), and the pairs, each at another k, no longer share what they read, about a third of a piece. The cut
+// is made where it saves more than 30 and that. Measured, whole tiles -> cut, with the norm's input behind a residual: 1300 x 4096 x
+// 14336 (96 tiles) 178 -> 139 us, 2500 x 4096 x 14336 (160) 287 -> 231, 256 x 6144 x 4096 (24) 32.2 -> 29.4, 350 x 28672 x 4096 gated (224)
+// 106 -> 99, and long gated ones about even at the power cap, 2048 x 28672 x 4096 (896) 351 -> 350, 3001 (1,344) 529 -> 535; not cut
+// because slower: 512 x 4096 x 4096 (32) 29.4 -> 33.8, 2048 x 4096 x 14336 (128) 203 -> 205, 2048 x 6144 x 4096 (192) 81 -> 91.
 PairWork plan_pairs(int M, int N, int K, int* n_pairs) {
     PairWork w;
     w.n_kblocks = (K + BK - 1) / BK;
@@ -2071,9 +2072,10 @@ Plan make_plan(int M, int N, int K) {
     Plan p;
     p.n_kblocks = (K + BK - 1) / BK;
     long long pair_tiles = (long long)((M + 255) / 256) * ((N + 255) / 256);
-    // (a pair's tile of 64 k-blocks takes 26 us alone, whatever fills the other pairs: with a short K the pairs win from 24
-    // tiles on, 512 x 4096 x 4096 in 26.1 against 38.3 us; with a long K the split products stay ahead until the pairs are
-    // well filled, 350 x 4096 x 14336 in 59 us against 69 cut along K)
+    // (a pair's tile of 64 k-blocks takes 18 us alone, whatever fills the other pairs: with a short K the pairs win from some 24
+    // tiles on, 512 x 6144 x 4096 in 27.3 against 31.8 us, 700 x 3072 x 2048 in 16.9 against 18.8; with a long K the split products
+    // stay ahead until the pairs are well filled, 350 x 4096 x 14336 in 48 us against 59. What leaves the next norm's input in its
+    // sum is ahead longer, 512 x 4096 x 4096 in 25.1 against 27.7 and 1000 x 2048 x 8192 in 38.6 against 43.3: the row side has most of those)
     bool few_tiles = p.n_kblocks <= 64 ? pair_tiles < 24 : pair_tiles * 5 < PAIRS * 3;
     p.swap = M <= SWAP_TOKENS || (M <= SWAP_TOKENS_MOST && few_tiles);
     if (p.swap) {
@@ -2105,7 +2107,8 @@ enum Target { TO_BF16, TO_F32, TO_RESIDUAL, TO_GATED };
 
 // Whether a product runs with its weights on the pairs' row side, and how: the width of the token tiles and the pairs a tile, if any,
 // whose estimate is below the other kernels' by 4 %, provided that it stays so when what leaves the tiles is counted. Estimates in us,
-// from the measured times of 1,700 products of 129 to 2,100 tokens with 256 to 131,000 outputs and K from 64 to 16,384:
+// from the measured times of 1,700 products of 129 to 2,100 tokens with 256 to 131,000 outputs and K from 64 to 16,384 (the layers'
+// among them stand in profiles/gemm_tc__row_side_or_not.txt):
 // * here, a round of 74 pairs takes 0.2 us a k-block up to 128 tokens a tile (the loads' pace) and 0.00151 us a token above, a call 4 us
 //   more, or 8 where pairs share a tile; a gated tile's activations take 0.06 us a token, under the next round's products and
 //   behind the last one's;

@@ -20,9 +20,11 @@
 // cluster (up to eight: blocks_a_row) each read their share of the row, tell each other how many elements they have from
 // their own cut on, gather what can be among the row's top_k and hand it to the first block, which ranks it and draws. The
 // row is read twice (the second time from L1), and two blocks an SM (64 registers a thread) keep the clusters of 32 rows in
-// one wave: with one, 42 us. Copying 32 rows of 128,256 logits and drawing from them with the default parameters: 76 us
-// with one block a row, 44 with the row's histograms summed over the cluster digit by digit, 36 now, of which the copy takes
-// 4.4, the penalty's four dependent reads 3.4, the cuts 4.4, the candidates 4.7, their sort 3.9 and the draw 2.2.
+// one wave: with one, 42 us. Copying 32 rows of 128,256 logits and drawing from them with the default parameters, call after
+// call from the host: 76 us with one block a row, 44 with the row's histograms summed over the cluster digit by digit, 35 now, of
+// which the copy takes 4.4, the penalty's four dependent reads 3.4, the cuts 4.4, the candidates 4.7, their sort 3.9 and the draw
+// 2.2. (The figures below are of calls in a graph, where the launches' gaps are shorter: 38 and 31 us.) Rows of which all but some
+// spread entries are -inf do the row's select behind the shares' cuts: 41 to 16,000 allowed ones 26 to 31 us, 36 to 38 before.
 #include <cooperative_groups.h>
 
 #include "common.cuh"
@@ -194,8 +196,8 @@ argmax_rows_kernel(const float* __restrict__ logits, int stride, int vocab, int*
 
 // How many blocks share a row. A row of a large vocabulary is long enough for several, as long as they fill no more than the
 // GPU. What a cluster costs a short row is its barriers. The default chain behind a copy of the logits, with the row's
-// histograms summed over the cluster -> as it is now: 8 rows of 128,256 35 -> 25 us, 32 rows 41 -> 31, 64 rows 49 -> 39, 32 rows
-// of 32,000 30 -> 23 (one block a row took 30 more at 8 rows of 128,256). Eight blocks where one is chosen, when that was
+// histograms summed over the cluster -> as it is now: 8 rows of 128,256 32 -> 25 us, 32 rows 38 -> 31, 64 rows 47 -> 39, 32 rows
+// of 32,000 27 -> 21 (one block a row took 30 more at 8 rows of 128,256). Eight blocks where one is chosen, when that was
 // decided: 256 rows of 128,256 147 -> 258, 148 rows of 32,000 36 -> 81, 1,024 rows of 4,096 82 -> 406.
 static int blocks_a_row(int n_rows, int vocab) {
     if (vocab < 16384) return 1;

@@ -57,7 +57,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 }
 // Loops that issue copies or products are run by a whole warp, and one elected lane issues: with a loop of one lane alone the
 // compiler keeps stages, phases and descriptors in the lanes' registers and moves each operand to the uniform ones in front
-// of every instruction. Four products of a k-block took 277 cycles of issue so and take some 50 run by the warp. Prefill attention
+// of every instruction. Four products of a k-block took 277 cycles of issue so and take 111 run by the warp. Prefill attention
 // of 350 / 1,024 / 2,048 tokens 10.4 -> 9.9, 20.2 -> 18.8, 46.0 -> 43.8 us, routed experts of 777 tokens 456 -> 448.
 __device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
 __device__ __forceinline__ bool elect_one() {

@@ -10,7 +10,9 @@ behind 0 to 8,000) of 16 combinations of heads, sizes and windows: the worst of 
 takes 13 % longer than the better kernel (0.9 us), all others at most 6 %. With tcgen05 at every
 step, up to 1.9 times as long as mma.sync (8 sequences of 16 tokens, 32 heads of 2 x 64: 17.8 us for
 9.3); with mma.sync at every step, up to 7.6 times as long as tcgen05 (8 sequences of 128 tokens
-behind 2,000, 32 mixed heads of 128 over 8: 1,583 us for 210).
+behind 2,000, 32 mixed heads of 128 over 8: 1,583 us for 210). Since then the tcgen05 kernels' loops are
+issued by whole warps and long walks on them take 5 to 7 % less; the numbers are still those of the 36 steps,
+so that a step near the line may be on mma.sync by that much.
 """
 from __future__ import annotations
 
