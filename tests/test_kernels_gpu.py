@@ -120,9 +120,9 @@ def _check_decode_product(m, n, k):
                                    (300, 4104, 2048), (256, 4096, 4096), (1000, 2304, 1536),
                                    (140, 19200, 128), (2500, 8192, 192)])
 def test_linear_tensor_core_kernel(m, n, k):
-    """tcgen05 product for more than 64 tokens: tile edges in M, N and K. Shapes with few output
-    tiles run with the weights on the 128-row side, several token tiles and split K (513 x 6144,
-    300 x 4104), the others as 256 x 256 tiles on pairs of SMs (2048 x 4096)."""
+    """tcgen05 product for more than 64 tokens: tile edges in M, N and K, on each of its kernels: weights on the 128-row side with
+    several token tiles and split K (256 x 4096), on the pairs' row side (513 x 6144, 300 x 4104), 256 x 256 tiles on pairs
+    of SMs (2500 x 8192)."""
     from llm_b200.ops import tactics
     assert tactics.choose_linear(m, n, k, torch.bfloat16, torch.bfloat16, k) == "gemm_tc"
     a = randn(m, k, dtype=torch.bfloat16, seed=84)
@@ -169,12 +169,16 @@ def test_linear_with_gated_epilogue(m, f, k):
     assert ops().tensor_core_status() == 0
 
 
-@pytest.mark.parametrize("m,n,k", [(350, 4096, 4096), (129, 2048, 14336), (257, 2048, 8192), (1300, 4096, 4096),
-                                   (300, 2112, 2056), (777, 28672, 1024), (2077, 6144, 1600)])
-def test_linear_cuts_the_last_round_of_tiles(m, n, k):
-    """Products whose last round of 256 x 256 tiles leaves pairs idle: its tiles are cut along K over all pairs and their parts
-    added, for each epilogue, with one part order (two runs give the same bits). Largest error of a sum of k products of
-    bfloat16 values in 32 bits: k 2^-24 of the sum of magnitudes, far inside 2e-3 of the largest result."""
+@pytest.mark.parametrize("m,n,k,cut", [(350, 4096, 4096, 0), (129, 2048, 14336, 0), (257, 2048, 8192, 0), (1300, 4096, 4096, 0),
+                                       (300, 2112, 2056, 0), (777, 28672, 1024, 0), (2077, 6144, 1600, 0),
+                                       (1153, 4128, 8200, 11), (1501, 9632, 4096, 6), (1501, 4120, 9608, 28), (2077, 6152, 4104, 3),
+                                       (2077, 2080, 8192, 7), (3001, 2080, 8192, 34)])
+def test_linear_cuts_the_last_round_of_tiles(m, n, k, cut):
+    """Products whose last round of 256 x 256 tiles leaves pairs idle: its `cut` tiles are cut along K over all pairs and their
+    parts added, for each epilogue, with one part order (two runs give the same bits); a few tiles in many parts and many in
+    few, tokens and outputs that end inside a tile. With 0, shapes around them that other kernels take. Largest error of a sum of
+    k products of bfloat16 values in 32 bits: k 2^-24 of the sum of magnitudes, far inside 2e-3 of the largest result."""
+    assert not cut or all(ops().product_plan(m, n, k, target).tail == cut for target in ops().TARGETS)
     a = randn(m, k, dtype=torch.bfloat16, seed=201)
     w = randn(n, k, dtype=torch.bfloat16, seed=202, scale=0.05)
     bias = randn(n, seed=203)
@@ -189,6 +193,11 @@ def test_linear_cuts_the_last_round_of_tiles(m, n, k):
     expect = residual.double() + want
     ops().linear(a, w, bias, residual=residual)
     assert float((residual - expect).abs().max()) <= 2e-3 * scale
+    if cut:
+        norm = ops().FoldedNorm(a, _sums_in_parts(a, 3, 205), 3, 1e-5, k)
+        rstd = 1.0 / torch.sqrt((a.double() ** 2).mean(dim=1, keepdim=True) + 1e-5)
+        got = ops().linear(a, w, bias, out_dtype=torch.float32, norm=norm)
+        assert float((got.double() - (plain * rstd + bias.double())).abs().max()) <= 2e-3 * scale
     if n % 32 == 0:
         f = n // 2
         gate, up = plain.view(m, f // 16, 2, 16).unbind(2)
@@ -199,12 +208,15 @@ def test_linear_cuts_the_last_round_of_tiles(m, n, k):
 
 @pytest.mark.parametrize("m,n,k", [(353, 6152, 1032), (350, 4102, 2056), (511, 4104, 4096), (256, 4104, 8192), (300, 4096, 4096),
                                    (190, 4096, 8192), (129, 6144, 4096), (1300, 4096, 1536), (140, 8224, 4104), (511, 4128, 4096),
-                                   (300, 8224, 4104), (350, 12320, 2056)])
+                                   (300, 8224, 4104), (350, 12320, 2056), (400, 4096, 14336), (300, 28704, 2056), (1150, 12320, 1544)])
 def test_linear_with_the_weights_on_the_row_side(m, n, k):
     """Products whose weights are the rows of the pairs' tiles: token tiles of several widths that end inside a tile and inside 16
     tokens, outputs that end inside a tile and a block, rows no tensor map can describe (4,102), K that ends inside a
-    k-block, one pair a tile and two or three in a cluster; every epilogue, with a folded norm and without, one order of the
-    sums (two runs give the same bits). Errors as in the test above."""
+    k-block, one pair a tile, up to six tiles a pair one after the other, and two or three pairs in a cluster; every epilogue, with a
+    folded norm and without, the next norm's input behind the residual, one order of the sums (two runs give the same bits).
+    Errors as in the test above; a square sum of n terms in 32 bits is off by n 2^-24 at most."""
+    plans = {target: ops().product_plan(m, n, k, target) for target in ops().TARGETS}
+    assert plans["float32"].kernel == plans["residual"].kernel == "row_side"
     a = randn(m, k, dtype=torch.bfloat16, seed=231)
     w = randn(n, k, dtype=torch.bfloat16, seed=232, scale=0.05)
     bias = randn(n, seed=233)
@@ -219,6 +231,12 @@ def test_linear_with_the_weights_on_the_row_side(m, n, k):
     expect = residual.double() + want
     ops().linear(a, w, bias, residual=residual)
     assert float((residual - expect).abs().max()) <= 2e-3 * scale
+    again = randn(m, n, seed=234)
+    emit = _emit(m, n)
+    ops().linear(a, w, bias, residual=again, emit=emit)
+    assert torch.equal(again, residual) and torch.equal(emit.rows, residual.to(torch.bfloat16))
+    squares = (residual.double() ** 2).sum(dim=1)
+    assert float((emit.sumsq[:, :emit.parts].double().sum(dim=1) / squares - 1).abs().max()) <= n * 2.0 ** -24
     norm = ops().FoldedNorm(a, _sums_in_parts(a, 5, 235), 5, 1e-5, k)
     rstd = 1.0 / torch.sqrt((a.double() ** 2).mean(dim=1, keepdim=True) + 1e-5)
     assert float((ops().linear(a, w, bias, norm=norm).double() - (plain * rstd + bias.double())).abs().max()) <= 1e-2 * scale
@@ -231,10 +249,14 @@ def test_linear_with_the_weights_on_the_row_side(m, n, k):
     assert ops().tensor_core_status() == 0
 
 
-def test_linear_on_two_streams_at_once():
-    """Products that leave parts in scratch, on two streams with nothing between them: each stream has its own."""
-    a = randn(350, 4096, dtype=torch.bfloat16, seed=205)
-    ws = [randn(4096, 4096, dtype=torch.bfloat16, seed=206 + i, scale=0.05) for i in range(2)]
+@pytest.mark.parametrize("m,n,k,kernel", [(350, 4096, 4096, "row_side"), (1153, 4128, 8200, "pairs"), (200, 2048, 4096, "blocks")])
+def test_linear_on_two_streams_at_once(m, n, k, kernel):
+    """Products on two streams with nothing between them, where the kernel leaves parts in scratch (tiles cut along K, split K) and
+    where it needs none: each stream has its own."""
+    plan = ops().product_plan(m, n, k)
+    assert plan.kernel == kernel and (plan.scratch_floats > 0) == (kernel != "row_side")
+    a = randn(m, k, dtype=torch.bfloat16, seed=205)
+    ws = [randn(n, k, dtype=torch.bfloat16, seed=206 + i, scale=0.05) for i in range(2)]
     want = [ops().linear(a, w) for w in ws]
     streams = [torch.cuda.Stream() for _ in ws]
     torch.cuda.synchronize()
@@ -247,7 +269,7 @@ def test_linear_on_two_streams_at_once():
     assert all(torch.equal(g, want[i]) for i in range(2) for g in got[i])
 
 
-@pytest.mark.parametrize("m,n,k", [(350, 4096, 4096), (64, 4096, 4096)])      # parts of tiles; K split over blocks
+@pytest.mark.parametrize("m,n,k", [(350, 4096, 4096), (64, 4096, 4096), (1153, 4128, 8200)])      # sums in a cluster; K split over blocks; parts of tiles
 def test_products_on_many_streams_and_in_a_graph_at_once(m, n, k):
     """More streams than keep scratch, and a captured product replayed on one more, with nothing between them: the bits of
     single calls."""
@@ -906,6 +928,10 @@ def _sums_in_parts(x, parts, seed):
     return sums
 
 
+def _emit(m, n):
+    return ops().Emit(torch.zeros(m, n, dtype=torch.bfloat16, device=DEV), torch.zeros(m, ops().SUMSQ_LD, device=DEV))
+
+
 @pytest.mark.parametrize("m,n,k,parts", [(8, 6144, 4096, 32), (1, 256, 64, 1), (16, 384, 512, 3),
                                          (40, 320, 1024, 5), (128, 512, 256, 64), (300, 512, 256, 2),
                                          (2048, 1024, 256, 16), (700, 200, 72, 1)])
@@ -980,8 +1006,8 @@ def test_qkv_product_rotates_and_writes_the_cache(tokens, heads, kv_heads, dim, 
     """The q/k/v product with the rotation and the cache write in its epilogue (and a folded norm
     with it) against the product followed by the plain rope_cache_write: sequences at different
     positions and pages, head sizes that fit a tile and one that does not (48: a kernel of its own
-    runs behind the product). 1,100 tokens run 256 x 256 tiles on pairs of SMs, which leave the
-    rotation to the kernel behind them."""
+    runs behind the product). 1,100 tokens run on pairs of SMs, as 256 x 256 tiles or with the weights on
+    the row side, which leave the rotation to the kernel behind them."""
     k = 256
     width = (heads + 2 * kv_heads) * dim
     counts = [tokens] if tokens < 3 else [tokens - 2, 1, 1]
