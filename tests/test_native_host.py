@@ -54,6 +54,38 @@ def test_a_step_is_refused_before_anything_changes():
     cache.check()
 
 
+def begin(cache, entries, vocab=100, max_seq_len=64 * 6):
+    batch = _Batch(entries)
+    native.check(native.lib().llmh_step_begin(cache._handle, *batch.arguments(), vocab, max_seq_len))
+
+
+def test_a_step_begins_with_its_pages_or_not_at_all():
+    """The engine's one call: a batch that is refused at its last entry, or whose pages are not all there, leaves lengths and
+    pages as they were; a batch that is taken holds the pages of its new lengths."""
+    cache = make_cache()                                       # twelve pages a group
+    a, b, c = cache.acquire(), cache.acquire(), cache.acquire()
+
+    def held():
+        return cache.held_tokens(), [cache.length(s) for s in (a, b, c)], [cache.block_table_rows(g, [a, b, c]).tolist() for g in range(2)]
+
+    before = held()
+    for last, error in ((Entry(b, [5, 100], [0]), FormatError), (Entry(b, [1], [1]), FormatError), (Entry(a, [1], [0]), FormatError),
+                        (Entry(b, [], []), FormatError), (Entry(3, [1], [0]), LlmError), (Entry(b, [1] * (64 * 6 + 1), []), ContextFull)):
+        with pytest.raises(error):
+            begin(cache, [Entry(a, [1] * 130, [0]), last])
+        assert held() == before
+    cache.reserve(c, 64 * 6)
+    before = held()
+    with pytest.raises(LlmError):
+        begin(cache, [Entry(a, [1] * 130, [0]), Entry(b, [1] * (64 * 4), [])])      # three pages and four, of six
+    assert held() == before
+    begin(cache, [Entry(a, [1] * 130, [129]), Entry(b, [1] * 64 * 3, [])])
+    with pytest.raises(LlmError):
+        cache.reserve(a, 64 * 3 + 1)                           # all twelve pages are held
+    assert held()[:2] == before[:2]
+    cache.check()
+
+
 def test_packing_of_an_unequal_batch():
     cache = make_cache()
     lib = native.lib()
